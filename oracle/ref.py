@@ -32,7 +32,7 @@ _params = None
 
 def build():
     """Compile the reference sources where the reference tree exists."""
-    if os.path.isdir(REF_TREE):
+    if os.path.isdir(os.path.join(REF_TREE, "src_compressible_stag")):
         subprocess.check_call(["make", "-s", "-C", _DIR, "ref", f"REF={REF_TREE}", f"-j{os.cpu_count() or 4}"])
 
 
