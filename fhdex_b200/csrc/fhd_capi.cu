@@ -33,7 +33,7 @@ struct fhd_ctx {
     fhd_fab sff[3]{};            // stage conservative face fluxes (f64)
     fhd_fab smc{}, sme{};        // stage total centre / edge momentum fluxes (f64)
     fhd_fab csrc{};              // zeroed source of a step given none (chemistry on)
-    int tile = 0;
+    int tile = -1;               // launch shape set by fhd_set_tile; -1: chosen by box, species and precision
     // physical boundaries: the periodic directions and the walls' values
     int per[3] = {1, 1, 1};
     bool walls = false;

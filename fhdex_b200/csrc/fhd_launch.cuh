@@ -165,6 +165,32 @@ StageArgs<NS, R, NZ> make_stage_args(const StageCall& c) {
     return a;
 }
 
+// The face kernel's launch shape when none was set (fhd_set_tile).  The kernel is
+// bound by latency and issue, so resident warps count until spills cost more:
+//   * a direction whose faces fit one wave of 128-register blocks (4 per SM, up to
+//     about 42^3) takes them: with no second wave, more residency buys nothing and
+//     spills cost (argon FP64 16^3: 170 us per step against 178 at 64 registers);
+//   * up to one wave of 80-register blocks (48^3: 258 us against 302 at 128
+//     registers and 263 at 64);
+//   * above, the shape measured fastest per precision and species count: FP64 64
+//     registers (256^3 argon 26.1 ms per step against 32.8 at 128 registers; 128^3
+//     four species 6.79 against 8.02); FP32 fluxes 64 registers for two species
+//     (192^3 8.13 against 8.90 ms), 48 for one (128^3 1.79 against 1.99), 80 for
+//     three and four (128^3 3.80 against 4.29).
+template <int NS, class R>
+int auto_face_tile(const int N[3]) {
+    int64_t most = 0;
+    for (int d = 0; d < 3; ++d) {
+        const int64_t f = (int64_t)(N[0] + (d == 0)) * (N[1] + (d == 1)) * (N[2] + (d == 2));
+        if (f > most) most = f;
+    }
+    const int64_t blocks = (most + 127) / 128;
+    if (blocks <= 4 * device_sms()) return 0;
+    if (blocks <= 6 * device_sms()) return 2;
+    if (sizeof(R) == 8) return 4;
+    return NS == 1 ? 3 : (NS == 2 ? 4 : 2);
+}
+
 inline int stage_block(const StageCall& c) {
     return (c.tile >= 0 && c.tile < kNumStageBlocks) ? kStageBlocks[c.tile] : 128;
 }
@@ -178,7 +204,7 @@ int launch_stage_part_t(const StageCall& c, int part) {
     if (part == 0) {
         k_taus<NS, R, NZ><<<grid_for((int64_t)(N[0] + 2) * (N[1] + 2) * (N[2] + 2), b), b, 0, c.stream>>>(a);
     } else if (part == 1) {
-        const int t = (c.tile >= 0 && c.tile < kNumStageBlocks) ? c.tile : 0;
+        const int t = (c.tile >= 0 && c.tile < kNumStageBlocks) ? c.tile : auto_face_tile<NS, R>(N);
 #define FHD_FACES(BS, MINB)                                                                                      \
         k_faces<NS, R, NZ, 0, BS, MINB><<<resident_grid<k_faces<NS, R, NZ, 0, BS, MINB>>(                     \
             (int64_t)(N[0] + 1) * N[1] * N[2], BS), BS, 0, c.stream>>>(a);                                     \

@@ -197,7 +197,8 @@ int fhd_status(fhd_ctx* ctx);
 /* Effective parameters (after GetHcGas and SetupCWallStag). */
 int fhd_get_params(const fhd_ctx* ctx, fhd_params* out);
 /* Launch shape of the stage kernels (index into fhd_tile_name's list); the
- * autotuner in the host layer times them and sets the fastest.  No reference
+ * autotuner in the host layer times them and sets the fastest.  Without a call the
+ * shape follows the box size, species count and precision.  No reference
  * counterpart (AMReX picks its own launch shapes). */
 int fhd_set_tile(fhd_ctx* ctx, int tile);
 int fhd_num_tiles(void);
