@@ -44,6 +44,11 @@ struct fhd_ctx {
     double* res_rec = nullptr;   // test hook: the particle reservoir's draws
     int res_cap = 0;
     WallParams wall{};
+    // the flux operator's stress scratch, its fabs, and the stream and end of its last use
+    double* fx = nullptr;
+    fhd_fab fxt{}, fxe{};
+    cudaStream_t fx_stream = nullptr;
+    cudaEvent_t fx_ev = nullptr;
     // the Valk/Waldmann model's pair constants (transport_type 2), device memory
     VWTable* vwt = nullptr;
     // x-line scratch of the spatial cross-correlations (fhd_stats_stag, FHD_STATS_CROSS)
@@ -245,6 +250,40 @@ int ensure_coef(fhd_ctx* c, int dtype) {
     c->ct = make_fab(p, n, CELLN, 1, 6, dtype); p += ctpts * 6 * es;
     c->et = make_fab(p, n, allnod, 0, 6, dtype);
     return FHD_OK;
+}
+
+// The flux operator's own stress scratch (ct, et), kept by the context.  It is apart
+// from the step's scratch, and a call on another stream than the last one's waits for
+// that one, so operator calls may overlap a step, and each other, on any streams.
+// false: no scratch (a stream under capture, whose graph may be replayed beside later
+// calls, or no memory left).
+bool flux_scratch(fhd_ctx* c) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &st) != cudaSuccess) { cudaGetLastError(); return false; }
+    if (st != cudaStreamCaptureStatusNone) return false;
+    if (!c->fx) {
+        const int* n = c->prm.n_cells;
+        const int allnod[3] = {1, 1, 1};
+        c->fxt = make_fab(nullptr, n, CELLN, 1, 6, FHD_F64);
+        c->fxe = make_fab(nullptr, n, allnod, 0, 6, FHD_F64);
+        const int64_t nt = fab_points(c->fxt) * 6, ne = fab_points(c->fxe) * 6;
+        if (!c->fx_ev && cudaEventCreateWithFlags(&c->fx_ev, cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            c->fx_ev = nullptr;
+            return false;
+        }
+        if (cudaMalloc(&c->fx, (size_t)(nt + ne) * sizeof(double)) != cudaSuccess) {
+            cudaGetLastError();
+            c->fx = nullptr;
+            return false;
+        }
+        c->fxt.data = c->fx;
+        c->fxe.data = c->fx + nt;
+    } else if (c->fx_stream != c->stream && cudaStreamWaitEvent(c->stream, c->fx_ev, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return true;
 }
 
 // brackets one launch with events when profiling is on
@@ -519,6 +558,8 @@ int fhd_destroy(fhd_ctx* c) {
     if (c->scratch) cudaFree(c->scratch);
     if (c->coef) cudaFree(c->coef);
     if (c->lines) cudaFree(c->lines);
+    if (c->fx) cudaFree(c->fx);
+    if (c->fx_ev) cudaEventDestroy(c->fx_ev);
     if (c->vwt) cudaFree(c->vwt);
     if (c->res.base) cudaFree(c->res.base);
     if (c->hbuf) cudaFree(c->hbuf);
@@ -670,7 +711,15 @@ int fhd_flux_stag(fhd_ctx* c, fhd_fab cu, const fhd_fab mom[3], fhd_fab prim, co
     }
     sc.status = c->d_status;
     sc.stream = c->stream;
-    return exact_aux_fluxes(sc);
+    // with the stress scratch every stress is computed once, without it once per face
+    if (!flux_scratch(c)) return exact_aux_fluxes(sc);
+    sc.ct = c->fxt;
+    sc.et = c->fxe;
+    int rc = exact_aux_stage(sc, 0);
+    if (!rc) rc = exact_aux_stage(sc, 1);
+    c->fx_stream = c->stream;
+    if (cudaEventRecord(c->fx_ev, c->stream) != cudaSuccess && !rc) { cudaGetLastError(); rc = FHD_ERR_CUDA; }
+    return rc;
 }
 
 int fhd_fill_boundary(fhd_ctx* c, fhd_fab f) {
@@ -1008,19 +1057,19 @@ static int walls_step_launches(fhd_ctx* c, fhd_fab cu, const fhd_fab mom[3], fhd
             }
         }
         if (rc) return rc;
-        if (s == 2 && aux_flux) {
+        const bool aux = s == 2 && aux_flux;
+        if (aux) {
             for (int d = 0; d < 3; ++d) { sc.ff[d] = faceflux[d]; sc.cf[d] = cenflux[d]; }
             for (int e = 0; e < 6; ++e) sc.ef[e] = edgeflux[e];
-            ProfScope ps(c, 6);
-            rc = exact_aux_fluxes(sc);
-            if (!rc && c->res4) rc = exact_res_reset(sc.P, c->res, faceflux, 0, 4, 5, edgeflux, -1, c->stream);
-            if (rc) return rc;
         }
         for (int part = 0; part < 3 && !rc; ++part) {
             ProfScope ps(c, 1 + part);
             // ResetReservoirFluxes between the fluxes and the update
-            if (part == 2 && c->res4) rc = exact_res_reset(sc.P, c->res, c->sff, 0, 1, 2, &c->sme, 0, c->stream);
-            if (!rc) rc = exact_walls_part(sc, part);
+            if (part == 2 && c->res4) {
+                if (aux) rc = exact_res_reset(sc.P, c->res, faceflux, 0, 4, 5, edgeflux, -1, c->stream);
+                if (!rc) rc = exact_res_reset(sc.P, c->res, c->sff, 0, 1, 2, &c->sme, 0, c->stream);
+            }
+            if (!rc) rc = aux && part < 2 ? exact_aux_stage(sc, part) : exact_walls_part(sc, part);
         }
         if (rc) return rc;
         {
@@ -1123,11 +1172,15 @@ static int step_launches(fhd_ctx* c, fhd_fab cu, const fhd_fab mom[3], fhd_fab p
                                  cmode == CN_AB ? &injected->chem[1] : nullptr, cmode, w[s], c->stream);
         }
         if (rc) return rc;
-        if (s == 2 && aux_flux) {
+        const bool aux = s == 2 && aux_flux;
+        if (aux) {
             for (int d = 0; d < 3; ++d) { sc.ff[d] = faceflux[d]; sc.cf[d] = cenflux[d]; }
             for (int e = 0; e < 6; ++e) sc.ef[e] = edgeflux[e];
+        }
+        if (aux && tile_fused(c->tile)) {
+            // the fused kernel keeps its fluxes in shared memory
             ProfScope ps(c, 6);
-            rc = exact_aux_fluxes(sc);
+            for (int part = 0; part < 2 && !rc; ++part) rc = exact_aux_stage(sc, part);
             if (rc) return rc;
         }
         if (tile_fused(c->tile)) {
@@ -1136,7 +1189,8 @@ static int step_launches(fhd_ctx* c, fhd_fab cu, const fhd_fab mom[3], fhd_fab p
         } else {
             for (int part = 0; part < 3 && !rc; ++part) {
                 ProfScope ps(c, 1 + part);
-                rc = mixed ? mixed_stage_part(sc, part) : exact_stage_part(sc, part);
+                rc = mixed ? mixed_stage_part(sc, part)
+                     : (aux && part < 2 ? exact_aux_stage(sc, part) : exact_stage_part(sc, part));
             }
         }
         if (rc) return rc;

@@ -18,23 +18,63 @@ namespace fhd {
 
 constexpr int MAXS = 8;
 
-// AMReX Array4 view: (i,j,k,n) at p[(i-lo0) + (j-lo1)*sy + (k-lo2)*sz + n*sn].
+// AMReX Array4 view: (i,j,k,n) at p[i + j*sy + k*sz + n*sn], with p already moved to
+// point (0,0,0) on the host (a point inside the fab: its low corner is at or below
+// zero), so that an access carries no subtraction of the low corner.
 // 32-bit offsets: the host rejects fabs with 2^31 or more elements.
 template <class T>
 struct Arr4 {
     T* p;
-    int lo0, lo1, lo2;
     int sy, sz, sn;
-    FHD_HD T& operator()(int i, int j, int k, int n = 0) const {
-        return p[(i - lo0) + (j - lo1) * sy + (k - lo2) * sz + n * sn];
-    }
+    FHD_HD T& operator()(int i, int j, int k, int n = 0) const { return p[i + j * sy + k * sz + n * sn]; }
 };
 
-// Parameters as the kernels see them (by value in the kernel parameter bank).
-// Cell-independent sub-expressions of the transport model are precomputed on the
-// host in the reference's own operation order (host IEEE double arithmetic gives
-// the identical values the reference computes inside its loops).
-struct DevParams {
+// Division of a 31-bit item number by a run constant: q / d = (q * m) >> s with
+// m = floor(2^(31+l) / d) + 1, l = ceil(log2 d), s = 31 + l (Granlund and Montgomery,
+// "Division by invariant integers using multiplication", PLDI 1994: exact for
+// 0 <= q < 2^31, as m*d - 2^(31+l) lies in (0, 2^l]).  Three instructions against
+// about twenty for a division by a value the compiler does not know.
+struct FastDiv {
+    uint32_t m, s;
+    FHD_HD uint32_t div(uint32_t q) const { return (uint32_t)(((uint64_t)q * m) >> s); }
+};
+inline FastDiv fast_div(uint32_t d) {
+    uint32_t l = 0;
+    while (((uint64_t)1 << l) < d) ++l;
+    FastDiv f;
+    f.m = (uint32_t)((((uint64_t)1 << (31 + l)) / d) + 1);
+    f.s = 31 + l;
+    return f;
+}
+
+// Items 0 .. nx*ny*nz - 1 of a box as points, x fastest
+struct Items {
+    int nx, nxy, n;      // row, plane, all (the host rejects boxes of 2^31 or more points)
+    FastDiv dx, dxy;
+    FHD_HD void point(int q, int& i, int& j, int& k) const {
+        k = (int)dxy.div((uint32_t)q);
+        const int r = q - k * nxy;
+        j = (int)dx.div((uint32_t)r);
+        i = r - j * nx;
+    }
+};
+inline Items make_items(int nx, int ny, int nz) {
+    Items t;
+    t.nx = nx;
+    t.nxy = nx * ny;
+    t.n = nx * ny * nz;
+    t.dx = fast_div((uint32_t)nx);
+    t.dxy = fast_div((uint32_t)(nx * ny));
+    return t;
+}
+
+// Parameters as the kernels see them.  RunParams holds what the stress, flux,
+// update and conversion kernels read; DevParams adds the transport model's tables,
+// whose cell-independent sub-expressions are precomputed on the host in the
+// reference's own operation order (host IEEE double arithmetic gives the identical
+// values the reference computes inside its loops).  The batched kernels copy their
+// member's argument block into shared memory once per block, so the two are apart.
+struct RunParams {
     int ns, nvars, nprim;
     int n[3];
     double dx[3];
@@ -50,6 +90,27 @@ struct DevParams {
     int bc_vel[6], bc_mass[6], bc_therm[6];
     double hdx[3], rhdx[3];          // 0.5*dx and RN(1/(0.5*dx)) (the wall faces' half-cell divisor)
     double molmass[MAXS], hcv[MAXS], hcp[MAXS], e0[MAXS];
+    double sqrt2, sqrt3;
+    // quasi-1-D / 2-D runs (do_1D / do_2D): dim 1 or 2, else 3; fac2d = (3+sqrt(3))/2,
+    // the 2-D trace factor (fluxStag.cpp:185); csd0 the deviation of the x centre
+    // noise (1 in 1-D, sqrt(2) otherwise: timeStepStag.cpp:208-222)
+    int dim;
+    double fac2d, csd0;
+    // noise
+    uint32_t key0, key1;             // Philox key
+    uint64_t step;                   // Philox counter words 2-3
+    const uint64_t* step_ptr;        // when set, the step is read here (batched graph replay)
+    // correctly rounded reciprocals (host 1.0 / x) of the constant divisors, for
+    // div_rcp; the dividend window is empty (div_span 0: plain divisions) when a
+    // divisor lies outside div_rcp's divisor window
+    double rdx[3];
+    double rmolmass[MAXS];
+    double rRdt;                     // 1/(Runiv*dt)
+    double rpi, r3;                  // 1/pi (the transport model's pi), 1/3
+    uint32_t div_lo, div_span;
+};
+
+struct DevParams : RunParams {
     // Giovangigli model constants (compressible_functions.H:1180-1222)
     double mm[MAXS];                 // molmass*(k_B/Runiv)
     double mmkB[MAXS];               // mm*k_B (first product of the eta1 sqrt argument)
@@ -62,29 +123,12 @@ struct DevParams {
     double koff;                     // 55.0/4.0-3.0*BKL-4.0*AKL
     double voff;                     // 0.6*AKL-1.0
     double cfac;                     // 6.0*CKL-5.0
-    double sqrt2, sqrt3;
-    // quasi-1-D / 2-D runs (do_1D / do_2D): dim 1 or 2, else 3; fac2d = (3+sqrt(3))/2,
-    // the 2-D trace factor (fluxStag.cpp:185); csd0 the deviation of the x centre
-    // noise (1 in 1-D, sqrt(2) otherwise: timeStepStag.cpp:208-222)
-    int dim;
-    double fac2d, csd0;
     // transport model (transCoeffs.cpp:58-73): 1 Giovangigli, 2 Valk/Waldmann (pair
     // constants in the device table vwt), 3 HCB binary
     int transport_type;
     const struct VWTable* vwt;
-    // noise
-    uint32_t key0, key1;             // Philox key
-    uint64_t step;                   // Philox counter words 2-3
-    const uint64_t* step_ptr;        // when set, the step is read here (batched graph replay)
-    // correctly rounded reciprocals (host 1.0 / x) of the constant divisors, for
-    // div_rcp; the dividend window is empty (div_span 0: plain divisions) when a
-    // divisor lies outside div_rcp's divisor window
-    double rdx[3];
-    double rmolmass[MAXS], rmm[MAXS];
+    double rmm[MAXS];
     double rmu[MAXS][MAXS], rmsum[MAXS][MAXS];
-    double rRdt;                     // 1/(Runiv*dt)
-    double rpi, r3;                  // 1/pi (the transport model's pi), 1/3
-    uint32_t div_lo, div_span;
 };
 
 // a / b in the compute type: FP64 the correctly rounded division (the reference's
@@ -96,21 +140,21 @@ FHD_D float rdiv(float a, float b) { return __fdividef(a, b); }
 // a / b for a constant divisor b with y = RN(1/b) from DevParams: bitwise a / b
 // (fhd_div.h).  In single precision (the mixed path, held to a tolerance against
 // FP64, not to bitwise parity) the product a * y: within about one FP32 ulp of a / b.
-FHD_D double divc(const DevParams& P, double a, double b, double y) { return div_rcp(a, b, y, P.div_lo, P.div_span); }
-FHD_D float divc(const DevParams&, float a, float, float y) { return a * y; }
+FHD_D double divc(const RunParams& P, double a, double b, double y) { return div_rcp(a, b, y, P.div_lo, P.div_span); }
+FHD_D float divc(const RunParams&, float a, float, float y) { return a * y; }
 // divc for call sites whose dividend is often exactly zero (zero handled inline)
-FHD_D double divc0(const DevParams& P, double a, double b, double y) {
+FHD_D double divc0(const RunParams& P, double a, double b, double y) {
     return div_rcp_z(a, b, y, P.div_lo, P.div_span);
 }
-FHD_D float divc0(const DevParams&, float a, float, float y) { return a * y; }
+FHD_D float divc0(const RunParams&, float a, float, float y) { return a * y; }
 // a / b for a cell value b used as a divisor several times, y = 1.0 / b
-FHD_D double divv(const DevParams& P, double a, double b, double y) {
+FHD_D double divv(const RunParams& P, double a, double b, double y) {
     return div_rcp_any(a, b, y, P.div_lo, P.div_span);
 }
-FHD_D float divv(const DevParams&, float a, float, float y) { return a * y; }
+FHD_D float divv(const RunParams&, float a, float, float y) { return a * y; }
 // a / Dbin with the reciprocal path for up to two species (see transport_gio)
 template <int NS, class R>
-FHD_D R div_dbin(const DevParams& P, R a, R b, R y) {
+FHD_D R div_dbin(const RunParams& P, R a, R b, R y) {
     if constexpr (NS <= 2) return divv(P, a, b, y);
     else return rdiv(a, b);
 }
@@ -119,7 +163,7 @@ FHD_D R div_dbin(const DevParams& P, R a, R b, R y) {
 FHD_D double divz(double a, double b) { return div_zero_short(a, b); }
 FHD_D float divz(float a, float b) { return rdiv(a, b); }
 
-FHD_D uint64_t noise_step(const DevParams& P) { return P.step_ptr ? *P.step_ptr : P.step; }
+FHD_D uint64_t noise_step(const RunParams& P) { return P.step_ptr ? *P.step_ptr : P.step; }
 
 // ---- persistent batched step: work units and run descriptor (k_batch_persist) -----------
 enum { PK_PREP = 0, PK_TAUS = 1, PK_FACEX = 2, PK_FACEY = 3, PK_FACEZ = 4, PK_UPDATE = 5, PK_CONVERT = 6,
@@ -157,14 +201,14 @@ struct WallParams {
 
 // the reference's is_<lo|hi>_<d>_dirichlet_mass (fluxStag.cpp:84-89): a side whose
 // bc_mass is neither -1 (periodic) nor 3
-FHD_HD bool dirichlet_side(const DevParams& P, int side) {
+FHD_HD bool dirichlet_side(const RunParams& P, int side) {
     const int b = P.bc_mass[side];
     return b != -1 && b != 3;
 }
 // the wall side (0 lo, 1 hi) of the face plane idx of direction d, or -1: the
 // reference's (i == 0 and is_lo_x_dirichlet_mass) / (i == n_cells[0] and
 // is_hi_x_dirichlet_mass) tests
-FHD_HD int wall_face(const DevParams& P, int d, int idx) {
+FHD_HD int wall_face(const RunParams& P, int d, int idx) {
     if (idx == 0 && dirichlet_side(P, 2 * d)) return 0;
     if (idx == P.n[d] && dirichlet_side(P, 2 * d + 1)) return 1;
     return -1;
@@ -172,7 +216,7 @@ FHD_HD int wall_face(const DevParams& P, int d, int idx) {
 // StochFluxStag's factors (boundaryStag.cpp:2086-3009) on a wall side: 0 for an
 // impermeable / adiabatic / slip wall (type 1), sqrt(2) for a concentration /
 // isothermal / no-slip wall (type 2), 1 otherwise
-FHD_HD double stoch_factor(const DevParams& P, int type) {
+FHD_HD double stoch_factor(const RunParams& P, int type) {
     return type == 1 ? 0. : (type == 2 ? P.sqrt2 : 1.0);
 }
 
@@ -187,7 +231,7 @@ FHD_D float mul_rn(float a, float b) { return a * b; }
 FHD_D float add_rn(float a, float b) { return a + b; }
 
 template <int NS, class R>
-FHD_D void GetMolfrac(const DevParams& P, const R (&Y)[NS], R (&X)[NS]) {
+FHD_D void GetMolfrac(const RunParams& P, const R (&Y)[NS], R (&X)[NS]) {
     R molmix = R(0.);
 #pragma unroll
     for (int n = 0; n < NS; ++n) molmix += divc(P, Y[n], R(P.molmass[n]), R(P.rmolmass[n]));
@@ -197,7 +241,7 @@ FHD_D void GetMolfrac(const DevParams& P, const R (&Y)[NS], R (&X)[NS]) {
 }
 
 template <int NS, class R>
-FHD_D R GetTemperature(const DevParams& P, R energy, const R (&Y)[NS]) {
+FHD_D R GetTemperature(const RunParams& P, R energy, const R (&Y)[NS]) {
     R cvmix = R(0.), e0mix = R(0.);
 #pragma unroll
     for (int n = 0; n < NS; ++n) {
@@ -208,7 +252,7 @@ FHD_D R GetTemperature(const DevParams& P, R energy, const R (&Y)[NS]) {
 }
 
 template <int NS, class R>
-FHD_D R GetPressureGas(const DevParams& P, const R (&Y)[NS], R density, R temp) {
+FHD_D R GetPressureGas(const RunParams& P, const R (&Y)[NS], R density, R temp) {
     R molmix = R(0.);
 #pragma unroll
     for (int n = 0; n < NS; ++n) molmix += divc(P, Y[n], R(P.molmass[n]), R(P.rmolmass[n]));
@@ -217,7 +261,7 @@ FHD_D R GetPressureGas(const DevParams& P, const R (&Y)[NS], R density, R temp) 
 }
 
 template <int NS, class R>
-FHD_D void GetEnthalpies(const DevParams& P, R T, R (&hk)[NS]) {
+FHD_D void GetEnthalpies(const RunParams& P, R T, R (&hk)[NS]) {
 #pragma unroll
     for (int i = 0; i < NS; ++i) hk[i] = R(P.e0[i]) + R(P.hcp[i]) * T;
 }
@@ -544,7 +588,7 @@ struct Prim {
 };
 
 template <int NS>
-FHD_D bool cons_to_prim(const DevParams& P, double rho, double rhoE, const double (&rhoY)[NS], double mxl,
+FHD_D bool cons_to_prim(const RunParams& P, double rho, double rhoE, const double (&rhoY)[NS], double mxl,
                         double mxh, double myl, double myh, double mzl, double mzh, Prim<NS>& q) {
     double kin = 0.;
     kin = add_rn(kin, mul_rn(mxh + mxl, mxh + mxl));

@@ -8,6 +8,7 @@ namespace fhd {
 int exact_cellprep_ns1(const StageCall&);
 int exact_stage_ns1(const StageCall&, int);
 int exact_aux_ns1(const StageCall&);
+int exact_aux_stage_ns1(const StageCall&, int);
 int mixed_cellprep_ns1(const StageCall&);
 int mixed_stage_ns1(const StageCall&, int);
 int exact_transport_ns1(const DevParams&, fhd_fab, fhd_fab, fhd_fab, fhd_fab, fhd_fab, fhd_fab, int*, cudaStream_t);
@@ -21,6 +22,7 @@ int exact_bc_seq_ns1(const DevParams&, const WallParams&, fhd_fab, fhd_fab, cons
 int exact_cellprep_ns2(const StageCall&);
 int exact_stage_ns2(const StageCall&, int);
 int exact_aux_ns2(const StageCall&);
+int exact_aux_stage_ns2(const StageCall&, int);
 int mixed_cellprep_ns2(const StageCall&);
 int mixed_stage_ns2(const StageCall&, int);
 int exact_transport_ns2(const DevParams&, fhd_fab, fhd_fab, fhd_fab, fhd_fab, fhd_fab, fhd_fab, int*, cudaStream_t);
@@ -34,6 +36,7 @@ int exact_bc_seq_ns2(const DevParams&, const WallParams&, fhd_fab, fhd_fab, cons
 int exact_cellprep_ns3(const StageCall&);
 int exact_stage_ns3(const StageCall&, int);
 int exact_aux_ns3(const StageCall&);
+int exact_aux_stage_ns3(const StageCall&, int);
 int mixed_cellprep_ns3(const StageCall&);
 int mixed_stage_ns3(const StageCall&, int);
 int exact_transport_ns3(const DevParams&, fhd_fab, fhd_fab, fhd_fab, fhd_fab, fhd_fab, fhd_fab, int*, cudaStream_t);
@@ -47,6 +50,7 @@ int exact_bc_seq_ns3(const DevParams&, const WallParams&, fhd_fab, fhd_fab, cons
 int exact_cellprep_ns4(const StageCall&);
 int exact_stage_ns4(const StageCall&, int);
 int exact_aux_ns4(const StageCall&);
+int exact_aux_stage_ns4(const StageCall&, int);
 int mixed_cellprep_ns4(const StageCall&);
 int mixed_stage_ns4(const StageCall&, int);
 int exact_transport_ns4(const DevParams&, fhd_fab, fhd_fab, fhd_fab, fhd_fab, fhd_fab, fhd_fab, int*, cudaStream_t);
@@ -102,6 +106,7 @@ int mixed_batch_persist_ns4(int, int, const PersistArgs&, cudaStream_t);
 
 int exact_cellprep(const StageCall& c) { FHD_DISPATCH(c.P.ns, exact_cellprep_ns, c) }
 int exact_stage_part(const StageCall& c, int part) { FHD_DISPATCH(c.P.ns, exact_stage_ns, c, part) }
+int exact_aux_stage(const StageCall& c, int part) { FHD_DISPATCH(c.P.ns, exact_aux_stage_ns, c, part) }
 int exact_aux_fluxes(const StageCall& c) { FHD_DISPATCH(c.P.ns, exact_aux_ns, c) }
 int mixed_cellprep(const StageCall& c) { FHD_DISPATCH(c.P.ns, mixed_cellprep_ns, c) }
 int mixed_stage_part(const StageCall& c, int part) { FHD_DISPATCH(c.P.ns, mixed_stage_ns, c, part) }
@@ -412,8 +417,8 @@ int noise_fill(const DevParams& P, const fhd_fab& f, int c0, int nc, double mean
 
 int init_uniform(const fhd_fab& cu, int ns, double rho0, double rhoE, const double* rhoY, cudaStream_t s) {
     InitArgs a;
-    a.cu = view<double>(cu);
-    a.npts = a.cu.sn;
+    a.cu = static_cast<double*>(cu.data);
+    a.sn = a.npts = (int64_t)(cu.hi[0] - cu.lo[0] + 1) * (cu.hi[1] - cu.lo[1] + 1) * (cu.hi[2] - cu.lo[2] + 1);
     a.nvars = cu.ncomp;
     a.ns = ns;
     a.rho0 = rho0;

@@ -50,7 +50,7 @@ struct Noise {
 
     FHD_D double comb(double A, double B) const { return 1.0 * A + w * B; }
     // fields fid0 and fid0+1 (fid0 even) at one point, each W = A + w B
-    FHD_D void gauss2(const DevParams& P, uint32_t fid0, int i, int j, int k, double sd, double& w0,
+    FHD_D void gauss2(const RunParams& P, uint32_t fid0, int i, int j, int k, double sd, double& w0,
                       double& w1) const {
         float z[4];
         normal_quad(P.key0, P.key1, canon(P, i, j, k), fid0 >> 1, noise_step(P), z);
@@ -58,20 +58,20 @@ struct Noise {
         w1 = comb(0.0 + sd * (double)z[2], 0.0 + sd * (double)z[3]);
     }
     // fields fid0 and fid0+1 with their own standard deviations
-    FHD_D void gauss2sd(const DevParams& P, uint32_t fid0, int i, int j, int k, double sd0, double sd1, double& w0,
+    FHD_D void gauss2sd(const RunParams& P, uint32_t fid0, int i, int j, int k, double sd0, double sd1, double& w0,
                         double& w1) const {
         float z[4];
         normal_quad(P.key0, P.key1, canon(P, i, j, k), fid0 >> 1, noise_step(P), z);
         w0 = comb(0.0 + sd0 * (double)z[0], 0.0 + sd0 * (double)z[1]);
         w1 = comb(0.0 + sd1 * (double)z[2], 0.0 + sd1 * (double)z[3]);
     }
-    FHD_D double gauss1(const DevParams& P, uint32_t fid, int i, int j, int k, double sd) const {
+    FHD_D double gauss1(const RunParams& P, uint32_t fid, int i, int j, int k, double sd) const {
         float za, zb;
         normal_pair(P.key0, P.key1, canon(P, i, j, k), fid, noise_step(P), za, zb);
         return comb(0.0 + sd * (double)za, 0.0 + sd * (double)zb);
     }
     template <int NC>
-    FHD_D void face_all(const DevParams& P, int d, int i, int j, int k, double (&out)[NC]) const {
+    FHD_D void face_all(const RunParams& P, int d, int i, int j, int k, double (&out)[NC]) const {
         if (MODE == NZ_PHILOX) {
 #pragma unroll
             for (int c = 0; c < NC; c += 2) {
@@ -83,7 +83,7 @@ struct Noise {
             for (int c = 0; c < NC; ++c) out[c] = face(P, d, c, i, j, k);
         }
     }
-    FHD_D void cen_all(const DevParams& P, int i, int j, int k, double (&out)[3]) const {
+    FHD_D void cen_all(const RunParams& P, int i, int j, int k, double (&out)[3]) const {
         if (MODE == NZ_PHILOX) {
             out[0] = gauss1(P, fid_cen(0), i, j, k, P.csd0);
             gauss2(P, fid_cen(1), i, j, k, P.sqrt2, out[1], out[2]);
@@ -95,7 +95,7 @@ struct Noise {
     // The six stress fields of point (i,j,k) in three Philox calls: the centre
     // fields of cell (i,j,k) with, when `edges`, the yz edge field of node (i,j,k)
     // (cen_and_yz_edge), then the xy and xz edge fields (xy_xz_edges)
-    FHD_D void cen_and_yz_edge(const DevParams& P, int i, int j, int k, bool edges, double (&wc)[3],
+    FHD_D void cen_and_yz_edge(const RunParams& P, int i, int j, int k, bool edges, double (&wc)[3],
                                double& we2) const {
         if (MODE == NZ_PHILOX) {
             gauss2sd(P, fid_edge(2), i, j, k, 1.0, P.csd0, we2, wc[0]);
@@ -105,7 +105,7 @@ struct Noise {
             if (edges) we2 = edge(P, 2, i, j, k);
         }
     }
-    FHD_D void xy_xz_edges(const DevParams& P, int i, int j, int k, double& we0, double& we1) const {
+    FHD_D void xy_xz_edges(const RunParams& P, int i, int j, int k, double& we0, double& we1) const {
         if (MODE == NZ_PHILOX) {
             gauss2(P, fid_edge(0), i, j, k, 1.0, we0, we1);
         } else {
@@ -113,7 +113,7 @@ struct Noise {
             we1 = edge(P, 1, i, j, k);
         }
     }
-    FHD_D void edge_all(const DevParams& P, int i, int j, int k, double (&out)[3]) const {
+    FHD_D void edge_all(const RunParams& P, int i, int j, int k, double (&out)[3]) const {
         if (MODE == NZ_PHILOX) {
             gauss2(P, fid_edge(0), i, j, k, 1.0, out[0], out[1]);
             out[2] = gauss1(P, fid_edge(2), i, j, k, 1.0);  // (shares its call with centre x)
@@ -122,19 +122,19 @@ struct Noise {
             for (int e = 0; e < 3; ++e) out[e] = edge(P, e, i, j, k);
         }
     }
-    FHD_D double face(const DevParams& P, int d, int c, int i, int j, int k) const {
+    FHD_D double face(const RunParams& P, int d, int c, int i, int j, int k) const {
         if (MODE == NZ_W) return a.fa[d](i, j, k, a.foa[d] + c);
         if (MODE == NZ_AB) return comb(a.fa[d](i, j, k, a.foa[d] + c), a.fb[d](i, j, k, a.fob[d] + c));
         if (MODE == NZ_PHILOX) return gauss1(P, fid_face(d, c), i, j, k, 1.0);
         return 0.0;
     }
-    FHD_D double edge(const DevParams& P, int e, int i, int j, int k) const {
+    FHD_D double edge(const RunParams& P, int e, int i, int j, int k) const {
         if (MODE == NZ_W) return a.ea[e](i, j, k);
         if (MODE == NZ_AB) return comb(a.ea[e](i, j, k), a.eb[e](i, j, k));
         if (MODE == NZ_PHILOX) return gauss1(P, fid_edge(e), i, j, k, 1.0);
         return 0.0;
     }
-    FHD_D double cen(const DevParams& P, int d, int i, int j, int k) const {
+    FHD_D double cen(const RunParams& P, int d, int i, int j, int k) const {
         if (MODE == NZ_W) return a.ca[d](i, j, k);
         if (MODE == NZ_AB) return comb(a.ca[d](i, j, k), a.cb[d](i, j, k));
         if (MODE == NZ_PHILOX) return gauss1(P, fid_cen(d), i, j, k, d == 0 ? P.csd0 : P.sqrt2);
@@ -159,7 +159,7 @@ struct CellTaus {
 // x (x and y) stresses, the 1-D amplitudes scaled by sqrt(3) and the 2-D trace
 // factor by (3+sqrt(3))/2 (fluxStag.cpp:171-192, 875-904)
 template <int NS, class R, int NZ, bool WL = false>
-FHD_D CellTaus<R> cell_taus_w(const DevParams& P, const Fields<NS, R>& F, const double (&wc)[3], int i, int j, int k) {
+FHD_D CellTaus<R> cell_taus_w(const RunParams& P, const Fields<NS, R>& F, const double (&wc)[3], int i, int j, int k) {
     CellTaus<R> t;
     const R eta = F.eta(i, j, k);
     const bool visc3 = (P.visc_type == 3 || P.visc_type == -3);
@@ -237,7 +237,7 @@ FHD_D CellTaus<R> cell_taus_w(const DevParams& P, const Fields<NS, R>& F, const 
 // velocity across the wall over the half cell (fluxStag.cpp:221-232, 250-261,
 // 279-290, 939-1019: the first direction's wall is tested last and wins a corner).
 template <int NS, class R, int NZ, int E, bool WL = false>
-FHD_D Taus<R> edge_taus_w(const DevParams& P, const Fields<NS, R>& F, double wnoise, int i, int j, int k) {
+FHD_D Taus<R> edge_taus_w(const RunParams& P, const Fields<NS, R>& F, double wnoise, int i, int j, int k) {
     // quasi-1-D: no shear stress; quasi-2-D: only xy (fluxStag.cpp:212-214, 241-243,
     // 270-272, 930-932, 962-964, 995-997)
     if (WL && (P.dim == 1 || (P.dim == 2 && E != 0))) {
@@ -324,14 +324,14 @@ FHD_D Taus<R> edge_taus_w(const DevParams& P, const Fields<NS, R>& F, double wno
 }
 
 template <int NS, class R, int NZ, bool WL = false>
-FHD_D CellTaus<R> cell_taus(const DevParams& P, const Fields<NS, R>& F, const Noise<NZ>& nz, int i, int j, int k) {
+FHD_D CellTaus<R> cell_taus(const RunParams& P, const Fields<NS, R>& F, const Noise<NZ>& nz, int i, int j, int k) {
     double wc[3] = {0.0, 0.0, 0.0};
     if (NZ != NZ_OFF) nz.cen_all(P, i, j, k, wc);
     return cell_taus_w<NS, R, NZ, WL>(P, F, wc, i, j, k);
 }
 
 template <int NS, class R, int NZ, int E, bool WL = false>
-FHD_D Taus<R> edge_taus(const DevParams& P, const Fields<NS, R>& F, const Noise<NZ>& nz, int i, int j, int k) {
+FHD_D Taus<R> edge_taus(const RunParams& P, const Fields<NS, R>& F, const Noise<NZ>& nz, int i, int j, int k) {
     return edge_taus_w<NS, R, NZ, E, WL>(P, F, NZ != NZ_OFF ? nz.edge(P, E, i, j, k) : 0.0, i, j, k);
 }
 
@@ -342,7 +342,51 @@ struct FaceFlux {
     double aux[4];        // comps nvars .. nvars+3 (heat, visc. heating diag/shear, Dufour)
 };
 
-// TauGet: .cell(i,j,k) -> CellTaus, .edge<E>(i,j,k) -> Taus.
+// Where face_flux reads its operands.  side 0 is the cell below the face in its
+// direction, side 1 the cell above.  FaceGen: whole fields and a direction known to
+// the compiler (the operator kernels and the fused stage kernel), with the stresses
+// from TauGet (.cell(i,j,k) -> CellTaus, .edge<E>(i,j,k) -> Taus).
+template <int NS, class R, int D, class TauGet>
+struct FaceGen {
+    const Fields<NS, R>& F;
+    const TauGet& tg;
+    int i, j, k;
+    FHD_D int dir() const { return D; }
+    FHD_D int ci(int s) const { return s ? i : i - (D == 0); }
+    FHD_D int cj(int s) const { return s ? j : j - (D == 1); }
+    FHD_D int ck(int s) const { return s ? k : k - (D == 2); }
+    FHD_D double T(int s) const { return F.T(ci(s), cj(s), ck(s)); }
+    FHD_D double p(int s) const { return F.p(ci(s), cj(s), ck(s)); }
+    FHD_D double Y(int s, int n) const { return F.Y(ci(s), cj(s), ck(s), n); }
+    FHD_D double X(int s, int n) const { return F.X(ci(s), cj(s), ck(s), n); }
+    FHD_D double cons(int s, int n) const { return F.cons(ci(s), cj(s), ck(s), n); }
+    FHD_D R kappa(int s) const { return F.kappa(ci(s), cj(s), ck(s)); }
+    FHD_D R chi(int s, int n) const { return F.chi(ci(s), cj(s), ck(s), n); }
+    FHD_D R Dc(int s, int n) const { return F.D(ci(s), cj(s), ck(s), n); }
+    FHD_D double u() const { return F.vel[D](i, j, k); }
+    FHD_D double m() const { return F.mom[D](i, j, k); }
+    FHD_D Taus<R> cell(int s) const {
+        const CellTaus<R> t = tg.cell(ci(s), cj(s), ck(s));
+        Taus<R> r;
+        r.s = t.s[D];
+        r.d = t.d[D];
+        return r;
+    }
+    // edge family f (the face's first / second transverse direction), position q (lo, hi)
+    FHD_D Taus<R> edge(int f, int q) const {
+        if (D == 0) return f == 0 ? tg.template edge<0>(i, j + q, k) : tg.template edge<1>(i, j, k + q);
+        if (D == 1) return f == 0 ? tg.template edge<0>(i + q, j, k) : tg.template edge<2>(i, j, k + q);
+        return f == 0 ? tg.template edge<1>(i + q, j, k) : tg.template edge<2>(i, j + q, k);
+    }
+    // that family's transverse velocity at position q on side s of the face
+    FHD_D double vt(int f, int q, int s) const {
+        if (D == 0) return f == 0 ? F.vel[1](ci(s), j + q, k) : F.vel[2](ci(s), j, k + q);
+        if (D == 1) return f == 0 ? F.vel[0](i + q, cj(s), k) : F.vel[2](i, cj(s), k + q);
+        return f == 0 ? F.vel[0](i + q, j, ck(s)) : F.vel[1](i, j + q, ck(s));
+    }
+};
+
+// conservative flux of one face; x: its operands (FaceGen, FaceRun).
 // WL: the box has physical walls.  A face on a wall plane (the reference's
 // "(i == 0) and is_lo_x_dirichlet_mass" faces) then takes the wall values from the
 // cell on the wall's ghost side with half-cell differences (fluxStag.cpp's
@@ -350,17 +394,13 @@ struct FaceFlux {
 // Dufour and shear-heating parts (boundaryStag.cpp:2086-3009),
 // BCWallReservoirFluxStag's zero species / Dufour fluxes on impermeable walls
 // (boundaryStag.cpp:300-580) and no advective flux (fluxStag.cpp:1511-1529).
-template <int NS, class R, int NZ, int D, class TauGet, bool WL = false>
-FHD_D FaceFlux<NS> face_flux(const DevParams& P, const Fields<NS, R>& F, const Noise<NZ>& nz, const TauGet& tg,
-                             int i, int j, int k) {
-    constexpr int e0 = D == 0, e1 = D == 1, e2 = D == 2;
-    const int im = i - e0, jm = j - e1, km = k - e2;
-    const Arr4<const double>& velx = F.vel[0];
-    const Arr4<const double>& vely = F.vel[1];
-    const Arr4<const double>& velz = F.vel[2];
-    // wall side of this face (0 lo, 1 hi, -1 none) and the cell holding the wall values
+template <int NS, class R, int NZ, bool WL, class X>
+FHD_D FaceFlux<NS> face_flux(const RunParams& P, const Fields<NS, R>& F, const Noise<NZ>& nz, const X& x, int i, int j,
+                             int k) {
+    const int D = x.dir();
+    // wall side of this face (0 lo, 1 hi, -1 none) and the side of the cell holding the wall values
     const int ws = WL ? wall_face(P, D, D == 0 ? i : (D == 1 ? j : k)) : -1;
-    const int gi = ws == 0 ? im : i, gj = ws == 0 ? jm : j, gk = ws == 0 ? km : k;
+    const int gs = ws == 0 ? 0 : 1;
     const int wside = 2 * D + (ws == 1 ? 1 : 0);
     // a transverse face of a quasi-1-D (y, z) or 2-D (z) run carries no heat,
     // species or Dufour flux, stochastic or diffusive (fluxStag.cpp:504-510,
@@ -372,42 +412,21 @@ FHD_D FaceFlux<NS> face_flux(const DevParams& P, const Fields<NS, R>& F, const N
 #pragma unroll
     for (int s = 0; s < NS; ++s) spec[s] = R(0.0);
 
-    const R un = R(F.vel[D](i, j, k));
+    const R un = R(x.u());
 
     // ---- viscous heating terms, complete (stochastic part assigned,
     // fluxStag.cpp:298-781, then the deterministic part added, :1026-1426).  Each
     // flux variable keeps the reference's own sequence of operations; finishing
     // these two first only shortens the live ranges of their operands.
     {
-    const CellTaus<R> tl = tg.cell(im, jm, km);
-    const CellTaus<R> th = tg.cell(i, j, k);
+    const Taus<R> tl = x.cell(0), th = x.cell(1);
     // the two transverse edge families touching this face and their (lo, hi) positions
-    Taus<R> ea0, ea1, eb0, eb1;  // ea: first transverse dir, eb: second
-    R va0l, va0h, va1l, va1h, vb0l, vb0h, vb1l, vb1h;  // transverse velocities (lo/hi sides of the face)
-    if (D == 0) {
-        ea0 = tg.template edge<0>(i, j, k);  ea1 = tg.template edge<0>(i, j + 1, k);
-        eb0 = tg.template edge<1>(i, j, k);  eb1 = tg.template edge<1>(i, j, k + 1);
-        va1h = R(vely(i, j + 1, k)); va1l = R(vely(i - 1, j + 1, k));
-        va0h = R(vely(i, j, k));     va0l = R(vely(i - 1, j, k));
-        vb1h = R(velz(i, j, k + 1)); vb1l = R(velz(i - 1, j, k + 1));
-        vb0h = R(velz(i, j, k));     vb0l = R(velz(i - 1, j, k));
-    } else if (D == 1) {
-        ea0 = tg.template edge<0>(i, j, k);  ea1 = tg.template edge<0>(i + 1, j, k);
-        eb0 = tg.template edge<2>(i, j, k);  eb1 = tg.template edge<2>(i, j, k + 1);
-        va1h = R(velx(i + 1, j, k)); va1l = R(velx(i + 1, j - 1, k));
-        va0h = R(velx(i, j, k));     va0l = R(velx(i, j - 1, k));
-        vb1h = R(velz(i, j, k + 1)); vb1l = R(velz(i, j - 1, k + 1));
-        vb0h = R(velz(i, j, k));     vb0l = R(velz(i, j - 1, k));
-    } else {
-        ea0 = tg.template edge<1>(i, j, k);  ea1 = tg.template edge<1>(i + 1, j, k);
-        eb0 = tg.template edge<2>(i, j, k);  eb1 = tg.template edge<2>(i, j + 1, k);
-        va1h = R(velx(i + 1, j, k)); va1l = R(velx(i + 1, j, k - 1));
-        va0h = R(velx(i, j, k));     va0l = R(velx(i, j, k - 1));
-        vb1h = R(vely(i, j + 1, k)); vb1l = R(vely(i, j + 1, k - 1));
-        vb0h = R(vely(i, j, k));     vb0l = R(vely(i, j, k - 1));
-    }
+    const Taus<R> ea0 = x.edge(0, 0), ea1 = x.edge(0, 1), eb0 = x.edge(1, 0), eb1 = x.edge(1, 1);
+    // transverse velocities (lo/hi sides of the face)
+    const R va1h = R(x.vt(0, 1, 1)), va1l = R(x.vt(0, 1, 0)), va0h = R(x.vt(0, 0, 1)), va0l = R(x.vt(0, 0, 0));
+    const R vb1h = R(x.vt(1, 1, 1)), vb1l = R(x.vt(1, 1, 0)), vb0h = R(x.vt(1, 0, 1)), vb0l = R(x.vt(1, 0, 0));
     if (NZ != NZ_OFF) {
-        vdiag = R(0.5) * un * (tl.s[D] + th.s[D]);
+        vdiag = R(0.5) * un * (tl.s + th.s);
         R vsh = R(0.0);
         if (WL && ws == 0) {
             vsh += R(0.5) * (va1l * ea1.s + va0l * ea0.s);
@@ -425,7 +444,7 @@ FHD_D FaceFlux<NS> face_flux(const DevParams& P, const Fields<NS, R>& F, const N
         if (WL && ws >= 0 && (P.bc_vel[wside] == 1 || P.bc_vel[wside] == 2) && P.bc_mass[wside] < 3)
             vshear *= R(stoch_factor(P, P.bc_vel[wside]));
     }
-    vdiag -= R(0.5) * un * (tl.d[D] + th.d[D]);
+    vdiag -= R(0.5) * un * (tl.d + th.d);
     R vsh = R(0.0);
     if (WL && ws == 0) {
         vsh -= R(0.5) * (va1l * ea1.d + va0l * ea0.d);
@@ -442,12 +461,12 @@ FHD_D FaceFlux<NS> face_flux(const DevParams& P, const Fields<NS, R>& F, const N
 
     // ---- stochastic part (fluxStag.cpp:298-781) ----
     if (NZ != NZ_OFF && !transverse) {
-        const R Th = R(F.T(i, j, k)), Tl = R(F.T(im, jm, km));
-        R kp = (F.kappa(i, j, k) * Th * Th + F.kappa(im, jm, km) * Tl * Tl);
+        const R Th = R(x.T(1)), Tl = R(x.T(0));
+        R kp = (x.kappa(1) * Th * Th + x.kappa(0) * Tl * Tl);
         R meanT = R(0.5) * (Th + Tl);
         if (WL && ws >= 0) {
-            const R Tg = R(F.T(gi, gj, gk));
-            kp = R(2.0) * F.kappa(gi, gj, gk) * Tg * Tg;
+            const R Tg = R(x.T(gs));
+            kp = R(2.0) * x.kappa(gs) * Tg * Tg;
             meanT = Tg;
         }
         double wf[NS + 1];
@@ -464,10 +483,10 @@ FHD_D FaceFlux<NS> face_flux(const DevParams& P, const Fields<NS, R>& F, const N
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
             wien[s] = R(0.);
-            yy[s] = clamp01(R(F.Y(im, jm, km, s)));
-            yyp[s] = clamp01(R(F.Y(i, j, k, s)));
-            if (WL && ws == 0) yyp[s] = clamp01(R(F.Y(im, jm, km, s)));
-            if (WL && ws == 1) yy[s] = clamp01(R(F.Y(i, j, k, s)));
+            yy[s] = clamp01(R(x.Y(0, s)));
+            yyp[s] = clamp01(R(x.Y(1, s)));
+            if (WL && ws == 0) yyp[s] = clamp01(R(x.Y(0, s)));
+            if (WL && ws == 1) yy[s] = clamp01(R(x.Y(1, s)));
         }
         R sumy = R(0.), sumyp = R(0.);
 #pragma unroll
@@ -481,11 +500,11 @@ FHD_D FaceFlux<NS> face_flux(const DevParams& P, const Fields<NS, R>& F, const N
 #pragma unroll
             for (int ll = 0; ll < NS; ++ll) {
                 if (WL && ws >= 0)
-                    DY[s * NS + ll] = R(0.5) * (F.D(gi, gj, gk, ll * NS + s) * yy[ll] + F.D(gi, gj, gk, ll * NS + s) * yyp[ll] +
-                                                (F.D(gi, gj, gk, s * NS + ll) * yy[s] + F.D(gi, gj, gk, s * NS + ll) * yyp[s]));
+                    DY[s * NS + ll] = R(0.5) * (x.Dc(gs, ll * NS + s) * yy[ll] + x.Dc(gs, ll * NS + s) * yyp[ll] +
+                                                (x.Dc(gs, s * NS + ll) * yy[s] + x.Dc(gs, s * NS + ll) * yyp[s]));
                 else
-                    DY[s * NS + ll] = R(0.5) * (F.D(im, jm, km, ll * NS + s) * yy[ll] + F.D(i, j, k, ll * NS + s) * yyp[ll] +
-                                                (F.D(im, jm, km, s * NS + ll) * yy[s] + F.D(i, j, k, s * NS + ll) * yyp[s]));
+                    DY[s * NS + ll] = R(0.5) * (x.Dc(0, ll * NS + s) * yy[ll] + x.Dc(1, ll * NS + s) * yyp[ll] +
+                                                (x.Dc(0, s * NS + ll) * yy[s] + x.Dc(1, s * NS + ll) * yyp[s]));
             }
         }
 #pragma unroll
@@ -513,10 +532,10 @@ FHD_D FaceFlux<NS> face_flux(const DevParams& P, const Fields<NS, R>& F, const N
             R soret_s;
             if (WL && ws >= 0)
                 soret_s = (hk[s] + divc(P, R(P.Runiv) * meanT, R(P.molmass[s]), R(P.rmolmass[s])) *
-                                       F.chi(gi, gj, gk, s)) * wien[s];
+                                       x.chi(gs, s)) * wien[s];
             else
                 soret_s = (hk[s] + divc(P, R(P.Runiv) * meanT, R(P.molmass[s]), R(P.rmolmass[s])) * R(0.5) *
-                                       (F.chi(im, jm, km, s) + F.chi(i, j, k, s))) * wien[s];
+                                       (x.chi(0, s) + x.chi(1, s))) * wien[s];
             soret += soret_s;
         }
         duf = soret;
@@ -535,15 +554,15 @@ FHD_D FaceFlux<NS> face_flux(const DevParams& P, const Fields<NS, R>& F, const N
         // wall faces difference over the half cell to the wall value
         const R h = (WL && ws >= 0) ? R(P.hdx[D]) : R(P.dx[D]);
         const R rh = (WL && ws >= 0) ? R(P.rhdx[D]) : R(P.rdx[D]);
-        const R Tl = R(F.T(im, jm, km)), Th = R(F.T(i, j, k));
-        const R pl = R(F.p(im, jm, km)), ph = R(F.p(i, j, k));
-        R kp = R(0.5) * (F.kappa(im, jm, km) + F.kappa(i, j, k));
+        const R Tl = R(x.T(0)), Th = R(x.T(1));
+        const R pl = R(x.p(0)), ph = R(x.p(1));
+        R kp = R(0.5) * (x.kappa(0) + x.kappa(1));
         R meanT = R(0.5) * (Tl + Th);
         R meanP = R(0.5) * (pl + ph);
         if (WL && ws >= 0) {
-            kp = F.kappa(gi, gj, gk);
-            meanT = R(F.T(gi, gj, gk));
-            meanP = R(F.p(gi, gj, gk));
+            kp = x.kappa(gs);
+            meanT = R(x.T(gs));
+            meanP = R(x.p(gs));
         }
         heat -= divc(P, kp * (Th - Tl), h, rh);
         // species diffusion, Dufour: mixtures only
@@ -551,18 +570,18 @@ FHD_D FaceFlux<NS> face_flux(const DevParams& P, const Fields<NS, R>& F, const N
         R dk[NS], sor[NS], Fk[NS], hk[NS];
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
-            const R Xl = R(F.X(im, jm, km, s)), Xh = R(F.X(i, j, k, s));
+            const R Xl = R(x.X(0, s)), Xh = R(x.X(1, s));
             const R term1 = divc(P, Xh - Xl, h, rh);
             R mX = R(0.5) * (Xl + Xh);
-            R mY = R(0.5) * (R(F.Y(im, jm, km, s)) + R(F.Y(i, j, k, s)));
+            R mY = R(0.5) * (R(x.Y(0, s)) + R(x.Y(1, s)));
             if (WL && ws >= 0) {
-                mX = R(F.X(gi, gj, gk, s));
-                mY = R(F.Y(gi, gj, gk, s));
+                mX = R(x.X(gs, s));
+                mY = R(x.Y(gs, s));
             }
             const R term2 = divz(divc0(P, (mX - mY) * (ph - pl), h, rh), meanP);
             dk[s] = term1 + term2;
-            R ChiX = R(0.5) * (F.chi(im, jm, km, s) * Xl + F.chi(i, j, k, s) * Xh);
-            if (WL && ws >= 0) ChiX = F.chi(gi, gj, gk, s) * R(F.X(gi, gj, gk, s));
+            R ChiX = R(0.5) * (x.chi(0, s) * Xl + x.chi(1, s) * Xh);
+            if (WL && ws >= 0) ChiX = x.chi(gs, s) * R(x.X(gs, s));
             sor[s] = divz(divc0(P, ChiX * (Th - Tl), h, rh), meanT);
         }
 #pragma unroll
@@ -571,8 +590,8 @@ FHD_D FaceFlux<NS> face_flux(const DevParams& P, const Fields<NS, R>& F, const N
 #pragma unroll
             for (int ll = 0; ll < NS; ++ll) {
                 R Fks;
-                if (WL && ws >= 0) Fks = F.D(gi, gj, gk, ll * NS + kk) * (dk[ll] + sor[ll]);
-                else Fks = R(0.5) * (F.D(im, jm, km, ll * NS + kk) + F.D(i, j, k, ll * NS + kk)) * (dk[ll] + sor[ll]);
+                if (WL && ws >= 0) Fks = x.Dc(gs, ll * NS + kk) * (dk[ll] + sor[ll]);
+                else Fks = R(0.5) * (x.Dc(0, ll * NS + kk) + x.Dc(1, ll * NS + kk)) * (dk[ll] + sor[ll]);
                 f -= Fks;
             }
             Fk[kk] = f;
@@ -582,11 +601,11 @@ FHD_D FaceFlux<NS> face_flux(const DevParams& P, const Fields<NS, R>& F, const N
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
             if (WL && ws >= 0) {
-                Q5 += (hk[s] + divc0(P, R(P.Runiv) * meanT * F.chi(gi, gj, gk, s), R(P.molmass[s]), R(P.rmolmass[s]))) *
+                Q5 += (hk[s] + divc0(P, R(P.Runiv) * meanT * x.chi(gs, s), R(P.molmass[s]), R(P.rmolmass[s]))) *
                       Fk[s];
             } else {
                 // z faces use chi(i,j,k)+chi(i,j,k), fluxStag.cpp:1407 (kept from the reference)
-                const R chs = (D == 2) ? (F.chi(i, j, k, s) + F.chi(i, j, k, s)) : (F.chi(im, jm, km, s) + F.chi(i, j, k, s));
+                const R chs = (D == 2) ? (x.chi(1, s) + x.chi(1, s)) : (x.chi(0, s) + x.chi(1, s));
                 Q5 += (hk[s] + divc0(P, R(0.5) * R(P.Runiv) * meanT * chs, R(P.molmass[s]), R(P.rmolmass[s]))) * Fk[s];
             }
         }
@@ -616,31 +635,32 @@ FHD_D FaceFlux<NS> face_flux(const DevParams& P, const Fields<NS, R>& F, const N
 #pragma unroll
         for (int s = 0; s < NS; ++s) fs[s] += 0.0;
     } else if (adv >= 0) {
-        const double m = F.mom[D](i, j, k);
-        const double u = F.vel[D](i, j, k);
+        const double m = x.m();
+        const double u = x.u();
         f0 += m;
-        const double pl = F.p(im, jm, km), ph = F.p(i, j, k);
+        const double pl = x.p(0), ph = x.p(1);
         if (adv == 2) {
-            f4 += 0.5 * (F.cons(im, jm, km, 4) + F.cons(i, j, k, 4)) * u + 0.5 * (pl + ph) * u;
+            f4 += 0.5 * (x.cons(0, 4) + x.cons(1, 4)) * u + 0.5 * (pl + ph) * u;
 #pragma unroll
-            for (int s = 0; s < NS; ++s) fs[s] += 0.5 * (F.cons(im, jm, km, 5 + s) + F.cons(i, j, k, 5 + s)) * u;
+            for (int s = 0; s < NS; ++s) fs[s] += 0.5 * (x.cons(0, 5 + s) + x.cons(1, 5 + s)) * u;
         } else {
-            const double meanT = 0.5 * (F.T(im, jm, km) + F.T(i, j, k));
-            const double meanRho = 0.5 * (F.cons(im, jm, km, 0) + F.cons(i, j, k, 0));
+            const double meanT = 0.5 * (x.T(0) + x.T(1));
+            const double meanRho = 0.5 * (x.cons(0, 0) + x.cons(1, 0));
             double hk[NS];
             GetEnthalpies<NS, double>(P, meanT, hk);
             if (adv == 1) {
-                const double meanE = 0.5 * (F.cons(im, jm, km, 4) + F.cons(i, j, k, 4)) / meanRho;
+                const double meanE = 0.5 * (x.cons(0, 4) + x.cons(1, 4)) / meanRho;
                 const double meanP = 0.5 * (pl + ph);
                 f4 += m * (meanE + (meanP / meanRho));
             }
 #pragma unroll
             for (int s = 0; s < NS; ++s) {
-                const double Yk = 0.5 * (F.Y(im, jm, km, s) + F.Y(i, j, k, s));
+                const double Yk = 0.5 * (x.Y(0, s) + x.Y(1, s));
                 fs[s] += Yk * m;
                 if (adv == 0) f4 += m * Yk * hk[s];
             }
             if (adv == 0) {
+                const int im = i - (D == 0), jm = j - (D == 1), km = k - (D == 2);
                 const Arr4<const double>& mx = F.mom[0];
                 const Arr4<const double>& my = F.mom[1];
                 const Arr4<const double>& mz = F.mom[2];
@@ -648,12 +668,12 @@ FHD_D FaceFlux<NS> face_flux(const DevParams& P, const Fields<NS, R>& F, const N
                 keP += (mx(i + 1, j, k) + mx(i, j, k)) * (mx(i + 1, j, k) + mx(i, j, k));
                 keP += (my(i, j + 1, k) + my(i, j, k)) * (my(i, j + 1, k) + my(i, j, k));
                 keP += (mz(i, j, k + 1) + mz(i, j, k)) * (mz(i, j, k + 1) + mz(i, j, k));
-                keP *= (0.125 / F.cons(i, j, k, 0) / F.cons(i, j, k, 0));
+                keP *= (0.125 / x.cons(1, 0) / x.cons(1, 0));
                 keM += (mx(im + 1, jm, km) + mx(im, jm, km)) * (mx(im + 1, jm, km) + mx(im, jm, km));
                 keM += (my(im, jm + 1, km) + my(im, jm, km)) * (my(im, jm + 1, km) + my(im, jm, km));
                 keM += (mz(im, jm, km + 1) + mz(im, jm, km)) * (mz(im, jm, km + 1) + mz(im, jm, km));
                 // z faces divide by cons(i,j-1,k,0), fluxStag.cpp:1755 (kept from the reference)
-                const double rm = (D == 2) ? F.cons(i, j - 1, k, 0) : F.cons(im, jm, km, 0);
+                const double rm = (D == 2) ? F.cons(i, j - 1, k, 0) : x.cons(0, 0);
                 keM *= (0.125 / rm / rm);
                 f4 += m * 0.5 * (keP + keM);
             }
@@ -681,7 +701,7 @@ FHD_D FaceFlux<NS> face_flux(const DevParams& P, const Fields<NS, R>& F, const N
 // side only (fluxStag.cpp:1774-1789, 1797-1812, 1820-1835: the second
 // direction's wall is tested first, the first direction's wins a corner).
 template <int NS, class R, int E, bool WL = false>
-FHD_D void edge_adv(const DevParams& P, const Fields<NS, R>& F, int i, int j, int k, double& a, double& b) {
+FHD_D void edge_adv(const RunParams& P, const Fields<NS, R>& F, int i, int j, int k, double& a, double& b) {
     const Arr4<const double>&mx = F.mom[0], &my = F.mom[1], &mz = F.mom[2];
     const Arr4<const double>&vx = F.vel[0], &vy = F.vel[1], &vz = F.vel[2];
     if (P.advection_type < 0) { a = b = 0.0; return; }
@@ -725,7 +745,7 @@ FHD_D double edge_total(const Taus<R>& t, double adv, int has_adv) {
 // of an edge of type E lying on wall planes, in its order (lo x, hi x, lo y, hi y,
 // lo z, hi z; boundaryStag.cpp:2456-3009)
 template <class R, int E>
-FHD_D double edge_total_w(const DevParams& P, const Taus<R>& t, double adv, int has_adv, int i, int j, int k) {
+FHD_D double edge_total_w(const RunParams& P, const Taus<R>& t, double adv, int has_adv, int i, int j, int k) {
     double v = (double)t.s;
     const int x[3] = {i, j, k};
 #pragma unroll
@@ -749,7 +769,7 @@ FHD_D double edge_total_w(const DevParams& P, const Taus<R>& t, double adv, int 
 // direction d is 0 (bc_mass 3) or, given as `inner` (bc_mass 4), that of the cell
 // inside it (BCWallReservoirFluxStag, boundaryStag.cpp:482-577).
 template <int NS, class R, bool WL = false>
-FHD_D double cen_total(const DevParams& P, const Fields<NS, R>& F, const CellTaus<R>& t, int d, int i, int j, int k,
+FHD_D double cen_total(const RunParams& P, const Fields<NS, R>& F, const CellTaus<R>& t, int d, int i, int j, int k,
                        const CellTaus<R>* inner = nullptr) {
     double v = (double)t.s[d];
     v -= (double)t.d[d];

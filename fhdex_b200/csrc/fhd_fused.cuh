@@ -121,7 +121,7 @@ template <int NS, class R, int NZ, int TX, int TY>
 FHD_D void zm_phase_a(const StageArgs<NS, R, NZ>& a, const ZmView<NS, R, TX, TY>& v, int k, bool xy_edges,
                       bool z_edges) {
     using G = ZmGeom<TX, TY>;
-    const DevParams& P = a.P;
+    const RunParams& P = a.P;
     const int s = v.slot(k);
     const int hadv = P.advection_type >= 0;
     for (int q = threadIdx.x; q < G::NC; q += blockDim.x) {
@@ -176,7 +176,7 @@ FHD_D void zm_phase_a(const StageArgs<NS, R, NZ>& a, const ZmView<NS, R, TX, TY>
 template <int NS, class R, int NZ, int TX, int TY>
 FHD_D void zm_phase_b(const StageArgs<NS, R, NZ>& a, const ZmView<NS, R, TX, TY>& v, int kz, int kxy) {
     using G = ZmGeom<TX, TY>;
-    const DevParams& P = a.P;
+    const RunParams& P = a.P;
     const ZmTaus<NS, R, TX, TY> tg{v};
     constexpr int NF = 2 + NS;
     const int nzi = kz >= 0 ? G::NT : 0;
@@ -185,7 +185,7 @@ FHD_D void zm_phase_b(const StageArgs<NS, R, NZ>& a, const ZmView<NS, R, TX, TY>
         if (q < nzi) {
             const int i = v.i0 + q % TX, j = v.j0 + q / TX;
             if (i >= P.n[0] || j >= P.n[1]) continue;
-            const FaceFlux<NS> f = face_flux<NS, R, NZ, 2>(P, a.F, a.noise, tg, i, j, kz);
+            const FaceFlux<NS> f = face_flux<NS, R, NZ, false>(P, a.F, a.noise, FaceGen<NS, R, 2, ZmTaus<NS, R, TX, TY>>{a.F, tg, i, j, kz}, i, j, kz);
             const int s = v.slot(kz);
 #pragma unroll
             for (int c = 0; c < NF; ++c) v.ffz(s, c)[q] = f.cons[c];
@@ -193,14 +193,14 @@ FHD_D void zm_phase_b(const StageArgs<NS, R, NZ>& a, const ZmView<NS, R, TX, TY>
             const int r = q - nzi;
             const int i = v.i0 + r % (TX + 1), j = v.j0 + r / (TX + 1);
             if (i > P.n[0] || j >= P.n[1]) continue;
-            const FaceFlux<NS> f = face_flux<NS, R, NZ, 0>(P, a.F, a.noise, tg, i, j, kxy);
+            const FaceFlux<NS> f = face_flux<NS, R, NZ, false>(P, a.F, a.noise, FaceGen<NS, R, 0, ZmTaus<NS, R, TX, TY>>{a.F, tg, i, j, kxy}, i, j, kxy);
 #pragma unroll
             for (int c = 0; c < NF; ++c) v.ffx(c)[r] = f.cons[c];
         } else {
             const int r = q - nzi - G::NFX;
             const int i = v.i0 + r % TX, j = v.j0 + r / TX;
             if (i >= P.n[0] || j > P.n[1]) continue;
-            const FaceFlux<NS> f = face_flux<NS, R, NZ, 1>(P, a.F, a.noise, tg, i, j, kxy);
+            const FaceFlux<NS> f = face_flux<NS, R, NZ, false>(P, a.F, a.noise, FaceGen<NS, R, 1, ZmTaus<NS, R, TX, TY>>{a.F, tg, i, j, kxy}, i, j, kxy);
 #pragma unroll
             for (int c = 0; c < NF; ++c) v.ffy(c)[r] = f.cons[c];
         }
@@ -212,7 +212,7 @@ FHD_D void zm_phase_b(const StageArgs<NS, R, NZ>& a, const ZmView<NS, R, TX, TY>
 template <int NS, class R, int NZ>
 FHD_D double zm_face_update(const StageArgs<NS, R, NZ>& a, int d, int i, int j, int k, double t1, double t2,
                             double t3) {
-    const DevParams& P = a.P;
+    const RunParams& P = a.P;
     const Fields<NS, R>& F = a.F;
     const double dt = P.dt;
     const int e0 = d == 0, e1 = d == 1, e2 = d == 2;
@@ -240,7 +240,7 @@ FHD_D double zm_face_update(const StageArgs<NS, R, NZ>& a, int d, int i, int j, 
 template <int NS, class R, int NZ, int TX, int TY>
 FHD_D void zm_phase_c(const StageArgs<NS, R, NZ>& a, const ZmView<NS, R, TX, TY>& v, int k, bool faces_only) {
     using G = ZmGeom<TX, TY>;
-    const DevParams& P = a.P;
+    const RunParams& P = a.P;
     const Fields<NS, R>& F = a.F;
     const double dt = P.dt;
     const int st = a.stage;

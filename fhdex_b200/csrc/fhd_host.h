@@ -150,6 +150,9 @@ struct StageCall {
 // exact (FP64) translation unit
 int exact_cellprep(const StageCall& c);
 int exact_stage_part(const StageCall& c, int part);  // 0 stresses, 1 face fluxes, 2 update, 3 fused (all three)
+// flux MultiFabs: exact_aux_stage writes them beside a stage's stresses (part 0) and
+// face fluxes (part 1), exact_aux_fluxes in kernels of their own without scratch
+int exact_aux_stage(const StageCall& c, int part);
 int exact_aux_fluxes(const StageCall& c);
 int exact_transport(const DevParams& P, fhd_fab prim, fhd_fab eta, fhd_fab zeta, fhd_fab kappa, fhd_fab chi,
                     fhd_fab D, int* status, cudaStream_t s);

@@ -85,6 +85,20 @@ int FHD_CAT(exact_aux_ns, FHD_NS)(const StageCall& c) {
     return (c.P.walls || c.P.dim < 3) ? aux_mode<true>(c) : aux_mode<false>(c);
 }
 
+template <bool WL>
+int aux_stage_mode(const StageCall& c, int part) {
+    switch (c.mode) {
+        case NM_OFF: return launch_aux_stage_t<FHD_NS, NZ_OFF, WL>(c, part);
+        case NM_W: return launch_aux_stage_t<FHD_NS, NZ_W, WL>(c, part);
+        case NM_AB: return launch_aux_stage_t<FHD_NS, NZ_AB, WL>(c, part);
+        case NM_PHILOX: return launch_aux_stage_t<FHD_NS, NZ_PHILOX, WL>(c, part);
+        default: return FHD_ERR_BAD_ARG;
+    }
+}
+int FHD_CAT(exact_aux_stage_ns, FHD_NS)(const StageCall& c, int part) {
+    return (c.P.walls || c.P.dim < 3) ? aux_stage_mode<true>(c, part) : aux_stage_mode<false>(c, part);
+}
+
 int FHD_CAT(exact_walls_ns, FHD_NS)(const StageCall& c, int part) { return launch_walls_part<FHD_NS>(c, part); }
 
 int FHD_CAT(exact_bc_prim_ns, FHD_NS)(const DevParams& P, const WallParams& W, fhd_fab prim, fhd_fab cons,
@@ -132,8 +146,9 @@ int FHD_CAT(exact_convert_ns, FHD_NS)(const DevParams& P, fhd_fab prim, const fh
         a.vel[d] = view<double>(vel[d]);
         a.mom[d] = view<const double>(mom[d]);
     }
+    a.it = make_items(P.n[0], P.n[1], P.n[2]);
     a.status = status;
-    const int64_t tot = (int64_t)P.n[0] * P.n[1] * P.n[2];
+    const int64_t tot = a.it.n;
     k_convert<FHD_NS><<<resident_grid<k_convert<FHD_NS>>(tot, 128), 128, 0, s>>>(a);
     return cuda_rc(cudaGetLastError());
 }

@@ -3,8 +3,8 @@
 //   k_cellprep  per stage: conservedToPrimitiveStag + calculateTransportCoeffs for
 //               every cell once (cells grown by 1, face velocities grown by 1)
 //   k_taus      per stage: stochastic + deterministic stresses on cells and edges
-//   k_faces<D>  per stage and direction: stochastic + diffusive + hyperbolic
-//               conservative face fluxes (one small kernel per direction)
+//   k_faces     per stage: stochastic + diffusive + hyperbolic conservative face
+//               fluxes of the three directions
 //   k_update    per stage: flux divergence, momentum update and the SSP-RK3
 //               combination
 //   k_convert   end of step / drop-in conversion (prim, vel, cons 1..3)
@@ -40,19 +40,19 @@ struct PrepArgs {
     Arr4<double> vel[3];
     Arr4<double> pr;   // view starting at the T component: T, p, Y[NS], X[NS]
     Arr4<R> eta, zeta, kappa, chi, D;
+    Items it;          // cells [-1, n + 1]^3
     int* status;
 };
 
 template <int NS, class R>
-FHD_D int cellprep_count(const PrepArgs<NS, R>& a) { return (a.P.n[0] + 3) * (a.P.n[1] + 3) * (a.P.n[2] + 3); }
+FHD_D int cellprep_count(const PrepArgs<NS, R>& a) { return a.it.n; }
 
 template <int NS, class R>
 FHD_D void cellprep_point(const PrepArgs<NS, R>& a, int q) {
     const DevParams& P = a.P;
-    const int nx = P.n[0] + 3, ny = P.n[1] + 3;
-    const int i = q % nx - 1;
-    const int j = (q / nx) % ny - 1;
-    const int k = q / (nx * ny) - 1;
+    int i, j, k;
+    a.it.point(q, i, j, k);
+    --i; --j; --k;
     const double rho = a.cons(i, j, k, 0);
     // low face velocities (conservedPrimitiveConversionsStag.cpp:61-67)
     a.vel[0](i, j, k) = 2 * a.mom[0](i, j, k) / (rho + a.cons(i - 1, j, k, 0));
@@ -105,7 +105,7 @@ static __global__ void __launch_bounds__(128, cellprep_min_blocks<NS, R>()) k_ce
 // bc_mass 4 side of direction d takes the stochastic and diffusive part of the cell
 // inside it (recomputed here with that cell's own noise)
 template <int NS, class R, int NZ, bool WL>
-FHD_D double cen_total_res(const DevParams& P, const Fields<NS, R>& F, const Noise<NZ>& nz, const CellTaus<R>& t,
+FHD_D double cen_total_res(const RunParams& P, const Fields<NS, R>& F, const Noise<NZ>& nz, const CellTaus<R>& t,
                            int d, int i, int j, int k) {
     if (WL) {
         const int x = d == 0 ? i : (d == 1 ? j : k);
@@ -121,7 +121,7 @@ FHD_D double cen_total_res(const DevParams& P, const Fields<NS, R>& F, const Noi
 }
 
 // ===================================================================================
-// stage pipeline: k_taus -> k_faces<D> (x3) -> k_update
+// stage pipeline: k_taus -> k_faces -> k_update
 // ===================================================================================
 // Scratch of one stage (owned by the context):
 //   ct: cell stresses on the cells grown by 1, comps 0-2 stochastic xx,yy,zz,
@@ -131,9 +131,37 @@ FHD_D double cen_total_res(const DevParams& P, const Fields<NS, R>& F, const Noi
 //   mc: total centre momentum fluxes (cenflux x, y, z) on the cells grown by 1
 //   me: total edge momentum fluxes on [0, n]^3 in the reference's order
 //       edgeflux_x[0..1], edgeflux_y[0..1], edgeflux_z[0..1]
+// What the face kernel reads, as one pointer per component at point (0,0,0) of its
+// fab and the strides of the fabs: an operand is then pointer + offset, with the
+// offset shared by the components of a fab.
+template <int NS, class R>
+struct FaceIn {
+    const double *T, *p, *Y[NS], *X[NS];          // prim
+    const double *E, *rY[NS];                     // cons 4, 5..
+    const R *kappa, *chi[NS], *D[NS * NS];
+    int psy, psz, csy, csz, ksy, ksz, hsy, hsz, dsy, dsz;   // prim, cons, kappa, chi, D
+    int tsy, tsz, esy, esz;                       // ct, et
+};
+// ... and what depends on the face direction: the same code serves the three
+template <int NS, class R>
+struct FaceDir {
+    const double *u, *m;                          // vel[d], mom[d]
+    int usy, usz, msy, msz;
+    const R *cs, *cd;                             // ct comps d, 3 + d
+    struct Family {                               // edge family f (first, second transverse direction)
+        const R *s, *d;                           // et comps (s, d)
+        const double* v;                          // transverse velocity
+        int eq, vsy, vsz, vq, vd;                 // et: step to position 1; v: strides, steps to position 1 and across the face
+    } f[2];
+    int pd, cd_, kd, hd, dd, td;                  // steps across the face in prim, cons, kappa, chi, D, ct
+    double* ff[2 + NS];                           // rho, rhoE, rhoY fluxes
+    int fsy, fsz;
+    Items it;
+};
+
 template <int NS, class R, int NZ>
 struct StageArgs {
-    DevParams P;
+    RunParams P;
     Fields<NS, R> F;             // stage-input state U^s + derived fields
     Noise<NZ> noise;
     Arr4<R> ct, et;
@@ -144,21 +172,54 @@ struct StageArgs {
     Arr4<double> cons_o;         // U^{s+1}
     Arr4<double> mom_o[3];
     Arr4<const double> src;      // source (nprimvars comps) or p == nullptr
+    FaceIn<NS, R> fi;
+    FaceDir<NS, R> fd[3];
+    Items it_taus, it_upd;       // cells [-1, n]^3, points [0, n]^3
     int stage;                   // 1, 2, 3
 };
 
 // stresses on cells (grown by 1) and edges; one thread per point of [-1, n]^3
 template <int NS, class R, int NZ>
-FHD_D int taus_count(const StageArgs<NS, R, NZ>& a) { return (a.P.n[0] + 2) * (a.P.n[1] + 2) * (a.P.n[2] + 2); }
+FHD_D int taus_count(const StageArgs<NS, R, NZ>& a) { return a.it_taus.n; }
+
+// The flux MultiFabs of a caller that wants them (the reference's by-products, and the
+// flux operator's outputs): the stress kernel has every edge and centre total and the
+// face kernel every face flux in registers when it stores its stage's scratch, so
+// AUX writes them from there.  Computing them in kernels of their own recomputed six
+// stresses with their noise for every face.
+template <bool AUX>
+struct StageAux {
+    Arr4<double> ff[3];   // faceflux (nvars+4 comps)
+    Arr4<double> ef[6];   // edgeflux_x[0..1], edgeflux_y[0..1], edgeflux_z[0..1]
+    Arr4<double> cf[3];   // cenflux (1 ghost)
+};
+template <>
+struct StageAux<false> {};
+
+// both edge totals of an edge into the stage's scratch (absent: the flux operator) and
+// the flux fabs; ca, cb: their components in the order edgeflux_x, _y, _z
+template <int NS, class R, int NZ, bool AUX>
+FHD_D void put_edge(const StageArgs<NS, R, NZ>& a, const StageAux<AUX>& x, int i, int j, int k, int ca, double va,
+                    int cb, double vb) {
+    if (!AUX || a.me.p) {
+        a.me(i, j, k, ca) = va;
+        a.me(i, j, k, cb) = vb;
+    }
+    if constexpr (AUX) {
+        x.ef[ca](i, j, k) = va;
+        x.ef[cb](i, j, k) = vb;
+    }
+}
 
 // WL: walls (the wall variants of the edge stresses, advective edge fluxes and
 // StochFluxStag's factors on the edge totals)
-template <int NS, class R, int NZ, bool WL = false>
-FHD_D void taus_point(const StageArgs<NS, R, NZ>& a, int q) {
-    const DevParams& P = a.P;
-    const int nx = P.n[0] + 2, ny = P.n[1] + 2;
+template <int NS, class R, int NZ, bool WL = false, bool AUX = false>
+FHD_D void taus_point(const StageArgs<NS, R, NZ>& a, int q, const StageAux<AUX>& x = StageAux<AUX>()) {
+    const RunParams& P = a.P;
     {
-        const int i = q % nx - 1, j = (q / nx) % ny - 1, k = q / (nx * ny) - 1;
+        int i, j, k;
+        a.it_taus.point(q, i, j, k);
+        --i; --j; --k;
         const bool edges = i >= 0 && j >= 0 && k >= 0;
         double wc[3] = {0.0, 0.0, 0.0}, we[3] = {0.0, 0.0, 0.0};
         if (NZ != NZ_OFF) a.noise.cen_and_yz_edge(P, i, j, k, edges, wc, we[2]);
@@ -167,7 +228,9 @@ FHD_D void taus_point(const StageArgs<NS, R, NZ>& a, int q) {
         for (int d = 0; d < 3; ++d) {
             a.ct(i, j, k, d) = t.s[d];
             a.ct(i, j, k, 3 + d) = t.d[d];
-            a.mc(i, j, k, d) = cen_total_res<NS, R, NZ, WL>(P, a.F, a.noise, t, d, i, j, k);
+            const double c = cen_total_res<NS, R, NZ, WL>(P, a.F, a.noise, t, d, i, j, k);
+            if (!AUX || a.mc.p) a.mc(i, j, k, d) = c;
+            if constexpr (AUX) x.cf[d](i, j, k) = c;
         }
         if (!edges) return;
         if (NZ != NZ_OFF) a.noise.xy_xz_edges(P, i, j, k, we[0], we[1]);
@@ -178,95 +241,148 @@ FHD_D void taus_point(const StageArgs<NS, R, NZ>& a, int q) {
             a.et(i, j, k, 0) = e.s;
             a.et(i, j, k, 1) = e.d;
             edge_adv<NS, R, 0, WL>(P, a.F, i, j, k, ea, eb);
-            a.me(i, j, k, 2) = WL ? edge_total_w<R, 0>(P, e, ea, hadv, i, j, k) : edge_total<R>(e, ea, hadv);  // edgey_u
-            a.me(i, j, k, 0) = WL ? edge_total_w<R, 0>(P, e, eb, hadv, i, j, k) : edge_total<R>(e, eb, hadv);  // edgex_v
+            put_edge(a, x, i, j, k, 2, WL ? edge_total_w<R, 0>(P, e, ea, hadv, i, j, k) : edge_total<R>(e, ea, hadv),  // edgey_u
+                     0, WL ? edge_total_w<R, 0>(P, e, eb, hadv, i, j, k) : edge_total<R>(e, eb, hadv));         // edgex_v
         }
         if (j < P.n[1]) {
             const Taus<R> e = edge_taus_w<NS, R, NZ, 1, WL>(P, a.F, we[1], i, j, k);
             a.et(i, j, k, 2) = e.s;
             a.et(i, j, k, 3) = e.d;
             edge_adv<NS, R, 1, WL>(P, a.F, i, j, k, ea, eb);
-            a.me(i, j, k, 4) = WL ? edge_total_w<R, 1>(P, e, ea, hadv, i, j, k) : edge_total<R>(e, ea, hadv);  // edgez_u
-            a.me(i, j, k, 1) = WL ? edge_total_w<R, 1>(P, e, eb, hadv, i, j, k) : edge_total<R>(e, eb, hadv);  // edgex_w
+            put_edge(a, x, i, j, k, 4, WL ? edge_total_w<R, 1>(P, e, ea, hadv, i, j, k) : edge_total<R>(e, ea, hadv),  // edgez_u
+                     1, WL ? edge_total_w<R, 1>(P, e, eb, hadv, i, j, k) : edge_total<R>(e, eb, hadv));         // edgex_w
         }
         if (i < P.n[0]) {
             const Taus<R> e = edge_taus_w<NS, R, NZ, 2, WL>(P, a.F, we[2], i, j, k);
             a.et(i, j, k, 4) = e.s;
             a.et(i, j, k, 5) = e.d;
             edge_adv<NS, R, 2, WL>(P, a.F, i, j, k, ea, eb);
-            a.me(i, j, k, 5) = WL ? edge_total_w<R, 2>(P, e, ea, hadv, i, j, k) : edge_total<R>(e, ea, hadv);  // edgez_v
-            a.me(i, j, k, 3) = WL ? edge_total_w<R, 2>(P, e, eb, hadv, i, j, k) : edge_total<R>(e, eb, hadv);  // edgey_w
+            put_edge(a, x, i, j, k, 5, WL ? edge_total_w<R, 2>(P, e, ea, hadv, i, j, k) : edge_total<R>(e, ea, hadv),  // edgez_v
+                     3, WL ? edge_total_w<R, 2>(P, e, eb, hadv, i, j, k) : edge_total<R>(e, eb, hadv));         // edgey_w
         }
     }
 }
 
-template <int NS, class R, int NZ, bool WL = false>
-static __global__ void __launch_bounds__(256) k_taus(StageArgs<NS, R, NZ> a) {
+template <int NS, class R, int NZ, bool WL = false, bool AUX = false>
+static __global__ void __launch_bounds__(256) k_taus(StageArgs<NS, R, NZ> a, StageAux<AUX> x) {
     const int tot = taus_count(a);
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < tot; q += gridDim.x * blockDim.x)
-        taus_point<NS, R, NZ, WL>(a, q);
+        taus_point<NS, R, NZ, WL, AUX>(a, q, x);
 }
 
-template <class R>
-struct GlobalTaus {
-    Arr4<R> ct, et;
-    FHD_D CellTaus<R> cell(int i, int j, int k) const {
-        CellTaus<R> t;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            t.s[d] = ct(i, j, k, d);
-            t.d[d] = ct(i, j, k, 3 + d);
-        }
+// operands of one face of a direction known only at run time (face_flux)
+template <int NS, class R, int NZ>
+struct FaceRun {
+    const StageArgs<NS, R, NZ>& a;
+    int d, op, oc, ok, oh, od, ot, oe, ou, om, ov[2];
+    FHD_D FaceRun(const StageArgs<NS, R, NZ>& a_, int d_, int i, int j, int k) : a(a_), d(d_) {
+        const FaceIn<NS, R>& fi = a.fi;
+        const FaceDir<NS, R>& f = a.fd[d];
+        op = i + j * fi.psy + k * fi.psz;
+        oc = i + j * fi.csy + k * fi.csz;
+        ok = i + j * fi.ksy + k * fi.ksz;
+        oh = i + j * fi.hsy + k * fi.hsz;
+        od = i + j * fi.dsy + k * fi.dsz;
+        ot = i + j * fi.tsy + k * fi.tsz;
+        oe = i + j * fi.esy + k * fi.esz;
+        ou = i + j * f.usy + k * f.usz;
+        om = i + j * f.msy + k * f.msz;
+        ov[0] = i + j * f.f[0].vsy + k * f.f[0].vsz;
+        ov[1] = i + j * f.f[1].vsy + k * f.f[1].vsz;
+    }
+    FHD_D const FaceDir<NS, R>& f() const { return a.fd[d]; }
+    FHD_D int dir() const { return d; }
+    FHD_D double T(int s) const { return a.fi.T[s ? op : op - f().pd]; }
+    FHD_D double p(int s) const { return a.fi.p[s ? op : op - f().pd]; }
+    FHD_D double Y(int s, int n) const { return a.fi.Y[n][s ? op : op - f().pd]; }
+    FHD_D double X(int s, int n) const { return a.fi.X[n][s ? op : op - f().pd]; }
+    FHD_D double cons(int s, int n) const {
+        const int o = s ? oc : oc - f().cd_;
+        if (n == 4) return a.fi.E[o];
+        if (n >= 5) return a.fi.rY[n - 5][o];
+        return a.F.cons.p[o];
+    }
+    FHD_D R kappa(int s) const { return a.fi.kappa[s ? ok : ok - f().kd]; }
+    FHD_D R chi(int s, int n) const { return a.fi.chi[n][s ? oh : oh - f().hd]; }
+    FHD_D R Dc(int s, int n) const { return a.fi.D[n][s ? od : od - f().dd]; }
+    FHD_D double u() const { return f().u[ou]; }
+    FHD_D double m() const { return f().m[om]; }
+    FHD_D Taus<R> cell(int s) const {
+        const int o = s ? ot : ot - f().td;
+        Taus<R> t;
+        t.s = f().cs[o];
+        t.d = f().cd[o];
         return t;
     }
-    template <int E>
-    FHD_D Taus<R> edge(int i, int j, int k) const {
+    FHD_D Taus<R> edge(int q, int pos) const {
+        const int o = pos ? oe + f().f[q].eq : oe;
         Taus<R> t;
-        t.s = et(i, j, k, 2 * E);
-        t.d = et(i, j, k, 2 * E + 1);
+        t.s = f().f[q].s[o];
+        t.d = f().f[q].d[o];
         return t;
+    }
+    FHD_D double vt(int q, int pos, int s) const {
+        const auto& v = f().f[q];
+        return v.v[ov[q] + (pos ? v.vq : 0) - (s ? 0 : v.vd)];
     }
 };
 
-// conservative fluxes of the faces of direction D; one thread per valid face.
-template <int NS, class R, int NZ, int D>
-FHD_D int faces_count(const StageArgs<NS, R, NZ>& a) {
-    return (a.P.n[0] + (D == 0)) * (a.P.n[1] + (D == 1)) * (a.P.n[2] + (D == 2));
-}
+template <int NS, class R, int NZ>
+FHD_D int faces_count(const StageArgs<NS, R, NZ>& a, int d) { return a.fd[d].it.n; }
 
-template <int NS, class R, int NZ, int D, bool WL = false>
-FHD_D void faces_point(const StageArgs<NS, R, NZ>& a, int q) {
-    const DevParams& P = a.P;
-    const int nx = P.n[0] + (D == 0), ny = P.n[1] + (D == 1);
-    const GlobalTaus<R> tg{a.ct, a.et};
-    const int i = q % nx, j = (q / nx) % ny, k = q / (nx * ny);
-    const FaceFlux<NS> f = face_flux<NS, R, NZ, D, GlobalTaus<R>, WL>(P, a.F, a.noise, tg, i, j, k);
+// conservative flux of face q of direction d
+template <int NS, class R, int NZ, bool WL = false, bool AUX = false>
+FHD_D void faces_point(const StageArgs<NS, R, NZ>& a, int d, int q, const StageAux<AUX>& aux = StageAux<AUX>()) {
+    int i, j, k;
+    a.fd[d].it.point(q, i, j, k);
+    const FaceRun<NS, R, NZ> x(a, d, i, j, k);
+    const FaceFlux<NS> f = face_flux<NS, R, NZ, WL>(a.P, a.F, a.noise, x, i, j, k);
+    if (!AUX || a.ff[d].p) {
+        const int o = i + j * a.fd[d].fsy + k * a.fd[d].fsz;
 #pragma unroll
-    for (int c = 0; c < 2 + NS; ++c) a.ff[D](i, j, k, c) = f.cons[c];
+        for (int c = 0; c < 2 + NS; ++c) a.fd[d].ff[c][o] = f.cons[c];
+    }
+    if constexpr (AUX) {
+        const Arr4<double>& o = aux.ff[d];
+        o(i, j, k, 0) = f.cons[0];
+        o(i, j, k, 1) = 0.0;
+        o(i, j, k, 2) = 0.0;
+        o(i, j, k, 3) = 0.0;
+        o(i, j, k, 4) = f.cons[1];
+#pragma unroll
+        for (int s = 0; s < NS; ++s) o(i, j, k, 5 + s) = f.cons[2 + s];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) o(i, j, k, 5 + NS + c) = f.aux[c];
+    }
 }
 
+// The faces of the three directions in one launch, block b on direction b % 3: the
+// blocks working at one time then read the same cells for all three directions, so
+// the second and third find them in L2, and a small box keeps three times as many SMs
+// busy as one launch per direction.
 // MINB = minimum resident blocks requested from the register allocator.
-template <int NS, class R, int NZ, int D, int BS, int MINB, bool WL = false>
-static __global__ void __launch_bounds__(BS, MINB) k_faces(StageArgs<NS, R, NZ> a) {
-    const int tot = faces_count<NS, R, NZ, D>(a);
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < tot; q += gridDim.x * blockDim.x)
-        faces_point<NS, R, NZ, D, WL>(a, q);
+template <int NS, class R, int NZ, int BS, int MINB, bool WL = false, bool AUX = false>
+static __global__ void __launch_bounds__(BS, MINB) k_faces(StageArgs<NS, R, NZ> a, int per, StageAux<AUX> x) {
+    const int d = blockIdx.x % 3;
+    const int tot = faces_count(a, d);
+    for (int q = (blockIdx.x / 3) * BS + threadIdx.x; q < tot; q += per * BS)
+        faces_point<NS, R, NZ, WL, AUX>(a, d, q, x);
 }
 
 // RK3 stage combination (timeStepStag.cpp:439-528, 771-861, 1106-1202): one thread
 // per point of [0, n]^3 updates the cell there (if valid) and the faces there
 template <int NS, class R, int NZ>
-FHD_D int update_count(const StageArgs<NS, R, NZ>& a) { return (a.P.n[0] + 1) * (a.P.n[1] + 1) * (a.P.n[2] + 1); }
+FHD_D int update_count(const StageArgs<NS, R, NZ>& a) { return a.it_upd.n; }
 
 template <int NS, class R, int NZ>
 FHD_D void update_point(const StageArgs<NS, R, NZ>& a, int q) {
-    const DevParams& P = a.P;
+    const RunParams& P = a.P;
     const Fields<NS, R>& F = a.F;
-    const int nx = P.n[0] + 1, ny = P.n[1] + 1;
     const double dt = P.dt;
     const int st = a.stage;
     {
-        const int i = q % nx, j = (q / nx) % ny, k = q / (nx * ny);
+        int i, j, k;
+        a.it_upd.point(q, i, j, k);
         const bool cell = i < P.n[0] && j < P.n[1] && k < P.n[2];
         if (cell) {
             double on[2 + NS];
@@ -343,7 +459,8 @@ static __global__ void __launch_bounds__(128, 16) k_update(StageArgs<NS, R, NZ> 
 // ===================================================================================
 template <int NS>
 struct ConvArgs {
-    DevParams P;
+    RunParams P;
+    Items it;
     Arr4<double> prim;   // reference layout (nprimvars comps)
     Arr4<double> vel[3];
     Arr4<double> cons;   // comps 1..3 rewritten
@@ -352,15 +469,14 @@ struct ConvArgs {
 };
 
 template <int NS>
-FHD_D int convert_count(const ConvArgs<NS>& a) { return a.P.n[0] * a.P.n[1] * a.P.n[2]; }
+FHD_D int convert_count(const ConvArgs<NS>& a) { return a.it.n; }
 
 template <int NS>
 FHD_D void convert_point(const ConvArgs<NS>& a, int q) {
-    const DevParams& P = a.P;
+    const RunParams& P = a.P;
     {
-        const int i = q % P.n[0];
-        const int j = (q / P.n[0]) % P.n[1];
-        const int k = q / (P.n[0] * P.n[1]);
+        int i, j, k;
+        a.it.point(q, i, j, k);
         const Arr4<double>& cons = a.cons;
         const double rho = cons(i, j, k, 0);
         const Arr4<const double>&mx = a.mom[0], &my = a.mom[1], &mz = a.mom[2];
@@ -559,7 +675,7 @@ static __global__ void __launch_bounds__(128) k_transport(TransArgs<NS> a) {
 // stresses recomputed on the fly (operator path)
 template <int NS, class R, int NZ, bool WL = false>
 struct DirectTaus {
-    const DevParams* P;
+    const RunParams* P;
     const Fields<NS, R>* F;
     const Noise<NZ>* nz;
     FHD_D CellTaus<R> cell(int i, int j, int k) const { return cell_taus<NS, R, NZ, WL>(*P, *F, *nz, i, j, k); }
@@ -569,7 +685,7 @@ struct DirectTaus {
 
 template <int NS, class R, int NZ>
 struct AuxArgs {
-    DevParams P;
+    RunParams P;
     Fields<NS, R> F;
     Noise<NZ> noise;
     Arr4<double> ff[3];   // faceflux (nvars+4 comps)
@@ -580,7 +696,7 @@ struct AuxArgs {
 // faceflux[d] on valid faces; items enumerate the three face boxes back to back
 template <int NS, class R, int NZ, bool WL = false>
 static __global__ void __launch_bounds__(128) k_aux_faces(AuxArgs<NS, R, NZ> a) {
-    const DevParams& P = a.P;
+    const RunParams& P = a.P;
     const int* N = P.n;
     const int64_t nxf = (int64_t)(N[0] + 1) * N[1] * N[2], nyf = (int64_t)N[0] * (N[1] + 1) * N[2],
                   nzf = (int64_t)N[0] * N[1] * (N[2] + 1);
@@ -592,9 +708,9 @@ static __global__ void __launch_bounds__(128) k_aux_faces(AuxArgs<NS, R, NZ> a) 
         else if (q < nxf + nyf) { const int64_t r = q - nxf; d = 1; i = (int)(r % N[0]); j = (int)((r / N[0]) % (N[1] + 1)); k = (int)(r / ((int64_t)N[0] * (N[1] + 1))); }
         else { const int64_t r = q - nxf - nyf; d = 2; i = (int)(r % N[0]); j = (int)((r / N[0]) % N[1]); k = (int)(r / ((int64_t)N[0] * N[1])); }
         FaceFlux<NS> f;
-        if (d == 0) f = face_flux<NS, R, NZ, 0, TG, WL>(P, a.F, a.noise, tg, i, j, k);
-        else if (d == 1) f = face_flux<NS, R, NZ, 1, TG, WL>(P, a.F, a.noise, tg, i, j, k);
-        else f = face_flux<NS, R, NZ, 2, TG, WL>(P, a.F, a.noise, tg, i, j, k);
+        if (d == 0) f = face_flux<NS, R, NZ, WL>(P, a.F, a.noise, FaceGen<NS, R, 0, TG>{a.F, tg, i, j, k}, i, j, k);
+        else if (d == 1) f = face_flux<NS, R, NZ, WL>(P, a.F, a.noise, FaceGen<NS, R, 1, TG>{a.F, tg, i, j, k}, i, j, k);
+        else f = face_flux<NS, R, NZ, WL>(P, a.F, a.noise, FaceGen<NS, R, 2, TG>{a.F, tg, i, j, k}, i, j, k);
         const Arr4<double>& o = a.ff[d];
         o(i, j, k, 0) = f.cons[0];
         o(i, j, k, 1) = 0.0;
@@ -611,7 +727,7 @@ static __global__ void __launch_bounds__(128) k_aux_faces(AuxArgs<NS, R, NZ> a) 
 // edge fluxes (6 fabs) on valid edges and centre fluxes on cells grown by 1
 template <int NS, class R, int NZ, bool WL = false>
 static __global__ void __launch_bounds__(128) k_aux_edges_cen(AuxArgs<NS, R, NZ> a) {
-    const DevParams& P = a.P;
+    const RunParams& P = a.P;
     const int* N = P.n;
     const int64_t nxy = (int64_t)(N[0] + 1) * (N[1] + 1) * N[2], nxz = (int64_t)(N[0] + 1) * N[1] * (N[2] + 1),
                   nyz = (int64_t)N[0] * (N[1] + 1) * (N[2] + 1), nc = (int64_t)(N[0] + 2) * (N[1] + 2) * (N[2] + 2);
@@ -659,7 +775,7 @@ static __global__ void __launch_bounds__(128) k_aux_edges_cen(AuxArgs<NS, R, NZ>
 // bits, 27 from the first and 26 from the second word of one Philox call on the
 // counter (canonical point, field = fid0 + comp, stream).
 struct NoiseFillArgs {
-    DevParams P;
+    RunParams P;
     Arr4<double> f;
     int vx, vy, vz;   // extents of the filled box
     int ox, oy, oz;   // its low corner (0, or -1 to take the ghost layer of a wall direction)
@@ -691,20 +807,20 @@ static __global__ void k_noise_fill(NoiseFillArgs a) {
 }
 
 struct InitArgs {
-    Arr4<double> cu;
-    int64_t npts;     // points of one component (whole fab incl. ghosts)
+    double* cu;       // the fab's first element
+    int64_t sn, npts; // component stride; points of one component (whole fab incl. ghosts)
     int nvars, ns;
     double rho0, rhoE, rhoY[MAXS];
 };
 static __global__ void k_init_uniform(InitArgs a) {
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < a.npts; q += (int64_t)gridDim.x * blockDim.x) {
-        double* p = a.cu.p + q;
+        double* p = a.cu + q;
         p[0] = a.rho0;
-        p[a.cu.sn] = 0.0;
-        p[2 * a.cu.sn] = 0.0;
-        p[3 * a.cu.sn] = 0.0;
-        p[4 * a.cu.sn] = a.rhoE;
-        for (int s = 0; s < a.ns; ++s) p[(5 + s) * a.cu.sn] = a.rhoY[s];
+        p[a.sn] = 0.0;
+        p[2 * a.sn] = 0.0;
+        p[3 * a.sn] = 0.0;
+        p[4 * a.sn] = a.rhoE;
+        for (int s = 0; s < a.ns; ++s) p[(5 + s) * a.sn] = a.rhoY[s];
     }
 }
 
@@ -758,13 +874,13 @@ static __global__ void __launch_bounds__(128) k_taus_b(const StageArgs<NS, R, NZ
 
 // Register cap of the batched face kernel: MINB resident blocks of 128 threads
 // (8: 64 registers, 6: 80, 4: 128), picked per batch by its autotuner.
-template <int NS, class R, int NZ, int D, int MINB>
+template <int NS, class R, int NZ, int MINB>
 static __global__ void __launch_bounds__(128, MINB) k_faces_b(const StageArgs<NS, R, NZ>* __restrict__ args,
-                                                   const int* __restrict__ bpref, int nmem) {
+                                                   const int* __restrict__ bpref, int nmem, int d) {
     const int m = member_of(bpref, nmem);
     const StageArgs<NS, R, NZ>& a = member_args(args, m);
     const int q = (blockIdx.x - bpref[m]) * blockDim.x + threadIdx.x;
-    if (q < faces_count<NS, R, NZ, D>(a)) faces_point<NS, R, NZ, D>(a, q);
+    if (q < faces_count(a, d)) faces_point(a, d, q);
 }
 
 template <int NS, class R, int NZ>
@@ -895,15 +1011,15 @@ static __global__ void __launch_bounds__(128, MINB) k_batch_persist(PersistArgs 
                 } break;
                 case PK_FACEX: {
                     const auto& A = *reinterpret_cast<const StageArgs<NS, R, NZ>*>(sbuf);
-                    for (int64_t x = q; x < q1; x += st) faces_point<NS, R, NZ, 0>(A, (int)x);
+                    for (int64_t x = q; x < q1; x += st) faces_point(A, 0, (int)x);
                 } break;
                 case PK_FACEY: {
                     const auto& A = *reinterpret_cast<const StageArgs<NS, R, NZ>*>(sbuf);
-                    for (int64_t x = q; x < q1; x += st) faces_point<NS, R, NZ, 1>(A, (int)x);
+                    for (int64_t x = q; x < q1; x += st) faces_point(A, 1, (int)x);
                 } break;
                 case PK_FACEZ: {
                     const auto& A = *reinterpret_cast<const StageArgs<NS, R, NZ>*>(sbuf);
-                    for (int64_t x = q; x < q1; x += st) faces_point<NS, R, NZ, 2>(A, (int)x);
+                    for (int64_t x = q; x < q1; x += st) faces_point(A, 2, (int)x);
                 } break;
                 case PK_UPDATE: {
                     const auto& A = *reinterpret_cast<const StageArgs<NS, R, NZ>*>(sbuf);

@@ -11,13 +11,10 @@ template <class T>
 inline Arr4<T> view(const fhd_fab& f, int comp0 = 0) {
     Arr4<T> a;
     const int64_t nx = f.hi[0] - f.lo[0] + 1, ny = f.hi[1] - f.lo[1] + 1, nz = f.hi[2] - f.lo[2] + 1;
-    a.lo0 = f.lo[0];
-    a.lo1 = f.lo[1];
-    a.lo2 = f.lo[2];
     a.sy = nx;
     a.sz = nx * ny;
     a.sn = nx * ny * nz;
-    a.p = f.data ? static_cast<T*>(f.data) + comp0 * a.sn : nullptr;
+    a.p = f.data ? static_cast<T*>(f.data) + comp0 * a.sn - (f.lo[0] + f.lo[1] * nx + f.lo[2] * nx * ny) : nullptr;
     return a;
 }
 
@@ -61,6 +58,20 @@ inline int resident_grid(int64_t items, int block) {
     if (g > cap) g = cap;
     if (g < 1) g = 1;
     return (int)g;
+}
+
+// blocks per direction of the face kernel: together as many as the SMs hold at once
+template <auto K>
+inline int face_grid(const int N[3], int block) {
+    int64_t most = 0;
+    for (int d = 0; d < 3; ++d) {
+        const int64_t f = (int64_t)(N[0] + (d == 0)) * (N[1] + (d == 1)) * (N[2] + (d == 2));
+        if (f > most) most = f;
+    }
+    int64_t g = (most + block - 1) / block;
+    const int cap = resident_blocks<K>(block) / 3;
+    if (g > cap) g = cap;
+    return (int)(g < 1 ? 1 : g);
 }
 
 inline int grid_for(int64_t items, int block, int cap = 148 * 32) {
@@ -122,8 +133,9 @@ int launch_cellprep(const StageCall& c) {
     a.kappa = view<R>(c.kappa);
     a.chi = view<R>(c.chi);
     a.D = view<R>(c.D);
+    a.it = make_items(c.P.n[0] + 3, c.P.n[1] + 3, c.P.n[2] + 3);
     a.status = c.status;
-    const int64_t tot = (int64_t)(c.P.n[0] + 3) * (c.P.n[1] + 3) * (c.P.n[2] + 3);
+    const int64_t tot = a.it.n;
     // (an occupancy-sized grid was measured slower here: blocks beyond the resident
     // set rebalance this kernel's uneven per-cell cost)
     k_cellprep<NS, R><<<grid_for(tot, 128), 128, 0, c.stream>>>(a);
@@ -142,6 +154,68 @@ constexpr int kZmThreads[] = {128, 256, 256, 384};
 constexpr int kZmChunks[] = {32, 32, 64, 32};
 constexpr int kNumZmTiles = 4;
 inline bool tile_is_fused(int t) { return t >= kNumStageBlocks && t < kNumStageBlocks + kNumZmTiles; }
+
+template <class T>
+int step_of(const Arr4<T>& a, int d) { return d == 0 ? 1 : (d == 1 ? a.sy : a.sz); }
+
+// the face kernel's operands from the stage's views
+template <int NS, class R, int NZ>
+void make_face_args(StageArgs<NS, R, NZ>& a, const int n[3]) {
+    const Fields<NS, R>& F = a.F;
+    FaceIn<NS, R>& f = a.fi;
+    // (a fab that the stage does not have has no views: its pointers stay null)
+    auto comp = [](const auto& v, int c) { return v.p ? v.p + (int64_t)c * v.sn : nullptr; };
+    f.T = comp(F.pr, F.pT);
+    f.p = comp(F.pr, F.pT + 1);
+    f.E = comp(F.cons, 4);
+    f.kappa = F.kappa.p;
+    for (int s = 0; s < NS; ++s) {
+        f.Y[s] = comp(F.pr, F.pT + 2 + s);
+        f.X[s] = comp(F.pr, F.pT + 2 + NS + s);
+        f.rY[s] = comp(F.cons, 5 + s);
+        f.chi[s] = comp(F.chi, s);
+    }
+    for (int s = 0; s < NS * NS; ++s) f.D[s] = comp(F.D, s);
+    f.psy = F.pr.sy;    f.psz = F.pr.sz;
+    f.csy = F.cons.sy;  f.csz = F.cons.sz;
+    f.ksy = F.kappa.sy; f.ksz = F.kappa.sz;
+    f.hsy = F.chi.sy;   f.hsz = F.chi.sz;
+    f.dsy = F.D.sy;     f.dsz = F.D.sz;
+    f.tsy = a.ct.sy;    f.tsz = a.ct.sz;
+    f.esy = a.et.sy;    f.esz = a.et.sz;
+    for (int d = 0; d < 3; ++d) {
+        FaceDir<NS, R>& x = a.fd[d];
+        x.u = F.vel[d].p;  x.usy = F.vel[d].sy; x.usz = F.vel[d].sz;
+        x.m = F.mom[d].p;  x.msy = F.mom[d].sy; x.msz = F.mom[d].sz;
+        x.cs = comp(a.ct, d);
+        x.cd = comp(a.ct, 3 + d);
+        x.td = step_of(a.ct, d);
+        x.pd = step_of(F.pr, d);
+        x.cd_ = step_of(F.cons, d);
+        x.kd = step_of(F.kappa, d);
+        x.hd = step_of(F.chi, d);
+        x.dd = step_of(F.D, d);
+        // transverse directions and their edges: x (y on xy, z on xz), y (x on xy, z
+        // on yz), z (x on xz, y on yz)
+        const int t[2] = {d == 0 ? 1 : 0, d == 2 ? 1 : 2};
+        for (int q = 0; q < 2; ++q) {
+            const int e = d + t[q] == 1 ? 0 : (d + t[q] == 2 ? 1 : 2);
+            auto& g = x.f[q];
+            g.s = comp(a.et, 2 * e);
+            g.d = comp(a.et, 2 * e + 1);
+            g.eq = step_of(a.et, t[q]);
+            g.v = F.vel[t[q]].p;
+            g.vsy = F.vel[t[q]].sy;
+            g.vsz = F.vel[t[q]].sz;
+            g.vq = step_of(F.vel[t[q]], t[q]);
+            g.vd = step_of(F.vel[t[q]], d);
+        }
+        for (int c = 0; c < 2 + NS; ++c) x.ff[c] = comp(a.ff[d], c);
+        x.fsy = a.ff[d].sy;
+        x.fsz = a.ff[d].sz;
+        x.it = make_items(n[0] + (d == 0), n[1] + (d == 1), n[2] + (d == 2));
+    }
+}
 
 template <int NS, class R, int NZ>
 StageArgs<NS, R, NZ> make_stage_args(const StageCall& c) {
@@ -162,6 +236,10 @@ StageArgs<NS, R, NZ> make_stage_args(const StageCall& c) {
     a.cons_o = view<double>(c.cons_o);
     a.src = view<const double>(c.src);
     a.stage = c.stage;
+    const int* n = c.P.n;
+    a.it_taus = make_items(n[0] + 2, n[1] + 2, n[2] + 2);
+    a.it_upd = make_items(n[0] + 1, n[1] + 1, n[2] + 1);
+    make_face_args(a, n);
     return a;
 }
 
@@ -184,7 +262,7 @@ int auto_face_tile(const int N[3]) {
         const int64_t f = (int64_t)(N[0] + (d == 0)) * (N[1] + (d == 1)) * (N[2] + (d == 2));
         if (f > most) most = f;
     }
-    const int64_t blocks = (most + 127) / 128;
+    const int64_t blocks = 3 * ((most + 127) / 128);
     if (blocks <= 4 * device_sms()) return 0;
     if (blocks <= 6 * device_sms()) return 2;
     if (sizeof(R) == 8) return 4;
@@ -202,16 +280,14 @@ int launch_stage_part_t(const StageCall& c, int part) {
     const int* N = c.P.n;
     const int b = stage_block(c);
     if (part == 0) {
-        k_taus<NS, R, NZ><<<grid_for((int64_t)(N[0] + 2) * (N[1] + 2) * (N[2] + 2), b), b, 0, c.stream>>>(a);
+        k_taus<NS, R, NZ><<<grid_for((int64_t)(N[0] + 2) * (N[1] + 2) * (N[2] + 2), b), b, 0, c.stream>>>(a, {});
     } else if (part == 1) {
         const int t = (c.tile >= 0 && c.tile < kNumStageBlocks) ? c.tile : auto_face_tile<NS, R>(N);
-#define FHD_FACES(BS, MINB)                                                                                      \
-        k_faces<NS, R, NZ, 0, BS, MINB><<<resident_grid<k_faces<NS, R, NZ, 0, BS, MINB>>(                     \
-            (int64_t)(N[0] + 1) * N[1] * N[2], BS), BS, 0, c.stream>>>(a);                                     \
-        k_faces<NS, R, NZ, 1, BS, MINB><<<resident_grid<k_faces<NS, R, NZ, 1, BS, MINB>>(                     \
-            (int64_t)N[0] * (N[1] + 1) * N[2], BS), BS, 0, c.stream>>>(a);                                     \
-        k_faces<NS, R, NZ, 2, BS, MINB><<<resident_grid<k_faces<NS, R, NZ, 2, BS, MINB>>(                     \
-            (int64_t)N[0] * N[1] * (N[2] + 1), BS), BS, 0, c.stream>>>(a);
+#define FHD_FACES(BS, MINB)                                                                    \
+        {                                                                                      \
+            const int per = face_grid<k_faces<NS, R, NZ, BS, MINB>>(N, BS);                    \
+            k_faces<NS, R, NZ, BS, MINB><<<3 * per, BS, 0, c.stream>>>(a, per, {});            \
+        }
         switch (t) {
             case 0: FHD_FACES(128, 4) break;
             case 1: FHD_FACES(256, 2) break;
@@ -270,6 +346,28 @@ int launch_stage_zm_t(const StageCall& c) {
     }
 }
 
+// the stress (part 0) and face (part 1) launches of a stage whose fluxes the caller
+// wants (StageAux), and of the flux operator, whose StageCall has no stage scratch but
+// the stresses
+template <int NS, int NZ, bool WL>
+int launch_aux_stage_t(const StageCall& c, int part) {
+    const StageArgs<NS, double, NZ> a = make_stage_args<NS, double, NZ>(c);
+    StageAux<true> x;
+    for (int d = 0; d < 3; ++d) {
+        x.ff[d] = view<double>(c.ff[d]);
+        x.cf[d] = view<double>(c.cf[d]);
+    }
+    for (int e = 0; e < 6; ++e) x.ef[e] = view<double>(c.ef[e]);
+    if (part == 0) {
+        k_taus<NS, double, NZ, WL, true><<<grid_for(a.it_taus.n, 128), 128, 0, c.stream>>>(a, x);
+    } else {
+        constexpr int MB = WL && NS > 2 ? 4 : 8;
+        const int per = face_grid<k_faces<NS, double, NZ, 128, MB, WL, true>>(c.P.n, 128);
+        k_faces<NS, double, NZ, 128, MB, WL, true><<<3 * per, 128, 0, c.stream>>>(a, per, x);
+    }
+    return cuda_rc(cudaGetLastError());
+}
+
 // the stage parts of a box with physical walls (FP64, one launch shape): the wall
 // variants of the stresses and face fluxes, and the common update
 template <int NS, int NZ>
@@ -277,17 +375,13 @@ int launch_walls_part_t(const StageCall& c, int part) {
     const StageArgs<NS, double, NZ> a = make_stage_args<NS, double, NZ>(c);
     const int* N = c.P.n;
     if (part == 0) {
-        k_taus<NS, double, NZ, true><<<grid_for((int64_t)(N[0] + 2) * (N[1] + 2) * (N[2] + 2), 128), 128, 0, c.stream>>>(a);
+        k_taus<NS, double, NZ, true><<<grid_for((int64_t)(N[0] + 2) * (N[1] + 2) * (N[2] + 2), 128), 128, 0, c.stream>>>(a, {});
     } else if (part == 1) {
         // register cap: 64 up to two species (the periodic autotuner's choice at 256^3;
         // 128 was measured twice as slow for the wall variant), 128 above
         constexpr int MB = NS <= 2 ? 8 : 4;
-        k_faces<NS, double, NZ, 0, 128, MB, true><<<resident_grid<k_faces<NS, double, NZ, 0, 128, MB, true>>(
-            (int64_t)(N[0] + 1) * N[1] * N[2], 128), 128, 0, c.stream>>>(a);
-        k_faces<NS, double, NZ, 1, 128, MB, true><<<resident_grid<k_faces<NS, double, NZ, 1, 128, MB, true>>(
-            (int64_t)N[0] * (N[1] + 1) * N[2], 128), 128, 0, c.stream>>>(a);
-        k_faces<NS, double, NZ, 2, 128, MB, true><<<resident_grid<k_faces<NS, double, NZ, 2, 128, MB, true>>(
-            (int64_t)N[0] * N[1] * (N[2] + 1), 128), 128, 0, c.stream>>>(a);
+        const int per = face_grid<k_faces<NS, double, NZ, 128, MB, true>>(N, 128);
+        k_faces<NS, double, NZ, 128, MB, true><<<3 * per, 128, 0, c.stream>>>(a, per, {});
     } else {
         k_update<NS, double, NZ><<<resident_grid<k_update<NS, double, NZ>>(
             (int64_t)(N[0] + 1) * (N[1] + 1) * (N[2] + 1), 128), 128, 0, c.stream>>>(a);
@@ -439,6 +533,7 @@ ConvArgs<NS> make_conv_args(const StageCall& c) {
         a.vel[d] = view<double>(c.vel[d]);
         a.mom[d] = view<const double>(c.mom_o[d]);
     }
+    a.it = make_items(c.P.n[0], c.P.n[1], c.P.n[2]);
     a.status = c.status;
     return a;
 }
@@ -458,6 +553,7 @@ PrepArgs<NS, R> make_prep_args(const StageCall& c) {
     a.kappa = view<R>(c.kappa);
     a.chi = view<R>(c.chi);
     a.D = view<R>(c.D);
+    a.it = make_items(c.P.n[0] + 3, c.P.n[1] + 3, c.P.n[2] + 3);
     a.status = c.status;
     return a;
 }
@@ -491,9 +587,7 @@ constexpr int kNumBatchFaceTiles = 3;
 
 template <int NS, class R, int NZ, int MINB>
 void batch_faces_t(int kind, const StageArgs<NS, R, NZ>* sa, const int* dbpref, int nmem, int nblocks, cudaStream_t s) {
-    if (kind == 2) k_faces_b<NS, R, NZ, 0, MINB><<<nblocks, 128, 0, s>>>(sa, dbpref, nmem);
-    else if (kind == 3) k_faces_b<NS, R, NZ, 1, MINB><<<nblocks, 128, 0, s>>>(sa, dbpref, nmem);
-    else k_faces_b<NS, R, NZ, 2, MINB><<<nblocks, 128, 0, s>>>(sa, dbpref, nmem);
+    k_faces_b<NS, R, NZ, MINB><<<nblocks, 128, 0, s>>>(sa, dbpref, nmem, kind - 2);
 }
 
 template <int NS, class R, int NZ>

@@ -82,10 +82,10 @@ FHD_HD int wrap1(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
 // shifted by one so that the ghost cell -1 and the cell/node n are distinct
 // (n + 2 indices: cells -1..n, nodes 0..n), as the reference's wall directions
 // neither OverrideSync nor FillBoundary their noise.
-FHD_HD uint32_t canon1(const DevParams& P, int d, int i) {
+FHD_HD uint32_t canon1(const RunParams& P, int d, int i) {
     return P.periodic[d] ? (uint32_t)wrap1(i, P.n[d]) : (uint32_t)(i + 1);
 }
-FHD_HD uint32_t canon(const DevParams& P, int i, int j, int k) {
+FHD_HD uint32_t canon(const RunParams& P, int i, int j, int k) {
     if (!P.walls)
         return (uint32_t)wrap1(i, P.n[0]) +
                (uint32_t)P.n[0] * ((uint32_t)wrap1(j, P.n[1]) + (uint32_t)P.n[1] * (uint32_t)wrap1(k, P.n[2]));
