@@ -6,10 +6,9 @@
 // amrex::FFT::R2C), the Hermitian half spectrum unpacked to the full grid and
 // divided by sqrt(N) (ComputeFFT, :322-519), then for each pair (a, b)
 //   cov_real += Re_a Re_b + Im_a Im_b,   cov_imag += -(Im_a Re_b) + Re_a Im_b.
-// Here the unpacking is not materialised: one fused kernel reads both half
-// spectra at the point or at its mirror (conjugated), applies the 1/sqrt(N) and
-// accumulates every pair in place — one pass over the spectra and the
-// accumulators per sample.
+// Here the unpacking is not materialised: the covariances are accumulated on the
+// half spectrum (see SfArgs) in one kernel per sample and unfolded by the output
+// kernels.
 // CallFinalize / Finalize (:598-641) and ShiftFFT (:643-719): optional zeroing of
 // k = 0, shift by N/2 in every direction, scaling by 1/nsamples and by
 // 1/var_scaling, magnitude sqrt(re^2 + im^2).
@@ -47,81 +46,110 @@ struct fhd_sf {
     int64_t nsamples = 0;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
-    double* cov = nullptr;           // [2][ncov][nmem][Nm]: real then imaginary accumulators
+    double* cov = nullptr;           // [2][ncov][nmem][mz][my][mx/2+1]: real then imaginary accumulators
     double2* spec = nullptr;         // [nvaru][nmem][mz][my][mx/2+1] half spectra
-    double* real = nullptr;          // [nmem][mz][my][mx] dense copy of one variable (FFT input)
-    int* dpairs = nullptr;           // [2][ncov] pair -> unique-variable slot
+    double* real = nullptr;          // [nvaru][nmem][mz][my][mx] dense copy of the variables (FFT input)
+    int* dpairs = nullptr;           // [2][ncov] pair -> unique-variable slot, then the variables' components
     double* dscale = nullptr;        // [ncov]
     cufftHandle plan = 0;
+    int per_plan = 0;                // variables per execution of the plan: all, or one where that plan failed
     bool have_plan = false;
 };
 
 namespace {
 
+// The covariances of real fields are Hermitian: at a mirrored point (i > nx/2, where the
+// reference's unpacking takes the conjugate of entry (nx-i, -j, -k)) both spectra have
+// negated imaginary parts, so the real covariance is the stored entry's and the
+// imaginary one its negation, to the bit.  The accumulators are therefore kept on the
+// half spectrum and unfolded at the output: half the traffic of a sample.
 struct SfArgs {
-    int nx, ny, nz, nxh1, ncov;      // one member's shape
-    int64_t N, half;                 // points and half-spectrum entries of all members
-    int64_t Nm, halfm;               // ... of one member
-    double sqrtnpts;
+    int nv, ncov;
+    int64_t half;                    // half-spectrum entries of all members
+    double sqrtnpts, rsqrtnpts;      // sqrt(N) of a member, and its reciprocal
     const double2* spec;
     const int* pairs;                // pa slots then pb slots
     double* cov;
     int reset;
 };
 
-// (re, im) of unique variable `v` at full-grid point (i, j, k): the stored half
-// spectrum for i <= nx/2, else the conjugate at the mirror point
-// (ComputeFFT's unpacking rule, StructFact.cpp:394-421), then divided by sqrt(N).
-__device__ __forceinline__ void spec_at(const SfArgs& a, int v, int64_t b, int i, int j, int k, double& re,
-                                        double& im) {
-    const double2* S = a.spec + (int64_t)v * a.half + b * a.halfm;
-    if (i <= a.nx / 2) {
-        const double2 s = S[i + (int64_t)a.nxh1 * (j + (int64_t)a.ny * k)];
-        re = s.x;
-        im = s.y;
-    } else {
-        const int iloc = a.nx - i;
-        const int jloc = (j == 0) ? 0 : a.ny - j;
-        const int kloc = (k == 0) ? 0 : a.nz - k;
-        const double2 s = S[iloc + (int64_t)a.nxh1 * (jloc + (int64_t)a.ny * kloc)];
-        re = s.x;
-        im = -s.y;
-    }
-    re /= a.sqrtnpts;
-    im /= a.sqrtnpts;
+// (re, im) of unique variable v at half-spectrum entry h, divided by sqrt(N)
+// (ComputeFFT, StructFact.cpp:394-421); sqrt(N) is a run constant (fhd_div.h)
+__device__ __forceinline__ double2 spec_at(const SfArgs& a, int v, int64_t h) {
+    double2 s = a.spec[(int64_t)v * a.half + h];
+    s.x = div_rcp(s.x, a.sqrtnpts, a.rsqrtnpts);
+    s.y = div_rcp(s.y, a.sqrtnpts, a.rsqrtnpts);
+    return s;
 }
 
-__global__ void __launch_bounds__(256) k_sf_accumulate(SfArgs a) {
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < a.N; q += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t b = q / a.Nm, l = q - b * a.Nm;   // member, point within it
-        const int i = int(l % a.nx), j = int((l / a.nx) % a.ny), k = int(l / ((int64_t)a.nx * a.ny));
-        for (int c = 0; c < a.ncov; ++c) {
-            double rA, iA, rB, iB;
-            spec_at(a, a.pairs[c], b, i, j, k, rA, iA);
-            spec_at(a, a.pairs[a.ncov + c], b, i, j, k, rB, iB);
-            // cov_temp = 0 + Re_a Re_b; += Im_a Im_b   (StructFact.cpp:265-268)
-            double tr = 0.0 + rA * rB;
-            tr = tr + iA * iB;
-            // cov_temp = 0 + Im_a Re_b; *= -1; += Re_a Im_b   (:276-280)
-            double ti = 0.0 + iA * rB;
-            ti = ti * -1.0;
-            ti = ti + rA * iB;
-            double* re = a.cov + (int64_t)c * a.N + q;
-            double* imv = a.cov + ((int64_t)a.ncov + c) * a.N + q;
-            if (a.reset) {
-                *re = tr;
-                *imv = ti;
-            } else {
-                *re = *re + tr;
-                *imv = *imv + ti;
+constexpr int kSfThreads = 256;
+constexpr int kSfStaged = 12;        // variables whose values fit 48 KiB of shared memory per block
+
+// One thread per half-spectrum entry.  STAGED (up to kSfStaged variables): the thread
+// scales each variable's value once and keeps it in its own column of shared memory (a
+// pair's two slots are known only at run time, which registers cannot be indexed by);
+// else every pair reads and scales its two.  The accumulators of four pairs are
+// loaded together before the first is stored.  Bound by HBM.  With a full-grid
+// accumulator and four divisions per pair it took 153 us per sample at 144x112x96 (4
+// variables, 10 pairs), more than half of the sample; two samples and the output of
+// such a box went from 888 to 388 us with this, the batched transform and the output below.
+template <bool STAGED>
+__global__ void __launch_bounds__(kSfThreads) k_sf_accumulate(SfArgs a) {
+    extern __shared__ double2 sv[];
+    for (int64_t h = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; h < a.half; h += (int64_t)gridDim.x * blockDim.x) {
+        if (STAGED)
+            for (int v = 0; v < a.nv; ++v) sv[v * kSfThreads + threadIdx.x] = spec_at(a, v, h);
+        auto value = [&](int v) { return STAGED ? sv[v * kSfThreads + threadIdx.x] : spec_at(a, v, h); };
+        constexpr int U = 4;
+        for (int c0 = 0; c0 < a.ncov; c0 += U) {
+            double re[U], im[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (c0 + u >= a.ncov || a.reset) continue;
+                re[u] = a.cov[(int64_t)(c0 + u) * a.half + h];
+                im[u] = a.cov[((int64_t)a.ncov + c0 + u) * a.half + h];
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int c = c0 + u;
+                if (c >= a.ncov) continue;
+                const double2 A = value(a.pairs[c]), B = value(a.pairs[a.ncov + c]);
+                // cov_temp = 0 + Re_a Re_b; += Im_a Im_b   (StructFact.cpp:265-268)
+                double tr = 0.0 + A.x * B.x;
+                tr = tr + A.y * B.y;
+                // cov_temp = 0 + Im_a Re_b; *= -1; += Re_a Im_b   (:276-280)
+                double ti = 0.0 + A.y * B.x;
+                ti = ti * -1.0;
+                ti = ti + A.x * B.y;
+                re[u] = a.reset ? tr : re[u] + tr;
+                im[u] = a.reset ? ti : im[u] + ti;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (c0 + u >= a.ncov) continue;
+                a.cov[(int64_t)(c0 + u) * a.half + h] = re[u];
+                a.cov[((int64_t)a.ncov + c0 + u) * a.half + h] = im[u];
             }
         }
     }
 }
 
+// half-spectrum entry and sign of the imaginary part of full-grid point (i, j, k) of one member
+__device__ __forceinline__ int64_t half_entry(int nx, int ny, int nz, int i, int j, int k, double& sign) {
+    sign = 1.0;
+    if (i > nx / 2) {
+        sign = -1.0;
+        i = nx - i;
+        j = j == 0 ? 0 : ny - j;
+        k = k == 0 ? 0 : nz - k;
+    }
+    return i + (int64_t)(nx / 2 + 1) * (j + (int64_t)ny * k);
+}
+
 struct SfFinArgs {
     int nx, ny, nz, ncov, zero_avg;
-    int64_t N;
+    int64_t N, half;
+    FastDiv dx, dxy;
     double nsinv;
     const double* cov;
     const double* scale;
@@ -132,12 +160,19 @@ struct SfFinArgs {
 // ((i + nx/2) % nx, ...) of source point (i, j, k).
 __global__ void __launch_bounds__(256) k_sf_finalize(SfFinArgs a) {
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < a.N; q += (int64_t)gridDim.x * blockDim.x) {
-        const int i = int(q % a.nx), j = int((q / a.nx) % a.ny), k = int(q / ((int64_t)a.nx * a.ny));
-        const int ip = (i + a.nx / 2) % a.nx, jp = (j + a.ny / 2) % a.ny, kp = (k + a.nz / 2) % a.nz;
+        const int k = (int)a.dxy.div((uint32_t)q), r = (int)q - k * a.nx * a.ny;
+        const int j = (int)a.dx.div((uint32_t)r), i = r - j * a.nx;
+        int ip = i + a.nx / 2, jp = j + a.ny / 2, kp = k + a.nz / 2;
+        ip -= ip >= a.nx ? a.nx : 0;
+        jp -= jp >= a.ny ? a.ny : 0;
+        kp -= kp >= a.nz ? a.nz : 0;
         const bool zero = a.zero_avg == 1 && i == 0 && j == 0 && k == 0;
+        double sign;
+        const int64_t h = half_entry(a.nx, a.ny, a.nz, i, j, k, sign);
+#pragma unroll 4
         for (int c = 0; c < a.ncov; ++c) {
-            double re = zero ? 0.0 : a.cov[(int64_t)c * a.N + q];
-            double im = zero ? 0.0 : a.cov[((int64_t)a.ncov + c) * a.N + q];
+            double re = zero ? 0.0 : __ldg(a.cov + (int64_t)c * a.half + h);
+            double im = zero ? 0.0 : sign * __ldg(a.cov + ((int64_t)a.ncov + c) * a.half + h);
             re = re * a.nsinv;
             re = re * a.scale[c];
             im = im * a.nsinv;
@@ -153,7 +188,7 @@ __global__ void __launch_bounds__(256) k_sf_finalize(SfFinArgs a) {
 
 struct SfAvgArgs {
     int nx, ny, nz, ncov, zero_avg;
-    int64_t N, Nm, nmem;
+    int64_t Nm, nmem, half, halfm;
     double nsinv, meminv;
     const double* cov;
     const double* scale;
@@ -175,11 +210,15 @@ __global__ void __launch_bounds__(256) k_sf_stack_avg(SfAvgArgs a) {
         const int ip = (i + a.nx / 2) % a.nx, jp = (j + a.ny / 2) % a.ny, kp = (k + a.nz / 2) % a.nz;
         const bool zero = a.zero_avg == 1 && i == 0 && j == 0 && k == 0;
         {
-            double sm = 0.0, sr = 0.0, si = 0.0;
+            double sm = 0.0, sr = 0.0, si = 0.0, sign;
+            const int64_t h = half_entry(a.nx, a.ny, a.nz, i, j, k, sign);
+            const double* cr = a.cov + (int64_t)c * a.half + h;
+            const double* ci = a.cov + ((int64_t)a.ncov + c) * a.half + h;
+            // the members' loads are independent of the sums: eight in flight per chain
+#pragma unroll 8
             for (int64_t b = 0; b < a.nmem; ++b) {
-                const int64_t q = b * a.Nm + l;
-                double re = zero ? 0.0 : a.cov[(int64_t)c * a.N + q];
-                double im = zero ? 0.0 : a.cov[((int64_t)a.ncov + c) * a.N + q];
+                double re = zero ? 0.0 : __ldg(cr + b * a.halfm);
+                double im = zero ? 0.0 : sign * __ldg(ci + b * a.halfm);
                 re = re * a.nsinv;
                 re = re * a.scale[c];
                 im = im * a.nsinv;
@@ -213,25 +252,24 @@ int sf_fab_ok(const fhd_sf* s, const fhd_fab& f, int min_nc) { return shape_fab_
 
 int cufft_rc(cufftResult r) { return r == CUFFT_SUCCESS ? FHD_OK : FHD_ERR_CUDA; }
 
-// Dense D2Z plan over the box (slowest dimension first: cuFFT is row-major),
-// writing the packed half spectrum nz x ny x (nx/2+1).  Its input is a dense,
-// aligned copy of one variable: cuFFT rejects an input pointer into a
-// ghost-inclusive fab whose valid region starts off a 16-byte boundary.
-// A stack: one plan of nmem transforms (2-D over a slice, 1-D over a pencil),
-// members contiguous in the dense copy and in the half spectra.
+// D2Z plan of every variable and member at once (slowest dimension first: cuFFT is
+// row-major): 3-D over the box, 2-D over a slice, 1-D over a pencil, transforms
+// contiguous in the input and in the half spectra.  One execution per sample: 144x112x96
+// with 4 variables took 12 kernels of about 10 us each with a plan per variable, 3 here.
 int sf_plan(fhd_sf* s) {
     if (s->have_plan) return FHD_OK;
     int rc;
-    if (s->kind == FHD_SF_BOX) {
-        rc = cufft_rc(cufftPlan3d(&s->plan, s->n[2], s->n[1], s->n[0], CUFFT_D2Z));
-    } else if (s->kind == FHD_SF_Z_SLICES) {
-        int dims[2] = {s->m[1], s->m[0]}, oemb[2] = {s->m[1], s->m[0] / 2 + 1};
-        rc = cufft_rc(cufftPlanMany(&s->plan, 2, dims, dims, 1, s->m[0] * s->m[1], oemb, 1,
-                                    s->m[1] * (s->m[0] / 2 + 1), CUFFT_D2Z, s->nmem));
-    } else {
-        int dims[1] = {s->m[0]}, oemb[1] = {s->m[0] / 2 + 1};
-        rc = cufft_rc(cufftPlanMany(&s->plan, 1, dims, dims, 1, s->m[0], oemb, 1, s->m[0] / 2 + 1, CUFFT_D2Z,
-                                    s->nmem));
+    const int rank = s->kind == FHD_SF_BOX ? 3 : (s->kind == FHD_SF_Z_SLICES ? 2 : 1);
+    int dims[3], oemb[3];
+    for (int r = 0; r < rank; ++r) dims[r] = oemb[r] = s->m[rank - 1 - r];
+    oemb[rank - 1] = s->m[0] / 2 + 1;
+    s->per_plan = (int)s->varu.size();
+    for (;;) {
+        rc = cufft_rc(cufftPlanMany(&s->plan, rank, dims, dims, 1, s->m[0] * s->m[1] * s->m[2], oemb, 1,
+                                    (s->m[0] / 2 + 1) * s->m[1] * s->m[2], CUFFT_D2Z, s->nmem * s->per_plan));
+        if (!rc || s->per_plan == 1) break;
+        cudaGetLastError();
+        s->per_plan = 1;   // no room for the workspace of all variables: one at a time
     }
     if (rc) return rc;
     rc = cufft_rc(cufftSetStream(s->plan, s->stream));
@@ -243,20 +281,43 @@ int sf_plan(fhd_sf* s) {
     return FHD_OK;
 }
 
-// dense copy of one component; x pencils in the reference's member order
+// dense copy of the variables (blockIdx.y); x pencils in the reference's member order
 // (member p at y = p / ny, z = p % ny, ExtractXPencil's arguments in
 // main_driver.cpp:1551), everything else in the box's own order
-__global__ void __launch_bounds__(256) k_sf_pack(Arr4<const double> v, int comp, int nx, int ny, int64_t N,
-                                                 int pencils, double* __restrict__ out) {
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < N; q += (int64_t)gridDim.x * blockDim.x) {
-        if (pencils) {
-            const int64_t p = q / nx;
-            out[q] = v(int(q - p * nx), int(p / ny), int(p % ny), comp);
+struct PackArgs {
+    Arr4<const double> v;
+    const int* comp;
+    int nx, ny;
+    int64_t N;
+    FastDiv dx, dxy, dy;
+    int pencils;
+    double* out;
+};
+__global__ void __launch_bounds__(256) k_sf_pack(PackArgs a) {
+    const int comp = a.comp[blockIdx.y];
+    double* out = a.out + (int64_t)blockIdx.y * a.N;
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < a.N; q += (int64_t)gridDim.x * blockDim.x) {
+        if (a.pencils) {
+            const int p = (int)a.dx.div((uint32_t)q), y = (int)a.dy.div((uint32_t)p);
+            out[q] = a.v((int)q - p * a.nx, y, p - y * a.ny, comp);
         } else {
-            const int i = int(q % nx), j = int((q / nx) % ny), k = int(q / ((int64_t)nx * ny));
-            out[q] = v(i, j, k, comp);
+            const int k = (int)a.dxy.div((uint32_t)q), r = (int)q - k * a.nx * a.ny;
+            const int j = (int)a.dx.div((uint32_t)r);
+            out[q] = a.v(r - j * a.nx, j, k, comp);
         }
     }
+}
+
+// Whether cuFFT can read the caller's fab itself: no ghosts, the used variables
+// consecutive components (then the transforms follow each other as in the dense copy),
+// members in the box's order, and a first element on the 16-byte boundary that cuFFT
+// asks of its input.  The out-of-place transform leaves its input unchanged.
+bool direct_input(const fhd_sf* s, const fhd_fab& f) {
+    if (s->kind == FHD_SF_X_PENCILS || f.lo[0] != 0) return false;
+    for (size_t u = 1; u < s->varu.size(); ++u)
+        if (s->varu[u] != s->varu[0] + (int)u) return false;
+    const int64_t N = (int64_t)s->n[0] * s->n[1] * s->n[2];
+    return ((uintptr_t)(static_cast<const double*>(f.data) + N * s->varu[0]) & 15) == 0;
 }
 
 }  // namespace
@@ -326,21 +387,22 @@ int fhd_sf_create_stack(fhd_sf** out, const int n_cells[3], int kind, int nvar, 
         hp[c] = slot[s->pa[c]];
         hp[s->ncov + c] = slot[s->pb[c]];
     }
+    hp.insert(hp.end(), s->varu.begin(), s->varu.end());
     const int64_t N = (int64_t)s->n[0] * s->n[1] * s->n[2];
     const int64_t half = (int64_t)(s->m[0] / 2 + 1) * s->m[1] * s->m[2] * s->nmem;
     int rc = FHD_OK;
     if (cudaSetDevice(device) != cudaSuccess) rc = FHD_ERR_CUDA;
     if (!rc && cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess) rc = FHD_ERR_CUDA;
     if (!rc) s->own_stream = true;
-    if (!rc && (cudaMalloc(&s->cov, sizeof(double) * 2 * s->ncov * N) != cudaSuccess ||
+    if (!rc && (cudaMalloc(&s->cov, sizeof(double) * 2 * s->ncov * half) != cudaSuccess ||
                 cudaMalloc(&s->spec, sizeof(double2) * s->varu.size() * half) != cudaSuccess ||
-                cudaMalloc(&s->real, sizeof(double) * N) != cudaSuccess ||
+                                cudaMalloc(&s->real, sizeof(double) * s->varu.size() * N) != cudaSuccess ||
                 cudaMalloc(&s->dpairs, sizeof(int) * hp.size()) != cudaSuccess ||
                 cudaMalloc(&s->dscale, sizeof(double) * s->ncov) != cudaSuccess))
         rc = FHD_ERR_OOM;
     if (!rc && (cudaMemcpy(s->dpairs, hp.data(), sizeof(int) * hp.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
                 cudaMemcpy(s->dscale, s->scaling.data(), sizeof(double) * s->ncov, cudaMemcpyHostToDevice) != cudaSuccess ||
-                cudaMemset(s->cov, 0, sizeof(double) * 2 * s->ncov * N) != cudaSuccess))
+                cudaMemset(s->cov, 0, sizeof(double) * 2 * s->ncov * half) != cudaSuccess))
         rc = FHD_ERR_CUDA;
     if (rc) {
         cudaGetLastError();
@@ -386,33 +448,46 @@ int fhd_sf_fort_structure(fhd_sf* s, fhd_fab variables, int reset) {
     cudaSetDevice(s->device);
     int rc = sf_plan(s);
     if (rc) return rc;
-    const Arr4<const double> v = view<const double>(variables);
     const int64_t N = (int64_t)s->n[0] * s->n[1] * s->n[2];
-    const int64_t halfm = (int64_t)(s->m[0] / 2 + 1) * s->m[1] * s->m[2], half = halfm * s->nmem;
-    for (size_t u = 0; u < s->varu.size(); ++u) {
-        k_sf_pack<<<grid_for(N, 256), 256, 0, s->stream>>>(v, s->varu[u], s->n[0], s->n[1], N,
-                                                          s->kind == FHD_SF_X_PENCILS ? 1 : 0, s->real);
-        rc = cuda_rc(cudaGetLastError());
-        if (rc) return rc;
-        rc = cufft_rc(cufftExecD2Z(s->plan, s->real, reinterpret_cast<cufftDoubleComplex*>(s->spec + u * half)));
-        if (rc) return rc;
+    const int64_t half = (int64_t)(s->m[0] / 2 + 1) * s->m[1] * s->m[2] * s->nmem;
+    const int nv = (int)s->varu.size();
+    auto exec = [&](double* in, int u) {
+        return cufft_rc(cufftExecD2Z(s->plan, in, reinterpret_cast<cufftDoubleComplex*>(s->spec + u * half)));
+    };
+    if (s->per_plan == nv && direct_input(s, variables)) {
+        rc = exec(static_cast<double*>(variables.data) + N * s->varu[0], 0);
+    } else {
+        PackArgs p;
+        p.v = view<const double>(variables);
+        p.nx = s->n[0];
+        p.ny = s->n[1];
+        p.N = N;
+        p.dx = fast_div((uint32_t)s->n[0]);
+        p.dxy = fast_div((uint32_t)(s->n[0] * s->n[1]));
+        p.dy = fast_div((uint32_t)s->n[1]);
+        p.pencils = s->kind == FHD_SF_X_PENCILS ? 1 : 0;
+        p.out = s->real;   // one variable at a time: each at the buffer's aligned start
+        for (int u = 0; u < nv && !rc; u += s->per_plan) {
+            p.comp = s->dpairs + 2 * s->ncov + u;
+            k_sf_pack<<<dim3(grid_for(N, 256, 148 * 8), s->per_plan), 256, 0, s->stream>>>(p);
+            rc = cuda_rc(cudaGetLastError());
+            if (!rc) rc = exec(s->real, u);
+        }
     }
+    if (rc) return rc;
     SfArgs a;
-    a.nx = s->m[0];
-    a.ny = s->m[1];
-    a.nz = s->m[2];
-    a.nxh1 = s->m[0] / 2 + 1;
+    a.nv = nv;
     a.ncov = s->ncov;
-    a.N = N;
     a.half = half;
-    a.Nm = (int64_t)s->m[0] * s->m[1] * s->m[2];
-    a.halfm = halfm;
-    a.sqrtnpts = std::sqrt((double)a.Nm);  // StructFact.cpp:348-350, over one member's box
+    a.sqrtnpts = std::sqrt((double)((int64_t)s->m[0] * s->m[1] * s->m[2]));  // StructFact.cpp:348-350, one member's box
+    a.rsqrtnpts = 1.0 / a.sqrtnpts;
     a.spec = s->spec;
     a.pairs = s->dpairs;
     a.cov = s->cov;
     a.reset = (reset == 1 || s->nsamples == 0) ? 1 : 0;
-    k_sf_accumulate<<<grid_for(a.N, 256), 256, 0, s->stream>>>(a);
+    const int grid = grid_for(half, kSfThreads);
+    if (nv <= kSfStaged) k_sf_accumulate<true><<<grid, kSfThreads, sizeof(double2) * kSfThreads * nv, s->stream>>>(a);
+    else k_sf_accumulate<false><<<grid, kSfThreads, 0, s->stream>>>(a);
     rc = cuda_rc(cudaGetLastError());
     if (rc) return rc;
     s->nsamples = (reset == 1) ? 1 : s->nsamples + 1;  // :307-311
@@ -431,6 +506,9 @@ int fhd_sf_finalize(fhd_sf* s, fhd_fab cov_real, fhd_fab cov_imag, fhd_fab cov_m
     a.ncov = s->ncov;
     a.zero_avg = zero_avg;
     a.N = (int64_t)s->n[0] * s->n[1] * s->n[2];
+    a.half = (int64_t)(s->n[0] / 2 + 1) * s->n[1] * s->n[2];
+    a.dx = fast_div((uint32_t)s->n[0]);
+    a.dxy = fast_div((uint32_t)(s->n[0] * s->n[1]));
     a.nsinv = 1.0 / (double)s->nsamples;  // StructFact.cpp:603
     a.cov = s->cov;
     a.scale = s->dscale;
@@ -453,7 +531,8 @@ int fhd_sf_stack_average(fhd_sf* s, fhd_fab mag, fhd_fab realimag, int zero_avg)
     a.zero_avg = zero_avg;
     a.Nm = (int64_t)s->m[0] * s->m[1] * s->m[2];
     a.nmem = s->nmem;
-    a.N = a.Nm * a.nmem;
+    a.halfm = (int64_t)(s->m[0] / 2 + 1) * s->m[1] * s->m[2];
+    a.half = a.halfm * a.nmem;
     a.nsinv = 1.0 / (double)s->nsamples;  // StructFact.cpp:603
     a.meminv = 1.0 / (double)s->nmem;     // ncellsinv (main_driver.cpp:1610, 1702)
     a.cov = s->cov;

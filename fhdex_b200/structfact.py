@@ -77,10 +77,15 @@ class StructFact:
         self._stream()
         check(self.lib.fhd_sf_fort_structure(self._h, variables.fab(), reset), "fhd_sf_fort_structure")
 
+    def _output(self, n_cells, ncomp) -> MultiFab:
+        """A MultiFab that the library writes whole (not zero-filled first)."""
+        t = torch.empty((ncomp,) + tuple(n_cells)[::-1], dtype=torch.float64, device=f"cuda:{self.device}")
+        return MultiFab(n_cells, CELL, ncomp, 0, tensor=t)
+
     def finalize(self, zero_avg: int = 1):
         """(cov_real, cov_imag, cov_mag) MultiFabs, StructFact::CallFinalize."""
         self._stream()
-        out = [MultiFab(self.n_cells, CELL, self.ncov, 0, device=f"cuda:{self.device}") for _ in range(3)]
+        out = [self._output(self.n_cells, self.ncov) for _ in range(3)]
         check(self.lib.fhd_sf_finalize(self._h, out[0].fab(), out[1].fab(), out[2].fab(), zero_avg),
               "fhd_sf_finalize")
         return tuple(out)
@@ -89,9 +94,7 @@ class StructFact:
         """(mag, realimag) MultiFabs of the member shape: AddToExternal of every
         member in order, then times 1/members (main_driver.cpp:1592-1618, 1683-1711)."""
         self._stream()
-        dev = f"cuda:{self.device}"
-        mag = MultiFab(self.member, CELL, self.ncov, 0, device=dev)
-        ri = MultiFab(self.member, CELL, 2 * self.ncov, 0, device=dev)
+        mag, ri = self._output(self.member, self.ncov), self._output(self.member, 2 * self.ncov)
         check(self.lib.fhd_sf_stack_average(self._h, mag.fab(), ri.fab(), zero_avg), "fhd_sf_stack_average")
         return mag, ri
 
