@@ -1,9 +1,9 @@
 """Build ``fhdex_b200/lib/libfhd_b200.so`` for sm_100a with nvcc (in-tree).
 
-The kernels are compiled once per (species count, precision) in parallel:
-the exact FP64 units with ``-fmad=false`` (no contraction of a*b+c, so the
-reference's operation order is kept), the mixed-precision units with FMA
-contraction allowed.  ``python -m fhdex_b200.build`` rebuilds what is stale.
+The kernels are compiled once per (species count, precision) in parallel, all
+with ``-fmad=false`` (no contraction of a*b+c): the FP64 path keeps the
+reference's operation order, and the mixed path's FMAs are the written ones, the
+same in every kernel.  ``python -m fhdex_b200.build`` rebuilds what is stale.
 """
 from __future__ import annotations
 
@@ -23,14 +23,14 @@ BASE = ARCH + ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contr
                "-Xptxas", "-v", f"-I{CSRC}", f"-I{os.path.join(ROOT, 'include')}"]
 SPECIES = (1, 2, 3, 4)
 
-HEADERS = ["fhd_div.h", "fhd_device.cuh", "philox.cuh", "fhd_flux.cuh", "fhd_kernels.cuh", "fhd_launch.cuh", "fhd_fused.cuh", "fhd_host.h", "fhd_chem.cuh", "fhd_vismf.h", "fhd_walls.cuh"]
+HEADERS = ["fhd_div.h", "fhd_items.h", "fhd_linesum.cuh", "fhd_transport_alt.cuh", "fhd_device.cuh", "philox.cuh", "fhd_flux.cuh", "fhd_kernels.cuh", "fhd_launch.cuh", "fhd_fused.cuh", "fhd_host.h", "fhd_chem.cuh", "fhd_vismf.h", "fhd_walls.cuh"]
 
 
 def _units():
     u = []
     for ns in SPECIES:
         u.append((f"kern_exact_ns{ns}", "fhd_kern_ns.cu", [f"-DFHD_NS={ns}", "-fmad=false"]))
-        u.append((f"kern_mixed_ns{ns}", "fhd_kern_ns.cu", [f"-DFHD_NS={ns}", "-DFHD_MIXED=1", "-fmad=true"]))
+        u.append((f"kern_mixed_ns{ns}", "fhd_kern_ns.cu", [f"-DFHD_NS={ns}", "-DFHD_MIXED=1", "-fmad=false"]))
     u.append(("exact_util", "fhd_exact.cu", ["-fmad=false"]))
     u.append(("capi", "fhd_capi.cu", ["-fmad=false"]))
     u.append(("noalloc", "fhd_noalloc.cu", ["-fmad=false"]))

@@ -224,17 +224,27 @@ int rebuild(fhd_batch* b) {
     const int ghost_sz = ghost_desc_size();
     size_t need = host.size();
     auto add = [&](size_t bytes) { need = ((need + 255) & ~(size_t)255) + bytes; };
+    // a block-prefix array and its start table of every 64th block; the ghost points of
+    // the five fabs of a fill are fewer than 64 per point of the box grown by three
+    auto add_bpref = [&](int kind, int entries) {
+        int64_t blocks = 0;
+        for (const Member& m : b->mem) {
+            const int* n = m.prm.n_cells;
+            blocks += (kind < 7 ? kind_items(kind, n) : 64ll * (n[0] + 5) * (n[1] + 5) * (n[2] + 5)) / 128 + 6;
+        }
+        add(sizeof(int) * (entries + 2 + blocks / 64));
+    };
     for (int s = 0; s < 3; ++s) {
         add(batch_args_size(b->ns, b->mixed, 0, b->mode) * M);
         add(batch_args_size(b->ns, b->mixed, 1, b->mode) * M);
-        for (int kind = 0; kind < 6; ++kind) add(sizeof(int) * (M + 1));
+        for (int kind = 0; kind < 6; ++kind) add_bpref(kind, M + 1);
         add((size_t)ghost_sz * 5 * M);
-        add(sizeof(int) * (5 * M + 1));
+        add_bpref(7, 5 * M + 1);
     }
     add(batch_args_size(b->ns, false, 6, b->mode) * M);
-    add(sizeof(int) * (M + 1));
+    add_bpref(6, M + 1);
     add((size_t)ghost_sz * 5 * M);
-    add(sizeof(int) * (5 * M + 1));
+    add_bpref(7, 5 * M + 1);
     // persistent step: 24 phases; 11 units per member and stage, 7 for the end
     const int kPhases = 24;
     add(sizeof(PUnit) * (size_t)40 * M);
@@ -254,6 +264,12 @@ int rebuild(fhd_batch* b) {
         std::vector<int> pref(items.size() + 1, 0);
         for (size_t q = 0; q < items.size(); ++q) pref[q + 1] = pref[q] + (int)((items[q] + bs - 1) / bs);
         nblocks = pref.back();
+        // the members of blocks 0, 64, 128, ... (member_of)
+        size_t m = 0;
+        for (int blk = 0; blk < nblocks; blk += 64) {
+            while (pref[m + 1] <= blk) ++m;
+            pref.push_back((int)m);
+        }
         const size_t off = align(256);
         host.resize(off + sizeof(int) * pref.size());
         memcpy(host.data() + off, pref.data(), sizeof(int) * pref.size());

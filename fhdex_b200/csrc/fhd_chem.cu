@@ -12,9 +12,10 @@
 namespace fhd {
 
 struct ChemArgs {
-    DevParams P;
+    RunParams P;
     ChemParams C;
     Arr4<const double> pr;   // prim: T comp 4, p comp 5, X comps 6+NS..
+    Items it;                // valid cells
     Arr4<double> src;        // species n -> comp 5+n
     Arr4<const double> na, nb;
     int mode;
@@ -23,10 +24,9 @@ struct ChemArgs {
 
 template <int NS>
 static __global__ void __launch_bounds__(128) k_chem(ChemArgs a) {
-    const int nx = a.P.n[0], ny = a.P.n[1], nz = a.P.n[2];
-    const int64_t tot = (int64_t)nx * ny * nz;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < tot; q += (int64_t)gridDim.x * blockDim.x) {
-        const int i = (int)(q % nx), j = (int)((q / nx) % ny), k = (int)(q / ((int64_t)nx * ny));
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < a.it.n; q += gridDim.x * blockDim.x) {
+        int i, j, k;
+        a.it.point(q, i, j, k);
         double W[MAXR];
 #pragma unroll
         for (int m = 0; m < MAXR; ++m) W[m] = 0.0;
@@ -56,8 +56,7 @@ static __global__ void __launch_bounds__(128) k_chem(ChemArgs a) {
 
 template <int NS>
 static int chem_launch_t(const ChemArgs& a, cudaStream_t s) {
-    const int64_t tot = (int64_t)a.P.n[0] * a.P.n[1] * a.P.n[2];
-    k_chem<NS><<<grid_for(tot, 128), 128, 0, s>>>(a);
+    k_chem<NS><<<grid_for(a.it.n, 128), 128, 0, s>>>(a);
     return cuda_rc(cudaGetLastError());
 }
 
@@ -72,6 +71,7 @@ int chem_launch(const DevParams& P, const ChemParams& C, const fhd_fab& prim, co
     if (na) a.na = view<const double>(*na);
     if (nb) a.nb = view<const double>(*nb);
     a.mode = mode;
+    a.it = make_items(P.n[0], P.n[1], P.n[2]);
     a.w = w;
     switch (P.ns) {
         case 1: return chem_launch_t<1>(a, s);

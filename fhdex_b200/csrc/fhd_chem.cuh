@@ -97,7 +97,7 @@ FHD_D double chem_ipow(double c, int r) {
 // source S_0..S_{NS-1} of one cell from p, T, X and the reaction noises W[m]
 // (chemistry_functions.cpp:147-190)
 template <int NS>
-FHD_D void chem_point(const DevParams& P, const ChemParams& C, double pres, double T, const double (&X)[NS],
+FHD_D void chem_point(const RunParams& P, const ChemParams& C, double pres, double T, const double (&X)[NS],
                       const double* W, double (&S)[NS]) {
     const double rT = 1 / T;
     const double ctot = div_rcp_any(div_rcp(pres, P.Runiv, C.rR, C.div_lo, C.div_span), T, rT);

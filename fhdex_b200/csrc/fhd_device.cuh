@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include "fhd_div.h"
+#include "fhd_items.h"
 
 #define FHD_HD __host__ __device__ __forceinline__
 #define FHD_D __device__ __forceinline__
@@ -29,51 +30,29 @@ struct Arr4 {
     FHD_HD T& operator()(int i, int j, int k, int n = 0) const { return p[i + j * sy + k * sz + n * sn]; }
 };
 
-// Division of a 31-bit item number by a run constant: q / d = (q * m) >> s with
-// m = floor(2^(31+l) / d) + 1, l = ceil(log2 d), s = 31 + l (Granlund and Montgomery,
-// "Division by invariant integers using multiplication", PLDI 1994: exact for
-// 0 <= q < 2^31, as m*d - 2^(31+l) lies in (0, 2^l]).  Three instructions against
-// about twenty for a division by a value the compiler does not know.
-struct FastDiv {
-    uint32_t m, s;
-    FHD_HD uint32_t div(uint32_t q) const { return (uint32_t)(((uint64_t)q * m) >> s); }
-};
-inline FastDiv fast_div(uint32_t d) {
-    uint32_t l = 0;
-    while (((uint64_t)1 << l) < d) ++l;
-    FastDiv f;
-    f.m = (uint32_t)((((uint64_t)1 << (31 + l)) / d) + 1);
-    f.s = 31 + l;
-    return f;
-}
-
-// Items 0 .. nx*ny*nz - 1 of a box as points, x fastest
-struct Items {
-    int nx, nxy, n;      // row, plane, all (the host rejects boxes of 2^31 or more points)
-    FastDiv dx, dxy;
-    FHD_HD void point(int q, int& i, int& j, int& k) const {
-        k = (int)dxy.div((uint32_t)q);
-        const int r = q - k * nxy;
-        j = (int)dx.div((uint32_t)r);
-        i = r - j * nx;
-    }
-};
-inline Items make_items(int nx, int ny, int nz) {
-    Items t;
-    t.nx = nx;
-    t.nxy = nx * ny;
-    t.n = nx * ny * nz;
-    t.dx = fast_div((uint32_t)nx);
-    t.dxy = fast_div((uint32_t)(nx * ny));
-    return t;
-}
-
 // Parameters as the kernels see them.  RunParams holds what the stress, flux,
 // update and conversion kernels read; DevParams adds the transport model's tables,
 // whose cell-independent sub-expressions are precomputed on the host in the
 // reference's own operation order (host IEEE double arithmetic gives the identical
 // values the reference computes inside its loops).  The batched kernels copy their
 // member's argument block into shared memory once per block, so the two are apart.
+//
+// The mixed path's FP32 arithmetic reads FP32 copies of the constants (the same
+// roundings the device conversion gives): converted at each use, a constant costs an
+// F2F on the quarter-rate conversion pipe per thread, over a hundred per cell in the
+// four-species transport model.
+struct RunConstsF {
+    float dx[3], hdx[3], rhdx[3], rdx[3];
+    float dt, volinv, dtinv, k_B, Runiv, zeta_ratio, sqrt3, fac2d, rRdt, rpi, r3;
+    float molmass[MAXS], rmolmass[MAXS], hcv[MAXS], hcp[MAXS], e0[MAXS];
+};
+struct TransConstsF {
+    float mm[MAXS], mmkB[MAXS], eta1pre[MAXS], rmm[MAXS];
+    float diam[MAXS][MAXS], mu[MAXS][MAXS], msum[MAXS][MAXS], vfac[MAXS][MAXS], kfac[MAXS][MAXS], rmu[MAXS][MAXS],
+        rmsum[MAXS][MAXS];
+    float koff, voff, cfac;
+};
+
 struct RunParams {
     int ns, nvars, nprim;
     int n[3];
@@ -108,6 +87,7 @@ struct RunParams {
     double rRdt;                     // 1/(Runiv*dt)
     double rpi, r3;                  // 1/pi (the transport model's pi), 1/3
     uint32_t div_lo, div_span;
+    RunConstsF f32;
 };
 
 struct DevParams : RunParams {
@@ -129,7 +109,25 @@ struct DevParams : RunParams {
     const struct VWTable* vwt;
     double rmm[MAXS];
     double rmu[MAXS][MAXS], rmsum[MAXS][MAXS];
+    TransConstsF t32;
 };
+
+// the constants in compute type R: rc the run's, tc the transport model's
+template <class R> FHD_HD const auto& rc(const RunParams& P) {
+    if constexpr (sizeof(R) == 8) return P;
+    else return P.f32;
+}
+template <class R> FHD_HD const auto& tc(const DevParams& P) {
+    if constexpr (sizeof(R) == 8) return P;
+    else return P.t32;
+}
+
+// c + a * b: FP64 with both roundings, as the reference's CPU build; FP32 (the mixed
+// path) one fused operation.  Every unit is built without contraction, so that where an
+// FMA is used does not depend on the kernel a function is inlined into: a batched member
+// and the same run alone then agree in the mixed path too.
+FHD_D double madd(double a, double b, double c) { return c + a * b; }
+FHD_D float madd(float a, float b, float c) { return fmaf(a, b, c); }
 
 // a / b in the compute type: FP64 the correctly rounded division (the reference's
 // arithmetic); FP32 (the mixed path, held to a tolerance against FP64) the fast
@@ -234,10 +232,10 @@ template <int NS, class R>
 FHD_D void GetMolfrac(const RunParams& P, const R (&Y)[NS], R (&X)[NS]) {
     R molmix = R(0.);
 #pragma unroll
-    for (int n = 0; n < NS; ++n) molmix += divc(P, Y[n], R(P.molmass[n]), R(P.rmolmass[n]));
+    for (int n = 0; n < NS; ++n) molmix += divc(P, Y[n], rc<R>(P).molmass[n], rc<R>(P).rmolmass[n]);
     molmix = rdiv(R(1.), molmix);
 #pragma unroll
-    for (int n = 0; n < NS; ++n) X[n] = divc(P, Y[n] * molmix, R(P.molmass[n]), R(P.rmolmass[n]));
+    for (int n = 0; n < NS; ++n) X[n] = divc(P, Y[n] * molmix, rc<R>(P).molmass[n], rc<R>(P).rmolmass[n]);
 }
 
 template <int NS, class R>
@@ -245,8 +243,8 @@ FHD_D R GetTemperature(const RunParams& P, R energy, const R (&Y)[NS]) {
     R cvmix = R(0.), e0mix = R(0.);
 #pragma unroll
     for (int n = 0; n < NS; ++n) {
-        cvmix = add_rn(cvmix, mul_rn(Y[n], R(P.hcv[n])));
-        e0mix = add_rn(e0mix, mul_rn(Y[n], R(P.e0[n])));
+        cvmix = add_rn(cvmix, mul_rn(Y[n], rc<R>(P).hcv[n]));
+        e0mix = add_rn(e0mix, mul_rn(Y[n], rc<R>(P).e0[n]));
     }
     return rdiv(energy - e0mix, cvmix);
 }
@@ -255,15 +253,15 @@ template <int NS, class R>
 FHD_D R GetPressureGas(const RunParams& P, const R (&Y)[NS], R density, R temp) {
     R molmix = R(0.);
 #pragma unroll
-    for (int n = 0; n < NS; ++n) molmix += divc(P, Y[n], R(P.molmass[n]), R(P.rmolmass[n]));
+    for (int n = 0; n < NS; ++n) molmix += divc(P, Y[n], rc<R>(P).molmass[n], rc<R>(P).rmolmass[n]);
     molmix = rdiv(R(1.), molmix);
-    return density * rdiv(R(P.Runiv), molmix) * temp;
+    return density * rdiv(rc<R>(P).Runiv, molmix) * temp;
 }
 
 template <int NS, class R>
 FHD_D void GetEnthalpies(const RunParams& P, R T, R (&hk)[NS]) {
 #pragma unroll
-    for (int i = 0; i < NS; ++i) hk[i] = R(P.e0[i]) + R(P.hcp[i]) * T;
+    for (int i = 0; i < NS; ++i) hk[i] = rc<R>(P).e0[i] + rc<R>(P).hcp[i] * T;
 }
 
 template <class R>
@@ -288,7 +286,7 @@ FHD_D void CholeskyDecomp(R (&a)[NS * NS], R (&sqda)[NS * NS]) {
         for (int j = i; j < NS; ++j) {
             R sum1 = a[i * NS + j];
 #pragma unroll
-            for (int k = i - 1; k >= 0; --k) sum1 = sum1 - a[i * NS + k] * a[j * NS + k];
+            for (int k = i - 1; k >= 0; --k) sum1 = madd(-a[i * NS + k], a[j * NS + k], sum1);
             if (i == j) {
                 if (sum1 <= R(0.)) { p[i] = R(0.); ising = 1; }
                 else p[i] = dsqrt(sum1);
@@ -356,7 +354,7 @@ FHD_D void D_GIO1(const DevParams& P, const R (&Dbin)[NS][NS], const R (&rDbin)[
         for (int j = 0; j < NS; ++j) {
             R s = R(0.);
 #pragma unroll
-            for (int k = 0; k < NS; ++k) s = s + Pmat[i * NS + k] * Jmat[k * NS + j];
+            for (int k = 0; k < NS; ++k) s = madd(Pmat[i * NS + k], Jmat[k * NS + j], s);
             PJ[i * NS + j] = s;
         }
 #pragma unroll
@@ -365,7 +363,7 @@ FHD_D void D_GIO1(const DevParams& P, const R (&Dbin)[NS][NS], const R (&rDbin)[
         for (int j = 0; j < NS; ++j) {
             R scr = R(0.);
 #pragma unroll
-            for (int k = 0; k < NS; ++k) scr = scr + Pmat[i * NS + k] * Minv[k] * Pmat[j * NS + k];
+            for (int k = 0; k < NS; ++k) scr = madd(Pmat[i * NS + k] * Minv[k], Pmat[j * NS + k], scr);
             M2[i * NS + j] = scr;
             Diff[i * NS + j] = scr;
         }
@@ -378,7 +376,7 @@ FHD_D void D_GIO1(const DevParams& P, const R (&Dbin)[NS][NS], const R (&rDbin)[
             for (int j = 0; j < NS; ++j) {
                 R scr = R(0.);
 #pragma unroll
-                for (int k = 0; k < NS; ++k) scr = scr + PJ[i * NS + k] * Diff[k * NS + j];
+                for (int k = 0; k < NS; ++k) scr = madd(PJ[i * NS + k], Diff[k * NS + j], scr);
                 M1[i * NS + j] = scr + M2[i * NS + j];
             }
 #pragma unroll
@@ -421,29 +419,29 @@ FHD_D bool transport_gio(const DevParams& P, R rho, R temperature, R pressure, c
     const R pi = R(3.1415926535897932);
     R mbar = R(0.0);
 #pragma unroll
-    for (int n = 0; n < NS; ++n) mbar += divc(P, Yk[n], R(P.mm[n]), R(P.rmm[n]));
+    for (int n = 0; n < NS; ++n) mbar += divc(P, Yk[n], tc<R>(P).mm[n], tc<R>(P).rmm[n]);
     mbar = rdiv(R(1.0), mbar);
     R Xk[NS], Xkp[NS], Ykp[NS];
     R Xksum = R(0.0);
 #pragma unroll
     for (int n = 0; n < NS; ++n) {
-        Xk[n] = divc(P, Yk[n] * mbar, R(P.mm[n]), R(P.rmm[n]));
+        Xk[n] = divc(P, Yk[n] * mbar, tc<R>(P).mm[n], tc<R>(P).rmm[n]);
         Xksum += Xk[n];
     }
 #pragma unroll
     for (int n = 0; n < NS; ++n) Xkp[n] = Xk[n] + R(1.0e-16) * (divc(P, Xksum, R(double(NS)), R(1.0 / double(NS))) - Xk[n]);
 #pragma unroll
-    for (int n = 0; n < NS; ++n) Ykp[n] = rdiv(Xkp[n] * R(P.mm[n]), mbar);
+    for (int n = 0; n < NS; ++n) Ykp[n] = rdiv(Xkp[n] * tc<R>(P).mm[n], mbar);
 
-    const R kT = R(P.k_B) * temperature;
+    const R kT = rc<R>(P).k_B * temperature;
     R Dbin[NS][NS];
 #pragma unroll
     for (int i = 0; i < NS; ++i)
 #pragma unroll
         for (int j = 0; j < NS; ++j) {
             if (j < i) { Dbin[i][j] = Dbin[j][i]; continue; }  // symmetric: bitwise equal
-            const R dij = R(P.diam[i][j]);
-            Dbin[i][j] = rdiv((R(3.0) / R(16.0)) * dsqrt(divc(P, R(2.0) * pi * kT * kT * kT, R(P.mu[i][j]), R(P.rmu[i][j]))),
+            const R dij = tc<R>(P).diam[i][j];
+            Dbin[i][j] = rdiv((R(3.0) / R(16.0)) * dsqrt(divc(P, R(2.0) * pi * kT * kT * kT, tc<R>(P).mu[i][j], tc<R>(P).rmu[i][j])),
                               pressure * pi * dij * dij);
         }
     // reciprocals of the off-diagonal binary diffusivities, each a divisor ~7 times below
@@ -459,7 +457,7 @@ FHD_D bool transport_gio(const DevParams& P, R rho, R temperature, R pressure, c
     R amat[NS][NS], Bi[NS], rhs[NS];
 #pragma unroll
     for (int i = 0; i < NS; ++i) {
-        const R eta1 = R(P.eta1pre[i]) * dsqrt(divc(P, R(P.mmkB[i]) * temperature, pi, R(P.rpi)));
+        const R eta1 = tc<R>(P).eta1pre[i] * dsqrt(divc(P, tc<R>(P).mmkB[i] * temperature, pi, rc<R>(P).rpi));
         rhs[i] = Xkp[i];
         Bi[i] = rhs[i];
 #pragma unroll
@@ -469,12 +467,12 @@ FHD_D bool transport_gio(const DevParams& P, R rho, R temperature, R pressure, c
 #pragma unroll
                 for (int k = 0; k < NS; ++k)
                     if (k != i)
-                        a += rdiv(R(2.0) * kT * Xkp[i] * Xkp[k], pressure * Dbin[i][k] * R(P.msum[i][k])) *
-                             R(P.vfac[i][k]);
+                        a += rdiv(R(2.0) * kT * Xkp[i] * Xkp[k], pressure * Dbin[i][k] * tc<R>(P).msum[i][k]) *
+                             tc<R>(P).vfac[i][k];
                 amat[i][i] = a;
             } else {
-                amat[i][j] = rdiv(R(2.0) * kT * Xkp[i] * Xkp[j], pressure * Dbin[i][j] * R(P.msum[i][j])) *
-                             R(P.voff);
+                amat[i][j] = rdiv(R(2.0) * kT * Xkp[i] * Xkp[j], pressure * Dbin[i][j] * tc<R>(P).msum[i][j]) *
+                             tc<R>(P).voff;
             }
         }
     }
@@ -484,20 +482,20 @@ FHD_D bool transport_gio(const DevParams& P, R rho, R temperature, R pressure, c
         for (int i = j + 1; i < NS; ++i) {
             const R fact1 = rdiv(amat[i][j], amat[j][j]);
 #pragma unroll
-            for (int k = 0; k < NS; ++k) amat[i][k] -= fact1 * amat[j][k];
-            Bi[i] -= fact1 * Bi[j];
+            for (int k = 0; k < NS; ++k) amat[i][k] = madd(-fact1, amat[j][k], amat[i][k]);
+            Bi[i] = madd(-fact1, Bi[j], Bi[i]);
         }
     Bi[NS - 1] = rdiv(Bi[NS - 1], amat[NS - 1][NS - 1]);
 #pragma unroll
     for (int i = NS - 2; i > -1; --i) {
         R sum1 = R(0.0);
 #pragma unroll
-        for (int j = NS - 1; j > i; --j) sum1 += amat[i][j] * Bi[j];
+        for (int j = NS - 1; j > i; --j) sum1 = madd(amat[i][j], Bi[j], sum1);
         Bi[i] = rdiv(Bi[i] - sum1, amat[i][i]);
     }
     R eta = R(0.0);
 #pragma unroll
-    for (int i = 0; i < NS; ++i) eta += Xkp[i] * Bi[i];
+    for (int i = 0; i < NS; ++i) eta = madd(Xkp[i], Bi[i], eta);
     c.eta = eta;
     c.zeta = R(0.);
     // thermal conductivity
@@ -512,12 +510,12 @@ FHD_D bool transport_gio(const DevParams& P, R rho, R temperature, R pressure, c
 #pragma unroll
                 for (int k = 0; k < NS; ++k)
                     if (k != i)
-                        a += divc(P, div_dbin<NS, R>(P, Xkp[i] * Xkp[k], Dbin[i][k], rDbin[i][k]) * R(P.mu[i][k]), R(P.msum[i][k]),
-                                  R(P.rmsum[i][k])) * R(P.kfac[i][k]);
+                        a += divc(P, div_dbin<NS, R>(P, Xkp[i] * Xkp[k], Dbin[i][k], rDbin[i][k]) * tc<R>(P).mu[i][k], tc<R>(P).msum[i][k],
+                                  tc<R>(P).rmsum[i][k]) * tc<R>(P).kfac[i][k];
                 amat[i][i] = a;
             } else {
-                amat[i][j] = divc(P, div_dbin<NS, R>(P, R(-1.0) * Xkp[i] * Xkp[j], Dbin[i][j], rDbin[i][j]) * R(P.mu[i][j]),
-                                  R(P.msum[i][j]), R(P.rmsum[i][j])) * R(P.koff);
+                amat[i][j] = divc(P, div_dbin<NS, R>(P, R(-1.0) * Xkp[i] * Xkp[j], Dbin[i][j], rDbin[i][j]) * tc<R>(P).mu[i][j],
+                                  tc<R>(P).msum[i][j], tc<R>(P).rmsum[i][j]) * tc<R>(P).koff;
             }
         }
     }
@@ -527,20 +525,20 @@ FHD_D bool transport_gio(const DevParams& P, R rho, R temperature, R pressure, c
         for (int i = j + 1; i < NS; ++i) {
             const R fact1 = rdiv(amat[i][j], amat[j][j]);
 #pragma unroll
-            for (int k = 0; k < NS; ++k) amat[i][k] -= fact1 * amat[j][k];
-            Bi[i] -= fact1 * Bi[j];
+            for (int k = 0; k < NS; ++k) amat[i][k] = madd(-fact1, amat[j][k], amat[i][k]);
+            Bi[i] = madd(-fact1, Bi[j], Bi[i]);
         }
     Bi[NS - 1] = rdiv(Bi[NS - 1], amat[NS - 1][NS - 1]);
 #pragma unroll
     for (int i = NS - 2; i > -1; --i) {
         R sum1 = R(0.0);
 #pragma unroll
-        for (int j = NS - 1; j > i; --j) sum1 += amat[i][j] * Bi[j];
+        for (int j = NS - 1; j > i; --j) sum1 = madd(amat[i][j], Bi[j], sum1);
         Bi[i] = rdiv(Bi[i] - sum1, amat[i][i]);
     }
     R kappa = R(0.0);
 #pragma unroll
-    for (int i = 0; i < NS; ++i) kappa += rhs[i] * Bi[i];
+    for (int i = 0; i < NS; ++i) kappa = madd(rhs[i], Bi[i], kappa);
     kappa *= rdiv(pressure, temperature);
     c.kappa = kappa;
     // thermal diffusion ratios
@@ -555,16 +553,16 @@ FHD_D bool transport_gio(const DevParams& P, R rho, R temperature, R pressure, c
 #pragma unroll
                 for (int k = 0; k < NS; ++k)
                     if (k != i)
-                        a -= divc(P, div_dbin<NS, R>(P, R(0.5) * Xkp[k], Dbin[i][k], rDbin[i][k]) * R(P.mm[k]), R(P.msum[i][k]),
-                                  R(P.rmsum[i][k])) * R(P.cfac);
+                        a -= divc(P, div_dbin<NS, R>(P, R(0.5) * Xkp[k], Dbin[i][k], rDbin[i][k]) * tc<R>(P).mm[k], tc<R>(P).msum[i][k],
+                                  tc<R>(P).rmsum[i][k]) * tc<R>(P).cfac;
                 row[j] = a;
             } else {
-                row[j] = divc(P, div_dbin<NS, R>(P, R(0.5) * Xkp[j], Dbin[i][j], rDbin[i][j]) * R(P.mm[i]), R(P.msum[i][j]),
-                              R(P.rmsum[i][j])) * R(P.cfac);
+                row[j] = divc(P, div_dbin<NS, R>(P, R(0.5) * Xkp[j], Dbin[i][j], rDbin[i][j]) * tc<R>(P).mm[i], tc<R>(P).msum[i][j],
+                              tc<R>(P).rmsum[i][j]) * tc<R>(P).cfac;
             }
         }
 #pragma unroll
-        for (int j = 0; j < NS; ++j) ch += row[j] * Bi[j];
+        for (int j = 0; j < NS; ++j) ch = madd(row[j], Bi[j], ch);
         c.chi[i] = ch;
     }
     if constexpr (NS == 1) {
@@ -575,7 +573,7 @@ FHD_D bool transport_gio(const DevParams& P, R rho, R temperature, R pressure, c
 #pragma unroll
         for (int q = 0; q < NS * NS; ++q) c.D[q] = Dl[q] * rho;
     }
-    if (P.visc_type == 3 || P.visc_type == -3) c.zeta = R(P.zeta_ratio) * c.eta;
+    if (P.visc_type == 3 || P.visc_type == -3) c.zeta = rc<R>(P).zeta_ratio * c.eta;
     return ok;
 }
 

@@ -285,27 +285,9 @@ int batch_face_min_blocks(int tile) { return (tile >= 0 && tile < kNumBatchFaceT
 int ghost_desc_size() { return (int)sizeof(GhostFab); }
 
 int64_t ghost_pack(const fhd_fab& f, int c0, int nc, const int ncell[3], void* dst) {
-    GhostFab g;
-    g.p = static_cast<double*>(f.data);
-    g.lo = f.lo[0];
-    const int gw = -f.lo[0];
-    int64_t ext[3];
-    for (int d = 0; d < 3; ++d) {
-        g.vhi[d] = ncell[d] - 1 + f.nodal[d];
-        ext[d] = f.hi[d] - f.lo[d] + 1;
-        g.n[d] = ncell[d];
-    }
-    g.sy = ext[0];
-    g.sz = ext[0] * ext[1];
-    g.sn = ext[0] * ext[1] * ext[2];
-    g.c0 = c0;
-    g.nc = nc;
-    for (int d = 0; d < 3; ++d) g.per[d] = 1;
-    g.mode = 0;
-    const int64_t VY = g.vhi[1] + 1, VZ = g.vhi[2] + 1;
-    g.npts = gw == 0 ? 0 : 2 * gw * ext[0] * ext[1] + 2 * gw * ext[0] * VZ + 2 * gw * VY * VZ;
+    const GhostFab g = make_ghost(f.data, f.lo, f.hi, f.nodal, c0, nc, ncell, nullptr, 0);
     memcpy(dst, &g, sizeof(g));
-    return g.npts * g.nc;
+    return (int64_t)g.npts * g.nc;
 }
 
 int ghost_launch_b(const void* dfabs, const int* dbpref, int nfab, int nblocks, cudaStream_t s) {
@@ -329,38 +311,15 @@ int fill_ghosts(const GhostReq* reqs, int n, const int ncell[3], cudaStream_t s,
     for (int base = 0; base < n; base += 16) {
         GhostArgs a;
         a.nf = 0;
-        int64_t maxpts = 0;
+        int64_t most = 0;
         for (int q = base; q < n && q < base + 16; ++q) {
             const fhd_fab& f = reqs[q].f;
-            GhostFab& g = a.f[a.nf++];
-            g.p = static_cast<double*>(f.data);
-            g.lo = f.lo[0];
-            const int gw = -f.lo[0];
-            int64_t ext[3];
-            for (int d = 0; d < 3; ++d) {
-                g.vhi[d] = ncell[d] - 1 + f.nodal[d];
-                ext[d] = f.hi[d] - f.lo[d] + 1;
-            }
-            g.sy = ext[0];
-            g.sz = ext[0] * ext[1];
-            g.sn = ext[0] * ext[1] * ext[2];
-            g.c0 = reqs[q].c0;
-            g.nc = reqs[q].nc;
-            for (int d = 0; d < 3; ++d) {
-                g.n[d] = ncell[d];
-                g.per[d] = periodic ? periodic[d] : 1;
-            }
-            g.mode = mode;
-            const int64_t VX = g.vhi[0] + 1, VY = g.vhi[1] + 1, VZ = g.vhi[2] + 1;
-            g.npts = 2 * gw * ext[0] * ext[1] + 2 * gw * ext[0] * VZ + 2 * gw * VY * VZ;
-            (void)VX;
-            if (gw == 0) g.npts = 0;
-            if (g.npts * g.nc > maxpts) maxpts = g.npts * g.nc;
+            const GhostFab& g = a.f[a.nf++] = make_ghost(f.data, f.lo, f.hi, f.nodal, reqs[q].c0, reqs[q].nc, ncell,
+                                                         periodic, mode);
+            if ((int64_t)g.npts * g.nc > most) most = (int64_t)g.npts * g.nc;
         }
-        for (int d = 0; d < 3; ++d) a.n[d] = ncell[d];
-        if (maxpts == 0) continue;
-        dim3 grid(grid_for(maxpts, 256, 148 * 8), a.nf);
-        k_ghosts<<<grid, 256, 0, s>>>(a);
+        if (most == 0) continue;
+        k_ghosts<<<dim3(grid_for(most, 256, 148 * 8), a.nf), 256, 0, s>>>(a);
         if (cudaGetLastError() != cudaSuccess) return FHD_ERR_CUDA;
     }
     return FHD_OK;

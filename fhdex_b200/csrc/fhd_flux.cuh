@@ -9,6 +9,8 @@
 // terms (double: reference order; float: mixed precision); hyperbolic terms and
 // all state sums stay in double.
 #pragma once
+#include <type_traits>
+
 #include "fhd_device.cuh"
 #include "philox.cuh"
 
@@ -43,9 +45,11 @@ struct NoiseArrays {
 // W = 1.0*A + w*B (MultiFab::LinComb, timeStepStag.cpp:258-326).  The *_all
 // accessors fetch every noise field needed at one point at once, so that the
 // in-kernel generator runs one Philox call per pair of fields.
+struct NoNoiseArrays {};
 template <int MODE>
 struct Noise {
-    NoiseArrays a;
+    // (empty where the mode reads no arrays: the batched kernels copy this per block)
+    std::conditional_t<MODE == NZ_W || MODE == NZ_AB, NoiseArrays, NoNoiseArrays> a;
     double w;
 
     FHD_D double comb(double A, double B) const { return 1.0 * A + w * B; }
@@ -123,21 +127,21 @@ struct Noise {
         }
     }
     FHD_D double face(const RunParams& P, int d, int c, int i, int j, int k) const {
-        if (MODE == NZ_W) return a.fa[d](i, j, k, a.foa[d] + c);
-        if (MODE == NZ_AB) return comb(a.fa[d](i, j, k, a.foa[d] + c), a.fb[d](i, j, k, a.fob[d] + c));
-        if (MODE == NZ_PHILOX) return gauss1(P, fid_face(d, c), i, j, k, 1.0);
+        if constexpr (MODE == NZ_W) return a.fa[d](i, j, k, a.foa[d] + c);
+        if constexpr (MODE == NZ_AB) return comb(a.fa[d](i, j, k, a.foa[d] + c), a.fb[d](i, j, k, a.fob[d] + c));
+        if constexpr (MODE == NZ_PHILOX) return gauss1(P, fid_face(d, c), i, j, k, 1.0);
         return 0.0;
     }
     FHD_D double edge(const RunParams& P, int e, int i, int j, int k) const {
-        if (MODE == NZ_W) return a.ea[e](i, j, k);
-        if (MODE == NZ_AB) return comb(a.ea[e](i, j, k), a.eb[e](i, j, k));
-        if (MODE == NZ_PHILOX) return gauss1(P, fid_edge(e), i, j, k, 1.0);
+        if constexpr (MODE == NZ_W) return a.ea[e](i, j, k);
+        if constexpr (MODE == NZ_AB) return comb(a.ea[e](i, j, k), a.eb[e](i, j, k));
+        if constexpr (MODE == NZ_PHILOX) return gauss1(P, fid_edge(e), i, j, k, 1.0);
         return 0.0;
     }
     FHD_D double cen(const RunParams& P, int d, int i, int j, int k) const {
-        if (MODE == NZ_W) return a.ca[d](i, j, k);
-        if (MODE == NZ_AB) return comb(a.ca[d](i, j, k), a.cb[d](i, j, k));
-        if (MODE == NZ_PHILOX) return gauss1(P, fid_cen(d), i, j, k, d == 0 ? P.csd0 : P.sqrt2);
+        if constexpr (MODE == NZ_W) return a.ca[d](i, j, k);
+        if constexpr (MODE == NZ_AB) return comb(a.ca[d](i, j, k), a.cb[d](i, j, k));
+        if constexpr (MODE == NZ_PHILOX) return gauss1(P, fid_cen(d), i, j, k, d == 0 ? P.csd0 : P.sqrt2);
         return 0.0;
     }
 };
@@ -166,17 +170,17 @@ FHD_D CellTaus<R> cell_taus_w(const RunParams& P, const Fields<NS, R>& F, const 
     if (WL && P.dim < 3) {
         if (NZ != NZ_OFF) {
             const R etaT = eta * R(F.T(i, j, k));
-            R fac1 = dsqrt(R(2.0) * R(P.k_B) * etaT * R(P.volinv) * R(P.dtinv));
-            R fac2 = R(-1.0 / 3.0) * dsqrt(R(2.0) * R(P.k_B) * etaT * R(P.volinv) * R(P.dtinv));
+            R fac1 = dsqrt(R(2.0) * rc<R>(P).k_B * etaT * rc<R>(P).volinv * rc<R>(P).dtinv);
+            R fac2 = R(-1.0 / 3.0) * dsqrt(R(2.0) * rc<R>(P).k_B * etaT * rc<R>(P).volinv * rc<R>(P).dtinv);
             const R w0 = R(wc[0]), w1 = R(wc[1]);
             if (P.dim == 1) {
-                fac1 *= R(P.sqrt3);
-                fac2 *= R(P.sqrt3);
+                fac1 *= rc<R>(P).sqrt3;
+                fac2 *= rc<R>(P).sqrt3;
                 const R traceZ = w0;
                 t.s[0] = (fac1 * w0) + (fac2 * traceZ);
                 t.s[1] = R(0.0);
             } else {
-                fac2 *= R(P.fac2d);
+                fac2 *= rc<R>(P).fac2d;
                 const R traceZ = w0 + w1;
                 t.s[0] = (fac1 * w0) + (fac2 * traceZ);
                 t.s[1] = (fac1 * w1) + (fac2 * traceZ);
@@ -185,14 +189,14 @@ FHD_D CellTaus<R> cell_taus_w(const RunParams& P, const Fields<NS, R>& F, const 
         } else {
             t.s[0] = t.s[1] = t.s[2] = R(0.);
         }
-        const R u_x = divc(P, R(F.vel[0](i + 1, j, k)) - R(F.vel[0](i, j, k)), R(P.dx[0]), R(P.rdx[0]));
-        const R eta23 = divc(P, R(2) * eta, R(3.), R(P.r3));
+        const R u_x = divc(P, R(F.vel[0](i + 1, j, k)) - R(F.vel[0](i, j, k)), rc<R>(P).dx[0], rc<R>(P).rdx[0]);
+        const R eta23 = divc(P, R(2) * eta, R(3.), rc<R>(P).r3);
         if (P.dim == 1) {
             const R div = u_x;
             t.d[0] = R(2) * eta * u_x + (R(0.0) - eta23) * div;
             t.d[1] = R(0.0);
         } else {
-            const R v_y = divc(P, R(F.vel[1](i, j + 1, k)) - R(F.vel[1](i, j, k)), R(P.dx[1]), R(P.rdx[1]));
+            const R v_y = divc(P, R(F.vel[1](i, j + 1, k)) - R(F.vel[1](i, j, k)), rc<R>(P).dx[1], rc<R>(P).rdx[1]);
             const R div = u_x + v_y;
             t.d[0] = R(2) * eta * u_x + (R(0.0) - eta23) * div;
             t.d[1] = R(2) * eta * v_y + (R(0.0) - eta23) * div;
@@ -204,11 +208,11 @@ FHD_D CellTaus<R> cell_taus_w(const RunParams& P, const Fields<NS, R>& F, const 
         const R Tc = R(F.T(i, j, k));
         const R etaT = eta * Tc;
         const R zetaT = F.zeta(i, j, k) * Tc;
-        const R fac1 = dsqrt(R(2.0) * R(P.k_B) * etaT * R(P.volinv) * R(P.dtinv));
-        R fac2 = R(-1.0 / 3.0) * dsqrt(R(2.0) * R(P.k_B) * etaT * R(P.volinv) * R(P.dtinv));
+        const R fac1 = dsqrt(R(2.0) * rc<R>(P).k_B * etaT * rc<R>(P).volinv * rc<R>(P).dtinv);
+        R fac2 = R(-1.0 / 3.0) * dsqrt(R(2.0) * rc<R>(P).k_B * etaT * rc<R>(P).volinv * rc<R>(P).dtinv);
         if (visc3)
-            fac2 = dsqrt(divc(P, R(P.k_B) * zetaT * R(P.volinv) * R(P.dtinv), R(3.0), R(P.r3))) -
-                   divc(P, dsqrt(R(2.0) * R(P.k_B) * etaT * R(P.volinv) * R(P.dtinv)), R(3.0), R(P.r3));
+            fac2 = dsqrt(divc(P, rc<R>(P).k_B * zetaT * rc<R>(P).volinv * rc<R>(P).dtinv, R(3.0), rc<R>(P).r3)) -
+                   divc(P, dsqrt(R(2.0) * rc<R>(P).k_B * etaT * rc<R>(P).volinv * rc<R>(P).dtinv), R(3.0), rc<R>(P).r3);
         const R w0 = R(wc[0]), w1 = R(wc[1]), w2 = R(wc[2]);
         const R traceZ = w0 + w1 + w2;
         t.s[0] = (fac1 * w0) + (fac2 * traceZ);
@@ -217,12 +221,12 @@ FHD_D CellTaus<R> cell_taus_w(const RunParams& P, const Fields<NS, R>& F, const 
     } else {
         t.s[0] = t.s[1] = t.s[2] = R(0.);
     }
-    const R u_x = divc(P, R(F.vel[0](i + 1, j, k)) - R(F.vel[0](i, j, k)), R(P.dx[0]), R(P.rdx[0]));
-    const R v_y = divc(P, R(F.vel[1](i, j + 1, k)) - R(F.vel[1](i, j, k)), R(P.dx[1]), R(P.rdx[1]));
-    const R w_z = divc(P, R(F.vel[2](i, j, k + 1)) - R(F.vel[2](i, j, k)), R(P.dx[2]), R(P.rdx[2]));
+    const R u_x = divc(P, R(F.vel[0](i + 1, j, k)) - R(F.vel[0](i, j, k)), rc<R>(P).dx[0], rc<R>(P).rdx[0]);
+    const R v_y = divc(P, R(F.vel[1](i, j + 1, k)) - R(F.vel[1](i, j, k)), rc<R>(P).dx[1], rc<R>(P).rdx[1]);
+    const R w_z = divc(P, R(F.vel[2](i, j, k + 1)) - R(F.vel[2](i, j, k)), rc<R>(P).dx[2], rc<R>(P).rdx[2]);
     const R div = u_x + v_y + w_z;
     const R zc = visc3 ? R(F.zeta(i, j, k)) : R(0.0);
-    const R eta23 = divc(P, R(2) * eta, R(3.), R(P.r3));
+    const R eta23 = divc(P, R(2) * eta, R(3.), rc<R>(P).r3);
     t.d[0] = R(2) * eta * u_x + (zc - eta23) * div;
     t.d[1] = R(2) * eta * v_y + (zc - eta23) * div;
     t.d[2] = R(2) * eta * w_z + (zc - eta23) * div;
@@ -267,21 +271,21 @@ FHD_D Taus<R> edge_taus_w(const RunParams& P, const Fields<NS, R>& F, double wno
             if (x1 == 0 && dirichlet_side(P, 2 * d1)) etaT = R(0.5) * (ta + tb);
             if (x1 == P.n[d1] && dirichlet_side(P, 2 * d1 + 1)) etaT = R(0.5) * (tc + td);
         }
-        const R fac = dsqrt(R(2.0) * R(P.k_B) * etaT * R(P.volinv) * R(P.dtinv));
+        const R fac = dsqrt(R(2.0) * rc<R>(P).k_B * etaT * rc<R>(P).volinv * rc<R>(P).dtinv);
         t.s = fac * R(wnoise);
     } else {
         t.s = R(0.);
     }
     R g1, g2;
     if (E == 0) {
-        g1 = divc(P, R(F.vel[0](i, j, k)) - R(F.vel[0](i, j - 1, k)), R(P.dx[1]), R(P.rdx[1]));  // u_y
-        g2 = divc(P, R(F.vel[1](i, j, k)) - R(F.vel[1](i - 1, j, k)), R(P.dx[0]), R(P.rdx[0]));  // v_x
+        g1 = divc(P, R(F.vel[0](i, j, k)) - R(F.vel[0](i, j - 1, k)), rc<R>(P).dx[1], rc<R>(P).rdx[1]);  // u_y
+        g2 = divc(P, R(F.vel[1](i, j, k)) - R(F.vel[1](i - 1, j, k)), rc<R>(P).dx[0], rc<R>(P).rdx[0]);  // v_x
     } else if (E == 1) {
-        g1 = divc(P, R(F.vel[0](i, j, k)) - R(F.vel[0](i, j, k - 1)), R(P.dx[2]), R(P.rdx[2]));  // u_z
-        g2 = divc(P, R(F.vel[2](i, j, k)) - R(F.vel[2](i - 1, j, k)), R(P.dx[0]), R(P.rdx[0]));  // w_x
+        g1 = divc(P, R(F.vel[0](i, j, k)) - R(F.vel[0](i, j, k - 1)), rc<R>(P).dx[2], rc<R>(P).rdx[2]);  // u_z
+        g2 = divc(P, R(F.vel[2](i, j, k)) - R(F.vel[2](i - 1, j, k)), rc<R>(P).dx[0], rc<R>(P).rdx[0]);  // w_x
     } else {
-        g1 = divc(P, R(F.vel[1](i, j, k)) - R(F.vel[1](i, j, k - 1)), R(P.dx[2]), R(P.rdx[2]));  // v_z
-        g2 = divc(P, R(F.vel[2](i, j, k)) - R(F.vel[2](i, j - 1, k)), R(P.dx[1]), R(P.rdx[1]));  // w_y
+        g1 = divc(P, R(F.vel[1](i, j, k)) - R(F.vel[1](i, j, k - 1)), rc<R>(P).dx[2], rc<R>(P).rdx[2]);  // v_z
+        g2 = divc(P, R(F.vel[2](i, j, k)) - R(F.vel[2](i, j - 1, k)), rc<R>(P).dx[1], rc<R>(P).rdx[1]);  // w_y
     }
     R ei = R(0.25) * (F.eta(ai, aj, ak) + F.eta(bi, bj, bk) + F.eta(ci, cj, ck) + F.eta(i, j, k));
     if (WL) {
@@ -303,19 +307,19 @@ FHD_D Taus<R> edge_taus_w(const RunParams& P, const Fields<NS, R>& F, double wno
             n2 = R(F.vel[2](i, j, k)) - R(F.vel[2](i, j - 1, k));
         }
         if (x2 == 0 && dirichlet_side(P, 2 * d2)) {
-            g1 = divc(P, n1, R(P.hdx[d2]), R(P.rhdx[d2]));
+            g1 = divc(P, n1, rc<R>(P).hdx[d2], rc<R>(P).rhdx[d2]);
             ei = R(0.5) * (ea + ec);
         }
         if (x2 == P.n[d2] && dirichlet_side(P, 2 * d2 + 1)) {
-            g1 = divc(P, n1, R(P.hdx[d2]), R(P.rhdx[d2]));
+            g1 = divc(P, n1, rc<R>(P).hdx[d2], rc<R>(P).rhdx[d2]);
             ei = R(0.5) * (eb + ed);
         }
         if (x1 == 0 && dirichlet_side(P, 2 * d1)) {
-            g2 = divc(P, n2, R(P.hdx[d1]), R(P.rhdx[d1]));
+            g2 = divc(P, n2, rc<R>(P).hdx[d1], rc<R>(P).rhdx[d1]);
             ei = R(0.5) * (ea + eb);
         }
         if (x1 == P.n[d1] && dirichlet_side(P, 2 * d1 + 1)) {
-            g2 = divc(P, n2, R(P.hdx[d1]), R(P.rhdx[d1]));
+            g2 = divc(P, n2, rc<R>(P).hdx[d1], rc<R>(P).rhdx[d1]);
             ei = R(0.5) * (ec + ed);
         }
     }
@@ -471,7 +475,7 @@ FHD_D FaceFlux<NS> face_flux(const RunParams& P, const Fields<NS, R>& F, const N
         }
         double wf[NS + 1];
         nz.template face_all<NS + 1>(P, D, i, j, k, wf);
-        const R fw0 = dsqrt(R(P.k_B) * kp * R(P.volinv) * R(P.dtinv));
+        const R fw0 = dsqrt(rc<R>(P).k_B * kp * rc<R>(P).volinv * rc<R>(P).dtinv);
         heat = fw0 * R(wf[0]);
         // StochFluxStag: thermal walls scale the stochastic heat flux (a reservoir
         // side keeps the factor 1)
@@ -496,15 +500,15 @@ FHD_D FaceFlux<NS> face_flux(const RunParams& P, const Fields<NS, R>& F, const N
         R MWmix = R(0.);
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
-            MWmix = MWmix + divc(P, R(0.5) * (yy[s] + yyp[s]), R(P.molmass[s]), R(P.rmolmass[s]));
+            MWmix = MWmix + divc(P, R(0.5) * (yy[s] + yyp[s]), rc<R>(P).molmass[s], rc<R>(P).rmolmass[s]);
 #pragma unroll
             for (int ll = 0; ll < NS; ++ll) {
                 if (WL && ws >= 0)
                     DY[s * NS + ll] = R(0.5) * (x.Dc(gs, ll * NS + s) * yy[ll] + x.Dc(gs, ll * NS + s) * yyp[ll] +
                                                 (x.Dc(gs, s * NS + ll) * yy[s] + x.Dc(gs, s * NS + ll) * yyp[s]));
                 else
-                    DY[s * NS + ll] = R(0.5) * (x.Dc(0, ll * NS + s) * yy[ll] + x.Dc(1, ll * NS + s) * yyp[ll] +
-                                                (x.Dc(0, s * NS + ll) * yy[s] + x.Dc(1, s * NS + ll) * yyp[s]));
+                    DY[s * NS + ll] = R(0.5) * (madd(x.Dc(0, ll * NS + s), yy[ll], x.Dc(1, ll * NS + s) * yyp[ll]) +
+                                                madd(x.Dc(0, s * NS + ll), yy[s], x.Dc(1, s * NS + ll) * yyp[s]));
             }
         }
 #pragma unroll
@@ -515,14 +519,14 @@ FHD_D FaceFlux<NS> face_flux(const RunParams& P, const Fields<NS, R>& F, const N
             }
         MWmix = rdiv(R(1.), MWmix);
         CholeskyDecomp<NS, R>(DY, sqD);
-        const R fwc = dsqrt(divc(P, R(P.k_B) * MWmix * R(P.volinv), R(P.Runiv) * R(P.dt), R(P.rRdt)));
+        const R fwc = dsqrt(divc(P, rc<R>(P).k_B * MWmix * rc<R>(P).volinv, rc<R>(P).Runiv * rc<R>(P).dt, rc<R>(P).rRdt));
         R zs[NS];
 #pragma unroll
         for (int ll = 0; ll < NS; ++ll) zs[ll] = R(wf[1 + ll]);
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
 #pragma unroll
-            for (int ll = 0; ll <= s; ++ll) wien[s] = wien[s] + fwc * sqD[s * NS + ll] * zs[ll];
+            for (int ll = 0; ll <= s; ++ll) wien[s] = madd(fwc * sqD[s * NS + ll], zs[ll], wien[s]);
             spec[s] = wien[s];
         }
         GetEnthalpies<NS, R>(P, meanT, hk);
@@ -531,10 +535,10 @@ FHD_D FaceFlux<NS> face_flux(const RunParams& P, const Fields<NS, R>& F, const N
         for (int s = 0; s < NS; ++s) {
             R soret_s;
             if (WL && ws >= 0)
-                soret_s = (hk[s] + divc(P, R(P.Runiv) * meanT, R(P.molmass[s]), R(P.rmolmass[s])) *
+                soret_s = (hk[s] + divc(P, rc<R>(P).Runiv * meanT, rc<R>(P).molmass[s], rc<R>(P).rmolmass[s]) *
                                        x.chi(gs, s)) * wien[s];
             else
-                soret_s = (hk[s] + divc(P, R(P.Runiv) * meanT, R(P.molmass[s]), R(P.rmolmass[s])) * R(0.5) *
+                soret_s = (hk[s] + divc(P, rc<R>(P).Runiv * meanT, rc<R>(P).molmass[s], rc<R>(P).rmolmass[s]) * R(0.5) *
                                        (x.chi(0, s) + x.chi(1, s))) * wien[s];
             soret += soret_s;
         }
@@ -552,8 +556,8 @@ FHD_D FaceFlux<NS> face_flux(const RunParams& P, const Fields<NS, R>& F, const N
     // ---- diffusive part (fluxStag.cpp:1026-1426) ----
     if (!transverse) {
         // wall faces difference over the half cell to the wall value
-        const R h = (WL && ws >= 0) ? R(P.hdx[D]) : R(P.dx[D]);
-        const R rh = (WL && ws >= 0) ? R(P.rhdx[D]) : R(P.rdx[D]);
+        const R h = (WL && ws >= 0) ? rc<R>(P).hdx[D] : rc<R>(P).dx[D];
+        const R rh = (WL && ws >= 0) ? rc<R>(P).rhdx[D] : rc<R>(P).rdx[D];
         const R Tl = R(x.T(0)), Th = R(x.T(1));
         const R pl = R(x.p(0)), ph = R(x.p(1));
         R kp = R(0.5) * (x.kappa(0) + x.kappa(1));
@@ -589,10 +593,9 @@ FHD_D FaceFlux<NS> face_flux(const RunParams& P, const Fields<NS, R>& F, const N
             R f = R(0.);
 #pragma unroll
             for (int ll = 0; ll < NS; ++ll) {
-                R Fks;
-                if (WL && ws >= 0) Fks = x.Dc(gs, ll * NS + kk) * (dk[ll] + sor[ll]);
-                else Fks = R(0.5) * (x.Dc(0, ll * NS + kk) + x.Dc(1, ll * NS + kk)) * (dk[ll] + sor[ll]);
-                f -= Fks;
+                const R Dm = (WL && ws >= 0) ? x.Dc(gs, ll * NS + kk)
+                                             : R(0.5) * (x.Dc(0, ll * NS + kk) + x.Dc(1, ll * NS + kk));
+                f = madd(-Dm, dk[ll] + sor[ll], f);
             }
             Fk[kk] = f;
         }
@@ -601,12 +604,12 @@ FHD_D FaceFlux<NS> face_flux(const RunParams& P, const Fields<NS, R>& F, const N
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
             if (WL && ws >= 0) {
-                Q5 += (hk[s] + divc0(P, R(P.Runiv) * meanT * x.chi(gs, s), R(P.molmass[s]), R(P.rmolmass[s]))) *
+                Q5 += (hk[s] + divc0(P, rc<R>(P).Runiv * meanT * x.chi(gs, s), rc<R>(P).molmass[s], rc<R>(P).rmolmass[s])) *
                       Fk[s];
             } else {
                 // z faces use chi(i,j,k)+chi(i,j,k), fluxStag.cpp:1407 (kept from the reference)
                 const R chs = (D == 2) ? (x.chi(1, s) + x.chi(1, s)) : (x.chi(0, s) + x.chi(1, s));
-                Q5 += (hk[s] + divc0(P, R(0.5) * R(P.Runiv) * meanT * chs, R(P.molmass[s]), R(P.rmolmass[s]))) * Fk[s];
+                Q5 += (hk[s] + divc0(P, R(0.5) * rc<R>(P).Runiv * meanT * chs, rc<R>(P).molmass[s], rc<R>(P).rmolmass[s])) * Fk[s];
             }
         }
         duf += Q5;

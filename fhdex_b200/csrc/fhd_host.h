@@ -121,6 +121,50 @@ inline DevParams dev_params(const fhd_params& p, double dt, uint64_t step) {
     P.r3 = rcp(3.0);
     P.div_lo = kDivAlo;
     P.div_span = in_window ? kDivAspan : 0u;
+    // the FP32 copies
+    auto cast = [](float& f, double d) { f = (float)d; };
+    RunConstsF& f = P.f32;
+    for (int d = 0; d < 3; ++d) {
+        cast(f.dx[d], P.dx[d]);
+        cast(f.hdx[d], P.hdx[d]);
+        cast(f.rhdx[d], P.rhdx[d]);
+        cast(f.rdx[d], P.rdx[d]);
+    }
+    cast(f.dt, P.dt);
+    cast(f.volinv, P.volinv);
+    cast(f.dtinv, P.dtinv);
+    cast(f.k_B, P.k_B);
+    cast(f.Runiv, P.Runiv);
+    cast(f.zeta_ratio, P.zeta_ratio);
+    cast(f.sqrt3, P.sqrt3);
+    cast(f.fac2d, P.fac2d);
+    cast(f.rRdt, P.rRdt);
+    cast(f.rpi, P.rpi);
+    cast(f.r3, P.r3);
+    TransConstsF& t = P.t32;
+    for (int i = 0; i < MAXS; ++i) {
+        cast(f.molmass[i], P.molmass[i]);
+        cast(f.rmolmass[i], P.rmolmass[i]);
+        cast(f.hcv[i], P.hcv[i]);
+        cast(f.hcp[i], P.hcp[i]);
+        cast(f.e0[i], P.e0[i]);
+        cast(t.mm[i], P.mm[i]);
+        cast(t.mmkB[i], P.mmkB[i]);
+        cast(t.eta1pre[i], P.eta1pre[i]);
+        cast(t.rmm[i], P.rmm[i]);
+        for (int j = 0; j < MAXS; ++j) {
+            cast(t.diam[i][j], P.diam[i][j]);
+            cast(t.mu[i][j], P.mu[i][j]);
+            cast(t.msum[i][j], P.msum[i][j]);
+            cast(t.vfac[i][j], P.vfac[i][j]);
+            cast(t.kfac[i][j], P.kfac[i][j]);
+            cast(t.rmu[i][j], P.rmu[i][j]);
+            cast(t.rmsum[i][j], P.rmsum[i][j]);
+        }
+    }
+    cast(t.koff, P.koff);
+    cast(t.voff, P.voff);
+    cast(t.cfac, P.cfac);
     return P;
 }
 

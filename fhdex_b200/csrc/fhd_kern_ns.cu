@@ -131,8 +131,9 @@ int FHD_CAT(exact_transport_ns, FHD_NS)(const DevParams& P, fhd_fab prim, fhd_fa
     if (P.dim == 1 && g > 1) g = 1;
     a.ng = g;
     a.status = status;
-    const int64_t tot = (int64_t)(P.n[0] + 2 * a.ng) * (P.n[1] + 2 * a.ng) * (P.n[2] + 2 * a.ng);
-    k_transport<FHD_NS><<<grid_for(tot, 128), 128, 0, s>>>(a);
+    a.it = make_items(P.n[0] + 2 * a.ng, P.n[1] + 2 * a.ng, P.n[2] + 2 * a.ng);
+    if (P.transport_type == 1) k_transport<FHD_NS><<<grid_for(a.it.n, 128), 128, 0, s>>>(a);
+    else k_transport_alt<FHD_NS><<<grid_for(a.it.n, 128), 128, 0, s>>>(a);
     return cuda_rc(cudaGetLastError());
 }
 

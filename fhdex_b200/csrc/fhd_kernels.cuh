@@ -33,7 +33,7 @@ FHD_D void flag(int* status, int code) {
 // cellprep: U^s -> (T, p, Y, X), coefficients, face velocities
 // ===================================================================================
 template <int NS, class R>
-struct PrepArgs {
+struct alignas(16) PrepArgs {
     DevParams P;
     Arr4<const double> cons;
     Arr4<const double> mom[3];
@@ -160,7 +160,7 @@ struct FaceDir {
 };
 
 template <int NS, class R, int NZ>
-struct StageArgs {
+struct alignas(16) StageArgs {
     RunParams P;
     Fields<NS, R> F;             // stage-input state U^s + derived fields
     Noise<NZ> noise;
@@ -448,8 +448,11 @@ FHD_D void update_point(const StageArgs<NS, R, NZ>& a, int q) {
     }
 }
 
-template <int NS, class R, int NZ>
-static __global__ void __launch_bounds__(128, 16) k_update(StageArgs<NS, R, NZ> a) {  // HBM-bound: full occupancy
+// MINB: 16 blocks of 128 (32 registers, full occupancy) where the kernel streams from
+// HBM; 4 for a box that fits one wave of them, where a point's loads cost its time and
+// more registers put more of them in flight (update_blocks)
+template <int NS, class R, int NZ, int MINB>
+static __global__ void __launch_bounds__(128, MINB) k_update(StageArgs<NS, R, NZ> a) {
     const int tot = update_count(a);
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < tot; q += gridDim.x * blockDim.x) update_point(a, q);
 }
@@ -458,7 +461,7 @@ static __global__ void __launch_bounds__(128, 16) k_update(StageArgs<NS, R, NZ> 
 // conservedToPrimitiveStag on valid cells/faces (conservedPrimitiveConversionsStag.cpp)
 // ===================================================================================
 template <int NS>
-struct ConvArgs {
+struct alignas(16) ConvArgs {
     RunParams P;
     Items it;
     Arr4<double> prim;   // reference layout (nprimvars comps)
@@ -528,11 +531,11 @@ static __global__ void __launch_bounds__(128) k_convert(ConvArgs<NS> a) {
 // periodic FillBoundary of up to 16 fabs in one launch
 // ===================================================================================
 struct GhostFab {
-    double* p;
-    int lo, vhi[3];   // ghost width = -lo; valid upper index per direction
-    int64_t sy, sz, sn;
+    double* p;        // point (0,0,0)
+    int g, vhi[3];    // ghost width; valid upper index per direction
+    int sy, sz, sn;
     int c0, nc;       // component range
-    int64_t npts;     // ghost points of one component
+    int npts;         // ghost points of one component
     int n[3];         // cells of the box (period)
     // periodic directions (walls elsewhere).  mode 0 (FillBoundary): a ghost point
     // is filled only when it lies outside the valid box in periodic directions
@@ -540,68 +543,104 @@ struct GhostFab {
     // periodic coordinates are wrapped and the wall coordinates kept.
     int per[3];
     int mode;
+    int zsl, ysl;     // points of the two z slabs (all x, y) and of the two y slabs (valid z)
+    int nx, vy, vz;   // row length with ghosts; valid rows and planes
+    FastDiv dpts, dzp, dnx, dyp, dxp, dvy;   // by npts, nx*(vy+2g), nx, nx*vz, vy*vz, vy
 };
 struct GhostArgs {
     GhostFab f[16];
     int nf;
-    int n[3];
 };
 
-FHD_D void ghost_point(const GhostFab& f, int64_t q) {
-    const int g = -f.lo;
-    const int NX = f.vhi[0] + 1 + 2 * g, NY = f.vhi[1] + 1 + 2 * g;
-    const int VX = f.vhi[0] + 1, VY = f.vhi[1] + 1, VZ = f.vhi[2] + 1;
-    const int64_t zsl = (int64_t)2 * g * NX * NY;        // two z slabs (all x, y)
-    const int64_t ysl = (int64_t)2 * g * NX * VZ;        // two y slabs (valid z)
-    {
-        const int c = f.c0 + (int)(q / f.npts);
-        int64_t r = q % f.npts;
-        int i, j, k;
-        if (r < zsl) {
-            const int kk = (int)(r / ((int64_t)NX * NY));
-            r -= (int64_t)kk * NX * NY;
-            j = (int)(r / NX) - g; i = (int)(r % NX) - g;
-            k = kk < g ? kk - g : VZ + (kk - g);
-        } else if (r < zsl + ysl) {
-            r -= zsl;
-            const int jj = (int)(r / ((int64_t)NX * VZ));
-            r -= (int64_t)jj * NX * VZ;
-            k = (int)(r / NX); i = (int)(r % NX) - g;
-            j = jj < g ? jj - g : VY + (jj - g);
-        } else {
-            r -= zsl + ysl;
-            const int ii = (int)(r / ((int64_t)VY * VZ));
-            r -= (int64_t)ii * VY * VZ;
-            k = (int)(r / VY); j = (int)(r % VY);
-            i = ii < g ? ii - g : VX + (ii - g);
-        }
-        int s[3] = {i, j, k};
-        bool wrapped = false;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            if (s[d] >= 0 && s[d] <= f.vhi[d]) continue;
-            if (!f.per[d]) {
-                if (f.mode == 0) return;
-                continue;
-            }
-            wrapped = true;
-            while (s[d] < 0) s[d] += f.n[d];
-            while (s[d] > f.vhi[d]) s[d] -= f.n[d];
-        }
-        if (!wrapped) return;
-        const int si = s[0], sj = s[1], sk = s[2];
-        const int64_t base = (int64_t)c * f.sn;
-        f.p[base + (i + g) + (j + g) * f.sy + (k + g) * f.sz] = f.p[base + (si + g) + (sj + g) * f.sy + (sk + g) * f.sz];
+// host: the ghost fill of components c0 .. c0+nc-1 of a fab of the box (a fab has fewer
+// than 2^31 values, so every index here is 32-bit and the divisions are FastDiv: with
+// 64-bit ones the fill of a statistics update took 39 us at 144x112x96, see fill_ghosts)
+inline GhostFab make_ghost(void* data, const int lo[3], const int hi[3], const int nodal[3], int c0, int nc,
+                           const int ncell[3], const int* periodic, int mode) {
+    GhostFab f;
+    f.g = -lo[0];
+    const int ex = hi[0] - lo[0] + 1, ey = hi[1] - lo[1] + 1, ez = hi[2] - lo[2] + 1;
+    f.sy = ex;
+    f.sz = ex * ey;
+    f.sn = ex * ey * ez;
+    f.p = static_cast<double*>(data) + f.g * (1 + f.sy + f.sz);
+    f.c0 = c0;
+    f.nc = nc;
+    for (int d = 0; d < 3; ++d) {
+        f.vhi[d] = ncell[d] - 1 + nodal[d];
+        f.n[d] = ncell[d];
+        f.per[d] = periodic ? periodic[d] : 1;
     }
+    f.mode = mode;
+    f.nx = ex;
+    f.vy = f.vhi[1] + 1;
+    f.vz = f.vhi[2] + 1;
+    f.zsl = 2 * f.g * ex * ey;
+    f.ysl = 2 * f.g * ex * f.vz;
+    f.npts = f.zsl + f.ysl + 2 * f.g * f.vy * f.vz;
+    auto div = [](int d) { return fast_div((uint32_t)(d > 0 ? d : 1)); };
+    f.dpts = div(f.npts);
+    f.dzp = div(ex * ey);
+    f.dnx = div(ex);
+    f.dyp = div(ex * f.vz);
+    f.dxp = div(f.vy * f.vz);
+    f.dvy = div(f.vy);
+    return f;
+}
+
+FHD_D void ghost_point(const GhostFab& f, int q) {
+    const int g = f.g;
+    const int cc = (int)f.dpts.div((uint32_t)q);
+    int r = q - cc * f.npts;
+    int s[3];
+    if (r < f.zsl) {
+        const int kk = (int)f.dzp.div((uint32_t)r);
+        r -= kk * f.sz;
+        const int jj = (int)f.dnx.div((uint32_t)r);
+        s[0] = r - jj * f.nx - g;
+        s[1] = jj - g;
+        s[2] = kk < g ? kk - g : f.vz + (kk - g);
+    } else if (r < f.zsl + f.ysl) {
+        r -= f.zsl;
+        const int jj = (int)f.dyp.div((uint32_t)r);
+        r -= jj * f.nx * f.vz;
+        const int kk = (int)f.dnx.div((uint32_t)r);
+        s[0] = r - kk * f.nx - g;
+        s[1] = jj < g ? jj - g : f.vy + (jj - g);
+        s[2] = kk;
+    } else {
+        r -= f.zsl + f.ysl;
+        const int ii = (int)f.dxp.div((uint32_t)r);
+        r -= ii * f.vy * f.vz;
+        const int kk = (int)f.dvy.div((uint32_t)r);
+        s[0] = ii < g ? ii - g : f.vhi[0] + 1 + (ii - g);
+        s[1] = r - kk * f.vy;
+        s[2] = kk;
+    }
+    double* base = f.p + (f.c0 + cc) * f.sn;
+    double* dst = base + s[0] + s[1] * f.sy + s[2] * f.sz;
+    bool wrapped = false;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        if (s[d] >= 0 && s[d] <= f.vhi[d]) continue;
+        if (!f.per[d]) {
+            if (f.mode == 0) return;
+            continue;
+        }
+        wrapped = true;
+        while (s[d] < 0) s[d] += f.n[d];
+        while (s[d] > f.vhi[d]) s[d] -= f.n[d];
+    }
+    if (!wrapped) return;
+    *dst = base[s[0] + s[1] * f.sy + s[2] * f.sz];
 }
 
 static __global__ void __launch_bounds__(256) k_ghosts(GhostArgs a) {
     const int fidx = blockIdx.y;
     if (fidx >= a.nf) return;
     const GhostFab& f = a.f[fidx];
-    const int64_t tot = f.npts * f.nc;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < tot; q += (int64_t)gridDim.x * blockDim.x)
-        ghost_point(f, q);
+    const int tot = f.npts * f.nc;
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < tot; q += gridDim.x * blockDim.x) ghost_point(f, q);
 }
 
 // OverrideSync: nodal point n_cells <- point 0 (per nodal direction)
@@ -639,24 +678,27 @@ struct TransArgs {
     DevParams P;
     Arr4<const double> prim;
     Arr4<double> eta, zeta, kappa, chi, D;
+    Items it;          // the box grown by ng
     int ng;
     int* status;
 };
 
-template <int NS>
-static __global__ void __launch_bounds__(128) k_transport(TransArgs<NS> a) {
+// ALT: the Valk/Waldmann or HCB binary model (runs with these models take this
+// kernel), else Giovangigli's.  One kernel with both models in it took 255 registers and
+// 620 B of spills for four species (160 registers for two); apart, Giovangigli's has
+// the cell kernel's register budget (cellprep_min_blocks).
+template <int NS, bool ALT>
+FHD_D void transport_body(const TransArgs<NS>& a) {
     const DevParams& P = a.P;
-    const int g = a.ng;
-    const int nx = P.n[0] + 2 * g, ny = P.n[1] + 2 * g, nz = P.n[2] + 2 * g;
-    const int64_t tot = (int64_t)nx * ny * nz;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < tot; q += (int64_t)gridDim.x * blockDim.x) {
-        const int i = (int)(q % nx) - g, j = (int)((q / nx) % ny) - g, k = (int)(q / ((int64_t)nx * ny)) - g;
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < a.it.n; q += gridDim.x * blockDim.x) {
+        int i, j, k;
+        a.it.point(q, i, j, k);
+        i -= a.ng; j -= a.ng; k -= a.ng;
         double Y[NS];
 #pragma unroll
         for (int n = 0; n < NS; ++n) Y[n] = a.prim(i, j, k, 6 + n);
         Coeffs<NS, double> c;
-        if (P.transport_type != 1) {
-            // Valk/Waldmann or HCB binary (runs with these models take this kernel)
+        if constexpr (ALT) {
             const int st = transport_alt<NS>(P, a.prim(i, j, k, 0), a.prim(i, j, k, 4), a.prim(i, j, k, 5), Y, c);
             if (st) flag(a.status, st);
         } else if (!transport_gio<NS, double>(P, a.prim(i, j, k, 0), a.prim(i, j, k, 4), a.prim(i, j, k, 5), Y, c)) {
@@ -670,6 +712,15 @@ static __global__ void __launch_bounds__(128) k_transport(TransArgs<NS> a) {
 #pragma unroll
         for (int n = 0; n < NS * NS; ++n) a.D(i, j, k, n) = c.D[n];
     }
+}
+
+template <int NS>
+static __global__ void __launch_bounds__(128, cellprep_min_blocks<NS, double>()) k_transport(TransArgs<NS> a) {
+    transport_body<NS, false>(a);
+}
+template <int NS>
+static __global__ void __launch_bounds__(128) k_transport_alt(TransArgs<NS> a) {
+    transport_body<NS, true>(a);
 }
 
 // stresses recomputed on the fly (operator path)
@@ -826,17 +877,16 @@ static __global__ void k_init_uniform(InitArgs a) {
 
 // ===================================================================================
 // batched launches: one launch covers the work items of every member of an
-// ensemble; block b belongs to the member m with bpref[m] <= b < bpref[m+1]
+// ensemble; block b belongs to the member m with bpref[m] <= b < bpref[m+1].  After the
+// nmem + 1 prefixes come the members of blocks 0, 64, 128, ...: a block starts there and
+// steps to its own (boxes of 64 and more blocks: at most one step), where a binary
+// search made log2(members) dependent loads before the block could start.
 // ===================================================================================
 FHD_D int member_of(const int* __restrict__ bpref, int nmem) {
-    int lo = 0, hi = nmem;
     const int b = blockIdx.x;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (bpref[mid] <= b) lo = mid;
-        else hi = mid;
-    }
-    return lo;
+    int m = __ldg(bpref + nmem + 1 + (b >> 6));
+    while (__ldg(bpref + m + 1) <= b) ++m;
+    return m;
 }
 
 // The member's argument block, copied once per block into shared memory (every
@@ -845,11 +895,11 @@ FHD_D int member_of(const int* __restrict__ bpref, int nmem) {
 // they read from global memory in registers.
 template <class A>
 FHD_D const A& member_args(const A* __restrict__ args, int m) {
-    static_assert(sizeof(A) % 8 == 0, "argument blocks are copied in 8-byte words");
+    static_assert(sizeof(A) % 16 == 0, "argument blocks are copied in 16-byte words");
     __shared__ A sa;
-    const unsigned long long* src = reinterpret_cast<const unsigned long long*>(args + m);
-    unsigned long long* dst = reinterpret_cast<unsigned long long*>(&sa);
-    for (int w = threadIdx.x; w < (int)(sizeof(A) / 8); w += blockDim.x) dst[w] = src[w];
+    const uint4* src = reinterpret_cast<const uint4*>(args + m);
+    uint4* dst = reinterpret_cast<uint4*>(&sa);
+    for (int w = threadIdx.x; w < (int)(sizeof(A) / 16); w += blockDim.x) dst[w] = src[w];
     __syncthreads();
     return sa;
 }
@@ -863,8 +913,9 @@ static __global__ void __launch_bounds__(128, cellprep_min_blocks<NS, R>()) k_ce
     if (q < cellprep_count(a)) cellprep_point(a, q);
 }
 
+// 64 registers (8 blocks of 128 per SM): uncapped, the FP32 kernel took 96 and ran 20 warps per SM
 template <int NS, class R, int NZ>
-static __global__ void __launch_bounds__(128) k_taus_b(const StageArgs<NS, R, NZ>* __restrict__ args,
+static __global__ void __launch_bounds__(128, 8) k_taus_b(const StageArgs<NS, R, NZ>* __restrict__ args,
                                                 const int* __restrict__ bpref, int nmem) {
     const int m = member_of(bpref, nmem);
     const StageArgs<NS, R, NZ>& a = member_args(args, m);
@@ -883,8 +934,9 @@ static __global__ void __launch_bounds__(128, MINB) k_faces_b(const StageArgs<NS
     if (q < faces_count(a, d)) faces_point(a, d, q);
 }
 
+// 48 registers (10 blocks per SM; the single-run kernel's 32 spill here)
 template <int NS, class R, int NZ>
-static __global__ void __launch_bounds__(128) k_update_b(const StageArgs<NS, R, NZ>* __restrict__ args,
+static __global__ void __launch_bounds__(128, 10) k_update_b(const StageArgs<NS, R, NZ>* __restrict__ args,
                                                   const int* __restrict__ bpref, int nmem) {
     const int m = member_of(bpref, nmem);
     const StageArgs<NS, R, NZ>& a = member_args(args, m);
@@ -905,7 +957,7 @@ static __global__ void __launch_bounds__(256) k_ghosts_b(const GhostFab* __restr
                                                          const int* __restrict__ bpref, int nfab) {
     const int m = member_of(bpref, nfab);
     const GhostFab& f = fabs[m];
-    const int64_t q = (int64_t)(blockIdx.x - bpref[m]) * blockDim.x + threadIdx.x;
+    const int q = (blockIdx.x - bpref[m]) * blockDim.x + threadIdx.x;
     if (q < f.npts * f.nc) ghost_point(f, q);
 }
 
@@ -958,7 +1010,7 @@ struct PersistBytes {
 
 template <int NS, class R, int NZ, int MINB>
 static __global__ void __launch_bounds__(128, MINB) k_batch_persist(PersistArgs a) {
-    __shared__ unsigned long long sbuf[PersistBytes<NS, R, NZ>::value / 8];
+    __shared__ __align__(16) unsigned long long sbuf[PersistBytes<NS, R, NZ>::value / 8];
     __shared__ int s_unit, s_go, s_end;
     __shared__ long long s_chunk;
     for (;;) {
@@ -1031,7 +1083,7 @@ static __global__ void __launch_bounds__(128, MINB) k_batch_persist(PersistArgs 
                 } break;
                 case PK_GHOST: {
                     const auto& G = *reinterpret_cast<const GhostFab*>(sbuf);
-                    for (int64_t x = q; x < q1; x += st) ghost_point(G, x);
+                    for (int64_t x = q; x < q1; x += st) ghost_point(G, (int)x);
                 } break;
                 default:
                     if (threadIdx.x == 0) a.steps[pu.member] += 1;

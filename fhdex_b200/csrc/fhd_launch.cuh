@@ -105,7 +105,7 @@ template <int MODE>
 Noise<MODE> make_noise(const StageCall& c) {
     Noise<MODE> n;
     n.w = c.w;
-    for (int d = 0; d < 3; ++d) {
+    if constexpr (MODE == NZ_W || MODE == NZ_AB) for (int d = 0; d < 3; ++d) {
         n.a.fa[d] = view<const double>(c.nz.fa[d]);
         n.a.fb[d] = view<const double>(c.nz.fb[d]);
         n.a.foa[d] = c.nz.fa[d].ncomp - (c.P.ns + 1);
@@ -273,6 +273,13 @@ inline int stage_block(const StageCall& c) {
     return (c.tile >= 0 && c.tile < kNumStageBlocks) ? kStageBlocks[c.tile] : 128;
 }
 
+template <int NS, class R, int NZ>
+void launch_update(const StageArgs<NS, R, NZ>& a, cudaStream_t s) {
+    const int blocks = (a.it_upd.n + 127) / 128;
+    if (blocks <= 4 * device_sms()) k_update<NS, R, NZ, 4><<<blocks, 128, 0, s>>>(a);
+    else k_update<NS, R, NZ, 16><<<resident_grid<k_update<NS, R, NZ, 16>>(a.it_upd.n, 128), 128, 0, s>>>(a);
+}
+
 // part: 0 stresses, 1 face fluxes (all three directions), 2 update
 template <int NS, class R, int NZ>
 int launch_stage_part_t(const StageCall& c, int part) {
@@ -280,13 +287,13 @@ int launch_stage_part_t(const StageCall& c, int part) {
     const int* N = c.P.n;
     const int b = stage_block(c);
     if (part == 0) {
-        k_taus<NS, R, NZ><<<grid_for((int64_t)(N[0] + 2) * (N[1] + 2) * (N[2] + 2), b), b, 0, c.stream>>>(a, {});
+        k_taus<NS, R, NZ><<<grid_for((int64_t)(N[0] + 2) * (N[1] + 2) * (N[2] + 2), b), b, 0, c.stream>>>(a, StageAux<false>{});
     } else if (part == 1) {
         const int t = (c.tile >= 0 && c.tile < kNumStageBlocks) ? c.tile : auto_face_tile<NS, R>(N);
 #define FHD_FACES(BS, MINB)                                                                    \
         {                                                                                      \
             const int per = face_grid<k_faces<NS, R, NZ, BS, MINB>>(N, BS);                    \
-            k_faces<NS, R, NZ, BS, MINB><<<3 * per, BS, 0, c.stream>>>(a, per, {});            \
+            k_faces<NS, R, NZ, BS, MINB><<<3 * per, BS, 0, c.stream>>>(a, per, StageAux<false>{}); \
         }
         switch (t) {
             case 0: FHD_FACES(128, 4) break;
@@ -297,10 +304,7 @@ int launch_stage_part_t(const StageCall& c, int part) {
         }
 #undef FHD_FACES
     } else {
-        // 128 threads whatever the tile: the update kernel is capped at 32 registers
-        // for full occupancy (16 blocks of 128 per SM)
-        k_update<NS, R, NZ><<<resident_grid<k_update<NS, R, NZ>>((int64_t)(N[0] + 1) * (N[1] + 1) * (N[2] + 1), 128),
-                               128, 0, c.stream>>>(a);
+        launch_update<NS, R, NZ>(a, c.stream);
     }
     return cuda_rc(cudaGetLastError());
 }
@@ -375,16 +379,15 @@ int launch_walls_part_t(const StageCall& c, int part) {
     const StageArgs<NS, double, NZ> a = make_stage_args<NS, double, NZ>(c);
     const int* N = c.P.n;
     if (part == 0) {
-        k_taus<NS, double, NZ, true><<<grid_for((int64_t)(N[0] + 2) * (N[1] + 2) * (N[2] + 2), 128), 128, 0, c.stream>>>(a, {});
+        k_taus<NS, double, NZ, true><<<grid_for((int64_t)(N[0] + 2) * (N[1] + 2) * (N[2] + 2), 128), 128, 0, c.stream>>>(a, StageAux<false>{});
     } else if (part == 1) {
         // register cap: 64 up to two species (the periodic autotuner's choice at 256^3;
         // 128 was measured twice as slow for the wall variant), 128 above
         constexpr int MB = NS <= 2 ? 8 : 4;
         const int per = face_grid<k_faces<NS, double, NZ, 128, MB, true>>(N, 128);
-        k_faces<NS, double, NZ, 128, MB, true><<<3 * per, 128, 0, c.stream>>>(a, per, {});
+        k_faces<NS, double, NZ, 128, MB, true><<<3 * per, 128, 0, c.stream>>>(a, per, StageAux<false>{});
     } else {
-        k_update<NS, double, NZ><<<resident_grid<k_update<NS, double, NZ>>(
-            (int64_t)(N[0] + 1) * (N[1] + 1) * (N[2] + 1), 128), 128, 0, c.stream>>>(a);
+        launch_update<NS, double, NZ>(a, c.stream);
     }
     return cuda_rc(cudaGetLastError());
 }

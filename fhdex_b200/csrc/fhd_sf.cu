@@ -147,9 +147,9 @@ __device__ __forceinline__ int64_t half_entry(int nx, int ny, int nz, int i, int
 }
 
 struct SfFinArgs {
-    int nx, ny, nz, ncov, zero_avg;
-    int64_t N, half;
-    FastDiv dx, dxy;
+    int nx, ny, nz, nxh1, ncov, zero_avg;
+    int64_t half;
+    FastDiv dx, dxy;                 // by nxh1, nxh1 * ny
     double nsinv;
     const double* cov;
     const double* scale;
@@ -157,31 +157,38 @@ struct SfFinArgs {
 };
 
 // Finalize (StructFact.cpp:598-620) with ShiftFFT (:643-719): destination point
-// ((i + nx/2) % nx, ...) of source point (i, j, k).
+// ((i + nx/2) % nx, ...) of source point (i, j, k).  One thread per half-spectrum entry
+// writes its point and, where that is beyond nx/2, the mirrored one (equal but for the
+// sign of the imaginary part), so that each entry is read, scaled and rooted once.
+// Bound by its writes (30 components of 10 pairs).
 __global__ void __launch_bounds__(256) k_sf_finalize(SfFinArgs a) {
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < a.N; q += (int64_t)gridDim.x * blockDim.x) {
-        const int k = (int)a.dxy.div((uint32_t)q), r = (int)q - k * a.nx * a.ny;
-        const int j = (int)a.dx.div((uint32_t)r), i = r - j * a.nx;
-        int ip = i + a.nx / 2, jp = j + a.ny / 2, kp = k + a.nz / 2;
-        ip -= ip >= a.nx ? a.nx : 0;
-        jp -= jp >= a.ny ? a.ny : 0;
-        kp -= kp >= a.nz ? a.nz : 0;
-        const bool zero = a.zero_avg == 1 && i == 0 && j == 0 && k == 0;
-        double sign;
-        const int64_t h = half_entry(a.nx, a.ny, a.nz, i, j, k, sign);
-#pragma unroll 4
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < a.half; q += (int64_t)gridDim.x * blockDim.x) {
+        const int k = (int)a.dxy.div((uint32_t)q), r = (int)q - k * a.nxh1 * a.ny;
+        const int j = (int)a.dx.div((uint32_t)r), i = r - j * a.nxh1;
+        auto shift = [](int x, int n) { const int s = x + n / 2; return s >= n ? s - n : s; };
+        const int ip = shift(i, a.nx), jp = shift(j, a.ny), kp = shift(k, a.nz);
+        const bool mirror = a.nx - i > a.nx / 2 && i > 0;
+        const int im = shift(a.nx - i, a.nx), jm = shift(j == 0 ? 0 : a.ny - j, a.ny),
+                  km = shift(k == 0 ? 0 : a.nz - k, a.nz);
+        const bool zero = a.zero_avg == 1 && q == 0;
+#pragma unroll 2
         for (int c = 0; c < a.ncov; ++c) {
-            double re = zero ? 0.0 : __ldg(a.cov + (int64_t)c * a.half + h);
-            double im = zero ? 0.0 : sign * __ldg(a.cov + ((int64_t)a.ncov + c) * a.half + h);
+            double re = zero ? 0.0 : __ldg(a.cov + (int64_t)c * a.half + q);
+            double im_ = zero ? 0.0 : __ldg(a.cov + ((int64_t)a.ncov + c) * a.half + q);
             re = re * a.nsinv;
             re = re * a.scale[c];
-            im = im * a.nsinv;
-            im = im * a.scale[c];
+            im_ = im_ * a.nsinv;
+            im_ = im_ * a.scale[c];
             double mag = 0.0 + re * re;
-            mag = mag + im * im;
+            mag = sqrt(mag + im_ * im_);
             a.ore(ip, jp, kp, c) = re;
-            a.oim(ip, jp, kp, c) = im;
-            a.omag(ip, jp, kp, c) = sqrt(mag);
+            a.oim(ip, jp, kp, c) = im_;
+            a.omag(ip, jp, kp, c) = mag;
+            if (mirror) {
+                a.ore(im, jm, km, c) = re;
+                a.oim(im, jm, km, c) = -im_;
+                a.omag(im, jm, km, c) = mag;
+            }
         }
     }
 }
@@ -505,17 +512,17 @@ int fhd_sf_finalize(fhd_sf* s, fhd_fab cov_real, fhd_fab cov_imag, fhd_fab cov_m
     a.nz = s->n[2];
     a.ncov = s->ncov;
     a.zero_avg = zero_avg;
-    a.N = (int64_t)s->n[0] * s->n[1] * s->n[2];
-    a.half = (int64_t)(s->n[0] / 2 + 1) * s->n[1] * s->n[2];
-    a.dx = fast_div((uint32_t)s->n[0]);
-    a.dxy = fast_div((uint32_t)(s->n[0] * s->n[1]));
+    a.nxh1 = s->n[0] / 2 + 1;
+    a.half = (int64_t)a.nxh1 * s->n[1] * s->n[2];
+    a.dx = fast_div((uint32_t)a.nxh1);
+    a.dxy = fast_div((uint32_t)(a.nxh1 * s->n[1]));
     a.nsinv = 1.0 / (double)s->nsamples;  // StructFact.cpp:603
     a.cov = s->cov;
     a.scale = s->dscale;
     a.ore = view<double>(cov_real);
     a.oim = view<double>(cov_imag);
     a.omag = view<double>(cov_mag);
-    k_sf_finalize<<<grid_for(a.N, 256), 256, 0, s->stream>>>(a);
+    k_sf_finalize<<<grid_for(a.half, 256), 256, 0, s->stream>>>(a);
     return cuda_rc(cudaGetLastError());
 }
 

@@ -24,10 +24,11 @@
 namespace fhd {
 
 struct StatsArgs {
-    DevParams P;
+    RunParams P;
     Arr4<const double> cu, prim, mom[3];
     Arr4<double> cum, cuv, pm, pv, cov, m3, m4;
     Arr4<double> vm[3], vv[3], mm[3], mv[3];
+    Items ita, itb;     // the cell box grown by 2; the points [0, n]^3
     double sm1, sinv;   // stepsminusone, stepsinv
     int mom3, mom4;     // plot_mom3 / plot_mom4
 };
@@ -35,10 +36,10 @@ struct StatsArgs {
 // pass A: one thread per point of the cell box grown by 2
 static __global__ void __launch_bounds__(256) k_stats_means_a(StatsArgs a) {
     const int* n = a.P.n;
-    const int gx = n[0] + 4, gy = n[1] + 4, gz = n[2] + 4;
-    const int64_t tot = (int64_t)gx * gy * gz;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < tot; q += (int64_t)gridDim.x * blockDim.x) {
-        const int i = int(q % gx) - 2, j = int((q / gx) % gy) - 2, k = int(q / ((int64_t)gx * gy)) - 2;
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < a.ita.n; q += gridDim.x * blockDim.x) {
+        int i, j, k;
+        a.ita.point(q, i, j, k);
+        i -= 2; j -= 2; k -= 2;
         // loads first, then the updates, then the stores (see pass B)
         const double r0 = a.cum(i, j, k, 0), u0 = a.cu(i, j, k, 0);
         bool on[3];
@@ -63,13 +64,12 @@ static __global__ void __launch_bounds__(256) k_stats_means_a(StatsArgs a) {
 // pass B: one thread per point of [0, n]^3
 template <int NS>
 static __global__ void __launch_bounds__(256) k_stats_means_b(StatsArgs a) {
-    const DevParams& P = a.P;
+    const RunParams& P = a.P;
     const int* n = P.n;
-    const int gx = n[0] + 1, gy = n[1] + 1, gz = n[2] + 1;
     const int nprim = 6 + 2 * NS;
-    const int64_t tot = (int64_t)gx * gy * gz;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < tot; q += (int64_t)gridDim.x * blockDim.x) {
-        const int i = int(q % gx), j = int((q / gx) % gy), k = int(q / ((int64_t)gx * gy));
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < a.itb.n; q += gridDim.x * blockDim.x) {
+        int i, j, k;
+        a.itb.point(q, i, j, k);
         if (i < n[0] && j < n[1] && k < n[2]) {
             // cell means (statsStag.cpp:275-316).  Every operand is loaded before
             // the first store (the statistics are distinct arrays the compiler
@@ -152,17 +152,19 @@ static __global__ void __launch_bounds__(256) k_stats_means_b(StatsArgs a) {
 }
 
 // pass C: one thread per point of [0, n]^3.  As in pass B, operands are loaded in
-// groups before the stores they feed, so each thread keeps many loads in flight.
+// groups before the stores they feed, so each thread keeps many loads in flight.  The
+// groups are of at most about 18 values, which lets 128 registers hold them: with all 26
+// covariances and both moments in one group each the kernel took 242 registers, eight
+// warps per SM (438 us at 144x112x96, two species, 4.3 TB/s of algorithmic bytes).
 template <int NS>
-static __global__ void __launch_bounds__(256) k_stats_vars(StatsArgs a) {
-    const DevParams& P = a.P;
+static __global__ void __launch_bounds__(128, 3) k_stats_vars(StatsArgs a) {
+    const RunParams& P = a.P;
     const int* n = P.n;
-    const int gx = n[0] + 1, gy = n[1] + 1, gz = n[2] + 1;
     const int nvars = 5 + NS, nprim = 6 + 2 * NS;
-    const int64_t tot = (int64_t)gx * gy * gz;
     const double sm1 = a.sm1, sinv = a.sinv;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < tot; q += (int64_t)gridDim.x * blockDim.x) {
-        const int i = int(q % gx), j = int((q / gx) % gy), k = int(q / ((int64_t)gx * gy));
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < a.itb.n; q += gridDim.x * blockDim.x) {
+        int i, j, k;
+        a.itb.point(q, i, j, k);
         const Arr4<const double>& cu = a.cu;
         const Arr4<double>& cm = a.cum;
         // momentum and velocity variances on faces (statsStag.cpp:416-435)
@@ -306,23 +308,23 @@ static __global__ void __launch_bounds__(256) k_stats_vars(StatsArgs a) {
                                       delvelx * delvelz, delrho * deltemp, delvelx * deltemp, delvely * deltemp,
                                       delvelz * deltemp, delYk[0] * delYk[NS - 1], delYk[0] * delvelx,
                                       delYk[NS - 1] * delvelx, delrhoYk[0] * delvelx, delrhoYk[NS - 1] * delvelx};
-            double oco[26];
+            double oco[13];
 #pragma unroll
-            for (int c = 0; c < 26; ++c) oco[c] = co(i, j, k, c);
+            for (int h = 0; h < 26; h += 13) {
 #pragma unroll
-            for (int c = 0; c < 26; ++c) co(i, j, k, c) = (oco[c] * sm1 + cterm[c]) * sinv;
+                for (int c = 0; c < 13; ++c) oco[c] = co(i, j, k, h + c);
+#pragma unroll
+                for (int c = 0; c < 13; ++c) co(i, j, k, h + c) = (oco[c] * sm1 + cterm[h + c]) * sinv;
+            }
         }
         // group 4: third and fourth moments (statsStag.cpp:639-688); their recomputed
         // inputs equal the values above
         if (a.mom3 || a.mom4) {
             const double dv[3] = {delvelx, delvely, delvelz};
-            double o3[6 + NS], o4[6 + NS];
-#pragma unroll
-            for (int c = 0; c < 6 + NS; ++c) {
-                if (a.mom3) o3[c] = a.m3(i, j, k, c);
-                if (a.mom4) o4[c] = a.m4(i, j, k, c);
-            }
             if (a.mom3) {
+                double o3[6 + NS];
+#pragma unroll
+                for (int c = 0; c < 6 + NS; ++c) o3[c] = a.m3(i, j, k, c);
                 o3[0] = (o3[0] * sm1 + delrho * delrho * delrho) * sinv;
                 o3[4] = (o3[4] * sm1 + delenergy * delenergy * delenergy) * sinv;
 #pragma unroll
@@ -334,6 +336,9 @@ static __global__ void __launch_bounds__(256) k_stats_vars(StatsArgs a) {
                 for (int c = 0; c < 6 + NS; ++c) a.m3(i, j, k, c) = o3[c];
             }
             if (a.mom4) {
+                double o4[6 + NS];
+#pragma unroll
+                for (int c = 0; c < 6 + NS; ++c) o4[c] = a.m4(i, j, k, c);
                 o4[0] = (o4[0] * sm1 + delrho * delrho * delrho * delrho) * sinv;
                 o4[4] = (o4[4] * sm1 + delenergy * delenergy * delenergy * delenergy) * sinv;
 #pragma unroll
@@ -353,8 +358,7 @@ template <int NS>
 static int stats_launch(const StatsArgs& a, bool means, bool vars, const fhd_fab& cuMeans,
                         const fhd_fab& primMeans, const fhd_fab& cuVars, const fhd_fab& primVars, cudaStream_t s) {
     const int* n = a.P.n;
-    const int64_t ga = (int64_t)(n[0] + 4) * (n[1] + 4) * (n[2] + 4);
-    const int64_t gb = (int64_t)(n[0] + 1) * (n[1] + 1) * (n[2] + 1);
+    const int64_t ga = a.ita.n, gb = a.itb.n;
     if (means) {
         k_stats_means_a<<<grid_for(ga, 256), 256, 0, s>>>(a);
         k_stats_means_b<NS><<<grid_for(gb, 256), 256, 0, s>>>(a);
@@ -363,7 +367,7 @@ static int stats_launch(const StatsArgs& a, bool means, bool vars, const fhd_fab
         if (rc) return rc;
     }
     if (vars) {
-        k_stats_vars<NS><<<grid_for(gb, 256), 256, 0, s>>>(a);
+        k_stats_vars<NS><<<grid_for(gb, 128), 128, 0, s>>>(a);
         const GhostReq g[2] = {{cuVars, 0, cuVars.ncomp}, {primVars, 0, primVars.ncomp}};
         const int rc = fill_ghosts(g, 2, n, s, a.P.periodic, 0);
         if (rc) return rc;
@@ -717,6 +721,8 @@ int exact_stats(const DevParams& P, const fhd_fab& cu, const fhd_fab& prim, cons
         a.mv[d] = view<double>(st.cumomVars[d]);
     }
     // statsStag.cpp:211-212 (and :383-384): computed on the host in the same order
+    a.ita = make_items(P.n[0] + 4, P.n[1] + 4, P.n[2] + 4);
+    a.itb = make_items(P.n[0] + 1, P.n[1] + 1, P.n[2] + 1);
     a.sm1 = (double)steps - 1.;
     a.sinv = 1. / (double)steps;
     const bool means = flags & FHD_STATS_MEANS, vars = flags & FHD_STATS_VARS;
