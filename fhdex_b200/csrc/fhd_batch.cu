@@ -57,7 +57,7 @@ struct Member {
     fhd_fab cu{}, mom[3]{}, prim{}, vel[3]{};
     void* scratch = nullptr;
     size_t bytes = 0;
-    fhd_fab cup{}, cup2{}, cupm[3]{}, cup2m[3]{}, eta{}, zeta{}, kappa{}, chi{}, D{}, ct{}, et{}, sff[3]{}, smc{}, sme{};
+    fhd_fab cup{}, cup2{}, cupm[3]{}, cup2m[3]{}, rec{}, ct{}, et{}, sff[3]{}, smc{}, sme{};
     int64_t cells = 0;
 };
 
@@ -130,11 +130,7 @@ int alloc_member(fhd_batch* b, Member& m) {
     m.cup = mk(n, CELLN, NGC, 5 + ns, FHD_F64);
     m.cup2 = m.cup;
     for (int d = 0; d < 3; ++d) m.cupm[d] = m.cup2m[d] = mk(n, FACEN[d], NGC, 1, FHD_F64);
-    m.eta = mk(n, CELLN, NGC, 1, rdt);
-    m.zeta = m.eta;
-    m.kappa = m.eta;
-    m.chi = mk(n, CELLN, NGC, ns, rdt);
-    m.D = mk(n, CELLN, NGC, ns * ns, rdt);
+    m.rec = mk(n, CELLN, 1, rec_words(ns, rdt), rdt);
     m.ct = mk(n, CELLN, 1, 6, rdt);
     m.et = mk(n, ALLN, 0, 6, rdt);
     for (int d = 0; d < 3; ++d) m.sff[d] = mk(n, ALLN, 0, 2 + ns, FHD_F64);
@@ -142,8 +138,7 @@ int alloc_member(fhd_batch* b, Member& m) {
     m.sme = mk(n, ALLN, 0, 6, FHD_F64);
     struct P { fhd_fab* f; size_t e; } parts[] = {
         {&m.cup, 8}, {&m.cup2, 8}, {&m.cupm[0], 8}, {&m.cupm[1], 8}, {&m.cupm[2], 8}, {&m.cup2m[0], 8},
-        {&m.cup2m[1], 8}, {&m.cup2m[2], 8}, {&m.eta, re}, {&m.zeta, re}, {&m.kappa, re}, {&m.chi, re}, {&m.D, re},
-        {&m.ct, re}, {&m.et, re}, {&m.sff[0], 8}, {&m.sff[1], 8}, {&m.sff[2], 8}, {&m.smc, 8}, {&m.sme, 8}};
+        {&m.cup2m[1], 8}, {&m.cup2m[2], 8}, {&m.rec, 16}, {&m.ct, re}, {&m.et, re}, {&m.sff[0], 8}, {&m.sff[1], 8}, {&m.sff[2], 8}, {&m.smc, 8}, {&m.sme, 8}};
     size_t total = 0;
     for (auto& q : parts) total += ((size_t)pts(*q.f) * q.f->ncomp * q.e + 255) & ~(size_t)255;
     if (cudaMallocAsync(&m.scratch, total, b->stream) != cudaSuccess) { cudaGetLastError(); return FHD_ERR_OOM; }
@@ -181,7 +176,9 @@ StageCall member_call(const fhd_batch* b, const Member& m, int s, const uint64_t
     }
     sc.pr = m.prim;
     sc.pT = 4;
-    sc.eta = m.eta; sc.zeta = m.zeta; sc.kappa = m.kappa; sc.chi = m.chi; sc.D = m.D;
+    sc.pack = 1;
+    sc.rec = m.rec;
+    sc.wprim = rec_wprim(m.prm);
     sc.ct = m.ct;
     sc.et = m.et;
     sc.smc = m.smc;

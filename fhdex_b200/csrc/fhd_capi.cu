@@ -29,6 +29,7 @@ struct fhd_ctx {
     size_t coef_bytes = 0;
     int coef_dtype = -1;
     fhd_fab ceta{}, czeta{}, ckappa{}, cchi{}, cD{};
+    fhd_fab crec{};              // cell records of the packed pipeline (in coef's memory)
     fhd_fab ct{}, et{};          // stage stresses (coefficient precision)
     fhd_fab sff[3]{};            // stage conservative face fluxes (f64)
     fhd_fab smc{}, sme{};        // stage total centre / edge momentum fluxes (f64)
@@ -173,7 +174,7 @@ int ensure_scratch(fhd_ctx* c) {
     const int64_t vpts = (int64_t)n[0] * n[1] * n[2];
     const int64_t srcpts = c->prm.nreaction > 0 ? vpts * nvars : 0;  // chemistry's source when the caller has none
     const size_t need = (size_t)(2 * cellpts * nvars + 2 * (fpts[0] + fpts[1] + fpts[2]) + 3 * npts * (2 + ns) +
-                                 3 * c1pts + 6 * npts + srcpts) * sizeof(double);
+                                 3 * c1pts + 6 * npts + srcpts + 4) * sizeof(double);
     if (c->scratch && c->scratch_bytes >= need) return FHD_OK;
     if (c->scratch) cudaFree(c->scratch);
     c->scratch = nullptr;
@@ -186,13 +187,17 @@ int ensure_scratch(fhd_ctx* c) {
     c->cup2 = make_fab(p, n, CELLN, NGC, nvars, FHD_F64); p += cellpts * nvars;
     for (int d = 0; d < 3; ++d) { c->cupm[d] = make_fab(p, n, FACEN[d], NGC, 1, FHD_F64); p += fpts[d]; }
     for (int d = 0; d < 3; ++d) { c->cup2m[d] = make_fab(p, n, FACEN[d], NGC, 1, FHD_F64); p += fpts[d]; }
-    // face fluxes on [0, n]^3 (lo = 0, hi = n: every face box fits)
+    // face fluxes on [0, n]^3 (lo = 0, hi = n: every face box fits); they and the edge
+    // totals hold 16-byte words
+    auto align2 = [&] { p += (p - c->scratch) & 1; };
     for (int d = 0; d < 3; ++d) {
+        align2();
         c->sff[d] = make_fab(p, n, allnod, 0, 2 + ns, FHD_F64);
         p += npts * (2 + ns);
     }
-    c->smc = make_fab(p, n, CELLN, 1, 3, FHD_F64); p += c1pts * 3;
+    align2();
     c->sme = make_fab(p, n, allnod, 0, 6, FHD_F64); p += npts * 6;
+    c->smc = make_fab(p, n, CELLN, 1, 3, FHD_F64); p += c1pts * 3;
     c->csrc = srcpts ? make_fab(p, n, CELLN, 0, nvars, FHD_F64) : fhd_fab{};
     return FHD_OK;
 }
@@ -234,21 +239,30 @@ int ensure_coef(fhd_ctx* c, int dtype) {
     const int64_t ctpts = fab_points(make_fab(nullptr, n, CELLN, 1, 1, dtype));
     const int64_t etpts = fab_points(make_fab(nullptr, n, allnod, 0, 1, dtype));
     const size_t es = dtype == FHD_F64 ? 8 : 4;
-    const size_t need = ((size_t)pts * ncomp + 6 * (size_t)(ctpts + etpts)) * es;
+    // The cell records of the packed pipeline and the coefficient fields of the others
+    // (walls, quasi-1-D / 2-D, the fused stage kernel) share one region: a step uses one
+    // of the two.  Then the stresses; each part starts on 16 bytes.
+    auto up = [](size_t b) { return (b + 15) & ~(size_t)15; };
+    const int words = rec_words(ns, dtype);
+    const size_t coef = (size_t)pts * ncomp * es, rec = (size_t)ctpts * words * 16;
+    const size_t head = up(coef > rec ? coef : rec), ctb = up(6 * (size_t)ctpts * es);
+    const size_t need = head + ctb + 6 * (size_t)etpts * es;
     if (c->coef && c->coef_bytes >= need && c->coef_dtype == dtype) return FHD_OK;
     if (c->coef) cudaFree(c->coef);
     c->coef = nullptr;
     if (cudaMalloc(&c->coef, need) != cudaSuccess) { cudaGetLastError(); return FHD_ERR_OOM; }
     c->coef_bytes = need;
     c->coef_dtype = dtype;
-    char* p = static_cast<char*>(c->coef);
+    char* const base = static_cast<char*>(c->coef);
+    char* p = base;
+    c->crec = make_fab(p, n, CELLN, 1, words, dtype);
     c->ceta = make_fab(p, n, CELLN, NGC, 1, dtype); p += pts * es;
     c->czeta = make_fab(p, n, CELLN, NGC, 1, dtype); p += pts * es;
     c->ckappa = make_fab(p, n, CELLN, NGC, 1, dtype); p += pts * es;
     c->cchi = make_fab(p, n, CELLN, NGC, ns, dtype); p += pts * ns * es;
-    c->cD = make_fab(p, n, CELLN, NGC, ns * ns, dtype); p += pts * ns * ns * es;
-    c->ct = make_fab(p, n, CELLN, 1, 6, dtype); p += ctpts * 6 * es;
-    c->et = make_fab(p, n, allnod, 0, 6, dtype);
+    c->cD = make_fab(p, n, CELLN, NGC, ns * ns, dtype);
+    c->ct = make_fab(base + head, n, CELLN, 1, 6, dtype);
+    c->et = make_fab(base + head + ctb, n, allnod, 0, 6, dtype);
     return FHD_OK;
 }
 
@@ -1133,6 +1147,11 @@ static int step_launches(fhd_ctx* c, fhd_fab cu, const fhd_fab mom[3], fhd_fab p
     sc.pT = 4;
     for (int d = 0; d < 3; ++d) { sc.vel[d] = vel[d]; sc.mom0[d] = mom[d]; }
     sc.cons0 = cu;
+    // the fused stage kernel reads the fields, the split pipeline's kernels cell records
+    const bool fused = tile_fused(c->tile);
+    sc.pack = !fused;
+    sc.rec = c->crec;
+    sc.wprim = rec_wprim(c->prm);
     if (aux_coef && !mixed) { sc.eta = eta; sc.zeta = zeta; sc.kappa = kappa; sc.chi = chi; sc.D = D; }
     else { sc.eta = c->ceta; sc.zeta = c->czeta; sc.kappa = c->ckappa; sc.chi = c->cchi; sc.D = c->cD; }
     sc.src = source;
@@ -1163,6 +1182,7 @@ static int step_launches(fhd_ctx* c, fhd_fab cu, const fhd_fab mom[3], fhd_fab p
         sc.w = w[s];
         sc.cons_s = *ins[s];
         sc.cons_o = *outs[s];
+        sc.wcoef = s == 2 && aux_coef;   // the stage-3 coefficients are the caller's
         for (int d = 0; d < 3; ++d) { sc.mom_s[d] = insm[s][d]; sc.mom_o[d] = outsm[s][d]; }
         {
             ProfScope ps(c, 0);
@@ -1177,13 +1197,13 @@ static int step_launches(fhd_ctx* c, fhd_fab cu, const fhd_fab mom[3], fhd_fab p
             for (int d = 0; d < 3; ++d) { sc.ff[d] = faceflux[d]; sc.cf[d] = cenflux[d]; }
             for (int e = 0; e < 6; ++e) sc.ef[e] = edgeflux[e];
         }
-        if (aux && tile_fused(c->tile)) {
+        if (aux && fused) {
             // the fused kernel keeps its fluxes in shared memory
             ProfScope ps(c, 6);
-            for (int part = 0; part < 2 && !rc; ++part) rc = exact_aux_stage(sc, part);
+            rc = exact_aux_fluxes(sc);
             if (rc) return rc;
         }
-        if (tile_fused(c->tile)) {
+        if (fused) {
             ProfScope ps(c, 7);
             rc = mixed ? mixed_stage_part(sc, 3) : exact_stage_part(sc, 3);
         } else {

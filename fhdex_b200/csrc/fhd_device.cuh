@@ -140,6 +140,9 @@ FHD_D float rdiv(float a, float b) { return __fdividef(a, b); }
 // FP64, not to bitwise parity) the product a * y: within about one FP32 ulp of a / b.
 FHD_D double divc(const RunParams& P, double a, double b, double y) { return div_rcp(a, b, y, P.div_lo, P.div_span); }
 FHD_D float divc(const RunParams&, float a, float, float y) { return a * y; }
+// c + a / b for a constant divisor
+FHD_D double divc_add(const RunParams& P, double a, double b, double y, double c) { return c + divc(P, a, b, y); }
+FHD_D float divc_add(const RunParams&, float a, float, float y, float c) { return fmaf(a, y, c); }
 // divc for call sites whose dividend is often exactly zero (zero handled inline)
 FHD_D double divc0(const RunParams& P, double a, double b, double y) {
     return div_rcp_z(a, b, y, P.div_lo, P.div_span);
@@ -261,7 +264,7 @@ FHD_D R GetPressureGas(const RunParams& P, const R (&Y)[NS], R density, R temp) 
 template <int NS, class R>
 FHD_D void GetEnthalpies(const RunParams& P, R T, R (&hk)[NS]) {
 #pragma unroll
-    for (int i = 0; i < NS; ++i) hk[i] = rc<R>(P).e0[i] + rc<R>(P).hcp[i] * T;
+    for (int i = 0; i < NS; ++i) hk[i] = madd(rc<R>(P).hcp[i], T, rc<R>(P).e0[i]);
 }
 
 template <class R>
@@ -419,7 +422,7 @@ FHD_D bool transport_gio(const DevParams& P, R rho, R temperature, R pressure, c
     const R pi = R(3.1415926535897932);
     R mbar = R(0.0);
 #pragma unroll
-    for (int n = 0; n < NS; ++n) mbar += divc(P, Yk[n], tc<R>(P).mm[n], tc<R>(P).rmm[n]);
+    for (int n = 0; n < NS; ++n) mbar = divc_add(P, Yk[n], tc<R>(P).mm[n], tc<R>(P).rmm[n], mbar);
     mbar = rdiv(R(1.0), mbar);
     R Xk[NS], Xkp[NS], Ykp[NS];
     R Xksum = R(0.0);
@@ -467,8 +470,8 @@ FHD_D bool transport_gio(const DevParams& P, R rho, R temperature, R pressure, c
 #pragma unroll
                 for (int k = 0; k < NS; ++k)
                     if (k != i)
-                        a += rdiv(R(2.0) * kT * Xkp[i] * Xkp[k], pressure * Dbin[i][k] * tc<R>(P).msum[i][k]) *
-                             tc<R>(P).vfac[i][k];
+                        a = madd(rdiv(R(2.0) * kT * Xkp[i] * Xkp[k], pressure * Dbin[i][k] * tc<R>(P).msum[i][k]),
+                                 tc<R>(P).vfac[i][k], a);
                 amat[i][i] = a;
             } else {
                 amat[i][j] = rdiv(R(2.0) * kT * Xkp[i] * Xkp[j], pressure * Dbin[i][j] * tc<R>(P).msum[i][j]) *
@@ -510,8 +513,8 @@ FHD_D bool transport_gio(const DevParams& P, R rho, R temperature, R pressure, c
 #pragma unroll
                 for (int k = 0; k < NS; ++k)
                     if (k != i)
-                        a += divc(P, div_dbin<NS, R>(P, Xkp[i] * Xkp[k], Dbin[i][k], rDbin[i][k]) * tc<R>(P).mu[i][k], tc<R>(P).msum[i][k],
-                                  tc<R>(P).rmsum[i][k]) * tc<R>(P).kfac[i][k];
+                        a = madd(divc(P, div_dbin<NS, R>(P, Xkp[i] * Xkp[k], Dbin[i][k], rDbin[i][k]) * tc<R>(P).mu[i][k], tc<R>(P).msum[i][k],
+                                  tc<R>(P).rmsum[i][k]), tc<R>(P).kfac[i][k], a);
                 amat[i][i] = a;
             } else {
                 amat[i][j] = divc(P, div_dbin<NS, R>(P, R(-1.0) * Xkp[i] * Xkp[j], Dbin[i][j], rDbin[i][j]) * tc<R>(P).mu[i][j],
@@ -553,8 +556,8 @@ FHD_D bool transport_gio(const DevParams& P, R rho, R temperature, R pressure, c
 #pragma unroll
                 for (int k = 0; k < NS; ++k)
                     if (k != i)
-                        a -= divc(P, div_dbin<NS, R>(P, R(0.5) * Xkp[k], Dbin[i][k], rDbin[i][k]) * tc<R>(P).mm[k], tc<R>(P).msum[i][k],
-                                  tc<R>(P).rmsum[i][k]) * tc<R>(P).cfac;
+                        a = madd(-divc(P, div_dbin<NS, R>(P, R(0.5) * Xkp[k], Dbin[i][k], rDbin[i][k]) * tc<R>(P).mm[k], tc<R>(P).msum[i][k],
+                                  tc<R>(P).rmsum[i][k]), tc<R>(P).cfac, a);
                 row[j] = a;
             } else {
                 row[j] = divc(P, div_dbin<NS, R>(P, R(0.5) * Xkp[j], Dbin[i][j], rDbin[i][j]) * tc<R>(P).mm[i], tc<R>(P).msum[i][j],

@@ -32,6 +32,55 @@ struct Fields {
     FHD_D double X(int i, int j, int k, int n) const { return pr(i, j, k, pT + 2 + NS + n); }
 };
 
+// ---- packed operands ------------------------------------------------------------
+// The stage kernels of a periodic box keep what they hand to one another in 16-byte
+// words: a cell's derived quantities as one record of the compute type (cellprep
+// writes it, the stress and face kernels read it), each stress as a (stochastic,
+// deterministic) pair, each edge's two momentum totals and the face fluxes as pairs.
+// One load then brings two FP64 (four FP32) operands: the kernels are bound by
+// instructions and by the latency of the loads they have in flight, and both halve.
+template <class R> using Vec = std::conditional_t<sizeof(R) == 8, double2, float4>;
+template <class R> using Pair = std::conditional_t<sizeof(R) == 8, double2, float2>;
+
+FHD_D double vget(const double2& v, int e) { return e ? v.y : v.x; }
+FHD_D float vget(const float4& v, int e) { return e == 0 ? v.x : (e == 1 ? v.y : (e == 2 ? v.z : v.w)); }
+FHD_D double2 vmake(const double* c) { return make_double2(c[0], c[1]); }
+FHD_D float4 vmake(const float* c) { return make_float4(c[0], c[1], c[2], c[3]); }
+FHD_D double2 pmake(double a, double b) { return make_double2(a, b); }
+FHD_D float2 pmake(float a, float b) { return make_float2(a, b); }
+
+// components of a cell record (a single gas has no species terms)
+template <int NS, class R>
+struct RecLayout {
+    static constexpr int T = 0, ETA = 1, KAPPA = 2, PR = 3, Y = 4, X = 4 + NS, CHI = 4 + 2 * NS, D = 4 + 3 * NS;
+    static constexpr int V = 16 / (int)sizeof(R);                  // components per word
+    static constexpr int N = NS == 1 ? 4 : 4 + 3 * NS + NS * NS;
+    static constexpr int NV = (N + V - 1) / V;                     // words per cell
+};
+template <int NS, class R>
+struct Rec {
+    const Vec<R>* p;     // word 0 of cell (0,0,0); cells grown by 1
+    int sy, sz, sn;
+    FHD_D R get(int o, int c) const { return vget(p[o + (c / RecLayout<NS, R>::V) * sn], c % RecLayout<NS, R>::V); }
+    FHD_D int at(int i, int j, int k) const { return i + j * sy + k * sz; }
+};
+
+// the fields of a stage with packed operands (the stress kernel's view; Fields' interface)
+template <int NS, class R>
+struct FieldsPack {
+    Rec<NS, R> q;
+    Arr4<const double> cons, mom[3], vel[3], pr;   // pr: prim, T at comp pT
+    int pT;
+    R zr;                                          // zeta = zeta_ratio * eta (|visc_type| = 3)
+    FHD_D R eta(int i, int j, int k) const { return q.get(q.at(i, j, k), RecLayout<NS, R>::ETA); }
+    FHD_D R zeta(int i, int j, int k) const { return zr * eta(i, j, k); }
+    FHD_D R T(int i, int j, int k) const { return q.get(q.at(i, j, k), RecLayout<NS, R>::T); }
+    FHD_D double p(int i, int j, int k) const {
+        if constexpr (sizeof(R) == 8) return q.get(q.at(i, j, k), RecLayout<NS, R>::PR);
+        else return pr(i, j, k, pT + 1);
+    }
+};
+
 // ---- noise sources --------------------------------------------------------------
 enum { NZ_OFF = 0, NZ_W = 1, NZ_AB = 2, NZ_PHILOX = 3 };
 
@@ -162,8 +211,8 @@ struct CellTaus {
 // pipeline, which also carries the quasi-1-D / 2-D runs (P.dim 1 / 2): only the
 // x (x and y) stresses, the 1-D amplitudes scaled by sqrt(3) and the 2-D trace
 // factor by (3+sqrt(3))/2 (fluxStag.cpp:171-192, 875-904)
-template <int NS, class R, int NZ, bool WL = false>
-FHD_D CellTaus<R> cell_taus_w(const RunParams& P, const Fields<NS, R>& F, const double (&wc)[3], int i, int j, int k) {
+template <int NS, class R, int NZ, bool WL = false, class FT>
+FHD_D CellTaus<R> cell_taus_w(const RunParams& P, const FT& F, const double (&wc)[3], int i, int j, int k) {
     CellTaus<R> t;
     const R eta = F.eta(i, j, k);
     const bool visc3 = (P.visc_type == 3 || P.visc_type == -3);
@@ -215,9 +264,9 @@ FHD_D CellTaus<R> cell_taus_w(const RunParams& P, const Fields<NS, R>& F, const 
                    divc(P, dsqrt(R(2.0) * rc<R>(P).k_B * etaT * rc<R>(P).volinv * rc<R>(P).dtinv), R(3.0), rc<R>(P).r3);
         const R w0 = R(wc[0]), w1 = R(wc[1]), w2 = R(wc[2]);
         const R traceZ = w0 + w1 + w2;
-        t.s[0] = (fac1 * w0) + (fac2 * traceZ);
-        t.s[1] = (fac1 * w1) + (fac2 * traceZ);
-        t.s[2] = (fac1 * w2) + (fac2 * traceZ);
+        t.s[0] = madd(fac1, w0, fac2 * traceZ);
+        t.s[1] = madd(fac1, w1, fac2 * traceZ);
+        t.s[2] = madd(fac1, w2, fac2 * traceZ);
     } else {
         t.s[0] = t.s[1] = t.s[2] = R(0.);
     }
@@ -227,9 +276,9 @@ FHD_D CellTaus<R> cell_taus_w(const RunParams& P, const Fields<NS, R>& F, const 
     const R div = u_x + v_y + w_z;
     const R zc = visc3 ? R(F.zeta(i, j, k)) : R(0.0);
     const R eta23 = divc(P, R(2) * eta, R(3.), rc<R>(P).r3);
-    t.d[0] = R(2) * eta * u_x + (zc - eta23) * div;
-    t.d[1] = R(2) * eta * v_y + (zc - eta23) * div;
-    t.d[2] = R(2) * eta * w_z + (zc - eta23) * div;
+    t.d[0] = madd(zc - eta23, div, R(2) * eta * u_x);
+    t.d[1] = madd(zc - eta23, div, R(2) * eta * v_y);
+    t.d[2] = madd(zc - eta23, div, R(2) * eta * w_z);
     return t;
 }
 
@@ -240,8 +289,8 @@ FHD_D CellTaus<R> cell_taus_w(const RunParams& P, const Fields<NS, R>& F, const 
 // ghost side for its stochastic amplitude and its viscosity, and differences the
 // velocity across the wall over the half cell (fluxStag.cpp:221-232, 250-261,
 // 279-290, 939-1019: the first direction's wall is tested last and wins a corner).
-template <int NS, class R, int NZ, int E, bool WL = false>
-FHD_D Taus<R> edge_taus_w(const RunParams& P, const Fields<NS, R>& F, double wnoise, int i, int j, int k) {
+template <int NS, class R, int NZ, int E, bool WL = false, class FT>
+FHD_D Taus<R> edge_taus_w(const RunParams& P, const FT& F, double wnoise, int i, int j, int k) {
     // quasi-1-D: no shear stress; quasi-2-D: only xy (fluxStag.cpp:212-214, 241-243,
     // 270-272, 930-932, 962-964, 995-997)
     if (WL && (P.dim == 1 || (P.dim == 2 && E != 0))) {
@@ -257,8 +306,10 @@ FHD_D Taus<R> edge_taus_w(const RunParams& P, const Fields<NS, R>& F, double wno
     else { ai = i; aj = j - 1; ak = k - 1; bi = i; bj = j - 1; bk = k; ci = i; cj = j; ck = k - 1; }
     Taus<R> t;
     if (NZ != NZ_OFF) {
-        R etaT = R(0.25) * (F.eta(ai, aj, ak) * R(F.T(ai, aj, ak)) + F.eta(bi, bj, bk) * R(F.T(bi, bj, bk)) +
-                            F.eta(ci, cj, ck) * R(F.T(ci, cj, ck)) + F.eta(i, j, k) * R(F.T(i, j, k)));
+        R etaT = F.eta(ai, aj, ak) * R(F.T(ai, aj, ak));
+        etaT = madd(F.eta(bi, bj, bk), R(F.T(bi, bj, bk)), etaT);
+        etaT = madd(F.eta(ci, cj, ck), R(F.T(ci, cj, ck)), etaT);
+        etaT = R(0.25) * madd(F.eta(i, j, k), R(F.T(i, j, k)), etaT);
         if (WL) {
             // cells a (lo, lo), b (lo, hi), c (hi, lo), d = (i, j, k) in the edge's
             // (first, second) directions; the wall of the second direction is tested first
@@ -367,6 +418,10 @@ struct FaceGen {
     FHD_D R kappa(int s) const { return F.kappa(ci(s), cj(s), ck(s)); }
     FHD_D R chi(int s, int n) const { return F.chi(ci(s), cj(s), ck(s), n); }
     FHD_D R Dc(int s, int n) const { return F.D(ci(s), cj(s), ck(s), n); }
+    // T, p and Y in FP64 for the hyperbolic part
+    FHD_D double Td(int s) const { return T(s); }
+    FHD_D double pd(int s) const { return p(s); }
+    FHD_D double Yd(int s, int n) const { return Y(s, n); }
     FHD_D double u() const { return F.vel[D](i, j, k); }
     FHD_D double m() const { return F.mom[D](i, j, k); }
     FHD_D Taus<R> cell(int s) const {
@@ -398,8 +453,8 @@ struct FaceGen {
 // Dufour and shear-heating parts (boundaryStag.cpp:2086-3009),
 // BCWallReservoirFluxStag's zero species / Dufour fluxes on impermeable walls
 // (boundaryStag.cpp:300-580) and no advective flux (fluxStag.cpp:1511-1529).
-template <int NS, class R, int NZ, bool WL, class X>
-FHD_D FaceFlux<NS> face_flux(const RunParams& P, const Fields<NS, R>& F, const Noise<NZ>& nz, const X& x, int i, int j,
+template <int NS, class R, int NZ, bool WL, class FT, class X>
+FHD_D FaceFlux<NS> face_flux(const RunParams& P, const FT& F, const Noise<NZ>& nz, const X& x, int i, int j,
                              int k) {
     const int D = x.dir();
     // wall side of this face (0 lo, 1 hi, -1 none) and the side of the cell holding the wall values
@@ -439,8 +494,8 @@ FHD_D FaceFlux<NS> face_flux(const RunParams& P, const Fields<NS, R>& F, const N
             vsh += R(0.5) * (va1h * ea1.s + va0h * ea0.s);
             vsh += R(0.5) * (vb1h * eb1.s + vb0h * eb0.s);
         } else {
-            vsh += R(0.25) * ((va1h + va1l) * ea1.s + (va0h + va0l) * ea0.s);
-            vsh += R(0.25) * ((vb1h + vb1l) * eb1.s + (vb0h + vb0l) * eb0.s);
+            vsh = madd(R(0.25), madd(va1h + va1l, ea1.s, (va0h + va0l) * ea0.s), vsh);
+            vsh = madd(R(0.25), madd(vb1h + vb1l, eb1.s, (vb0h + vb0l) * eb0.s), vsh);
         }
         vshear = vsh;
         // StochFluxStag: velocity walls scale the stochastic shear heating (a
@@ -457,8 +512,8 @@ FHD_D FaceFlux<NS> face_flux(const RunParams& P, const Fields<NS, R>& F, const N
         vsh -= R(0.5) * (va1h * ea1.d + va0h * ea0.d);
         vsh -= R(0.5) * (vb1h * eb1.d + vb0h * eb0.d);
     } else {
-        vsh -= R(0.25) * ((va1h + va1l) * ea1.d + (va0h + va0l) * ea0.d);
-        vsh -= R(0.25) * ((vb1h + vb1l) * eb1.d + (vb0h + vb0l) * eb0.d);
+        vsh = madd(R(-0.25), madd(va1h + va1l, ea1.d, (va0h + va0l) * ea0.d), vsh);
+        vsh = madd(R(-0.25), madd(vb1h + vb1l, eb1.d, (vb0h + vb0l) * eb0.d), vsh);
     }
     vshear += vsh;
     }
@@ -466,7 +521,7 @@ FHD_D FaceFlux<NS> face_flux(const RunParams& P, const Fields<NS, R>& F, const N
     // ---- stochastic part (fluxStag.cpp:298-781) ----
     if (NZ != NZ_OFF && !transverse) {
         const R Th = R(x.T(1)), Tl = R(x.T(0));
-        R kp = (x.kappa(1) * Th * Th + x.kappa(0) * Tl * Tl);
+        R kp = madd(x.kappa(0) * Tl, Tl, x.kappa(1) * Th * Th);
         R meanT = R(0.5) * (Th + Tl);
         if (WL && ws >= 0) {
             const R Tg = R(x.T(gs));
@@ -500,7 +555,7 @@ FHD_D FaceFlux<NS> face_flux(const RunParams& P, const Fields<NS, R>& F, const N
         R MWmix = R(0.);
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
-            MWmix = MWmix + divc(P, R(0.5) * (yy[s] + yyp[s]), rc<R>(P).molmass[s], rc<R>(P).rmolmass[s]);
+            MWmix = divc_add(P, R(0.5) * (yy[s] + yyp[s]), rc<R>(P).molmass[s], rc<R>(P).rmolmass[s], MWmix);
 #pragma unroll
             for (int ll = 0; ll < NS; ++ll) {
                 if (WL && ws >= 0)
@@ -535,12 +590,11 @@ FHD_D FaceFlux<NS> face_flux(const RunParams& P, const Fields<NS, R>& F, const N
         for (int s = 0; s < NS; ++s) {
             R soret_s;
             if (WL && ws >= 0)
-                soret_s = (hk[s] + divc(P, rc<R>(P).Runiv * meanT, rc<R>(P).molmass[s], rc<R>(P).rmolmass[s]) *
-                                       x.chi(gs, s)) * wien[s];
+                soret_s = madd(divc(P, rc<R>(P).Runiv * meanT, rc<R>(P).molmass[s], rc<R>(P).rmolmass[s]), x.chi(gs, s), hk[s]);
             else
-                soret_s = (hk[s] + divc(P, rc<R>(P).Runiv * meanT, rc<R>(P).molmass[s], rc<R>(P).rmolmass[s]) * R(0.5) *
-                                       (x.chi(0, s) + x.chi(1, s))) * wien[s];
-            soret += soret_s;
+                soret_s = madd(divc(P, rc<R>(P).Runiv * meanT, rc<R>(P).molmass[s], rc<R>(P).rmolmass[s]) * R(0.5),
+                               x.chi(0, s) + x.chi(1, s), hk[s]);
+            soret = madd(soret_s, wien[s], soret);
         }
         duf = soret;
         // StochFluxStag: mass walls scale the stochastic species and Dufour fluxes
@@ -584,7 +638,7 @@ FHD_D FaceFlux<NS> face_flux(const RunParams& P, const Fields<NS, R>& F, const N
             }
             const R term2 = divz(divc0(P, (mX - mY) * (ph - pl), h, rh), meanP);
             dk[s] = term1 + term2;
-            R ChiX = R(0.5) * (x.chi(0, s) * Xl + x.chi(1, s) * Xh);
+            R ChiX = R(0.5) * madd(x.chi(0, s), Xl, x.chi(1, s) * Xh);
             if (WL && ws >= 0) ChiX = x.chi(gs, s) * R(x.X(gs, s));
             sor[s] = divz(divc0(P, ChiX * (Th - Tl), h, rh), meanT);
         }
@@ -604,12 +658,13 @@ FHD_D FaceFlux<NS> face_flux(const RunParams& P, const Fields<NS, R>& F, const N
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
             if (WL && ws >= 0) {
-                Q5 += (hk[s] + divc0(P, rc<R>(P).Runiv * meanT * x.chi(gs, s), rc<R>(P).molmass[s], rc<R>(P).rmolmass[s])) *
-                      Fk[s];
+                Q5 = madd(hk[s] + divc0(P, rc<R>(P).Runiv * meanT * x.chi(gs, s), rc<R>(P).molmass[s], rc<R>(P).rmolmass[s]),
+                          Fk[s], Q5);
             } else {
                 // z faces use chi(i,j,k)+chi(i,j,k), fluxStag.cpp:1407 (kept from the reference)
                 const R chs = (D == 2) ? (x.chi(1, s) + x.chi(1, s)) : (x.chi(0, s) + x.chi(1, s));
-                Q5 += (hk[s] + divc0(P, R(0.5) * rc<R>(P).Runiv * meanT * chs, rc<R>(P).molmass[s], rc<R>(P).rmolmass[s])) * Fk[s];
+                Q5 = madd(hk[s] + divc0(P, R(0.5) * rc<R>(P).Runiv * meanT * chs, rc<R>(P).molmass[s], rc<R>(P).rmolmass[s]),
+                          Fk[s], Q5);
             }
         }
         duf += Q5;
@@ -641,13 +696,13 @@ FHD_D FaceFlux<NS> face_flux(const RunParams& P, const Fields<NS, R>& F, const N
         const double m = x.m();
         const double u = x.u();
         f0 += m;
-        const double pl = x.p(0), ph = x.p(1);
+        const double pl = x.pd(0), ph = x.pd(1);
         if (adv == 2) {
             f4 += 0.5 * (x.cons(0, 4) + x.cons(1, 4)) * u + 0.5 * (pl + ph) * u;
 #pragma unroll
             for (int s = 0; s < NS; ++s) fs[s] += 0.5 * (x.cons(0, 5 + s) + x.cons(1, 5 + s)) * u;
         } else {
-            const double meanT = 0.5 * (x.T(0) + x.T(1));
+            const double meanT = 0.5 * (x.Td(0) + x.Td(1));
             const double meanRho = 0.5 * (x.cons(0, 0) + x.cons(1, 0));
             double hk[NS];
             GetEnthalpies<NS, double>(P, meanT, hk);
@@ -658,7 +713,7 @@ FHD_D FaceFlux<NS> face_flux(const RunParams& P, const Fields<NS, R>& F, const N
             }
 #pragma unroll
             for (int s = 0; s < NS; ++s) {
-                const double Yk = 0.5 * (x.Y(0, s) + x.Y(1, s));
+                const double Yk = 0.5 * (x.Yd(0, s) + x.Yd(1, s));
                 fs[s] += Yk * m;
                 if (adv == 0) f4 += m * Yk * hk[s];
             }
@@ -703,8 +758,8 @@ FHD_D FaceFlux<NS> face_flux(const RunParams& P, const Fields<NS, R>& F, const N
 // WL: walls; an edge on a wall plane takes the momentum / velocity of its wall
 // side only (fluxStag.cpp:1774-1789, 1797-1812, 1820-1835: the second
 // direction's wall is tested first, the first direction's wins a corner).
-template <int NS, class R, int E, bool WL = false>
-FHD_D void edge_adv(const RunParams& P, const Fields<NS, R>& F, int i, int j, int k, double& a, double& b) {
+template <int NS, class R, int E, bool WL = false, class FT>
+FHD_D void edge_adv(const RunParams& P, const FT& F, int i, int j, int k, double& a, double& b) {
     const Arr4<const double>&mx = F.mom[0], &my = F.mom[1], &mz = F.mom[2];
     const Arr4<const double>&vx = F.vel[0], &vy = F.vel[1], &vz = F.vel[2];
     if (P.advection_type < 0) { a = b = 0.0; return; }
@@ -771,8 +826,8 @@ FHD_D double edge_total_w(const RunParams& P, const Taus<R>& t, double adv, int 
 // WL: the stochastic and diffusive part of a ghost cell beyond a reservoir side of
 // direction d is 0 (bc_mass 3) or, given as `inner` (bc_mass 4), that of the cell
 // inside it (BCWallReservoirFluxStag, boundaryStag.cpp:482-577).
-template <int NS, class R, bool WL = false>
-FHD_D double cen_total(const RunParams& P, const Fields<NS, R>& F, const CellTaus<R>& t, int d, int i, int j, int k,
+template <int NS, class R, bool WL = false, class FT>
+FHD_D double cen_total(const RunParams& P, const FT& F, const CellTaus<R>& t, int d, int i, int j, int k,
                        const CellTaus<R>* inner = nullptr) {
     double v = (double)t.s[d];
     v -= (double)t.d[d];

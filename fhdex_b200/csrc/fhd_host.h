@@ -186,10 +186,29 @@ struct StageCall {
     fhd_fab ff[3], ef[6], cf[3];        // flux outputs of the operator path
     fhd_fab ct, et, sff[3];             // stage scratch: cell/edge stresses, face fluxes
     fhd_fab smc, sme;                   // stage scratch: total centre / edge momentum fluxes
+    // Packed operands (the stage kernels of a periodic box): rec holds the cell records,
+    // and ct, et, sff, sme hold words of two (StageScratch; 16-byte aligned).  wprim: what
+    // the cell kernel writes of prim besides (1: p, 2: T, p, Y, X); wcoef: whether it
+    // writes the coefficient fabs.  Not packed: the cell kernel writes all of them.
+    int pack;
+    fhd_fab rec;
+    int wprim, wcoef;
     int* status;
     cudaStream_t stream;
     int tile;               // tile-shape index of k_stage (autotuned)
 };
+
+// words of 16 bytes in one cell record (RecLayout)
+inline int rec_words(int ns, int dtype) {
+    const int n = ns == 1 ? 4 : 4 + 3 * ns + ns * ns, v = dtype == FHD_F64 ? 2 : 4;
+    return (n + v - 1) / v;
+}
+// what the packed cell kernel must leave in prim: the FP64 pressure for the mixed path's
+// momentum and hyperbolic fluxes, everything for the other advection forms and reactions
+inline int rec_wprim(const fhd_params& p) {
+    if (p.nreaction > 0 || p.advection_type == 0 || p.advection_type == 1) return 2;
+    return p.precision == FHD_PREC_MIXED ? 1 : 0;
+}
 
 // exact (FP64) translation unit
 int exact_cellprep(const StageCall& c);

@@ -85,18 +85,30 @@ int FHD_CAT(exact_aux_ns, FHD_NS)(const StageCall& c) {
     return (c.P.walls || c.P.dim < 3) ? aux_mode<true>(c) : aux_mode<false>(c);
 }
 
-template <bool WL>
-int aux_stage_mode(const StageCall& c, int part) {
-    switch (c.mode) {
-        case NM_OFF: return launch_aux_stage_t<FHD_NS, NZ_OFF, WL>(c, part);
-        case NM_W: return launch_aux_stage_t<FHD_NS, NZ_W, WL>(c, part);
-        case NM_AB: return launch_aux_stage_t<FHD_NS, NZ_AB, WL>(c, part);
-        case NM_PHILOX: return launch_aux_stage_t<FHD_NS, NZ_PHILOX, WL>(c, part);
-        default: return FHD_ERR_BAD_ARG;
-    }
-}
+// a stage of the packed pipeline, of a box with walls or a quasi-1-D / 2-D run, or the
+// flux operator (no packed operands; its noise is W)
 int FHD_CAT(exact_aux_stage_ns, FHD_NS)(const StageCall& c, int part) {
-    return (c.P.walls || c.P.dim < 3) ? aux_stage_mode<true>(c, part) : aux_stage_mode<false>(c, part);
+    const bool wl = c.P.walls || c.P.dim < 3;
+    if (wl) {
+        switch (c.mode) {
+            case NM_OFF: return launch_aux_stage_t<FHD_NS, NZ_OFF, true, false>(c, part);
+            case NM_W: return launch_aux_stage_t<FHD_NS, NZ_W, true, false>(c, part);
+            case NM_AB: return launch_aux_stage_t<FHD_NS, NZ_AB, true, false>(c, part);
+            case NM_PHILOX: return launch_aux_stage_t<FHD_NS, NZ_PHILOX, true, false>(c, part);
+        }
+    } else if (c.pack) {
+        switch (c.mode) {
+            case NM_OFF: return launch_aux_stage_t<FHD_NS, NZ_OFF, false, true>(c, part);
+            case NM_AB: return launch_aux_stage_t<FHD_NS, NZ_AB, false, true>(c, part);
+            case NM_PHILOX: return launch_aux_stage_t<FHD_NS, NZ_PHILOX, false, true>(c, part);
+        }
+    } else {
+        switch (c.mode) {
+            case NM_OFF: return launch_aux_stage_t<FHD_NS, NZ_OFF, false, false>(c, part);
+            case NM_W: return launch_aux_stage_t<FHD_NS, NZ_W, false, false>(c, part);
+        }
+    }
+    return FHD_ERR_BAD_ARG;
 }
 
 int FHD_CAT(exact_walls_ns, FHD_NS)(const StageCall& c, int part) { return launch_walls_part<FHD_NS>(c, part); }

@@ -40,6 +40,11 @@ struct alignas(16) PrepArgs {
     Arr4<double> vel[3];
     Arr4<double> pr;   // view starting at the T component: T, p, Y[NS], X[NS]
     Arr4<R> eta, zeta, kappa, chi, D;
+    // packed pipeline: the cell records, else q null; which of prim (1: p, 2: T, p, Y, X)
+    // and whether the coefficient fields are written
+    Vec<R>* q;
+    int qsy, qsz, qsn;
+    int prim, coef;
     Items it;          // cells [-1, n + 1]^3
     int* status;
 };
@@ -67,18 +72,54 @@ FHD_D void cellprep_point(const PrepArgs<NS, R>& a, int q) {
                                       a.mom[1](i, j, k), a.mom[1](i, j + 1, k), a.mom[2](i, j, k),
                                       a.mom[2](i, j, k + 1), q2);
     if (!fin) flag(a.status, ST_NONFINITE);
-    a.pr(i, j, k, 0) = q2.T;
-    a.pr(i, j, k, 1) = q2.p;
+    if (a.prim) a.pr(i, j, k, 1) = q2.p;
+    if (a.prim > 1) {
+        a.pr(i, j, k, 0) = q2.T;
 #pragma unroll
-    for (int n = 0; n < NS; ++n) {
-        a.pr(i, j, k, 2 + n) = q2.Y[n];
-        a.pr(i, j, k, 2 + NS + n) = q2.X[n];
+        for (int n = 0; n < NS; ++n) {
+            a.pr(i, j, k, 2 + n) = q2.Y[n];
+            a.pr(i, j, k, 2 + NS + n) = q2.X[n];
+        }
     }
     R Yr[NS];
 #pragma unroll
     for (int n = 0; n < NS; ++n) Yr[n] = R(q2.Y[n]);
+    // The cell record, each word as soon as its components are known (the ones of Y and
+    // X alone before the transport model: fewer values live through it)
+    using L = RecLayout<NS, R>;
+    R v[L::NV * L::V];
+    Vec<R>* const o = a.q + (i + j * a.qsy + k * a.qsz);
+    auto early = [](int w) { return NS > 1 && w * L::V >= L::Y && (w + 1) * L::V <= L::CHI; };
+    if constexpr (NS > 1) {
+#pragma unroll
+        for (int n = 0; n < NS; ++n) {
+            v[L::Y + n] = R(q2.Y[n]);
+            v[L::X + n] = R(q2.X[n]);
+        }
+#pragma unroll
+        for (int w = 0; w < L::NV; ++w)
+            if (early(w) && a.q) o[w * a.qsn] = vmake(v + w * L::V);
+    }
     Coeffs<NS, R> c;
     if (!transport_gio<NS, R>(P, R(rho), R(q2.T), R(q2.p), Yr, c)) flag(a.status, ST_MASSFRAC);
+    if (a.q) {
+        v[L::T] = R(q2.T);
+        v[L::ETA] = c.eta;
+        v[L::KAPPA] = c.kappa;
+        v[L::PR] = R(q2.p);
+        if constexpr (NS > 1) {
+#pragma unroll
+            for (int n = 0; n < NS; ++n) v[L::CHI + n] = c.chi[n];
+#pragma unroll
+            for (int n = 0; n < NS * NS; ++n) v[L::D + n] = c.D[n];
+        }
+#pragma unroll
+        for (int n = L::N; n < L::NV * L::V; ++n) v[n] = R(0.);
+#pragma unroll
+        for (int w = 0; w < L::NV; ++w)
+            if (!early(w)) o[w * a.qsn] = vmake(v + w * L::V);
+    }
+    if (!a.coef) return;
     a.eta(i, j, k) = c.eta;
     a.kappa(i, j, k) = c.kappa;
     a.zeta(i, j, k) = c.zeta;
@@ -104,10 +145,10 @@ static __global__ void __launch_bounds__(128, cellprep_min_blocks<NS, R>()) k_ce
 // centre momentum flux with the particle reservoir's rule: a ghost cell beyond a
 // bc_mass 4 side of direction d takes the stochastic and diffusive part of the cell
 // inside it (recomputed here with that cell's own noise)
-template <int NS, class R, int NZ, bool WL>
-FHD_D double cen_total_res(const RunParams& P, const Fields<NS, R>& F, const Noise<NZ>& nz, const CellTaus<R>& t,
+template <int NS, class R, int NZ, bool WL, class FT>
+FHD_D double cen_total_res(const RunParams& P, const FT& F, const Noise<NZ>& nz, const CellTaus<R>& t,
                            int d, int i, int j, int k) {
-    if (WL) {
+    if constexpr (WL) {
         const int x = d == 0 ? i : (d == 1 ? j : k);
         const int side = x < 0 ? 2 * d : (x > P.n[d] - 1 ? 2 * d + 1 : -1);
         if (side >= 0 && P.bc_mass[side] == 4) {
@@ -131,10 +172,83 @@ FHD_D double cen_total_res(const RunParams& P, const Fields<NS, R>& F, const Noi
 //   mc: total centre momentum fluxes (cenflux x, y, z) on the cells grown by 1
 //   me: total edge momentum fluxes on [0, n]^3 in the reference's order
 //       edgeflux_x[0..1], edgeflux_y[0..1], edgeflux_z[0..1]
+// PACK (periodic boxes): the same values in words of two; ct and et hold (s, d), me the
+// two totals of edge E (edgey_u, edgex_v; edgez_u, edgex_w; edgez_v, edgey_w), ff
+// (rho, rhoE), (rhoY_0, rhoY_1), ... with a last odd component by itself (fl).
+template <int NS, class R, bool PACK>
+struct StageScratch {
+    Arr4<R> ct, et;
+    Arr4<double> ff[3], me;
+    FHD_D void put_ct(int i, int j, int k, int d, R s, R dd) const {
+        ct(i, j, k, d) = s;
+        ct(i, j, k, 3 + d) = dd;
+    }
+    FHD_D void put_et(int E, int i, int j, int k, const Taus<R>& t) const {
+        et(i, j, k, 2 * E) = t.s;
+        et(i, j, k, 2 * E + 1) = t.d;
+    }
+    // component of edgeflux_x[0..1], _y, _z that total q of edge E is
+    static FHD_D int me_comp(int E, int q) { return q == 0 ? (E == 0 ? 2 : (E == 1 ? 4 : 5)) : (E == 0 ? 0 : (E == 1 ? 1 : 3)); }
+    FHD_D bool has_me() const { return me.p != nullptr; }
+    FHD_D void put_me(int E, int i, int j, int k, double va, double vb) const {
+        me(i, j, k, me_comp(E, 0)) = va;
+        me(i, j, k, me_comp(E, 1)) = vb;
+    }
+    FHD_D double get_me(int E, int q, int i, int j, int k) const { return me(i, j, k, me_comp(E, q)); }
+    FHD_D bool has_ff(int d) const { return ff[d].p != nullptr; }
+    FHD_D void put_ff(int d, int i, int j, int k, const double (&f)[2 + NS]) const {
+#pragma unroll
+        for (int c = 0; c < 2 + NS; ++c) ff[d](i, j, k, c) = f[c];
+    }
+    // Fluxes in words: word w holds components cw .. cw + n - 1 (n = 1, PACK 2); their
+    // differences of the faces above and below (i, j, k) in direction d
+    static constexpr int NW = 2 + NS;
+    static FHD_D int first(int w) { return w; }
+    static FHD_D int count(int) { return 1; }
+    FHD_D void ff_diff(int w, int d, int i, int j, int k, double (&f)[2]) const {
+        f[0] = ff[d](i + (d == 0), j + (d == 1), k + (d == 2), w) - ff[d](i, j, k, w);
+    }
+};
+template <int NS, class R>
+struct StageScratch<NS, R, true> {
+    static constexpr int NP = (2 + NS) / 2;     // whole words of a face's fluxes
+    Arr4<Pair<R>> ct, et;
+    Arr4<double2> ff[3], me;
+    Arr4<double> fl[3];
+    FHD_D void put_ct(int i, int j, int k, int d, R s, R dd) const { ct(i, j, k, d) = pmake(s, dd); }
+    FHD_D void put_et(int E, int i, int j, int k, const Taus<R>& t) const { et(i, j, k, E) = pmake(t.s, t.d); }
+    FHD_D bool has_me() const { return true; }
+    FHD_D void put_me(int E, int i, int j, int k, double va, double vb) const { me(i, j, k, E) = make_double2(va, vb); }
+    FHD_D double get_me(int E, int q, int i, int j, int k) const {
+        const double2& v = me(i, j, k, E);
+        return q ? v.y : v.x;
+    }
+    FHD_D bool has_ff(int) const { return true; }
+    FHD_D void put_ff(int d, int i, int j, int k, const double (&f)[2 + NS]) const {
+#pragma unroll
+        for (int c = 0; c < NP; ++c) ff[d](i, j, k, c) = make_double2(f[2 * c], f[2 * c + 1]);
+        if constexpr (NS % 2) fl[d](i, j, k) = f[1 + NS];
+    }
+    static constexpr int NW = NP + NS % 2;
+    static FHD_D int first(int w) { return 2 * w; }
+    static FHD_D int count(int w) { return w < NP ? 2 : 1; }
+    FHD_D void ff_diff(int w, int d, int i, int j, int k, double (&f)[2]) const {
+        const int ip = i + (d == 0), jp = j + (d == 1), kp = k + (d == 2);
+        if (w < NP) {
+            const double2 h = ff[d](ip, jp, kp, w), l = ff[d](i, j, k, w);
+            f[0] = h.x - l.x;
+            f[1] = h.y - l.y;
+        } else {
+            f[0] = fl[d](ip, jp, kp) - fl[d](i, j, k);
+        }
+    }
+};
+
 // What the face kernel reads, as one pointer per component at point (0,0,0) of its
 // fab and the strides of the fabs: an operand is then pointer + offset, with the
-// offset shared by the components of a fab.
-template <int NS, class R>
+// offset shared by the components of a fab.  FaceDir: what depends on the face
+// direction (the same code serves the three).
+template <int NS, class R, bool PACK>
 struct FaceIn {
     const double *T, *p, *Y[NS], *X[NS];          // prim
     const double *E, *rY[NS];                     // cons 4, 5..
@@ -142,45 +256,47 @@ struct FaceIn {
     int psy, psz, csy, csz, ksy, ksz, hsy, hsz, dsy, dsz;   // prim, cons, kappa, chi, D
     int tsy, tsz, esy, esz;                       // ct, et
 };
-// ... and what depends on the face direction: the same code serves the three
 template <int NS, class R>
+struct FaceIn<NS, R, true> {
+    const double *T, *p, *Y[NS];                  // prim, for the hyperbolic part
+    const double *E, *rY[NS];
+    int psy, psz, csy, csz, tsy, tsz, esy, esz;
+};
+template <int NS, class R, bool PACK>
 struct FaceDir {
     const double *u, *m;                          // vel[d], mom[d]
     int usy, usz, msy, msz;
-    const R *cs, *cd;                             // ct comps d, 3 + d
+    const std::conditional_t<PACK, Pair<R>, R>*cs, *cd;   // ct comps d, 3 + d (PACK: cs the pair)
     struct Family {                               // edge family f (first, second transverse direction)
-        const R *s, *d;                           // et comps (s, d)
+        const std::conditional_t<PACK, Pair<R>, R>*s, *d; // et comps (s, d) (PACK: s the pair)
         const double* v;                          // transverse velocity
         int eq, vsy, vsz, vq, vd;                 // et: step to position 1; v: strides, steps to position 1 and across the face
     } f[2];
-    int pd, cd_, kd, hd, dd, td;                  // steps across the face in prim, cons, kappa, chi, D, ct
-    double* ff[2 + NS];                           // rho, rhoE, rhoY fluxes
-    int fsy, fsz;
+    int pd, cd_, kd, hd, dd, td, qd;              // steps across the face in prim, cons, kappa, chi, D, ct, records
     Items it;
 };
 
-template <int NS, class R, int NZ>
+template <int NS, class R, int NZ, bool PACK = false>
 struct alignas(16) StageArgs {
     RunParams P;
-    Fields<NS, R> F;             // stage-input state U^s + derived fields
+    std::conditional_t<PACK, FieldsPack<NS, R>, Fields<NS, R>> F;   // stage-input state U^s + derived fields
     Noise<NZ> noise;
-    Arr4<R> ct, et;
-    Arr4<double> ff[3];
-    Arr4<double> mc, me;
+    StageScratch<NS, R, PACK> S;
+    Arr4<double> mc;
     Arr4<const double> cons0;    // U^0 (for the RK combination)
     Arr4<const double> mom0[3];
     Arr4<double> cons_o;         // U^{s+1}
     Arr4<double> mom_o[3];
     Arr4<const double> src;      // source (nprimvars comps) or p == nullptr
-    FaceIn<NS, R> fi;
-    FaceDir<NS, R> fd[3];
+    FaceIn<NS, R, PACK> fi;
+    FaceDir<NS, R, PACK> fd[3];
     Items it_taus, it_upd;       // cells [-1, n]^3, points [0, n]^3
     int stage;                   // 1, 2, 3
 };
 
 // stresses on cells (grown by 1) and edges; one thread per point of [-1, n]^3
-template <int NS, class R, int NZ>
-FHD_D int taus_count(const StageArgs<NS, R, NZ>& a) { return a.it_taus.n; }
+template <int NS, class R, int NZ, bool PACK>
+FHD_D int taus_count(const StageArgs<NS, R, NZ, PACK>& a) { return a.it_taus.n; }
 
 // The flux MultiFabs of a caller that wants them (the reference's by-products, and the
 // flux operator's outputs): the stress kernel has every edge and centre total and the
@@ -196,93 +312,82 @@ struct StageAux {
 template <>
 struct StageAux<false> {};
 
-// both edge totals of an edge into the stage's scratch (absent: the flux operator) and
-// the flux fabs; ca, cb: their components in the order edgeflux_x, _y, _z
-template <int NS, class R, int NZ, bool AUX>
-FHD_D void put_edge(const StageArgs<NS, R, NZ>& a, const StageAux<AUX>& x, int i, int j, int k, int ca, double va,
-                    int cb, double vb) {
-    if (!AUX || a.me.p) {
-        a.me(i, j, k, ca) = va;
-        a.me(i, j, k, cb) = vb;
-    }
+// both edge totals of edge E into the stage's scratch (absent: the flux operator) and
+// the flux fabs
+template <int E, bool AUX, class A>
+FHD_D void put_edge(const A& a, const StageAux<AUX>& x, int i, int j, int k, double va, double vb) {
+    if (!AUX || a.S.has_me()) a.S.put_me(E, i, j, k, va, vb);
     if constexpr (AUX) {
+        constexpr int ca = E == 0 ? 2 : (E == 1 ? 4 : 5), cb = E == 0 ? 0 : (E == 1 ? 1 : 3);
         x.ef[ca](i, j, k) = va;
         x.ef[cb](i, j, k) = vb;
     }
 }
 
-// WL: walls (the wall variants of the edge stresses, advective edge fluxes and
-// StochFluxStag's factors on the edge totals)
-template <int NS, class R, int NZ, bool WL = false, bool AUX = false>
-FHD_D void taus_point(const StageArgs<NS, R, NZ>& a, int q, const StageAux<AUX>& x = StageAux<AUX>()) {
+// stress and edge totals of edge E at point (i, j, k)
+template <int NS, class R, int NZ, int E, bool WL, bool AUX, bool PACK>
+FHD_D void taus_edge(const StageArgs<NS, R, NZ, PACK>& a, const StageAux<AUX>& x, double w, int i, int j, int k) {
     const RunParams& P = a.P;
-    {
-        int i, j, k;
-        a.it_taus.point(q, i, j, k);
-        --i; --j; --k;
-        const bool edges = i >= 0 && j >= 0 && k >= 0;
-        double wc[3] = {0.0, 0.0, 0.0}, we[3] = {0.0, 0.0, 0.0};
-        if (NZ != NZ_OFF) a.noise.cen_and_yz_edge(P, i, j, k, edges, wc, we[2]);
-        const CellTaus<R> t = cell_taus_w<NS, R, NZ, WL>(P, a.F, wc, i, j, k);
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            a.ct(i, j, k, d) = t.s[d];
-            a.ct(i, j, k, 3 + d) = t.d[d];
-            const double c = cen_total_res<NS, R, NZ, WL>(P, a.F, a.noise, t, d, i, j, k);
-            if (!AUX || a.mc.p) a.mc(i, j, k, d) = c;
-            if constexpr (AUX) x.cf[d](i, j, k) = c;
-        }
-        if (!edges) return;
-        if (NZ != NZ_OFF) a.noise.xy_xz_edges(P, i, j, k, we[0], we[1]);
-        const int hadv = P.advection_type >= 0;
-        double ea, eb;
-        if (k < P.n[2]) {
-            const Taus<R> e = edge_taus_w<NS, R, NZ, 0, WL>(P, a.F, we[0], i, j, k);
-            a.et(i, j, k, 0) = e.s;
-            a.et(i, j, k, 1) = e.d;
-            edge_adv<NS, R, 0, WL>(P, a.F, i, j, k, ea, eb);
-            put_edge(a, x, i, j, k, 2, WL ? edge_total_w<R, 0>(P, e, ea, hadv, i, j, k) : edge_total<R>(e, ea, hadv),  // edgey_u
-                     0, WL ? edge_total_w<R, 0>(P, e, eb, hadv, i, j, k) : edge_total<R>(e, eb, hadv));         // edgex_v
-        }
-        if (j < P.n[1]) {
-            const Taus<R> e = edge_taus_w<NS, R, NZ, 1, WL>(P, a.F, we[1], i, j, k);
-            a.et(i, j, k, 2) = e.s;
-            a.et(i, j, k, 3) = e.d;
-            edge_adv<NS, R, 1, WL>(P, a.F, i, j, k, ea, eb);
-            put_edge(a, x, i, j, k, 4, WL ? edge_total_w<R, 1>(P, e, ea, hadv, i, j, k) : edge_total<R>(e, ea, hadv),  // edgez_u
-                     1, WL ? edge_total_w<R, 1>(P, e, eb, hadv, i, j, k) : edge_total<R>(e, eb, hadv));         // edgex_w
-        }
-        if (i < P.n[0]) {
-            const Taus<R> e = edge_taus_w<NS, R, NZ, 2, WL>(P, a.F, we[2], i, j, k);
-            a.et(i, j, k, 4) = e.s;
-            a.et(i, j, k, 5) = e.d;
-            edge_adv<NS, R, 2, WL>(P, a.F, i, j, k, ea, eb);
-            put_edge(a, x, i, j, k, 5, WL ? edge_total_w<R, 2>(P, e, ea, hadv, i, j, k) : edge_total<R>(e, ea, hadv),  // edgez_v
-                     3, WL ? edge_total_w<R, 2>(P, e, eb, hadv, i, j, k) : edge_total<R>(e, eb, hadv));         // edgey_w
-        }
-    }
+    const int hadv = P.advection_type >= 0;
+    const Taus<R> e = edge_taus_w<NS, R, NZ, E, WL>(P, a.F, w, i, j, k);
+    a.S.put_et(E, i, j, k, e);
+    double ea, eb;
+    edge_adv<NS, R, E, WL>(P, a.F, i, j, k, ea, eb);
+    put_edge<E>(a, x, i, j, k, WL ? edge_total_w<R, E>(P, e, ea, hadv, i, j, k) : edge_total<R>(e, ea, hadv),
+                WL ? edge_total_w<R, E>(P, e, eb, hadv, i, j, k) : edge_total<R>(e, eb, hadv));
 }
 
-template <int NS, class R, int NZ, bool WL = false, bool AUX = false>
-static __global__ void __launch_bounds__(256) k_taus(StageArgs<NS, R, NZ> a, StageAux<AUX> x) {
+// WL: walls (the wall variants of the edge stresses, advective edge fluxes and
+// StochFluxStag's factors on the edge totals)
+template <int NS, class R, int NZ, bool WL = false, bool AUX = false, bool PACK = false>
+FHD_D void taus_point(const StageArgs<NS, R, NZ, PACK>& a, int q, const StageAux<AUX>& x = StageAux<AUX>()) {
+    const RunParams& P = a.P;
+    int i, j, k;
+    a.it_taus.point(q, i, j, k);
+    --i; --j; --k;
+    const bool edges = i >= 0 && j >= 0 && k >= 0;
+    double wc[3] = {0.0, 0.0, 0.0}, we[3] = {0.0, 0.0, 0.0};
+    if (NZ != NZ_OFF) a.noise.cen_and_yz_edge(P, i, j, k, edges, wc, we[2]);
+    const CellTaus<R> t = cell_taus_w<NS, R, NZ, WL>(P, a.F, wc, i, j, k);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        a.S.put_ct(i, j, k, d, t.s[d], t.d[d]);
+        const double c = cen_total_res<NS, R, NZ, WL>(P, a.F, a.noise, t, d, i, j, k);
+        if (!AUX || a.mc.p) a.mc(i, j, k, d) = c;
+        if constexpr (AUX) x.cf[d](i, j, k) = c;
+    }
+    if (!edges) return;
+    if (NZ != NZ_OFF) a.noise.xy_xz_edges(P, i, j, k, we[0], we[1]);
+    if (k < P.n[2]) taus_edge<NS, R, NZ, 0, WL>(a, x, we[0], i, j, k);
+    if (j < P.n[1]) taus_edge<NS, R, NZ, 1, WL>(a, x, we[1], i, j, k);
+    if (i < P.n[0]) taus_edge<NS, R, NZ, 2, WL>(a, x, we[2], i, j, k);
+}
+
+template <int NS, class R, int NZ, bool WL = false, bool AUX = false, bool PACK = false>
+static __global__ void __launch_bounds__(256) k_taus(StageArgs<NS, R, NZ, PACK> a, StageAux<AUX> x) {
     const int tot = taus_count(a);
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < tot; q += gridDim.x * blockDim.x)
         taus_point<NS, R, NZ, WL, AUX>(a, q, x);
 }
 
 // operands of one face of a direction known only at run time (face_flux)
-template <int NS, class R, int NZ>
+template <int NS, class R, int NZ, bool PACK>
 struct FaceRun {
-    const StageArgs<NS, R, NZ>& a;
-    int d, op, oc, ok, oh, od, ot, oe, ou, om, ov[2];
-    FHD_D FaceRun(const StageArgs<NS, R, NZ>& a_, int d_, int i, int j, int k) : a(a_), d(d_) {
-        const FaceIn<NS, R>& fi = a.fi;
-        const FaceDir<NS, R>& f = a.fd[d];
+    using L = RecLayout<NS, R>;
+    const StageArgs<NS, R, NZ, PACK>& a;
+    int d, op, oc, ok, oh, od, ot, oe, ou, om, ov[2];   // (ok: records when PACK)
+    FHD_D FaceRun(const StageArgs<NS, R, NZ, PACK>& a_, int d_, int i, int j, int k) : a(a_), d(d_) {
+        const auto& fi = a.fi;
+        const auto& f = a.fd[d];
         op = i + j * fi.psy + k * fi.psz;
         oc = i + j * fi.csy + k * fi.csz;
-        ok = i + j * fi.ksy + k * fi.ksz;
-        oh = i + j * fi.hsy + k * fi.hsz;
-        od = i + j * fi.dsy + k * fi.dsz;
+        if constexpr (PACK) {
+            ok = a.F.q.at(i, j, k);
+        } else {
+            ok = i + j * fi.ksy + k * fi.ksz;
+            oh = i + j * fi.hsy + k * fi.hsz;
+            od = i + j * fi.dsy + k * fi.dsz;
+        }
         ot = i + j * fi.tsy + k * fi.tsz;
         oe = i + j * fi.esy + k * fi.esz;
         ou = i + j * f.usy + k * f.usz;
@@ -290,35 +395,76 @@ struct FaceRun {
         ov[0] = i + j * f.f[0].vsy + k * f.f[0].vsz;
         ov[1] = i + j * f.f[1].vsy + k * f.f[1].vsz;
     }
-    FHD_D const FaceDir<NS, R>& f() const { return a.fd[d]; }
+    FHD_D const FaceDir<NS, R, PACK>& f() const { return a.fd[d]; }
     FHD_D int dir() const { return d; }
-    FHD_D double T(int s) const { return a.fi.T[s ? op : op - f().pd]; }
-    FHD_D double p(int s) const { return a.fi.p[s ? op : op - f().pd]; }
-    FHD_D double Y(int s, int n) const { return a.fi.Y[n][s ? op : op - f().pd]; }
-    FHD_D double X(int s, int n) const { return a.fi.X[n][s ? op : op - f().pd]; }
+    FHD_D R rec(int s, int c) const { return a.F.q.get(s ? ok : ok - f().qd, c); }
+    FHD_D auto T(int s) const {
+        if constexpr (PACK) return rec(s, L::T);
+        else return a.fi.T[s ? op : op - f().pd];
+    }
+    FHD_D auto p(int s) const {
+        if constexpr (PACK) return rec(s, L::PR);
+        else return a.fi.p[s ? op : op - f().pd];
+    }
+    FHD_D auto Y(int s, int n) const {
+        if constexpr (PACK) return rec(s, L::Y + n);
+        else return a.fi.Y[n][s ? op : op - f().pd];
+    }
+    FHD_D auto X(int s, int n) const {
+        if constexpr (PACK) return rec(s, L::X + n);
+        else return a.fi.X[n][s ? op : op - f().pd];
+    }
+    // T, p and Y in FP64 for the hyperbolic part
+    FHD_D double Td(int s) const { return a.fi.T[s ? op : op - f().pd]; }
+    FHD_D double pd(int s) const {
+        if constexpr (PACK && sizeof(R) == 8) return rec(s, L::PR);
+        else return a.fi.p[s ? op : op - f().pd];
+    }
+    FHD_D double Yd(int s, int n) const { return a.fi.Y[n][s ? op : op - f().pd]; }
     FHD_D double cons(int s, int n) const {
         const int o = s ? oc : oc - f().cd_;
         if (n == 4) return a.fi.E[o];
         if (n >= 5) return a.fi.rY[n - 5][o];
         return a.F.cons.p[o];
     }
-    FHD_D R kappa(int s) const { return a.fi.kappa[s ? ok : ok - f().kd]; }
-    FHD_D R chi(int s, int n) const { return a.fi.chi[n][s ? oh : oh - f().hd]; }
-    FHD_D R Dc(int s, int n) const { return a.fi.D[n][s ? od : od - f().dd]; }
+    FHD_D R kappa(int s) const {
+        if constexpr (PACK) return rec(s, L::KAPPA);
+        else return a.fi.kappa[s ? ok : ok - f().kd];
+    }
+    FHD_D R chi(int s, int n) const {
+        if constexpr (PACK) return rec(s, L::CHI + n);
+        else return a.fi.chi[n][s ? oh : oh - f().hd];
+    }
+    FHD_D R Dc(int s, int n) const {
+        if constexpr (PACK) return rec(s, L::D + n);
+        else return a.fi.D[n][s ? od : od - f().dd];
+    }
     FHD_D double u() const { return f().u[ou]; }
     FHD_D double m() const { return f().m[om]; }
     FHD_D Taus<R> cell(int s) const {
         const int o = s ? ot : ot - f().td;
         Taus<R> t;
-        t.s = f().cs[o];
-        t.d = f().cd[o];
+        if constexpr (PACK) {
+            const Pair<R> v = f().cs[o];
+            t.s = v.x;
+            t.d = v.y;
+        } else {
+            t.s = f().cs[o];
+            t.d = f().cd[o];
+        }
         return t;
     }
     FHD_D Taus<R> edge(int q, int pos) const {
         const int o = pos ? oe + f().f[q].eq : oe;
         Taus<R> t;
-        t.s = f().f[q].s[o];
-        t.d = f().f[q].d[o];
+        if constexpr (PACK) {
+            const Pair<R> v = f().f[q].s[o];
+            t.s = v.x;
+            t.d = v.y;
+        } else {
+            t.s = f().f[q].s[o];
+            t.d = f().f[q].d[o];
+        }
         return t;
     }
     FHD_D double vt(int q, int pos, int s) const {
@@ -327,21 +473,17 @@ struct FaceRun {
     }
 };
 
-template <int NS, class R, int NZ>
-FHD_D int faces_count(const StageArgs<NS, R, NZ>& a, int d) { return a.fd[d].it.n; }
+template <int NS, class R, int NZ, bool PACK>
+FHD_D int faces_count(const StageArgs<NS, R, NZ, PACK>& a, int d) { return a.fd[d].it.n; }
 
 // conservative flux of face q of direction d
-template <int NS, class R, int NZ, bool WL = false, bool AUX = false>
-FHD_D void faces_point(const StageArgs<NS, R, NZ>& a, int d, int q, const StageAux<AUX>& aux = StageAux<AUX>()) {
+template <int NS, class R, int NZ, bool WL = false, bool AUX = false, bool PACK = false>
+FHD_D void faces_point(const StageArgs<NS, R, NZ, PACK>& a, int d, int q, const StageAux<AUX>& aux = StageAux<AUX>()) {
     int i, j, k;
     a.fd[d].it.point(q, i, j, k);
-    const FaceRun<NS, R, NZ> x(a, d, i, j, k);
+    const FaceRun<NS, R, NZ, PACK> x(a, d, i, j, k);
     const FaceFlux<NS> f = face_flux<NS, R, NZ, WL>(a.P, a.F, a.noise, x, i, j, k);
-    if (!AUX || a.ff[d].p) {
-        const int o = i + j * a.fd[d].fsy + k * a.fd[d].fsz;
-#pragma unroll
-        for (int c = 0; c < 2 + NS; ++c) a.fd[d].ff[c][o] = f.cons[c];
-    }
+    if (!AUX || a.S.has_ff(d)) a.S.put_ff(d, i, j, k, f.cons);
     if constexpr (AUX) {
         const Arr4<double>& o = aux.ff[d];
         o(i, j, k, 0) = f.cons[0];
@@ -361,8 +503,8 @@ FHD_D void faces_point(const StageArgs<NS, R, NZ>& a, int d, int q, const StageA
 // the second and third find them in L2, and a small box keeps three times as many SMs
 // busy as one launch per direction.
 // MINB = minimum resident blocks requested from the register allocator.
-template <int NS, class R, int NZ, int BS, int MINB, bool WL = false, bool AUX = false>
-static __global__ void __launch_bounds__(BS, MINB) k_faces(StageArgs<NS, R, NZ> a, int per, StageAux<AUX> x) {
+template <int NS, class R, int NZ, int BS, int MINB, bool WL = false, bool AUX = false, bool PACK = false>
+static __global__ void __launch_bounds__(BS, MINB) k_faces(StageArgs<NS, R, NZ, PACK> a, int per, StageAux<AUX> x) {
     const int d = blockIdx.x % 3;
     const int tot = faces_count(a, d);
     for (int q = (blockIdx.x / 3) * BS + threadIdx.x; q < tot; q += per * BS)
@@ -371,13 +513,13 @@ static __global__ void __launch_bounds__(BS, MINB) k_faces(StageArgs<NS, R, NZ> 
 
 // RK3 stage combination (timeStepStag.cpp:439-528, 771-861, 1106-1202): one thread
 // per point of [0, n]^3 updates the cell there (if valid) and the faces there
-template <int NS, class R, int NZ>
-FHD_D int update_count(const StageArgs<NS, R, NZ>& a) { return a.it_upd.n; }
+template <int NS, class R, int NZ, bool PACK>
+FHD_D int update_count(const StageArgs<NS, R, NZ, PACK>& a) { return a.it_upd.n; }
 
-template <int NS, class R, int NZ>
-FHD_D void update_point(const StageArgs<NS, R, NZ>& a, int q) {
+template <int NS, class R, int NZ, bool PACK>
+FHD_D void update_point(const StageArgs<NS, R, NZ, PACK>& a, int q) {
     const RunParams& P = a.P;
-    const Fields<NS, R>& F = a.F;
+    const auto& F = a.F;
     const double dt = P.dt;
     const int st = a.stage;
     {
@@ -385,20 +527,28 @@ FHD_D void update_point(const StageArgs<NS, R, NZ>& a, int q) {
         a.it_upd.point(q, i, j, k);
         const bool cell = i < P.n[0] && j < P.n[1] && k < P.n[2];
         if (cell) {
+            using S = std::remove_const_t<std::remove_reference_t<decltype(a.S)>>;
             double on[2 + NS];
 #pragma unroll
-            for (int c = 0; c < 2 + NS; ++c) {
-                const int n = (c == 0) ? 0 : 3 + c;  // conserved component index
-                const double div = divc(P, a.ff[0](i + 1, j, k, c) - a.ff[0](i, j, k, c), P.dx[0], P.rdx[0]) +
-                                   divc(P, a.ff[1](i, j + 1, k, c) - a.ff[1](i, j, k, c), P.dx[1], P.rdx[1]) +
-                                   divc(P, a.ff[2](i, j, k + 1, c) - a.ff[2](i, j, k, c), P.dx[2], P.rdx[2]);
-                const double src = a.src.p ? a.src(i, j, k, n) : 0.0;
-                const double u0 = a.cons0(i, j, k, n);
-                double v;
-                if (st == 1) v = u0 - dt * (div) + dt * src;
-                else if (st == 2) v = 0.25 * (3.0 * u0 + F.cons(i, j, k, n) - dt * (div) + dt * src);
-                else v = (2. / 3.) * (0.5 * u0 + F.cons(i, j, k, n) - dt * (div) + dt * src);
-                on[c] = v;
+            for (int w = 0; w < S::NW; ++w) {
+                double fx[2], fy[2], fz[2];
+                a.S.ff_diff(w, 0, i, j, k, fx);
+                a.S.ff_diff(w, 1, i, j, k, fy);
+                a.S.ff_diff(w, 2, i, j, k, fz);
+#pragma unroll
+                for (int e = 0; e < S::count(w); ++e) {
+                    const int c = S::first(w) + e;
+                    const int n = (c == 0) ? 0 : 3 + c;  // conserved component index
+                    const double div = divc(P, fx[e], P.dx[0], P.rdx[0]) + divc(P, fy[e], P.dx[1], P.rdx[1]) +
+                                       divc(P, fz[e], P.dx[2], P.rdx[2]);
+                    const double src = a.src.p ? a.src(i, j, k, n) : 0.0;
+                    const double u0 = a.cons0(i, j, k, n);
+                    double v;
+                    if (st == 1) v = u0 - dt * (div) + dt * src;
+                    else if (st == 2) v = 0.25 * (3.0 * u0 + F.cons(i, j, k, n) - dt * (div) + dt * src);
+                    else v = (2. / 3.) * (0.5 * u0 + F.cons(i, j, k, n) - dt * (div) + dt * src);
+                    on[c] = v;
+                }
             }
             // gravity work on the energy with the stage-input momenta
             const double gfac = (st == 1) ? 0.5 * dt : (st == 2) ? 0.5 * 0.25 * dt : 0.5 * (2. / 3.) * dt;
@@ -417,15 +567,15 @@ FHD_D void update_point(const StageArgs<NS, R, NZ>& a, int q) {
             double t1, t2, t3;
             if (d == 0) {
                 t1 = a.mc(i, j, k, 0) - a.mc(i - 1, j, k, 0);
-                t2 = a.me(i, j + 1, k, 2) - a.me(i, j, k, 2);   // edgey_u
-                t3 = a.me(i, j, k + 1, 4) - a.me(i, j, k, 4);   // edgez_u
+                t2 = a.S.get_me(0, 0, i, j + 1, k) - a.S.get_me(0, 0, i, j, k);   // edgey_u
+                t3 = a.S.get_me(1, 0, i, j, k + 1) - a.S.get_me(1, 0, i, j, k);   // edgez_u
             } else if (d == 1) {
-                t1 = a.me(i + 1, j, k, 0) - a.me(i, j, k, 0);   // edgex_v
+                t1 = a.S.get_me(0, 1, i + 1, j, k) - a.S.get_me(0, 1, i, j, k);   // edgex_v
                 t2 = a.mc(i, j, k, 1) - a.mc(i, j - 1, k, 1);
-                t3 = a.me(i, j, k + 1, 5) - a.me(i, j, k, 5);   // edgez_v
+                t3 = a.S.get_me(2, 0, i, j, k + 1) - a.S.get_me(2, 0, i, j, k);   // edgez_v
             } else {
-                t1 = a.me(i + 1, j, k, 1) - a.me(i, j, k, 1);   // edgex_w
-                t2 = a.me(i, j + 1, k, 3) - a.me(i, j, k, 3);   // edgey_w
+                t1 = a.S.get_me(1, 1, i + 1, j, k) - a.S.get_me(1, 1, i, j, k);   // edgex_w
+                t2 = a.S.get_me(2, 1, i, j + 1, k) - a.S.get_me(2, 1, i, j, k);   // edgey_w
                 t3 = a.mc(i, j, k, 2) - a.mc(i, j, k - 1, 2);
             }
             const double rsum = F.cons(i - e0, j - e1, k - e2, 0) + F.cons(i, j, k, 0);
@@ -448,11 +598,11 @@ FHD_D void update_point(const StageArgs<NS, R, NZ>& a, int q) {
     }
 }
 
-// MINB: 16 blocks of 128 (32 registers, full occupancy) where the kernel streams from
-// HBM; 4 for a box that fits one wave of them, where a point's loads cost its time and
-// more registers put more of them in flight (update_blocks)
-template <int NS, class R, int NZ, int MINB>
-static __global__ void __launch_bounds__(128, MINB) k_update(StageArgs<NS, R, NZ> a) {
+// MINB: 16 blocks of 128 (32 registers, full occupancy; packed 12 or 10) where the kernel
+// streams from HBM; 4 for a box that fits one wave of them, where a point's loads cost
+// its time and more registers put more of them in flight (launch_update)
+template <int NS, class R, int NZ, int MINB, bool PACK>
+static __global__ void __launch_bounds__(128, MINB) k_update(StageArgs<NS, R, NZ, PACK> a) {
     const int tot = update_count(a);
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < tot; q += gridDim.x * blockDim.x) update_point(a, q);
 }
@@ -915,10 +1065,10 @@ static __global__ void __launch_bounds__(128, cellprep_min_blocks<NS, R>()) k_ce
 
 // 64 registers (8 blocks of 128 per SM): uncapped, the FP32 kernel took 96 and ran 20 warps per SM
 template <int NS, class R, int NZ>
-static __global__ void __launch_bounds__(128, 8) k_taus_b(const StageArgs<NS, R, NZ>* __restrict__ args,
+static __global__ void __launch_bounds__(128, 8) k_taus_b(const StageArgs<NS, R, NZ, true>* __restrict__ args,
                                                 const int* __restrict__ bpref, int nmem) {
     const int m = member_of(bpref, nmem);
-    const StageArgs<NS, R, NZ>& a = member_args(args, m);
+    const StageArgs<NS, R, NZ, true>& a = member_args(args, m);
     const int q = (blockIdx.x - bpref[m]) * blockDim.x + threadIdx.x;
     if (q < taus_count(a)) taus_point(a, q);
 }
@@ -926,20 +1076,20 @@ static __global__ void __launch_bounds__(128, 8) k_taus_b(const StageArgs<NS, R,
 // Register cap of the batched face kernel: MINB resident blocks of 128 threads
 // (8: 64 registers, 6: 80, 4: 128), picked per batch by its autotuner.
 template <int NS, class R, int NZ, int MINB>
-static __global__ void __launch_bounds__(128, MINB) k_faces_b(const StageArgs<NS, R, NZ>* __restrict__ args,
+static __global__ void __launch_bounds__(128, MINB) k_faces_b(const StageArgs<NS, R, NZ, true>* __restrict__ args,
                                                    const int* __restrict__ bpref, int nmem, int d) {
     const int m = member_of(bpref, nmem);
-    const StageArgs<NS, R, NZ>& a = member_args(args, m);
+    const StageArgs<NS, R, NZ, true>& a = member_args(args, m);
     const int q = (blockIdx.x - bpref[m]) * blockDim.x + threadIdx.x;
     if (q < faces_count(a, d)) faces_point(a, d, q);
 }
 
-// 48 registers (10 blocks per SM; the single-run kernel's 32 spill here)
+// 64 registers (8 blocks per SM; fewer spill)
 template <int NS, class R, int NZ>
-static __global__ void __launch_bounds__(128, 10) k_update_b(const StageArgs<NS, R, NZ>* __restrict__ args,
+static __global__ void __launch_bounds__(128, 8) k_update_b(const StageArgs<NS, R, NZ, true>* __restrict__ args,
                                                   const int* __restrict__ bpref, int nmem) {
     const int m = member_of(bpref, nmem);
-    const StageArgs<NS, R, NZ>& a = member_args(args, m);
+    const StageArgs<NS, R, NZ, true>& a = member_args(args, m);
     const int q = (blockIdx.x - bpref[m]) * blockDim.x + threadIdx.x;
     if (q < update_count(a)) update_point(a, q);
 }
@@ -1002,7 +1152,7 @@ FHD_D int wait_phase(const PersistArgs& a, int m, int p) {
 
 template <int NS, class R, int NZ>
 struct PersistBytes {
-    static constexpr size_t a = sizeof(PrepArgs<NS, R>), b = sizeof(StageArgs<NS, R, NZ>), c = sizeof(ConvArgs<NS>),
+    static constexpr size_t a = sizeof(PrepArgs<NS, R>), b = sizeof(StageArgs<NS, R, NZ, true>), c = sizeof(ConvArgs<NS>),
                             d = sizeof(GhostFab);
     static constexpr size_t m1 = a > b ? a : b, m2 = c > d ? c : d;
     static constexpr size_t value = ((m1 > m2 ? m1 : m2) + 7) / 8 * 8;
@@ -1043,7 +1193,7 @@ static __global__ void __launch_bounds__(128, MINB) k_batch_persist(PersistArgs 
             if (kind != PK_STEP) {
                 const size_t bytes = kind == PK_PREP ? sizeof(PrepArgs<NS, R>)
                                      : kind == PK_CONVERT ? sizeof(ConvArgs<NS>)
-                                     : kind == PK_GHOST ? sizeof(GhostFab) : sizeof(StageArgs<NS, R, NZ>);
+                                     : kind == PK_GHOST ? sizeof(GhostFab) : sizeof(StageArgs<NS, R, NZ, true>);
                 const unsigned long long* src = static_cast<const unsigned long long*>(pu.args);
                 for (int w = threadIdx.x; w < (int)((bytes + 7) / 8); w += blockDim.x) sbuf[w] = src[w];
             }
@@ -1058,23 +1208,23 @@ static __global__ void __launch_bounds__(128, MINB) k_batch_persist(PersistArgs 
                     for (int64_t x = q; x < q1; x += st) cellprep_point(A, (int)x);
                 } break;
                 case PK_TAUS: {
-                    const auto& A = *reinterpret_cast<const StageArgs<NS, R, NZ>*>(sbuf);
+                    const auto& A = *reinterpret_cast<const StageArgs<NS, R, NZ, true>*>(sbuf);
                     for (int64_t x = q; x < q1; x += st) taus_point(A, (int)x);
                 } break;
                 case PK_FACEX: {
-                    const auto& A = *reinterpret_cast<const StageArgs<NS, R, NZ>*>(sbuf);
+                    const auto& A = *reinterpret_cast<const StageArgs<NS, R, NZ, true>*>(sbuf);
                     for (int64_t x = q; x < q1; x += st) faces_point(A, 0, (int)x);
                 } break;
                 case PK_FACEY: {
-                    const auto& A = *reinterpret_cast<const StageArgs<NS, R, NZ>*>(sbuf);
+                    const auto& A = *reinterpret_cast<const StageArgs<NS, R, NZ, true>*>(sbuf);
                     for (int64_t x = q; x < q1; x += st) faces_point(A, 1, (int)x);
                 } break;
                 case PK_FACEZ: {
-                    const auto& A = *reinterpret_cast<const StageArgs<NS, R, NZ>*>(sbuf);
+                    const auto& A = *reinterpret_cast<const StageArgs<NS, R, NZ, true>*>(sbuf);
                     for (int64_t x = q; x < q1; x += st) faces_point(A, 2, (int)x);
                 } break;
                 case PK_UPDATE: {
-                    const auto& A = *reinterpret_cast<const StageArgs<NS, R, NZ>*>(sbuf);
+                    const auto& A = *reinterpret_cast<const StageArgs<NS, R, NZ, true>*>(sbuf);
                     for (int64_t x = q; x < q1; x += st) update_point(A, (int)x);
                 } break;
                 case PK_CONVERT: {

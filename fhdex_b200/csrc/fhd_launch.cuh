@@ -101,6 +101,28 @@ Fields<NS, R> make_fields(const StageCall& c) {
     return F;
 }
 
+// the cell records of a packed stage (c.rec: their first word and geometry)
+template <int NS, class R>
+Rec<NS, R> make_rec(const StageCall& c) {
+    const Arr4<const Vec<R>> v = view<const Vec<R>>(c.rec);
+    return Rec<NS, R>{c.pack ? v.p : nullptr, v.sy, v.sz, v.sn};
+}
+
+template <int NS, class R>
+FieldsPack<NS, R> make_fields_pack(const StageCall& c) {
+    FieldsPack<NS, R> F;
+    F.q = make_rec<NS, R>(c);
+    F.cons = view<const double>(c.cons_s);
+    for (int d = 0; d < 3; ++d) {
+        F.mom[d] = view<const double>(c.mom_s[d]);
+        F.vel[d] = view<const double>(c.vel[d]);
+    }
+    F.pr = view<const double>(c.pr);
+    F.pT = c.pT;
+    F.zr = R(c.P.zeta_ratio);
+    return F;
+}
+
 template <int MODE>
 Noise<MODE> make_noise(const StageCall& c) {
     Noise<MODE> n;
@@ -119,7 +141,7 @@ Noise<MODE> make_noise(const StageCall& c) {
 }
 
 template <int NS, class R>
-int launch_cellprep(const StageCall& c) {
+PrepArgs<NS, R> make_prep_args(const StageCall& c) {
     PrepArgs<NS, R> a;
     a.P = c.P;
     a.cons = view<const double>(c.cons_s);
@@ -133,12 +155,24 @@ int launch_cellprep(const StageCall& c) {
     a.kappa = view<R>(c.kappa);
     a.chi = view<R>(c.chi);
     a.D = view<R>(c.D);
+    const Rec<NS, R> q = make_rec<NS, R>(c);
+    a.q = const_cast<Vec<R>*>(q.p);
+    a.qsy = q.sy;
+    a.qsz = q.sz;
+    a.qsn = q.sn;
+    a.prim = c.pack ? c.wprim : 2;
+    a.coef = c.pack ? c.wcoef : 1;
     a.it = make_items(c.P.n[0] + 3, c.P.n[1] + 3, c.P.n[2] + 3);
     a.status = c.status;
-    const int64_t tot = a.it.n;
+    return a;
+}
+
+template <int NS, class R>
+int launch_cellprep(const StageCall& c) {
+    const PrepArgs<NS, R> a = make_prep_args<NS, R>(c);
     // (an occupancy-sized grid was measured slower here: blocks beyond the resident
     // set rebalance this kernel's uneven per-cell cost)
-    k_cellprep<NS, R><<<grid_for(tot, 128), 128, 0, c.stream>>>(a);
+    k_cellprep<NS, R><<<grid_for(a.it.n, 128), 128, 0, c.stream>>>(a);
     return cuda_rc(cudaGetLastError());
 }
 
@@ -159,76 +193,96 @@ template <class T>
 int step_of(const Arr4<T>& a, int d) { return d == 0 ? 1 : (d == 1 ? a.sy : a.sz); }
 
 // the face kernel's operands from the stage's views
-template <int NS, class R, int NZ>
-void make_face_args(StageArgs<NS, R, NZ>& a, const int n[3]) {
-    const Fields<NS, R>& F = a.F;
-    FaceIn<NS, R>& f = a.fi;
+template <int NS, class R, int NZ, bool PACK>
+void make_face_args(StageArgs<NS, R, NZ, PACK>& a, const int n[3]) {
+    const auto& F = a.F;
+    auto& f = a.fi;
     // (a fab that the stage does not have has no views: its pointers stay null)
     auto comp = [](const auto& v, int c) { return v.p ? v.p + (int64_t)c * v.sn : nullptr; };
     f.T = comp(F.pr, F.pT);
     f.p = comp(F.pr, F.pT + 1);
     f.E = comp(F.cons, 4);
-    f.kappa = F.kappa.p;
     for (int s = 0; s < NS; ++s) {
         f.Y[s] = comp(F.pr, F.pT + 2 + s);
-        f.X[s] = comp(F.pr, F.pT + 2 + NS + s);
         f.rY[s] = comp(F.cons, 5 + s);
-        f.chi[s] = comp(F.chi, s);
     }
-    for (int s = 0; s < NS * NS; ++s) f.D[s] = comp(F.D, s);
     f.psy = F.pr.sy;    f.psz = F.pr.sz;
     f.csy = F.cons.sy;  f.csz = F.cons.sz;
-    f.ksy = F.kappa.sy; f.ksz = F.kappa.sz;
-    f.hsy = F.chi.sy;   f.hsz = F.chi.sz;
-    f.dsy = F.D.sy;     f.dsz = F.D.sz;
-    f.tsy = a.ct.sy;    f.tsz = a.ct.sz;
-    f.esy = a.et.sy;    f.esz = a.et.sz;
+    f.tsy = a.S.ct.sy;  f.tsz = a.S.ct.sz;
+    f.esy = a.S.et.sy;  f.esz = a.S.et.sz;
+    if constexpr (!PACK) {
+        f.kappa = F.kappa.p;
+        for (int s = 0; s < NS; ++s) {
+            f.X[s] = comp(F.pr, F.pT + 2 + NS + s);
+            f.chi[s] = comp(F.chi, s);
+        }
+        for (int s = 0; s < NS * NS; ++s) f.D[s] = comp(F.D, s);
+        f.ksy = F.kappa.sy; f.ksz = F.kappa.sz;
+        f.hsy = F.chi.sy;   f.hsz = F.chi.sz;
+        f.dsy = F.D.sy;     f.dsz = F.D.sz;
+    }
     for (int d = 0; d < 3; ++d) {
-        FaceDir<NS, R>& x = a.fd[d];
+        auto& x = a.fd[d];
         x.u = F.vel[d].p;  x.usy = F.vel[d].sy; x.usz = F.vel[d].sz;
         x.m = F.mom[d].p;  x.msy = F.mom[d].sy; x.msz = F.mom[d].sz;
-        x.cs = comp(a.ct, d);
-        x.cd = comp(a.ct, 3 + d);
-        x.td = step_of(a.ct, d);
+        x.cs = comp(a.S.ct, d);
+        x.cd = PACK ? nullptr : comp(a.S.ct, 3 + d);
+        x.td = step_of(a.S.ct, d);
         x.pd = step_of(F.pr, d);
         x.cd_ = step_of(F.cons, d);
-        x.kd = step_of(F.kappa, d);
-        x.hd = step_of(F.chi, d);
-        x.dd = step_of(F.D, d);
+        x.kd = x.hd = x.dd = x.qd = 0;
+        if constexpr (PACK) {
+            x.qd = d == 0 ? 1 : (d == 1 ? F.q.sy : F.q.sz);
+        } else {
+            x.kd = step_of(F.kappa, d);
+            x.hd = step_of(F.chi, d);
+            x.dd = step_of(F.D, d);
+        }
         // transverse directions and their edges: x (y on xy, z on xz), y (x on xy, z
         // on yz), z (x on xz, y on yz)
         const int t[2] = {d == 0 ? 1 : 0, d == 2 ? 1 : 2};
         for (int q = 0; q < 2; ++q) {
             const int e = d + t[q] == 1 ? 0 : (d + t[q] == 2 ? 1 : 2);
             auto& g = x.f[q];
-            g.s = comp(a.et, 2 * e);
-            g.d = comp(a.et, 2 * e + 1);
-            g.eq = step_of(a.et, t[q]);
+            g.s = comp(a.S.et, PACK ? e : 2 * e);
+            g.d = PACK ? nullptr : comp(a.S.et, 2 * e + 1);
+            g.eq = step_of(a.S.et, t[q]);
             g.v = F.vel[t[q]].p;
             g.vsy = F.vel[t[q]].sy;
             g.vsz = F.vel[t[q]].sz;
             g.vq = step_of(F.vel[t[q]], t[q]);
             g.vd = step_of(F.vel[t[q]], d);
         }
-        for (int c = 0; c < 2 + NS; ++c) x.ff[c] = comp(a.ff[d], c);
-        x.fsy = a.ff[d].sy;
-        x.fsz = a.ff[d].sz;
         x.it = make_items(n[0] + (d == 0), n[1] + (d == 1), n[2] + (d == 2));
     }
 }
 
-template <int NS, class R, int NZ>
-StageArgs<NS, R, NZ> make_stage_args(const StageCall& c) {
-    StageArgs<NS, R, NZ> a;
+template <int NS, class R, int NZ, bool PACK>
+StageArgs<NS, R, NZ, PACK> make_stage_args(const StageCall& c) {
+    StageArgs<NS, R, NZ, PACK> a;
     a.P = c.P;
-    a.F = make_fields<NS, R>(c);
+    if constexpr (PACK) a.F = make_fields_pack<NS, R>(c);
+    else a.F = make_fields<NS, R>(c);
     a.noise = make_noise<NZ>(c);
-    a.ct = view<R>(c.ct);
-    a.et = view<R>(c.et);
     a.mc = view<double>(c.smc);
-    a.me = view<double>(c.sme);
+    if constexpr (PACK) {
+        // the same buffers with words of two (StageScratch): half the components
+        a.S.ct = view<Pair<R>>(c.ct);
+        a.S.et = view<Pair<R>>(c.et);
+        a.S.me = view<double2>(c.sme);
+        for (int d = 0; d < 3; ++d) {
+            a.S.ff[d] = view<double2>(c.sff[d]);
+            fhd_fab last = c.sff[d];
+            last.data = static_cast<double*>(last.data) + (int64_t)2 * ((2 + NS) / 2) * a.S.ff[d].sn;
+            a.S.fl[d] = view<double>(last);
+        }
+    } else {
+        a.S.ct = view<R>(c.ct);
+        a.S.et = view<R>(c.et);
+        a.S.me = view<double>(c.sme);
+        for (int d = 0; d < 3; ++d) a.S.ff[d] = view<double>(c.sff[d]);
+    }
     for (int d = 0; d < 3; ++d) {
-        a.ff[d] = view<double>(c.sff[d]);
         a.mom0[d] = view<const double>(c.mom0[d]);
         a.mom_o[d] = view<double>(c.mom_o[d]);
     }
@@ -273,27 +327,28 @@ inline int stage_block(const StageCall& c) {
     return (c.tile >= 0 && c.tile < kNumStageBlocks) ? kStageBlocks[c.tile] : 128;
 }
 
-template <int NS, class R, int NZ>
-void launch_update(const StageArgs<NS, R, NZ>& a, cudaStream_t s) {
+template <int NS, class R, int NZ, bool PACK>
+void launch_update(const StageArgs<NS, R, NZ, PACK>& a, cudaStream_t s) {
     const int blocks = (a.it_upd.n + 127) / 128;
-    if (blocks <= 4 * device_sms()) k_update<NS, R, NZ, 4><<<blocks, 128, 0, s>>>(a);
-    else k_update<NS, R, NZ, 16><<<resident_grid<k_update<NS, R, NZ, 16>>(a.it_upd.n, 128), 128, 0, s>>>(a);
+    constexpr int MB = !PACK ? 16 : (NS <= 2 ? 12 : 10);
+    if (blocks <= 4 * device_sms()) k_update<NS, R, NZ, 4, PACK><<<blocks, 128, 0, s>>>(a);
+    else k_update<NS, R, NZ, MB, PACK><<<resident_grid<k_update<NS, R, NZ, MB, PACK>>(a.it_upd.n, 128), 128, 0, s>>>(a);
 }
 
 // part: 0 stresses, 1 face fluxes (all three directions), 2 update
 template <int NS, class R, int NZ>
 int launch_stage_part_t(const StageCall& c, int part) {
-    const StageArgs<NS, R, NZ> a = make_stage_args<NS, R, NZ>(c);
-    const int* N = c.P.n;
+    const StageArgs<NS, R, NZ, true> a = make_stage_args<NS, R, NZ, true>(c);
     const int b = stage_block(c);
     if (part == 0) {
-        k_taus<NS, R, NZ><<<grid_for((int64_t)(N[0] + 2) * (N[1] + 2) * (N[2] + 2), b), b, 0, c.stream>>>(a, StageAux<false>{});
+        k_taus<NS, R, NZ, false, false, true><<<grid_for(a.it_taus.n, b), b, 0, c.stream>>>(a, StageAux<false>{});
     } else if (part == 1) {
-        const int t = (c.tile >= 0 && c.tile < kNumStageBlocks) ? c.tile : auto_face_tile<NS, R>(N);
-#define FHD_FACES(BS, MINB)                                                                    \
-        {                                                                                      \
-            const int per = face_grid<k_faces<NS, R, NZ, BS, MINB>>(N, BS);                    \
-            k_faces<NS, R, NZ, BS, MINB><<<3 * per, BS, 0, c.stream>>>(a, per, StageAux<false>{}); \
+        const int t = (c.tile >= 0 && c.tile < kNumStageBlocks) ? c.tile : auto_face_tile<NS, R>(c.P.n);
+#define FHD_FACES(BS, MINB)                                                                             \
+        {                                                                                               \
+            constexpr auto K = k_faces<NS, R, NZ, BS, MINB, false, false, true>;                        \
+            const int per = face_grid<K>(c.P.n, BS);                                                    \
+            K<<<3 * per, BS, 0, c.stream>>>(a, per, StageAux<false>{});                                 \
         }
         switch (t) {
             case 0: FHD_FACES(128, 4) break;
@@ -304,7 +359,25 @@ int launch_stage_part_t(const StageCall& c, int part) {
         }
 #undef FHD_FACES
     } else {
-        launch_update<NS, R, NZ>(a, c.stream);
+        launch_update(a, c.stream);
+    }
+    return cuda_rc(cudaGetLastError());
+}
+
+// the same without packed operands, for the allocation-free step: its 16 MiB of static
+// scratch hold the boxes that they were sized for only without the records.  FP64,
+// small boxes.
+template <int NS, int NZ>
+int launch_stage_plain_t(const StageCall& c, int part) {
+    const StageArgs<NS, double, NZ> a = make_stage_args<NS, double, NZ, false>(c);
+    if (part == 0) {
+        k_taus<NS, double, NZ><<<grid_for(a.it_taus.n, 128), 128, 0, c.stream>>>(a, StageAux<false>{});
+    } else if (part == 1) {
+        constexpr auto K = k_faces<NS, double, NZ, 128, 4>;
+        const int per = face_grid<K>(c.P.n, 128);
+        K<<<3 * per, 128, 0, c.stream>>>(a, per, StageAux<false>{});
+    } else {
+        launch_update(a, c.stream);
     }
     return cuda_rc(cudaGetLastError());
 }
@@ -333,7 +406,7 @@ int launch_stage_zm_bt(const StageCall& c, int zc) {
         }
         set[dev] = true;
     }
-    const StageArgs<NS, R, NZ> a = make_stage_args<NS, R, NZ>(c);
+    const StageArgs<NS, R, NZ> a = make_stage_args<NS, R, NZ, false>(c);
     const int* N = c.P.n;
     const dim3 grid((N[0] + TX - 1) / TX, (N[1] + TY - 1) / TY, (N[2] + zc - 1) / zc);
     kern<<<grid, BT, smem, c.stream>>>(a, zc);
@@ -353,9 +426,9 @@ int launch_stage_zm_t(const StageCall& c) {
 // the stress (part 0) and face (part 1) launches of a stage whose fluxes the caller
 // wants (StageAux), and of the flux operator, whose StageCall has no stage scratch but
 // the stresses
-template <int NS, int NZ, bool WL>
+template <int NS, int NZ, bool WL, bool PACK>
 int launch_aux_stage_t(const StageCall& c, int part) {
-    const StageArgs<NS, double, NZ> a = make_stage_args<NS, double, NZ>(c);
+    const StageArgs<NS, double, NZ, PACK> a = make_stage_args<NS, double, NZ, PACK>(c);
     StageAux<true> x;
     for (int d = 0; d < 3; ++d) {
         x.ff[d] = view<double>(c.ff[d]);
@@ -363,11 +436,11 @@ int launch_aux_stage_t(const StageCall& c, int part) {
     }
     for (int e = 0; e < 6; ++e) x.ef[e] = view<double>(c.ef[e]);
     if (part == 0) {
-        k_taus<NS, double, NZ, WL, true><<<grid_for(a.it_taus.n, 128), 128, 0, c.stream>>>(a, x);
+        k_taus<NS, double, NZ, WL, true, PACK><<<grid_for(a.it_taus.n, 128), 128, 0, c.stream>>>(a, x);
     } else {
-        constexpr int MB = WL && NS > 2 ? 4 : 8;
-        const int per = face_grid<k_faces<NS, double, NZ, 128, MB, WL, true>>(c.P.n, 128);
-        k_faces<NS, double, NZ, 128, MB, WL, true><<<3 * per, 128, 0, c.stream>>>(a, per, x);
+        constexpr auto K = k_faces<NS, double, NZ, 128, (WL && NS > 2 ? 4 : 8), WL, true, PACK>;
+        const int per = face_grid<K>(c.P.n, 128);
+        K<<<3 * per, 128, 0, c.stream>>>(a, per, x);
     }
     return cuda_rc(cudaGetLastError());
 }
@@ -376,18 +449,17 @@ int launch_aux_stage_t(const StageCall& c, int part) {
 // variants of the stresses and face fluxes, and the common update
 template <int NS, int NZ>
 int launch_walls_part_t(const StageCall& c, int part) {
-    const StageArgs<NS, double, NZ> a = make_stage_args<NS, double, NZ>(c);
-    const int* N = c.P.n;
+    const StageArgs<NS, double, NZ> a = make_stage_args<NS, double, NZ, false>(c);
     if (part == 0) {
-        k_taus<NS, double, NZ, true><<<grid_for((int64_t)(N[0] + 2) * (N[1] + 2) * (N[2] + 2), 128), 128, 0, c.stream>>>(a, StageAux<false>{});
+        k_taus<NS, double, NZ, true><<<grid_for(a.it_taus.n, 128), 128, 0, c.stream>>>(a, StageAux<false>{});
     } else if (part == 1) {
         // register cap: 64 up to two species (the periodic autotuner's choice at 256^3;
         // 128 was measured twice as slow for the wall variant), 128 above
         constexpr int MB = NS <= 2 ? 8 : 4;
-        const int per = face_grid<k_faces<NS, double, NZ, 128, MB, true>>(N, 128);
+        const int per = face_grid<k_faces<NS, double, NZ, 128, MB, true>>(c.P.n, 128);
         k_faces<NS, double, NZ, 128, MB, true><<<3 * per, 128, 0, c.stream>>>(a, per, StageAux<false>{});
     } else {
-        launch_update<NS, double, NZ>(a, c.stream);
+        launch_update(a, c.stream);
     }
     return cuda_rc(cudaGetLastError());
 }
@@ -515,6 +587,13 @@ int launch_stage_part(const StageCall& c, int part) {
             default: return FHD_ERR_BAD_ARG;
         }
     }
+    if (!c.pack) {
+        if constexpr (sizeof(R) == 8) {
+            if (c.mode == NM_OFF) return launch_stage_plain_t<NS, NZ_OFF>(c, part);
+            if (c.mode == NM_PHILOX) return launch_stage_plain_t<NS, NZ_PHILOX>(c, part);
+        }
+        return FHD_ERR_BAD_ARG;
+    }
     switch (c.mode) {
         case NM_OFF: return launch_stage_part_t<NS, R, NZ_OFF>(c, part);
         case NM_AB: return launch_stage_part_t<NS, R, NZ_AB>(c, part);
@@ -541,31 +620,11 @@ ConvArgs<NS> make_conv_args(const StageCall& c) {
     return a;
 }
 
-template <int NS, class R>
-PrepArgs<NS, R> make_prep_args(const StageCall& c) {
-    PrepArgs<NS, R> a;
-    a.P = c.P;
-    a.cons = view<const double>(c.cons_s);
-    for (int d = 0; d < 3; ++d) {
-        a.mom[d] = view<const double>(c.mom_s[d]);
-        a.vel[d] = view<double>(c.vel[d]);
-    }
-    a.pr = view<double>(c.pr, c.pT);
-    a.eta = view<R>(c.eta);
-    a.zeta = view<R>(c.zeta);
-    a.kappa = view<R>(c.kappa);
-    a.chi = view<R>(c.chi);
-    a.D = view<R>(c.D);
-    a.it = make_items(c.P.n[0] + 3, c.P.n[1] + 3, c.P.n[2] + 3);
-    a.status = c.status;
-    return a;
-}
-
 template <int NS, class R, int NZ>
 size_t batch_args_size_t(int kind) {
     if (kind == 0) return sizeof(PrepArgs<NS, R>);
     if (kind == 6) return sizeof(ConvArgs<NS>);
-    return sizeof(StageArgs<NS, R, NZ>);
+    return sizeof(StageArgs<NS, R, NZ, true>);
 }
 
 template <int NS, class R, int NZ>
@@ -577,7 +636,7 @@ void batch_pack_t(int kind, const StageCall& c, void* dst) {
         const ConvArgs<NS> a = make_conv_args<NS>(c);
         memcpy(dst, &a, sizeof(a));
     } else {
-        const StageArgs<NS, R, NZ> a = make_stage_args<NS, R, NZ>(c);
+        const StageArgs<NS, R, NZ, true> a = make_stage_args<NS, R, NZ, true>(c);
         memcpy(dst, &a, sizeof(a));
     }
 }
@@ -589,14 +648,14 @@ constexpr int kBatchFaceMinBlocks[] = {8, 6, 4};
 constexpr int kNumBatchFaceTiles = 3;
 
 template <int NS, class R, int NZ, int MINB>
-void batch_faces_t(int kind, const StageArgs<NS, R, NZ>* sa, const int* dbpref, int nmem, int nblocks, cudaStream_t s) {
+void batch_faces_t(int kind, const StageArgs<NS, R, NZ, true>* sa, const int* dbpref, int nmem, int nblocks, cudaStream_t s) {
     k_faces_b<NS, R, NZ, MINB><<<nblocks, 128, 0, s>>>(sa, dbpref, nmem, kind - 2);
 }
 
 template <int NS, class R, int NZ>
 int batch_launch_t(int kind, int tile, const void* dargs, const int* dbpref, int nmem, int nblocks, cudaStream_t s) {
     if (nblocks <= 0 || nmem <= 0) return FHD_OK;
-    using SA = StageArgs<NS, R, NZ>;
+    using SA = StageArgs<NS, R, NZ, true>;
     const SA* sa = static_cast<const SA*>(dargs);
     switch (kind) {
         case 0: k_cellprep_b<NS, R><<<nblocks, 128, 0, s>>>(static_cast<const PrepArgs<NS, R>*>(dargs), dbpref, nmem); break;
