@@ -269,35 +269,51 @@ int ensure_coef(fhd_ctx* c, int dtype) {
 // The flux operator's own stress scratch (ct, et), kept by the context.  It is apart
 // from the step's scratch, and a call on another stream than the last one's waits for
 // that one, so operator calls may overlap a step, and each other, on any streams.
-// false: no scratch (a stream under capture, whose graph may be replayed beside later
-// calls, or no memory left).
-bool flux_scratch(fhd_ctx* c) {
+// false: no scratch (not allocated yet, or a stream under capture, whose graph may be
+// replayed beside later calls).
+bool capturing(fhd_ctx* c) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(c->stream, &st) != cudaSuccess) { cudaGetLastError(); return false; }
-    if (st != cudaStreamCaptureStatusNone) return false;
-    if (!c->fx) {
-        const int* n = c->prm.n_cells;
-        const int allnod[3] = {1, 1, 1};
-        c->fxt = make_fab(nullptr, n, CELLN, 1, 6, FHD_F64);
-        c->fxe = make_fab(nullptr, n, allnod, 0, 6, FHD_F64);
-        const int64_t nt = fab_points(c->fxt) * 6, ne = fab_points(c->fxe) * 6;
-        if (!c->fx_ev && cudaEventCreateWithFlags(&c->fx_ev, cudaEventDisableTiming) != cudaSuccess) {
-            cudaGetLastError();
-            c->fx_ev = nullptr;
-            return false;
-        }
-        if (cudaMalloc(&c->fx, (size_t)(nt + ne) * sizeof(double)) != cudaSuccess) {
-            cudaGetLastError();
-            c->fx = nullptr;
-            return false;
-        }
-        c->fxt.data = c->fx;
-        c->fxe.data = c->fx + nt;
-    } else if (c->fx_stream != c->stream && cudaStreamWaitEvent(c->stream, c->fx_ev, 0) != cudaSuccess) {
+    if (cudaStreamIsCapturing(c->stream, &st) != cudaSuccess) { cudaGetLastError(); return true; }
+    return st != cudaStreamCaptureStatusNone;
+}
+bool flux_scratch(fhd_ctx* c) {
+    if (!c->fx || capturing(c)) return false;
+    if (c->fx_stream != c->stream && cudaStreamWaitEvent(c->stream, c->fx_ev, 0) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
     return true;
+}
+// Allocates it behind the first call's kernels, which go without, in stream order: at 72^3
+// a context's first call takes 523 us, 841 with cudaMalloc in front of the kernels and 705
+// with cudaMalloc (which waits for them) behind.
+// Without memory left the operator stays without.
+void flux_scratch_alloc(fhd_ctx* c) {
+    if (c->fx || capturing(c)) return;
+    const int* n = c->prm.n_cells;
+    const int allnod[3] = {1, 1, 1};
+    c->fxt = make_fab(nullptr, n, CELLN, 1, 6, FHD_F64);
+    c->fxe = make_fab(nullptr, n, allnod, 0, 6, FHD_F64);
+    const int64_t nt = fab_points(c->fxt) * 6, ne = fab_points(c->fxe) * 6;
+    if (!c->fx_ev && cudaEventCreateWithFlags(&c->fx_ev, cudaEventDisableTiming) != cudaSuccess) {
+        cudaGetLastError();
+        c->fx_ev = nullptr;
+        return;
+    }
+    if (cudaMallocAsync(&c->fx, (size_t)(nt + ne) * sizeof(double), c->stream) != cudaSuccess) {
+        cudaGetLastError();
+        c->fx = nullptr;
+        return;
+    }
+    if (cudaEventRecord(c->fx_ev, c->stream) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(c->fx);
+        c->fx = nullptr;
+        return;
+    }
+    c->fx_stream = c->stream;
+    c->fxt.data = c->fx;
+    c->fxe.data = c->fx + nt;
 }
 
 // brackets one launch with events when profiling is on
@@ -726,7 +742,11 @@ int fhd_flux_stag(fhd_ctx* c, fhd_fab cu, const fhd_fab mom[3], fhd_fab prim, co
     sc.status = c->d_status;
     sc.stream = c->stream;
     // with the stress scratch every stress is computed once, without it once per face
-    if (!flux_scratch(c)) return exact_aux_fluxes(sc);
+    if (!flux_scratch(c)) {
+        const int rc = exact_aux_fluxes(sc);
+        if (!rc) flux_scratch_alloc(c);
+        return rc;
+    }
     sc.ct = c->fxt;
     sc.et = c->fxe;
     int rc = exact_aux_stage(sc, 0);
