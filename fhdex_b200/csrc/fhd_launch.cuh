@@ -298,17 +298,18 @@ StageArgs<NS, R, NZ, PACK> make_stage_args(const StageCall& c) {
 }
 
 // The face kernel's launch shape when none was set (fhd_set_tile).  The kernel is
-// bound by latency and issue, so resident warps count until spills cost more:
-//   * a direction whose faces fit one wave of 128-register blocks (4 per SM, up to
-//     about 42^3) takes them: with no second wave, more residency buys nothing and
-//     spills cost (argon FP64 16^3: 170 us per step against 178 at 64 registers);
-//   * up to one wave of 80-register blocks (48^3: 258 us against 302 at 128
-//     registers and 263 at 64);
-//   * above, the shape measured fastest per precision and species count: FP64 64
-//     registers (256^3 argon 26.1 ms per step against 32.8 at 128 registers; 128^3
-//     four species 6.79 against 8.02); FP32 fluxes 64 registers for two species
-//     (192^3 8.13 against 8.90 ms), 48 for one (128^3 1.79 against 1.99), 80 for
-//     three and four (128^3 3.80 against 4.29).
+// bound by latency and issue, so resident warps count until spills cost more
+// (us per step, all kernels, unless ms):
+//   * faces that fit one wave of 128-register blocks (4 per SM; up to about 29^3) take
+//     them: with no second wave, more residency buys nothing and spills cost (argon FP64
+//     24^3 88.2 against 90.8 at 64 registers; 32^3 110.8 against 102.6);
+//   * up to one wave of 80-register blocks (about 33^3): 32^3, faces alone, 44.6 against 47.5
+//     at 64 registers; 40^3 138.5 against 135.9;
+//   * above, 64 registers (argon FP64 48^3 191 against 213 at 128 registers, 128^3 2905
+//     against 2933 at 80; mixed 128^3 1908 against 1975 at 80; four species FP64 64^3 803
+//     against 841, mixed 405 against 418), with two exceptions: 48 for one species (96^3
+//     FP64 703 against 732, mixed 632 against 644), and 80 for three and four species in
+//     mixed precision beyond about 93^3 (128^3 2940 against 3014).
 template <int NS, class R>
 int auto_face_tile(const int N[3]) {
     int64_t most = 0;
@@ -319,8 +320,8 @@ int auto_face_tile(const int N[3]) {
     const int64_t blocks = 3 * ((most + 127) / 128);
     if (blocks <= 4 * device_sms()) return 0;
     if (blocks <= 6 * device_sms()) return 2;
-    if (sizeof(R) == 8) return 4;
-    return NS == 1 ? 3 : (NS == 2 ? 4 : 2);
+    if (NS == 1) return 3;
+    return sizeof(R) == 4 && NS >= 3 && blocks > 128 * device_sms() ? 2 : 4;
 }
 
 inline int stage_block(const StageCall& c) {
