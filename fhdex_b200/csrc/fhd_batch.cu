@@ -101,6 +101,7 @@ struct fhd_batch {
     size_t counters_bytes = 0;   // next, abort, done[] (zeroed before each launch)
     double wait_limit_s = 1.0;
     int hold_phase = -1;
+    bool images = false;         // the update and the conversion store the periodic ghosts (image_width), for every member
     int persist_tile = -1;       // register cap of the persistent kernel (batch face tiles; -1 default)
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
@@ -179,6 +180,7 @@ StageCall member_call(const fhd_batch* b, const Member& m, int s, const uint64_t
     sc.pack = 1;
     sc.rec = m.rec;
     sc.wprim = rec_wprim(m.prm);
+    sc.img = b->images ? -m.cu.lo[0] : 0;
     sc.ct = m.ct;
     sc.et = m.et;
     sc.smc = m.smc;
@@ -208,6 +210,12 @@ int rebuild(fhd_batch* b) {
     b->plan.clear();
     const int M = (int)b->mem.size();
     if (M == 0) { b->dirty = false; return FHD_OK; }
+    b->images = true;
+    for (const Member& m : b->mem) {
+        const fhd_fab* f[16] = {&m.cu, &m.prim, &m.mom[0], &m.mom[1], &m.mom[2], &m.vel[0], &m.vel[1], &m.vel[2],
+                                &m.cup, &m.cup2, &m.cupm[0], &m.cupm[1], &m.cupm[2], &m.cup2m[0], &m.cup2m[1], &m.cup2m[2]};
+        if (!image_width(m.prm.n_cells, f, 16)) b->images = false;
+    }
     std::vector<char> host;
     auto align = [&](size_t a) { size_t o = (host.size() + a - 1) & ~(a - 1); host.resize(o); return o; };
     // steps and statuses first
@@ -347,6 +355,7 @@ int rebuild(fhd_batch* b) {
         }
         int nfab = 0, nb = 0;
         std::vector<int64_t> gitems;
+        if (b->images) continue;
         auto g = push_ghosts(s, nfab, nb, gitems);
         b->plan.push_back(Launch{7, g.first, g.second, nfab, nb, (size_t)ghost_sz, gitems});
     }
@@ -357,10 +366,12 @@ int rebuild(fhd_batch* b) {
         int nb = 0;
         const size_t bpo = push_bpref(items, 128, nb);
         b->plan.push_back(Launch{6, conv, bpo, M, nb, batch_args_size(b->ns, false, 6, b->mode), items});
-        int nfab = 0;
-        std::vector<int64_t> gitems;
-        auto g = push_final_ghosts(nfab, nb, gitems);
-        b->plan.push_back(Launch{7, g.first, g.second, nfab, nb, (size_t)ghost_sz, gitems});
+        if (!b->images) {
+            int nfab = 0;
+            std::vector<int64_t> gitems;
+            auto g = push_final_ghosts(nfab, nb, gitems);
+            b->plan.push_back(Launch{7, g.first, g.second, nfab, nb, (size_t)ghost_sz, gitems});
+        }
         b->plan.push_back(Launch{8, 0, 0, M, 0, 0, std::vector<int64_t>(M, 1)});
     }
     // the persistent step's work units, phase-major over members, with each

@@ -1203,6 +1203,8 @@ static int step_launches(fhd_ctx* c, fhd_fab cu, const fhd_fab mom[3], fhd_fab p
         sc.cons_s = *ins[s];
         sc.cons_o = *outs[s];
         sc.wcoef = s == 2 && aux_coef;   // the stage-3 coefficients are the caller's
+        const fhd_fab* of[4] = {outs[s], &outsm[s][0], &outsm[s][1], &outsm[s][2]};
+        sc.img = fused ? 0 : image_width(c->prm.n_cells, of, 4);
         for (int d = 0; d < 3; ++d) { sc.mom_s[d] = insm[s][d]; sc.mom_o[d] = outsm[s][d]; }
         {
             ProfScope ps(c, 0);
@@ -1234,6 +1236,7 @@ static int step_launches(fhd_ctx* c, fhd_fab cu, const fhd_fab mom[3], fhd_fab p
             }
         }
         if (rc) return rc;
+        if (sc.img) continue;
         GhostReq g[5] = {{*outs[s], 0, 1}, {*outs[s], 4, 1 + ns}, {outsm[s][0], 0, 1}, {outsm[s][1], 0, 1},
                          {outsm[s][2], 0, 1}};
         {
@@ -1243,16 +1246,20 @@ static int step_launches(fhd_ctx* c, fhd_fab cu, const fhd_fab mom[3], fhd_fab p
         if (rc) return rc;
     }
     // final conservedToPrimitiveStag + FillBoundary (timeStepStag.cpp:1216-1230)
+    const fhd_fab* cf[5] = {&cu, &prim, &vel[0], &vel[1], &vel[2]};
+    const int img = image_width(c->prm.n_cells, cf, 5);
     {
         ProfScope ps(c, 5);
-        rc = exact_convert(sc.P, prim, vel, cu, mom, c->d_status, c->stream);
+        rc = exact_convert(sc.P, prim, vel, cu, mom, c->d_status, c->stream, img);
     }
     if (rc) return rc;
     GhostReq g[10];
     int ng = 0;
-    g[ng++] = GhostReq{cu, 1, 3};
-    g[ng++] = GhostReq{prim, 0, nprim};
-    for (int d = 0; d < 3; ++d) g[ng++] = GhostReq{vel[d], 0, 1};
+    if (!img) {
+        g[ng++] = GhostReq{cu, 1, 3};
+        g[ng++] = GhostReq{prim, 0, nprim};
+        for (int d = 0; d < 3; ++d) g[ng++] = GhostReq{vel[d], 0, 1};
+    }
     if (aux_coef) {
         g[ng++] = GhostReq{eta, 0, 1};
         g[ng++] = GhostReq{zeta, 0, 1};
@@ -1260,10 +1267,10 @@ static int step_launches(fhd_ctx* c, fhd_fab cu, const fhd_fab mom[3], fhd_fab p
         g[ng++] = GhostReq{chi, 0, ns};
         g[ng++] = GhostReq{D, 0, ns * ns};
     }
+    if (!ng) return FHD_OK;
     ProfScope ps(c, 4);
     return fill_ghosts(g, ng, c->prm.n_cells, c->stream);
 }
-
 
 int fhd_rk3_step_stag(fhd_ctx* c, fhd_fab cu, const fhd_fab mom[3], fhd_fab prim, const fhd_fab vel[3], fhd_fab source,
                       fhd_fab eta, fhd_fab zeta, fhd_fab kappa, fhd_fab chi, fhd_fab D, const fhd_fab* faceflux,

@@ -223,9 +223,7 @@ FHD_HD double stoch_factor(const RunParams& P, int type) {
 
 // ---- EOS helpers (compressible_functions.H:138-219, 1497-1520) ----------------------
 // Products summed in double go through mul_rn / add_rn, which are never fused into
-// an FMA: the conversion then gives the same bits in the FP64 units (built without
-// contraction) and in the mixed units (built with it), where the persistent batched
-// step converts the state.  FP32 code keeps the compiler's contraction.
+// an FMA: the conversion gives the same bits however a unit is built.
 FHD_D double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 FHD_D double add_rn(double a, double b) { return __dadd_rn(a, b); }
 FHD_D float mul_rn(float a, float b) { return a * b; }

@@ -12,7 +12,7 @@ int exact_aux_stage_ns1(const StageCall&, int);
 int mixed_cellprep_ns1(const StageCall&);
 int mixed_stage_ns1(const StageCall&, int);
 int exact_transport_ns1(const DevParams&, fhd_fab, fhd_fab, fhd_fab, fhd_fab, fhd_fab, fhd_fab, int*, cudaStream_t);
-int exact_convert_ns1(const DevParams&, fhd_fab, const fhd_fab*, fhd_fab, const fhd_fab*, int*, cudaStream_t);
+int exact_convert_ns1(const DevParams&, fhd_fab, const fhd_fab*, fhd_fab, const fhd_fab*, int*, cudaStream_t, int);
 int exact_walls_ns1(const StageCall&, int);
 int exact_reservoir_ns1(const ResArgs&, cudaStream_t);
 int exact_res_reset_ns1(const ResResetArgs&, cudaStream_t);
@@ -26,7 +26,7 @@ int exact_aux_stage_ns2(const StageCall&, int);
 int mixed_cellprep_ns2(const StageCall&);
 int mixed_stage_ns2(const StageCall&, int);
 int exact_transport_ns2(const DevParams&, fhd_fab, fhd_fab, fhd_fab, fhd_fab, fhd_fab, fhd_fab, int*, cudaStream_t);
-int exact_convert_ns2(const DevParams&, fhd_fab, const fhd_fab*, fhd_fab, const fhd_fab*, int*, cudaStream_t);
+int exact_convert_ns2(const DevParams&, fhd_fab, const fhd_fab*, fhd_fab, const fhd_fab*, int*, cudaStream_t, int);
 int exact_walls_ns2(const StageCall&, int);
 int exact_reservoir_ns2(const ResArgs&, cudaStream_t);
 int exact_res_reset_ns2(const ResResetArgs&, cudaStream_t);
@@ -40,7 +40,7 @@ int exact_aux_stage_ns3(const StageCall&, int);
 int mixed_cellprep_ns3(const StageCall&);
 int mixed_stage_ns3(const StageCall&, int);
 int exact_transport_ns3(const DevParams&, fhd_fab, fhd_fab, fhd_fab, fhd_fab, fhd_fab, fhd_fab, int*, cudaStream_t);
-int exact_convert_ns3(const DevParams&, fhd_fab, const fhd_fab*, fhd_fab, const fhd_fab*, int*, cudaStream_t);
+int exact_convert_ns3(const DevParams&, fhd_fab, const fhd_fab*, fhd_fab, const fhd_fab*, int*, cudaStream_t, int);
 int exact_walls_ns3(const StageCall&, int);
 int exact_reservoir_ns3(const ResArgs&, cudaStream_t);
 int exact_res_reset_ns3(const ResResetArgs&, cudaStream_t);
@@ -54,7 +54,7 @@ int exact_aux_stage_ns4(const StageCall&, int);
 int mixed_cellprep_ns4(const StageCall&);
 int mixed_stage_ns4(const StageCall&, int);
 int exact_transport_ns4(const DevParams&, fhd_fab, fhd_fab, fhd_fab, fhd_fab, fhd_fab, fhd_fab, int*, cudaStream_t);
-int exact_convert_ns4(const DevParams&, fhd_fab, const fhd_fab*, fhd_fab, const fhd_fab*, int*, cudaStream_t);
+int exact_convert_ns4(const DevParams&, fhd_fab, const fhd_fab*, fhd_fab, const fhd_fab*, int*, cudaStream_t, int);
 int exact_walls_ns4(const StageCall&, int);
 int exact_reservoir_ns4(const ResArgs&, cudaStream_t);
 int exact_res_reset_ns4(const ResResetArgs&, cudaStream_t);
@@ -115,8 +115,8 @@ int exact_transport(const DevParams& P, fhd_fab prim, fhd_fab eta, fhd_fab zeta,
     FHD_DISPATCH(P.ns, exact_transport_ns, P, prim, eta, zeta, kappa, chi, D, status, s)
 }
 int exact_convert(const DevParams& P, fhd_fab prim, const fhd_fab vel[3], fhd_fab cons, const fhd_fab mom[3],
-                  int* status, cudaStream_t s) {
-    FHD_DISPATCH(P.ns, exact_convert_ns, P, prim, vel, cons, mom, status, s)
+                  int* status, cudaStream_t s, int img) {
+    FHD_DISPATCH(P.ns, exact_convert_ns, P, prim, vel, cons, mom, status, s, img)
 }
 
 int exact_walls_part(const StageCall& c, int part) { FHD_DISPATCH(c.P.ns, exact_walls_ns, c, part) }

@@ -760,8 +760,8 @@ FHD_D FaceFlux<NS> face_flux(const RunParams& P, const FT& F, const Noise<NZ>& n
 // direction's wall is tested first, the first direction's wins a corner).
 template <int NS, class R, int E, bool WL = false, class FT>
 FHD_D void edge_adv(const RunParams& P, const FT& F, int i, int j, int k, double& a, double& b) {
-    const Arr4<const double>&mx = F.mom[0], &my = F.mom[1], &mz = F.mom[2];
-    const Arr4<const double>&vx = F.vel[0], &vy = F.vel[1], &vz = F.vel[2];
+    const auto &mx = F.mom[0], &my = F.mom[1], &mz = F.mom[2];
+    const auto &vx = F.vel[0], &vy = F.vel[1], &vz = F.vel[2];
     if (P.advection_type < 0) { a = b = 0.0; return; }
     // edge of directions (p, q) = xy, xz or yz: a carries the p-momentum along q
     // (m0, m1 the p-face momenta on the q-1 / q sides, u0, u1 the q-face velocities
@@ -844,8 +844,8 @@ FHD_D double cen_total(const RunParams& P, const FT& F, const CellTaus<R>& t, in
         if (WL && d >= P.dim) {
             v += 0.0;   // no transverse pressure / advection term in 1-D and 2-D (fluxStag.cpp:1850-1860)
         } else {
-            const Arr4<const double>& m = F.mom[d];
-            const Arr4<const double>& u = F.vel[d];
+            const auto& m = F.mom[d];
+            const auto& u = F.vel[d];
             const int e0 = d == 0, e1 = d == 1, e2 = d == 2;
             v += 0.25 * (m(i, j, k) + m(i + e0, j + e1, k + e2)) * (u(i, j, k) + u(i + e0, j + e1, k + e2)) +
                  F.p(i, j, k);

@@ -1,6 +1,6 @@
 // fhd_host.h — host-side launch descriptors shared by the C ABI and the kernel
-// translation units (fhd_exact.cu: FP64 in the reference's operation order,
-// built with -fmad=false; fhd_mixed.cu: FP32 fluxes/coefficients).
+// translation units (exact_*: FP64 in the reference's operation order; mixed_*: FP32
+// fluxes and coefficients).
 #pragma once
 #include <cmath>
 #include <cstring>
@@ -193,6 +193,7 @@ struct StageCall {
     int pack;
     fhd_fab rec;
     int wprim, wcoef;
+    int img;                // packed update and conversion: ghost width of the periodic images they store (0: none)
     int* status;
     cudaStream_t stream;
     int tile;               // tile-shape index of k_stage (autotuned)
@@ -210,6 +211,18 @@ inline int rec_wprim(const fhd_params& p) {
     return p.precision == FHD_PREC_MIXED ? 1 : 0;
 }
 
+// Ghost width of the periodic images that the update and the conversion can store
+// themselves (images, fhd_kernels.cuh) into cell or face fabs of the box: the fabs' common
+// width when every direction has more than twice as many cells, so that a point has one
+// image per direction at most.  0: fill_ghosts after the kernel.
+inline int image_width(const int n[3], const fhd_fab* const* f, int nf) {
+    const int g = -f[0]->lo[0];
+    for (int q = 0; q < nf; ++q)
+        for (int d = 0; d < 3; ++d)
+            if (-f[q]->lo[d] != g) return 0;
+    return n[0] > 2 * g && n[1] > 2 * g && n[2] > 2 * g ? g : 0;
+}
+
 // exact (FP64) translation unit
 int exact_cellprep(const StageCall& c);
 int exact_stage_part(const StageCall& c, int part);  // 0 stresses, 1 face fluxes, 2 update, 3 fused (all three)
@@ -219,8 +232,9 @@ int exact_aux_stage(const StageCall& c, int part);
 int exact_aux_fluxes(const StageCall& c);
 int exact_transport(const DevParams& P, fhd_fab prim, fhd_fab eta, fhd_fab zeta, fhd_fab kappa, fhd_fab chi,
                     fhd_fab D, int* status, cudaStream_t s);
+// img: as StageCall::img
 int exact_convert(const DevParams& P, fhd_fab prim, const fhd_fab vel[3], fhd_fab cons, const fhd_fab mom[3],
-                  int* status, cudaStream_t s);
+                  int* status, cudaStream_t s, int img = 0);
 // boxes with physical walls (FP64): the stage parts (0 stresses, 1 face fluxes, 2
 // update), BCMassTempPress + BCRhoRhoE on prim / cons, BCMomNormal + BCMomTrans on
 // the face momenta and velocities

@@ -1,7 +1,8 @@
 // fhd_kern_ns.cu — kernel instantiations for one species count, compiled once per
 // (FHD_NS, precision) pair so the build runs in parallel:
-//   -DFHD_NS=<n>                 exact FP64 (built with -fmad=false)
+//   -DFHD_NS=<n>                 exact FP64
 //   -DFHD_NS=<n> -DFHD_MIXED=1   mixed precision (FP32 compute)
+// Both are built with -fmad=false; FP32 fused multiply-adds are explicit (madd).
 #include "fhd_launch.cuh"
 
 #ifndef FHD_NS
@@ -150,7 +151,7 @@ int FHD_CAT(exact_transport_ns, FHD_NS)(const DevParams& P, fhd_fab prim, fhd_fa
 }
 
 int FHD_CAT(exact_convert_ns, FHD_NS)(const DevParams& P, fhd_fab prim, const fhd_fab vel[3], fhd_fab cons,
-                                      const fhd_fab mom[3], int* status, cudaStream_t s) {
+                                      const fhd_fab mom[3], int* status, cudaStream_t s, int img) {
     ConvArgs<FHD_NS> a;
     a.P = P;
     a.prim = view<double>(prim);
@@ -161,6 +162,7 @@ int FHD_CAT(exact_convert_ns, FHD_NS)(const DevParams& P, fhd_fab prim, const fh
     }
     a.it = make_items(P.n[0], P.n[1], P.n[2]);
     a.status = status;
+    a.img = img;
     const int64_t tot = a.it.n;
     k_convert<FHD_NS><<<resident_grid<k_convert<FHD_NS>>(tot, 128), 128, 0, s>>>(a);
     return cuda_rc(cudaGetLastError());

@@ -3,10 +3,12 @@
 //   k_cellprep  per stage: conservedToPrimitiveStag + calculateTransportCoeffs for
 //               every cell once (cells grown by 1, face velocities grown by 1)
 //   k_taus      per stage: stochastic + deterministic stresses on cells and edges
+//               (k_taus_staged: small boxes)
 //   k_faces     per stage: stochastic + diffusive + hyperbolic conservative face
 //               fluxes of the three directions
 //   k_update    per stage: flux divergence, momentum update and the SSP-RK3
-//               combination
+//               combination, with the results' periodic ghosts (k_update_split: the
+//               smallest boxes)
 //   k_convert   end of step / drop-in conversion (prim, vel, cons 1..3)
 //   k_ghosts    periodic FillBoundary of several fabs in one launch
 //   k_transport, k_aux_*  drop-in operators (transport coefficients, flux MultiFabs)
@@ -17,11 +19,10 @@
 
 namespace fhd {
 
-// Every kernel here has internal linkage (static): the FP64 units (built with
-// -fmad=false) and the mixed units (-fmad=true) both instantiate the kernels that
-// do not depend on the precision (e.g. k_convert_b<NS>) under the same name.
-// With external linkage a launch could reach the other unit's device code, and
-// which one depends on the order the modules are loaded in.
+// Every kernel here has internal linkage (static): the FP64 and the mixed units both
+// instantiate the kernels that do not depend on the precision (e.g. k_convert_b<NS>)
+// under the same name.  With external linkage a launch could reach the other unit's
+// device code, and which one depends on the order the modules are loaded in.
 
 enum { ST_OK = 0, ST_MASSFRAC = 2, ST_NONFINITE = 3, ST_TIMEOUT = 5 };
 
@@ -292,6 +293,7 @@ struct alignas(16) StageArgs {
     FaceDir<NS, R, PACK> fd[3];
     Items it_taus, it_upd;       // cells [-1, n]^3, points [0, n]^3
     int stage;                   // 1, 2, 3
+    int img;                     // packed: ghost width of the periodic images the update stores (0: none)
 };
 
 // stresses on cells (grown by 1) and edges; one thread per point of [-1, n]^3
@@ -312,6 +314,102 @@ struct StageAux {
 template <>
 struct StageAux<false> {};
 
+// ---- staged operands ---------------------------------------------------------------
+// In a box of a few waves the stress kernel's time is one thread's: registers hold only a
+// few of a point's 32 operands at a time, so it waits for memory several times in turn,
+// then draws its noise.  Staged, a thread issues all of them at once as asynchronous
+// copies into its own column of shared memory, draws the noise meanwhile, waits once and
+// computes from there (launch_stage_part_t has the figures and the size up to which it is
+// used; more registers without it gave 38.5 us for 38.6).  A column is read by its own
+// thread alone, so cp.async.wait_all orders it and no barrier is needed.
+template <int N>
+FHD_D void stage_copy(void* dst, const void* src) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(d), "l"(src), "n"(N) : "memory");
+}
+FHD_D void stage_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+constexpr int kStagedThreads = 128;
+
+// stress kernel: (T, eta) words of the point's cell and the six below it that its edges
+// touch, its pressure, and four values of each face velocity and momentum
+template <int NS, class R>
+struct TausStage {
+    static constexpr bool f64 = sizeof(R) == 8;
+    static constexpr int n16 = 7 + (f64 ? 1 : 0), n8 = 24 + (f64 ? 0 : 1);
+    static constexpr int bytes = (n16 * 16 + n8 * 8) * kStagedThreads;
+};
+template <int NS, class R>
+struct FieldsStaged {
+    // values of one face field: (0), one above in its own direction, one below in the
+    // first and in the second of the other two
+    struct Face {
+        const double* s;
+        int d, i, j, k;
+        FHD_D static int slot(int d, int dx, int dy, int dz) {
+            if (dx + dy + dz > 0) return 1;
+            if (dx < 0) return 2;
+            if (dy < 0) return d == 0 ? 2 : 3;
+            return dz < 0 ? 3 : 0;
+        }
+        FHD_D double operator()(int a, int b, int c) const { return s[slot(d, a - i, b - j, c - k) * kStagedThreads]; }
+    };
+    const Vec<R>* s16;   // the thread's columns
+    const double* s8;
+    int i, j, k;
+    R zr;
+    Face vel[3], mom[3];
+    FHD_D FieldsStaged(const unsigned char* smem, int i_, int j_, int k_, R zr_) : i(i_), j(j_), k(k_), zr(zr_) {
+        s16 = reinterpret_cast<const Vec<R>*>(smem) + threadIdx.x;
+        s8 = reinterpret_cast<const double*>(smem + TausStage<NS, R>::n16 * 16 * kStagedThreads) + threadIdx.x;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            vel[d] = Face{s8 + 4 * d * kStagedThreads, d, i, j, k};
+            mom[d] = Face{s8 + (12 + 4 * d) * kStagedThreads, d, i, j, k};
+        }
+    }
+    FHD_D R word(int a, int b, int c, int e) const {
+        return vget(s16[((i - a) + 2 * (j - b) + 4 * (k - c)) * kStagedThreads], e);
+    }
+    FHD_D R T(int a, int b, int c) const { return word(a, b, c, RecLayout<NS, R>::T); }
+    FHD_D R eta(int a, int b, int c) const { return word(a, b, c, RecLayout<NS, R>::ETA); }
+    FHD_D R zeta(int a, int b, int c) const { return zr * eta(a, b, c); }
+    FHD_D double p(int, int, int) const {
+        if constexpr (sizeof(R) == 8) return vget(s16[7 * kStagedThreads], RecLayout<NS, R>::PR % 2);
+        else return s8[24 * kStagedThreads];
+    }
+};
+template <int NS, class R>
+FHD_D void taus_issue(const FieldsPack<NS, R>& F, unsigned char* smem, int i, int j, int k, bool edges) {
+    constexpr int B = kStagedThreads;
+    Vec<R>* s16 = reinterpret_cast<Vec<R>*>(smem) + threadIdx.x;
+    double* s8 = reinterpret_cast<double*>(smem + TausStage<NS, R>::n16 * 16 * B) + threadIdx.x;
+    const int oq = F.q.at(i, j, k);
+    stage_copy<16>(s16, F.q.p + oq);
+    if constexpr (sizeof(R) == 8) stage_copy<16>(s16 + 7 * B, F.q.p + oq + F.q.sn);
+    else stage_copy<8>(s8 + 24 * B, &F.pr(i, j, k, F.pT + 1));
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+            const Arr4<const double>& f = m ? F.mom[d] : F.vel[d];
+            double* s = s8 + (12 * m + 4 * d) * B;
+            const double* g = &f(i, j, k);
+            stage_copy<8>(s, g);
+            stage_copy<8>(s + B, g + (d == 0 ? 1 : (d == 1 ? f.sy : f.sz)));
+            if (edges) {
+                stage_copy<8>(s + 2 * B, g - (d == 0 ? f.sy : 1));
+                stage_copy<8>(s + 3 * B, g - (d == 2 ? f.sy : f.sz));
+            }
+        }
+    }
+    if (edges) {
+#pragma unroll
+        for (int c = 1; c < 7; ++c)
+            stage_copy<16>(s16 + c * B, F.q.p + oq - ((c & 1) + ((c >> 1) & 1) * F.q.sy + (c >> 2) * F.q.sz));
+    }
+}
+
 // both edge totals of edge E into the stage's scratch (absent: the flux operator) and
 // the flux fabs
 template <int E, bool AUX, class A>
@@ -325,49 +423,73 @@ FHD_D void put_edge(const A& a, const StageAux<AUX>& x, int i, int j, int k, dou
 }
 
 // stress and edge totals of edge E at point (i, j, k)
-template <int NS, class R, int NZ, int E, bool WL, bool AUX, bool PACK>
-FHD_D void taus_edge(const StageArgs<NS, R, NZ, PACK>& a, const StageAux<AUX>& x, double w, int i, int j, int k) {
+template <int NS, class R, int NZ, int E, bool WL, bool AUX, bool PACK, class FT>
+FHD_D void taus_edge(const StageArgs<NS, R, NZ, PACK>& a, const FT& F, const StageAux<AUX>& x, double w, int i, int j,
+                     int k) {
     const RunParams& P = a.P;
     const int hadv = P.advection_type >= 0;
-    const Taus<R> e = edge_taus_w<NS, R, NZ, E, WL>(P, a.F, w, i, j, k);
+    const Taus<R> e = edge_taus_w<NS, R, NZ, E, WL>(P, F, w, i, j, k);
     a.S.put_et(E, i, j, k, e);
     double ea, eb;
-    edge_adv<NS, R, E, WL>(P, a.F, i, j, k, ea, eb);
+    edge_adv<NS, R, E, WL>(P, F, i, j, k, ea, eb);
     put_edge<E>(a, x, i, j, k, WL ? edge_total_w<R, E>(P, e, ea, hadv, i, j, k) : edge_total<R>(e, ea, hadv),
                 WL ? edge_total_w<R, E>(P, e, eb, hadv, i, j, k) : edge_total<R>(e, eb, hadv));
 }
 
 // WL: walls (the wall variants of the edge stresses, advective edge fluxes and
 // StochFluxStag's factors on the edge totals)
-template <int NS, class R, int NZ, bool WL = false, bool AUX = false, bool PACK = false>
-FHD_D void taus_point(const StageArgs<NS, R, NZ, PACK>& a, int q, const StageAux<AUX>& x = StageAux<AUX>()) {
+// STAGED: the operands come through shared memory (smem, TausStage)
+template <int NS, class R, int NZ, bool WL = false, bool AUX = false, bool STAGED = false, bool PACK = false>
+FHD_D void taus_point(const StageArgs<NS, R, NZ, PACK>& a, int q, const StageAux<AUX>& x = StageAux<AUX>(),
+                      unsigned char* smem = nullptr) {
     const RunParams& P = a.P;
     int i, j, k;
     a.it_taus.point(q, i, j, k);
     --i; --j; --k;
     const bool edges = i >= 0 && j >= 0 && k >= 0;
     double wc[3] = {0.0, 0.0, 0.0}, we[3] = {0.0, 0.0, 0.0};
+    if constexpr (STAGED) taus_issue<NS, R>(a.F, smem, i, j, k, edges);
     if (NZ != NZ_OFF) a.noise.cen_and_yz_edge(P, i, j, k, edges, wc, we[2]);
-    const CellTaus<R> t = cell_taus_w<NS, R, NZ, WL>(P, a.F, wc, i, j, k);
+    auto work = [&](const auto& F) {
+        const CellTaus<R> t = cell_taus_w<NS, R, NZ, WL>(P, F, wc, i, j, k);
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        a.S.put_ct(i, j, k, d, t.s[d], t.d[d]);
-        const double c = cen_total_res<NS, R, NZ, WL>(P, a.F, a.noise, t, d, i, j, k);
-        if (!AUX || a.mc.p) a.mc(i, j, k, d) = c;
-        if constexpr (AUX) x.cf[d](i, j, k) = c;
+        for (int d = 0; d < 3; ++d) {
+            a.S.put_ct(i, j, k, d, t.s[d], t.d[d]);
+            const double c = cen_total_res<NS, R, NZ, WL>(P, F, a.noise, t, d, i, j, k);
+            if (!AUX || a.mc.p) a.mc(i, j, k, d) = c;
+            if constexpr (AUX) x.cf[d](i, j, k) = c;
+        }
+        if (!edges) return;
+        if (NZ != NZ_OFF && !STAGED) a.noise.xy_xz_edges(P, i, j, k, we[0], we[1]);
+        if (k < P.n[2]) taus_edge<NS, R, NZ, 0, WL>(a, F, x, we[0], i, j, k);
+        if (j < P.n[1]) taus_edge<NS, R, NZ, 1, WL>(a, F, x, we[1], i, j, k);
+        if (i < P.n[0]) taus_edge<NS, R, NZ, 2, WL>(a, F, x, we[2], i, j, k);
+    };
+    if constexpr (STAGED) {
+        if (NZ != NZ_OFF && edges) a.noise.xy_xz_edges(P, i, j, k, we[0], we[1]);
+        stage_wait();
+        work(FieldsStaged<NS, R>(smem, i, j, k, a.F.zr));
+    } else {
+        work(a.F);
     }
-    if (!edges) return;
-    if (NZ != NZ_OFF) a.noise.xy_xz_edges(P, i, j, k, we[0], we[1]);
-    if (k < P.n[2]) taus_edge<NS, R, NZ, 0, WL>(a, x, we[0], i, j, k);
-    if (j < P.n[1]) taus_edge<NS, R, NZ, 1, WL>(a, x, we[1], i, j, k);
-    if (i < P.n[0]) taus_edge<NS, R, NZ, 2, WL>(a, x, we[2], i, j, k);
 }
 
+// Packed, beyond the sizes of k_taus_staged: bound by the latency of its loads, where 48
+// registers (40 warps per SM; a few spilled values) beat 64 (32 warps): 510 against 529 us
+// per step at 128^3 argon FP64, 654 at 80.  (0: no minimum.)
 template <int NS, class R, int NZ, bool WL = false, bool AUX = false, bool PACK = false>
-static __global__ void __launch_bounds__(256) k_taus(StageArgs<NS, R, NZ, PACK> a, StageAux<AUX> x) {
+static __global__ void __launch_bounds__(256, PACK ? 5 : 0) k_taus(StageArgs<NS, R, NZ, PACK> a, StageAux<AUX> x) {
     const int tot = taus_count(a);
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < tot; q += gridDim.x * blockDim.x)
         taus_point<NS, R, NZ, WL, AUX>(a, q, x);
+}
+
+template <int NS, class R, int NZ>
+static __global__ void __launch_bounds__(kStagedThreads, 5) k_taus_staged(StageArgs<NS, R, NZ, true> a) {
+    extern __shared__ __align__(16) unsigned char stage_smem[];
+    const int tot = taus_count(a);
+    for (int q = blockIdx.x * kStagedThreads + threadIdx.x; q < tot; q += gridDim.x * kStagedThreads)
+        taus_point<NS, R, NZ, false, false, true>(a, q, StageAux<false>{}, stage_smem);
 }
 
 // operands of one face of a direction known only at run time (face_flux)
@@ -511,13 +633,36 @@ static __global__ void __launch_bounds__(BS, MINB) k_faces(StageArgs<NS, R, NZ, 
         faces_point<NS, R, NZ, WL, AUX>(a, d, q, x);
 }
 
+// Periodic ghosts from the kernel that computes the values (FillBoundary fused into its
+// producer): a point within g of a face of the box also stores its values at the ghost
+// points they wrap to, instead of a launch per stage that reads and writes them again
+// (argon FP64 per step, before and after: 32^3 125 and 117 us, 64^3 423 and 403 us, 128^3
+// 2760 and 2732 us).  With n > 2 g (image_width) that is at most one shift per direction.
+// image_shift: that shift of index i in a direction of n cells (0: no image)
+FHD_D int image_shift(int i, int n, int g, int nodal) {
+    return i >= nodal && i < g + nodal ? n : (i >= n - g && i < n ? -n : 0);
+}
+// put(di, dj, dk) for the point itself, (0, 0, 0), and each of its images
+template <class F>
+FHD_D void images(int sx, int sy, int sz, F&& put) {
+    for (int dk = 0;; dk = sz) {
+        for (int dj = 0;; dj = sy) {
+            put(0, dj, dk);
+            if (sx) put(sx, dj, dk);
+            if (dj == sy) break;
+        }
+        if (dk == sz) break;
+    }
+}
+
 // RK3 stage combination (timeStepStag.cpp:439-528, 771-861, 1106-1202): one thread
 // per point of [0, n]^3 updates the cell there (if valid) and the faces there
 template <int NS, class R, int NZ, bool PACK>
 FHD_D int update_count(const StageArgs<NS, R, NZ, PACK>& a) { return a.it_upd.n; }
 
-template <int NS, class R, int NZ, bool PACK>
-FHD_D void update_point(const StageArgs<NS, R, NZ, PACK>& a, int q) {
+// SPLIT: one part of it alone, 0 the cell, 1 + d the face of direction d
+template <bool SPLIT = false, int NS, class R, int NZ, bool PACK>
+FHD_D void update_point(const StageArgs<NS, R, NZ, PACK>& a, int q, int part = 0) {
     const RunParams& P = a.P;
     const auto& F = a.F;
     const double dt = P.dt;
@@ -526,7 +671,7 @@ FHD_D void update_point(const StageArgs<NS, R, NZ, PACK>& a, int q) {
         int i, j, k;
         a.it_upd.point(q, i, j, k);
         const bool cell = i < P.n[0] && j < P.n[1] && k < P.n[2];
-        if (cell) {
+        if (cell && (!SPLIT || part == 0)) {
             using S = std::remove_const_t<std::remove_reference_t<decltype(a.S)>>;
             double on[2 + NS];
 #pragma unroll
@@ -555,12 +700,20 @@ FHD_D void update_point(const StageArgs<NS, R, NZ, PACK>& a, int q) {
             on[1] += gfac * (P.grav[0] * (F.mom[0](i + 1, j, k) + F.mom[0](i, j, k)) +
                              P.grav[1] * (F.mom[1](i, j + 1, k) + F.mom[1](i, j, k)) +
                              P.grav[2] * (F.mom[2](i, j, k + 1) + F.mom[2](i, j, k)));
+            auto put = [&](int di, int dj, int dk) {
 #pragma unroll
-            for (int c = 0; c < 2 + NS; ++c) a.cons_o(i, j, k, (c == 0) ? 0 : 3 + c) = on[c];
+                for (int c = 0; c < 2 + NS; ++c) a.cons_o(i + di, j + dj, k + dk, (c == 0) ? 0 : 3 + c) = on[c];
+            };
+            if constexpr (PACK)
+                images(image_shift(i, P.n[0], a.img, 0), image_shift(j, P.n[1], a.img, 0),
+                       image_shift(k, P.n[2], a.img, 0), put);
+            else
+                put(0, 0, 0);
         }
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             const int e0 = d == 0, e1 = d == 1, e2 = d == 2;
+            if (SPLIT && part != 1 + d) continue;
             if (i >= P.n[0] + e0 || j >= P.n[1] + e1 || k >= P.n[2] + e2) continue;
             // momentum flux differences (timeStepStag.cpp:452-482): centre and edge
             // totals stored by k_taus
@@ -593,18 +746,29 @@ FHD_D void update_point(const StageArgs<NS, R, NZ, PACK>& a, int q) {
                     divc(P, (2. / 3.) * dt * t2, P.dx[1], P.rdx[1]) - divc(P, (2. / 3.) * dt * t3, P.dx[2], P.rdx[2]) +
                     0.5 * (2. / 3.) * dt * P.grav[d] * rsum;
             }
-            a.mom_o[d](i, j, k) = v;
+            auto put = [&](int di, int dj, int dk) { a.mom_o[d](i + di, j + dj, k + dk) = v; };
+            if constexpr (PACK)
+                images(image_shift(i, P.n[0], a.img, e0), image_shift(j, P.n[1], a.img, e1),
+                       image_shift(k, P.n[2], a.img, e2), put);
+            else
+                put(0, 0, 0);
         }
     }
 }
 
 // MINB: 16 blocks of 128 (32 registers, full occupancy; packed 12 or 10) where the kernel
-// streams from HBM; 4 for a box that fits one wave of them, where a point's loads cost
-// its time and more registers put more of them in flight (launch_update)
+// streams from HBM; 4 for a small box that is not packed (launch_update)
 template <int NS, class R, int NZ, int MINB, bool PACK>
 static __global__ void __launch_bounds__(128, MINB) k_update(StageArgs<NS, R, NZ, PACK> a) {
     const int tot = update_count(a);
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < tot; q += gridDim.x * blockDim.x) update_point(a, q);
+}
+
+// one part of a point per thread, block b on part b % 4
+template <int NS, class R, int NZ>
+static __global__ void __launch_bounds__(128, 6) k_update_split(StageArgs<NS, R, NZ, true> a) {
+    const int q = (blockIdx.x / 4) * 128 + threadIdx.x;
+    if (q < update_count(a)) update_point<true>(a, q, blockIdx.x % 4);
 }
 
 // ===================================================================================
@@ -619,6 +783,7 @@ struct alignas(16) ConvArgs {
     Arr4<double> cons;   // comps 1..3 rewritten
     Arr4<const double> mom[3];
     int* status;
+    int img;             // ghost width of the periodic images to store too (0: none)
 };
 
 template <int NS>
@@ -640,20 +805,21 @@ FHD_D void convert_point(const ConvArgs<NS>& a, int q) {
         const double vxh = 2 * mx(i + 1, j, k) / (cons(i + 1, j, k, 0) + rho);
         const double vyh = 2 * my(i, j + 1, k) / (cons(i, j + 1, k, 0) + rho);
         const double vzh = 2 * mz(i, j, k + 1) / (cons(i, j, k + 1, 0) + rho);
-        a.vel[0](i, j, k) = vxl;
-        a.vel[1](i, j, k) = vyl;
-        a.vel[2](i, j, k) = vzl;
-        if (i == P.n[0] - 1) a.vel[0](i + 1, j, k) = vxh;
-        if (j == P.n[1] - 1) a.vel[1](i, j + 1, k) = vyh;
-        if (k == P.n[2] - 1) a.vel[2](i, j, k + 1) = vzh;
-        const Arr4<double>& prim = a.prim;
-        prim(i, j, k, 0) = rho;
-        prim(i, j, k, 1) = 0.5 * (vxl + vxh);
-        prim(i, j, k, 2) = 0.5 * (vyl + vyh);
-        prim(i, j, k, 3) = 0.5 * (vzl + vzh);
-        cons(i, j, k, 1) = 0.5 * (mx(i, j, k) + mx(i + 1, j, k));
-        cons(i, j, k, 2) = 0.5 * (my(i, j, k) + my(i, j + 1, k));
-        cons(i, j, k, 3) = 0.5 * (mz(i, j, k) + mz(i, j, k + 1));
+        const int g = a.img;
+        const int s0 = image_shift(i, P.n[0], g, 0), s1 = image_shift(j, P.n[1], g, 0), s2 = image_shift(k, P.n[2], g, 0);
+        images(image_shift(i, P.n[0], g, 1), s1, s2,
+               [&](int di, int dj, int dk) { a.vel[0](i + di, j + dj, k + dk) = vxl; });
+        images(s0, image_shift(j, P.n[1], g, 1), s2,
+               [&](int di, int dj, int dk) { a.vel[1](i + di, j + dj, k + dk) = vyl; });
+        images(s0, s1, image_shift(k, P.n[2], g, 1),
+               [&](int di, int dj, int dk) { a.vel[2](i + di, j + dj, k + dk) = vzl; });
+        // (the node of the high side has images in the other two directions alone)
+        if (i == P.n[0] - 1) images(0, s1, s2, [&](int, int dj, int dk) { a.vel[0](i + 1, j + dj, k + dk) = vxh; });
+        if (j == P.n[1] - 1) images(s0, 0, s2, [&](int di, int, int dk) { a.vel[1](i + di, j + 1, k + dk) = vyh; });
+        if (k == P.n[2] - 1) images(s0, s1, 0, [&](int di, int dj, int) { a.vel[2](i + di, j + dj, k + 1) = vzh; });
+        const double vc[3] = {0.5 * (vxl + vxh), 0.5 * (vyl + vyh), 0.5 * (vzl + vzh)};
+        const double mc[3] = {0.5 * (mx(i, j, k) + mx(i + 1, j, k)), 0.5 * (my(i, j, k) + my(i, j + 1, k)),
+                              0.5 * (mz(i, j, k) + mz(i, j, k + 1))};
         double rY[NS];
 #pragma unroll
         for (int n = 0; n < NS; ++n) rY[n] = cons(i, j, k, 5 + n);
@@ -661,13 +827,23 @@ FHD_D void convert_point(const ConvArgs<NS>& a, int q) {
         if (!cons_to_prim<NS>(P, rho, cons(i, j, k, 4), rY, mx(i, j, k), mx(i + 1, j, k), my(i, j, k), my(i, j + 1, k),
                               mz(i, j, k), mz(i, j, k + 1), q2))
             flag(a.status, ST_NONFINITE);
-        prim(i, j, k, 4) = q2.T;
-        prim(i, j, k, 5) = q2.p;
+        images(s0, s1, s2, [&](int di, int dj, int dk) {
+            double* u = &cons(i + di, j + dj, k + dk);
+            double* w = &a.prim(i + di, j + dj, k + dk);
+            w[0] = rho;
 #pragma unroll
-        for (int n = 0; n < NS; ++n) {
-            prim(i, j, k, 6 + n) = q2.Y[n];
-            prim(i, j, k, 6 + NS + n) = q2.X[n];
-        }
+            for (int d = 0; d < 3; ++d) {
+                u[(1 + d) * cons.sn] = mc[d];
+                w[(1 + d) * a.prim.sn] = vc[d];
+            }
+            w[4 * a.prim.sn] = q2.T;
+            w[5 * a.prim.sn] = q2.p;
+#pragma unroll
+            for (int n = 0; n < NS; ++n) {
+                w[(6 + n) * a.prim.sn] = q2.Y[n];
+                w[(6 + NS + n) * a.prim.sn] = q2.X[n];
+            }
+        });
     }
 }
 
@@ -1120,7 +1296,8 @@ static __global__ void __launch_bounds__(256) k_ghosts_b(const GhostFab* __restr
 // ===================================================================================
 // persistent batched step: one launch runs every phase of one RK3 step for every
 // member.  Phases per member: for each stage cellprep, stresses, faces x / y / z,
-// update, ghost fill; then the conversion, its ghost fill and the step counter.
+// update, ghost fill; then the conversion, its ghost fill and the step counter (no ghost
+// fills when the update and the conversion store the images).
 // Work is cut into chunks of `chunk` items; a unit is one member's (or one ghost
 // fab's) part of a phase.  Blocks take chunks in order from one counter (phase-
 // major over members) and, before working on a chunk of phase p > 0, wait until

@@ -1,5 +1,7 @@
 // fhd_launch.cuh — templated launchers included by each kernel translation unit.
 #pragma once
+#include <atomic>
+
 #include "fhd_host.h"
 #include "fhd_kernels.cuh"
 #include "fhd_fused.cuh"
@@ -72,6 +74,26 @@ inline int face_grid(const int N[3], int block) {
     const int cap = resident_blocks<K>(block) / 3;
     if (g > cap) g = cap;
     return (int)(g < 1 ? 1 : g);
+}
+
+// opts a kernel into dynamic shared memory above 48 KiB on the current device, once per
+// device, and returns the blocks its SMs hold at once with it (0: not available)
+template <auto K>
+inline int staged_blocks(int block, int bytes) {
+    static std::atomic<int> blocks[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); return 0; }
+    int nb = blocks[dev].load(std::memory_order_relaxed);
+    if (!nb) {
+        if (cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, K, block, bytes) != cudaSuccess || nb < 1) {
+            cudaGetLastError();
+            return 0;
+        }
+        nb *= device_sms();
+        blocks[dev].store(nb, std::memory_order_relaxed);
+    }
+    return nb;
 }
 
 inline int grid_for(int64_t items, int block, int cap = 148 * 32) {
@@ -290,6 +312,7 @@ StageArgs<NS, R, NZ, PACK> make_stage_args(const StageCall& c) {
     a.cons_o = view<double>(c.cons_o);
     a.src = view<const double>(c.src);
     a.stage = c.stage;
+    a.img = c.img;
     const int* n = c.P.n;
     a.it_taus = make_items(n[0] + 2, n[1] + 2, n[2] + 2);
     a.it_upd = make_items(n[0] + 1, n[1] + 1, n[2] + 1);
@@ -328,12 +351,22 @@ inline int stage_block(const StageCall& c) {
     return (c.tile >= 0 && c.tile < kNumStageBlocks) ? kStageBlocks[c.tile] : 128;
 }
 
+// Up to 4 blocks of points per SM (about 42^3) the launch's time is one thread's chain of
+// loads and FP64 operations: four threads per point cut it (argon FP64, per step: 16^3 30.6
+// against 38.3 us with one, 32^3 32.4 against 38.6, 40^3 38.3 against 42.2; 44^3 44.3 against
+// 43.2, 64^3 91 against 83, 128^3 512 against 393: there the kernel streams).  Not packed
+// (walls, low dimensions, allocation-free) a small box takes one thread with all the
+// registers it wants.
 template <int NS, class R, int NZ, bool PACK>
 void launch_update(const StageArgs<NS, R, NZ, PACK>& a, cudaStream_t s) {
     const int blocks = (a.it_upd.n + 127) / 128;
     constexpr int MB = !PACK ? 16 : (NS <= 2 ? 12 : 10);
-    if (blocks <= 4 * device_sms()) k_update<NS, R, NZ, 4, PACK><<<blocks, 128, 0, s>>>(a);
-    else k_update<NS, R, NZ, MB, PACK><<<resident_grid<k_update<NS, R, NZ, MB, PACK>>(a.it_upd.n, 128), 128, 0, s>>>(a);
+    if (blocks > 4 * device_sms()) {
+        k_update<NS, R, NZ, MB, PACK><<<resident_grid<k_update<NS, R, NZ, MB, PACK>>(a.it_upd.n, 128), 128, 0, s>>>(a);
+    } else {
+        if constexpr (PACK) k_update_split<NS, R, NZ><<<4 * blocks, 128, 0, s>>>(a);
+        else k_update<NS, R, NZ, 4, PACK><<<blocks, 128, 0, s>>>(a);
+    }
 }
 
 // part: 0 stresses, 1 face fluxes (all three directions), 2 update
@@ -342,7 +375,18 @@ int launch_stage_part_t(const StageCall& c, int part) {
     const StageArgs<NS, R, NZ, true> a = make_stage_args<NS, R, NZ, true>(c);
     const int b = stage_block(c);
     if (part == 0) {
-        k_taus<NS, R, NZ, false, false, true><<<grid_for(a.it_taus.n, b), b, 0, c.stream>>>(a, StageAux<false>{});
+        // Staged up to five waves of its blocks (about 76^3): 16^3 argon FP64 26.1 against
+        // 38.6 us per step, 64^3 75.0 against 87.5, 72^3 103.9 against 116.9; even at 80^3
+        // (143); beyond, L1 holds more of the neighbours' operands than the columns leave
+        // of it, 88^3 184 against 181, 128^3 535 against 511.
+        constexpr auto S = k_taus_staged<NS, R, NZ>;
+        constexpr int bytes = TausStage<NS, R>::bytes;
+        const int wave = staged_blocks<S>(kStagedThreads, bytes);
+        const int need = (a.it_taus.n + kStagedThreads - 1) / kStagedThreads;
+        if (need <= 5 * wave)
+            S<<<need < wave ? need : wave, kStagedThreads, bytes, c.stream>>>(a);
+        else
+            k_taus<NS, R, NZ, false, false, true><<<grid_for(a.it_taus.n, b), b, 0, c.stream>>>(a, StageAux<false>{});
     } else if (part == 1) {
         const int t = (c.tile >= 0 && c.tile < kNumStageBlocks) ? c.tile : auto_face_tile<NS, R>(c.P.n);
 #define FHD_FACES(BS, MINB)                                                                             \
@@ -618,6 +662,7 @@ ConvArgs<NS> make_conv_args(const StageCall& c) {
     }
     a.it = make_items(c.P.n[0], c.P.n[1], c.P.n[2]);
     a.status = c.status;
+    a.img = c.img;
     return a;
 }
 

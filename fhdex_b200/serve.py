@@ -108,9 +108,11 @@ def footprint_bytes(p: Params) -> int:
     pts = (n[0] + 1) * (n[1] + 1) * (n[2] + 1)
     ns = p.nspecies
     re = 4 if p.precision == 1 else 8
+    vals = 4 if ns == 1 else 4 + 3 * ns + ns * ns              # values of a cell record
+    rec = 16 * -(-vals // (16 // re))
     state = 8 * (cells_g * (p.nvars + p.nprimvars) + 2 * faces_g)
     scratch = (8 * (2 * cells_g * p.nvars + 2 * faces_g + 3 * pts * (2 + ns) + 3 * cells_g + 6 * pts)
-               + re * (cells_g * (3 + ns + ns * ns) + 6 * cells_g + 6 * pts))
+               + rec * cells_g + re * (6 * cells_g + 6 * pts))
     return state + scratch
 
 

@@ -540,7 +540,8 @@ int fhd_stats_stag(fhd_ctx* ctx, fhd_fab cu, fhd_fab prim, const fhd_fab vel[3],
  * nvar (nvar + 1) / 2 pairs (A = j, B = i for i <= j) as the reference's define
  * without pairs does (StructFact.cpp:45-69).  var_scaling has one entry per pair
  * (the result is divided by it).  The accumulators live in device memory owned
- * by the object (2 x ncov doubles per cell). */
+ * by the object (2 x ncov doubles per
+ * point of the half spectrum). */
 typedef struct fhd_sf fhd_sf;
 int fhd_sf_create(fhd_sf** sf, const int n_cells[3], int nvar, int ncov, const int* pairA, const int* pairB,
                   const double* var_scaling, int device);
@@ -565,8 +566,8 @@ int fhd_sf_finalize(fhd_sf* sf, fhd_fab cov_real, fhd_fab cov_imag, fhd_fab cov_
  * n_cells[1] x 1, ExtractSlice) or per x pencil (FHD_SF_X_PENCILS, do_1D: member
  * i at y = i / n_cells[1], z = i % n_cells[1] of n_cells[0] x 1 x 1,
  * ExtractXPencil; needs n_cells[1] == n_cells[2], since for other shapes that
- * enumeration reads pencils outside the box).  All members transform in one
- * batched cuFFT per variable.  fhd_sf_fort_structure takes the whole box's
+ * enumeration reads pencils outside the box).  All members and variables
+ * transform in one batched cuFFT (one per variable where its work area does not fit).  fhd_sf_fort_structure takes the whole box's
  * variables fab and samples every member; fhd_sf_stack_average is the
  * reference's output loop: zeroed mag (ncov comps) and realimag (2 ncov comps:
  * real then imaginary) fabs of the member shape, AddToExternal of every member

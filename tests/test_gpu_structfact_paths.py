@@ -1,0 +1,35 @@
+"""The structure factor's routes: more variables than a block's shared memory holds
+(13 and up) and the input transformed in place or packed first, odd and even half
+spectra, against the NumPy restatement within 1e-12 (the FFT libraries' rounding, as in
+the tests of the default route)."""
+import numpy as np
+import pytest
+import torch
+
+from fhdex_b200.fab import CELL, MultiFab
+from fhdex_b200.structfact import StructFact
+from oracle.structfact import StructFactOracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nvar", [12, 13])
+@pytest.mark.parametrize("shape_xyz,ng", [((6, 4, 5), 0), ((7, 3, 4), 1), ((2, 6, 3), 0)])
+def test_routes_match_oracle(nvar, shape_xyz, ng):
+    rng = np.random.default_rng(17)
+    ncov = nvar * (nvar + 1) // 2
+    scaling = list(rng.uniform(0.5, 2.0, ncov))
+    sf = StructFact(shape_xyz, [f"v{i}" for i in range(nvar)], scaling)
+    zyx = shape_xyz[::-1]
+    ora = StructFactOracle(zyx, nvar, scaling)
+    mf = MultiFab(shape_xyz, CELL, nvar, ng, device="cuda")
+    for _ in range(2):
+        v = rng.standard_normal((nvar,) + zyx)
+        mf.valid().copy_(torch.from_numpy(v))
+        sf.fort_structure(mf)
+        ora.fort_structure(v)
+    for zero_avg in (0, 1):
+        got = [m.valid().cpu().numpy() for m in sf.finalize(zero_avg)]
+        for g, r in zip(got, ora.finalize(zero_avg)):
+            assert np.abs(g - r).max() < 1e-12 * max(np.abs(r).max(), 1e-300)
+    sf.close()
