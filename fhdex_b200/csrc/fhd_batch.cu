@@ -237,7 +237,7 @@ int rebuild(fhd_batch* b) {
             const int* n = m.prm.n_cells;
             blocks += (kind < 7 ? kind_items(kind, n) : 64ll * (n[0] + 5) * (n[1] + 5) * (n[2] + 5)) / 128 + 6;
         }
-        add(sizeof(int) * (entries + 3 + blocks / 64));
+        add(sizeof(int) * (entries + 2 + blocks / 64));
     };
     for (int s = 0; s < 3; ++s) {
         add(batch_args_size(b->ns, b->mixed, 0, b->mode) * M);
@@ -265,20 +265,9 @@ int rebuild(fhd_batch* b) {
     char* dbase = static_cast<char*>(b->dbuf);
     b->dsteps = reinterpret_cast<uint64_t*>(dbase + steps_off);
     b->dstatus = reinterpret_cast<int*>(dbase + status_off);
-    int sms = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device) != cudaSuccess) return cuda_ok(cudaGetLastError());
     auto push_bpref = [&](const std::vector<int64_t>& items, int bs, int& nblocks) {
-        // Chunks of bs points per block, stored in front of the prefix.  A stage block starts
-        // with three loads in a row (member, argument block, points); two chunks share them
-        // where more than eight waves of eight blocks per SM are left to fill it (48 members
-        // of 32^3 and 64^3: mixed 7.79 against 7.99 ms with one chunk, 7.94 with four; FP64
-        // 12.42, 12.47 and 12.65).
-        int64_t total = 0;
-        for (int64_t n : items) total += (n + bs - 1) / bs;
-        const int ch = bs == 128 && total > 64 * (int64_t)sms ? 2 : 1;
         std::vector<int> pref(items.size() + 1, 0);
-        for (size_t q = 0; q < items.size(); ++q)
-            pref[q + 1] = pref[q] + (int)((items[q] + bs * ch - 1) / (bs * ch));
+        for (size_t q = 0; q < items.size(); ++q) pref[q + 1] = pref[q] + (int)((items[q] + bs - 1) / bs);
         nblocks = pref.back();
         // the members of blocks 0, 64, 128, ... (member_of)
         size_t m = 0;
@@ -286,11 +275,10 @@ int rebuild(fhd_batch* b) {
             while (pref[m + 1] <= blk) ++m;
             pref.push_back((int)m);
         }
-        pref.insert(pref.begin(), ch);
         const size_t off = align(256);
         host.resize(off + sizeof(int) * pref.size());
         memcpy(host.data() + off, pref.data(), sizeof(int) * pref.size());
-        return off + sizeof(int);
+        return off;
     };
     auto push_args = [&](int kind, bool mixed, int s) {
         const size_t sz = batch_args_size(b->ns, mixed, kind, b->mode);

@@ -1207,7 +1207,6 @@ static __global__ void k_init_uniform(InitArgs a) {
 // nmem + 1 prefixes come the members of blocks 0, 64, 128, ...: a block starts there and
 // steps to its own (boxes of 64 and more blocks: at most one step), where a binary
 // search made log2(members) dependent loads before the block could start.
-// bpref[-1]: chunks of 128 points per block.
 // ===================================================================================
 FHD_D int member_of(const int* __restrict__ bpref, int nmem) {
     const int b = blockIdx.x;
@@ -1236,9 +1235,8 @@ static __global__ void __launch_bounds__(128, cellprep_min_blocks<NS, R>()) k_ce
                                                     const int* __restrict__ bpref, int nmem) {
     const int m = member_of(bpref, nmem);
     const PrepArgs<NS, R>& a = member_args(args, m);
-    const int ch = bpref[-1], end = cellprep_count(a);
-    int q = (blockIdx.x - bpref[m]) * ch * 128 + threadIdx.x;
-    for (int c = 0; c < ch && q < end; ++c, q += 128) cellprep_point(a, q);
+    const int q = (blockIdx.x - bpref[m]) * blockDim.x + threadIdx.x;
+    if (q < cellprep_count(a)) cellprep_point(a, q);
 }
 
 // 64 registers (8 blocks of 128 per SM): uncapped, the FP32 kernel took 96 and ran 20 warps per SM
@@ -1247,9 +1245,8 @@ static __global__ void __launch_bounds__(128, 8) k_taus_b(const StageArgs<NS, R,
                                                 const int* __restrict__ bpref, int nmem) {
     const int m = member_of(bpref, nmem);
     const StageArgs<NS, R, NZ, true>& a = member_args(args, m);
-    const int ch = bpref[-1], end = taus_count(a);
-    int q = (blockIdx.x - bpref[m]) * ch * 128 + threadIdx.x;
-    for (int c = 0; c < ch && q < end; ++c, q += 128) taus_point(a, q);
+    const int q = (blockIdx.x - bpref[m]) * blockDim.x + threadIdx.x;
+    if (q < taus_count(a)) taus_point(a, q);
 }
 
 // Register cap of the batched face kernel: MINB resident blocks of 128 threads
@@ -1259,20 +1256,18 @@ static __global__ void __launch_bounds__(128, MINB) k_faces_b(const StageArgs<NS
                                                    const int* __restrict__ bpref, int nmem, int d) {
     const int m = member_of(bpref, nmem);
     const StageArgs<NS, R, NZ, true>& a = member_args(args, m);
-    const int ch = bpref[-1], end = faces_count(a, d);
-    int q = (blockIdx.x - bpref[m]) * ch * 128 + threadIdx.x;
-    for (int c = 0; c < ch && q < end; ++c, q += 128) faces_point(a, d, q);
+    const int q = (blockIdx.x - bpref[m]) * blockDim.x + threadIdx.x;
+    if (q < faces_count(a, d)) faces_point(a, d, q);
 }
 
-// 64 registers (8 blocks per SM): 80 or 48 made the 48-member ensemble 8.35 and 7.95 ms for 7.99
+// 64 registers (8 blocks per SM; fewer spill)
 template <int NS, class R, int NZ>
 static __global__ void __launch_bounds__(128, 8) k_update_b(const StageArgs<NS, R, NZ, true>* __restrict__ args,
                                                   const int* __restrict__ bpref, int nmem) {
     const int m = member_of(bpref, nmem);
     const StageArgs<NS, R, NZ, true>& a = member_args(args, m);
-    const int ch = bpref[-1], end = update_count(a);
-    int q = (blockIdx.x - bpref[m]) * ch * 128 + threadIdx.x;
-    for (int c = 0; c < ch && q < end; ++c, q += 128) update_point(a, q);
+    const int q = (blockIdx.x - bpref[m]) * blockDim.x + threadIdx.x;
+    if (q < update_count(a)) update_point(a, q);
 }
 
 template <int NS>
@@ -1280,9 +1275,8 @@ static __global__ void __launch_bounds__(128) k_convert_b(const ConvArgs<NS>* __
                                                    const int* __restrict__ bpref, int nmem) {
     const int m = member_of(bpref, nmem);
     const ConvArgs<NS>& a = member_args(args, m);
-    const int ch = bpref[-1], end = convert_count(a);
-    int q = (blockIdx.x - bpref[m]) * ch * 128 + threadIdx.x;
-    for (int c = 0; c < ch && q < end; ++c, q += 128) convert_point(a, q);
+    const int q = (blockIdx.x - bpref[m]) * blockDim.x + threadIdx.x;
+    if (q < convert_count(a)) convert_point(a, q);
 }
 
 static __global__ void __launch_bounds__(256) k_ghosts_b(const GhostFab* __restrict__ fabs,

@@ -143,26 +143,3 @@ def test_flux_operator_under_capture_equals_eager():
         for c in range(r.ncomp):
             assert torch.equal(a.valid(c).cpu(), r.valid(c).cpu()), (n, c)
     ctx.close()
-
-
-def test_batch_blocks_of_two_chunks():
-    """More than 64 blocks of 128 points per SM: two chunks a block, whose last may hold one
-    chunk, a remainder or nothing."""
-    ps = [argon((100, 97, 95), dx=8e-6, seed=71), argon((9, 5, 6), dx=8e-6, seed=72), argon((90, 95, 99), dx=8e-6, seed=73)]
-    dts = [stable_dt(p) for p in ps]
-    b = Batch(2, 0)
-    sts = [StagState(p, "cuda", aux=False) for p in ps]
-    for p, st, dt in zip(ps, sts, dts):
-        b.add(p, st, dt)
-    b.step(2)
-    b.synchronize()
-    for p, st, dt in zip(ps, sts, dts):
-        r = StagState(p, "cuda", aux=False)
-        ctx = Context(p)
-        ctx.init_state(r)
-        ctx.rk3_steps(r, dt, 0, 2)
-        torch.cuda.synchronize()
-        bad, _ = compare_named(st.named(), r.named())
-        assert not bad, (p.n_cells, bad[:6])
-        ctx.close()
-    b.close()
