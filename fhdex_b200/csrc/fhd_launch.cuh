@@ -332,7 +332,8 @@ StageArgs<NS, R, NZ, PACK> make_stage_args(const StageCall& c) {
 //     against 2933 at 80; mixed 128^3 1908 against 1975 at 80; four species FP64 64^3 803
 //     against 841, mixed 405 against 418), with two exceptions: 48 for one species (96^3
 //     FP64 703 against 732, mixed 632 against 644), and 80 for three and four species in
-//     mixed precision beyond about 93^3 (128^3 2940 against 3014).
+//     mixed precision beyond about 108^3 (100^3 1441 against 1408, 128^3 2940 against
+//     3014).
 template <int NS, class R>
 int auto_face_tile(const int N[3]) {
     int64_t most = 0;
@@ -344,7 +345,7 @@ int auto_face_tile(const int N[3]) {
     if (blocks <= 4 * device_sms()) return 0;
     if (blocks <= 6 * device_sms()) return 2;
     if (NS == 1) return 3;
-    return sizeof(R) == 4 && NS >= 3 && blocks > 128 * device_sms() ? 2 : 4;
+    return sizeof(R) == 4 && NS >= 3 && blocks > 200 * device_sms() ? 2 : 4;
 }
 
 inline int stage_block(const StageCall& c) {
