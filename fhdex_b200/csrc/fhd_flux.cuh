@@ -147,7 +147,10 @@ struct Noise {
     }
     // The six stress fields of point (i,j,k) in three Philox calls: the centre
     // fields of cell (i,j,k) with, when `edges`, the yz edge field of node (i,j,k)
-    // (cen_and_yz_edge), then the xy and xz edge fields (xy_xz_edges)
+    // (cen_and_yz_edge), then the xy and xz edge fields (xy_xz_edges).  The points of a
+    // launch are the nodes of every direction, an edge field ends one short of them in its
+    // edge's own: there the arrays are not read (they may have no ghosts) and the value,
+    // which no edge uses, is left as it was.
     FHD_D void cen_and_yz_edge(const RunParams& P, int i, int j, int k, bool edges, double (&wc)[3],
                                double& we2) const {
         if (MODE == NZ_PHILOX) {
@@ -155,15 +158,15 @@ struct Noise {
             gauss2(P, fid_cen(1), i, j, k, P.sqrt2, wc[1], wc[2]);
         } else {
             cen_all(P, i, j, k, wc);
-            if (edges) we2 = edge(P, 2, i, j, k);
+            if (edges && i < P.n[0]) we2 = edge(P, 2, i, j, k);
         }
     }
     FHD_D void xy_xz_edges(const RunParams& P, int i, int j, int k, double& we0, double& we1) const {
         if (MODE == NZ_PHILOX) {
             gauss2(P, fid_edge(0), i, j, k, 1.0, we0, we1);
         } else {
-            we0 = edge(P, 0, i, j, k);
-            we1 = edge(P, 1, i, j, k);
+            if (k < P.n[2]) we0 = edge(P, 0, i, j, k);
+            if (j < P.n[1]) we1 = edge(P, 1, i, j, k);
         }
     }
     FHD_D void edge_all(const RunParams& P, int i, int j, int k, double (&out)[3]) const {
