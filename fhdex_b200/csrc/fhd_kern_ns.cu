@@ -86,10 +86,11 @@ int FHD_CAT(exact_aux_ns, FHD_NS)(const StageCall& c) {
     return (c.P.walls || c.P.dim < 3) ? aux_mode<true>(c) : aux_mode<false>(c);
 }
 
-// a stage of the packed pipeline, of a box with walls or a quasi-1-D / 2-D run, or the
-// flux operator (no packed operands; its noise is W)
+// a stage of the packed pipeline, of the reference-ordered one (walls, quasi-1-D / 2-D
+// runs, the transport models 2 and 3 on any box: the wall variants, as its other parts), or
+// the flux operator (no packed operands; its noise is W, and a stage's is not)
 int FHD_CAT(exact_aux_stage_ns, FHD_NS)(const StageCall& c, int part) {
-    const bool wl = c.P.walls || c.P.dim < 3;
+    const bool wl = c.P.walls || c.P.dim < 3 || (!c.pack && (c.mode == NM_AB || c.mode == NM_PHILOX));
     if (wl) {
         switch (c.mode) {
             case NM_OFF: return launch_aux_stage_t<FHD_NS, NZ_OFF, true, false>(c, part);
