@@ -45,10 +45,9 @@ struct fhd_ctx {
     double* res_rec = nullptr;   // test hook: the particle reservoir's draws
     int res_cap = 0;
     WallParams wall{};
-    // the flux operator's stress scratch, its fabs, and the stream and end of its last use
+    // the flux operator's stress scratch, its fabs, and the end of its last use
     double* fx = nullptr;
     fhd_fab fxt{}, fxe{};
-    cudaStream_t fx_stream = nullptr;
     cudaEvent_t fx_ev = nullptr;
     // the Valk/Waldmann model's pair constants (transport_type 2), device memory
     VWTable* vwt = nullptr;
@@ -267,8 +266,9 @@ int ensure_coef(fhd_ctx* c, int dtype) {
 }
 
 // The flux operator's own stress scratch (ct, et), kept by the context.  It is apart
-// from the step's scratch, and a call on another stream than the last one's waits for
-// that one, so operator calls may overlap a step, and each other, on any streams.
+// from the step's scratch, and a call's stream waits for the last call's end, so operator
+// calls may overlap a step, and follow each other on any streams.  (The wait is made
+// whatever the streams: a handle may be that of a destroyed stream whose work still runs.)
 // false: no scratch (not allocated yet, or a stream under capture, whose graph may be
 // replayed beside later calls).
 bool capturing(fhd_ctx* c) {
@@ -278,7 +278,7 @@ bool capturing(fhd_ctx* c) {
 }
 bool flux_scratch(fhd_ctx* c) {
     if (!c->fx || capturing(c)) return false;
-    if (c->fx_stream != c->stream && cudaStreamWaitEvent(c->stream, c->fx_ev, 0) != cudaSuccess) {
+    if (cudaStreamWaitEvent(c->stream, c->fx_ev, 0) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
@@ -311,7 +311,6 @@ void flux_scratch_alloc(fhd_ctx* c) {
         c->fx = nullptr;
         return;
     }
-    c->fx_stream = c->stream;
     c->fxt.data = c->fx;
     c->fxe.data = c->fx + nt;
 }
@@ -751,7 +750,6 @@ int fhd_flux_stag(fhd_ctx* c, fhd_fab cu, const fhd_fab mom[3], fhd_fab prim, co
     sc.et = c->fxe;
     int rc = exact_aux_stage(sc, 0);
     if (!rc) rc = exact_aux_stage(sc, 1);
-    c->fx_stream = c->stream;
     if (cudaEventRecord(c->fx_ev, c->stream) != cudaSuccess && !rc) { cudaGetLastError(); rc = FHD_ERR_CUDA; }
     return rc;
 }
