@@ -307,7 +307,7 @@ void flux_scratch_alloc(fhd_ctx* c) {
     }
     if (cudaEventRecord(c->fx_ev, c->stream) != cudaSuccess) {
         cudaGetLastError();
-        cudaFree(c->fx);
+        cudaFreeAsync(c->fx, c->stream);
         c->fx = nullptr;
         return;
     }
@@ -587,7 +587,13 @@ int fhd_destroy(fhd_ctx* c) {
     if (c->scratch) cudaFree(c->scratch);
     if (c->coef) cudaFree(c->coef);
     if (c->lines) cudaFree(c->lines);
-    if (c->fx) cudaFree(c->fx);
+    // fx is pool memory: it goes back in stream order, behind its last use on whatever
+    // stream (cudaFree would not wait for that)
+    if (c->fx) {
+        cudaStreamWaitEvent(c->own, c->fx_ev, 0);
+        cudaFreeAsync(c->fx, c->own);
+        cudaStreamSynchronize(c->own);
+    }
     if (c->fx_ev) cudaEventDestroy(c->fx_ev);
     if (c->vwt) cudaFree(c->vwt);
     if (c->res.base) cudaFree(c->res.base);

@@ -76,3 +76,33 @@ def test_a_call_waits_for_the_last_on_a_recycled_stream():
             assert torch.equal(v, w[n]), n
     assert ctx.status() == 0      # (and the context is back on a stream that exists)
     ctx.close()
+
+
+def test_close_ends_the_scratch_s_last_use():
+    """The operator on one stream, a later call on another, and close(): the first stream is
+    done when close returns, and the scratch is back in the device's memory pool."""
+    p = argon((24, 20, 16), dx=8e-6, seed=73)
+    st, nz = prepared(p)
+    ctx = Context(p)
+    operator(ctx, st, nz)
+    torch.cuda.synchronize()
+    rt = ctypes.CDLL("libcudart.so.12")
+    pool, used = ctypes.c_void_p(), ctypes.c_uint64()
+    assert rt.cudaDeviceGetDefaultMemPool(ctypes.byref(pool), torch.cuda.current_device()) == 0
+
+    def in_use():
+        assert rt.cudaMemPoolGetAttribute(pool, 7, ctypes.byref(used)) == 0     # cudaMemPoolAttrUsedMemCurrent
+        return used.value
+
+    before = in_use()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(600_000_000)
+        operator(ctx, st, nz)
+        done = torch.cuda.Event()
+        done.record()
+    assert ctx.status() == 0      # on the current stream, which the context then keeps
+    ctx.close()
+    assert done.query()
+    torch.cuda.synchronize()
+    assert in_use() < before
