@@ -82,6 +82,11 @@ __device__ __forceinline__ double2 spec_at(const SfArgs& a, int v, int64_t h) {
     return s;
 }
 
+// A component of an output or input fab.  One component has fewer than 2^31 points
+// (shape_fab_ok), all of them together may have more: 21 pairs at 512^3 are 2.8e9 values.
+template <class T>
+__device__ __forceinline__ T* sf_comp(const Arr4<T>& a, int n) { return a.p + (int64_t)n * a.sn; }
+
 constexpr int kSfThreads = 256;
 constexpr int kSfStaged = 12;        // variables whose values fit 48 KiB of shared memory per block
 
@@ -171,6 +176,10 @@ __global__ void __launch_bounds__(256) k_sf_finalize(SfFinArgs a) {
         const int im = shift(a.nx - i, a.nx), jm = shift(j == 0 ? 0 : a.ny - j, a.ny),
                   km = shift(k == 0 ? 0 : a.nz - k, a.nz);
         const bool zero = a.zero_avg == 1 && q == 0;
+        // (the three outputs have the box's cells and ghosts of their own)
+        auto at = [](const Arr4<double>& v, int x, int y, int z) { return x + y * v.sy + z * v.sz; };
+        const int ro = at(a.ore, ip, jp, kp), io = at(a.oim, ip, jp, kp), mo = at(a.omag, ip, jp, kp);
+        const int rm = at(a.ore, im, jm, km), imm = at(a.oim, im, jm, km), mm = at(a.omag, im, jm, km);
 #pragma unroll 2
         for (int c = 0; c < a.ncov; ++c) {
             double re = zero ? 0.0 : __ldg(a.cov + (int64_t)c * a.half + q);
@@ -181,13 +190,14 @@ __global__ void __launch_bounds__(256) k_sf_finalize(SfFinArgs a) {
             im_ = im_ * a.scale[c];
             double mag = 0.0 + re * re;
             mag = sqrt(mag + im_ * im_);
-            a.ore(ip, jp, kp, c) = re;
-            a.oim(ip, jp, kp, c) = im_;
-            a.omag(ip, jp, kp, c) = mag;
+            double *const ore = sf_comp(a.ore, c), *const oim = sf_comp(a.oim, c), *const omag = sf_comp(a.omag, c);
+            ore[ro] = re;
+            oim[io] = im_;
+            omag[mo] = mag;
             if (mirror) {
-                a.ore(im, jm, km, c) = re;
-                a.oim(im, jm, km, c) = -im_;
-                a.omag(im, jm, km, c) = mag;
+                ore[rm] = re;
+                oim[imm] = -im_;
+                omag[mm] = mag;
             }
         }
     }
@@ -236,9 +246,9 @@ __global__ void __launch_bounds__(256) k_sf_stack_avg(SfAvgArgs a) {
                 sr = sr + re;
                 si = si + im;
             }
-            a.omag(ip, jp, kp, c) = sm * a.meminv;
-            a.ori(ip, jp, kp, c) = sr * a.meminv;
-            a.ori(ip, jp, kp, a.ncov + c) = si * a.meminv;
+            sf_comp(a.omag, c)[ip + jp * a.omag.sy + kp * a.omag.sz] = sm * a.meminv;
+            sf_comp(a.ori, c)[ip + jp * a.ori.sy + kp * a.ori.sz] = sr * a.meminv;
+            sf_comp(a.ori, a.ncov + c)[ip + jp * a.ori.sy + kp * a.ori.sz] = si * a.meminv;
         }
     }
 }
@@ -251,8 +261,12 @@ int shape_fab_ok(const int n[3], const fhd_fab& f, int min_nc) {
     if (!f.data || f.dtype != FHD_F64 || f.ncomp < min_nc) return 0;
     const int g = -f.lo[0];
     if (g < 0) return 0;
-    for (int d = 0; d < 3; ++d)
+    int64_t points = 1;
+    for (int d = 0; d < 3; ++d) {
         if (f.nodal[d] != 0 || f.lo[d] != -g || f.hi[d] != n[d] - 1 + g) return 0;
+        points *= n[d] + 2 * (int64_t)g;
+        if (points > INT32_MAX) return 0;   // the kernels index a component with 32 bits
+    }
     return 1;
 }
 int sf_fab_ok(const fhd_sf* s, const fhd_fab& f, int min_nc) { return shape_fab_ok(s->n, f, min_nc); }
@@ -270,7 +284,7 @@ int sf_plan(fhd_sf* s) {
     int dims[3], oemb[3];
     for (int r = 0; r < rank; ++r) dims[r] = oemb[r] = s->m[rank - 1 - r];
     oemb[rank - 1] = s->m[0] / 2 + 1;
-    s->per_plan = (int)s->varu.size();
+    s->per_plan = (int64_t)s->nmem * (int64_t)s->varu.size() > INT32_MAX ? 1 : (int)s->varu.size();
     for (;;) {
         rc = cufft_rc(cufftPlanMany(&s->plan, rank, dims, dims, 1, s->m[0] * s->m[1] * s->m[2], oemb, 1,
                                     (s->m[0] / 2 + 1) * s->m[1] * s->m[2], CUFFT_D2Z, s->nmem * s->per_plan));
@@ -301,16 +315,16 @@ struct PackArgs {
     double* out;
 };
 __global__ void __launch_bounds__(256) k_sf_pack(PackArgs a) {
-    const int comp = a.comp[blockIdx.y];
+    const double* const v = sf_comp(a.v, a.comp[blockIdx.y]);
     double* out = a.out + (int64_t)blockIdx.y * a.N;
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < a.N; q += (int64_t)gridDim.x * blockDim.x) {
         if (a.pencils) {
             const int p = (int)a.dx.div((uint32_t)q), y = (int)a.dy.div((uint32_t)p);
-            out[q] = a.v((int)q - p * a.nx, y, p - y * a.ny, comp);
+            out[q] = v[(int)q - p * a.nx + y * a.v.sy + (p - y * a.ny) * a.v.sz];
         } else {
             const int k = (int)a.dxy.div((uint32_t)q), r = (int)q - k * a.nx * a.ny;
             const int j = (int)a.dx.div((uint32_t)r);
-            out[q] = a.v(r - j * a.nx, j, k, comp);
+            out[q] = v[r - j * a.nx + j * a.v.sy + k * a.v.sz];
         }
     }
 }
@@ -343,6 +357,11 @@ int fhd_sf_create_stack(fhd_sf** out, const int n_cells[3], int kind, int nvar, 
     for (int d = 0; d < 3; ++d)
         if (n_cells[d] < (kind == FHD_SF_BOX || d == 0 ? 2 : 1)) return FHD_ERR_BAD_ARG;
     if (kind == FHD_SF_Z_SLICES && n_cells[1] < 2) return FHD_ERR_BAD_ARG;
+    int64_t cells = 1;
+    for (int d = 0; d < 3; ++d) {
+        cells *= n_cells[d];
+        if (cells > INT32_MAX) return FHD_ERR_UNSUPPORTED;
+    }
     if (kind == FHD_SF_X_PENCILS && n_cells[1] != n_cells[2]) return FHD_ERR_UNSUPPORTED;
     fhd_sf* s = new (std::nothrow) fhd_sf;
     if (!s) return FHD_ERR_OOM;

@@ -33,3 +33,23 @@ def test_routes_match_oracle(nvar, shape_xyz, ng):
         for g, r in zip(got, ora.finalize(zero_avg)):
             assert np.abs(g - r).max() < 1e-12 * max(np.abs(r).max(), 1e-300)
     sf.close()
+
+
+def test_outputs_of_more_than_2_31_values():
+    """1030 pairs at 128^3 are 2.16e9 values per output, with the components from 1024 on
+    beyond 32-bit offsets (about 70 GB in all).  Every pair is the same one."""
+    shape, ncov = (128, 128, 128), 1030
+    mf = MultiFab(shape, CELL, 2, 0, device="cuda")
+    mf.valid().copy_(torch.randn((2,) + shape, dtype=torch.float64, generator=torch.Generator().manual_seed(18)))
+    one = StructFact(shape, ["a", "b"], [1.0], pairs=([1], [0]))
+    many = StructFact(shape, ["a", "b"], [1.0] * ncov, pairs=([1] * ncov, [0] * ncov))
+    for sf in (one, many):
+        sf.fort_structure(mf)
+    want, got = one.finalize(), many.finalize()
+    for g, w in zip(got, want):
+        for c in (0, 511, 1023, 1024, 1029):
+            assert torch.equal(g.valid(c), w.valid(0)), c
+    del got, g
+    one.close()
+    many.close()
+    torch.cuda.empty_cache()

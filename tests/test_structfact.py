@@ -67,6 +67,17 @@ def test_structure_factor_stack_refusals():
     assert lib.fhd_sf_create_stack(C.byref(h), n1, 2, 1, 1, None, None, sc, 0) == capi.FHD_ERR_BAD_ARG
 
 
+@pytest.mark.parametrize("kind", [0, 1])
+def test_boxes_beyond_32_bit_indices_are_refused(kind):
+    """2^31 cells, more than the kernels index, before a device is touched."""
+    import ctypes as C
+    from fhdex_b200 import capi
+    h = C.c_void_p()
+    n = (C.c_int * 3)(2048, 1024, 1024)
+    rc = capi.load().fhd_sf_create_stack(C.byref(h), n, kind, 1, 1, None, None, (C.c_double * 1)(1.0), 0)
+    assert rc == capi.FHD_ERR_UNSUPPORTED
+
+
 def test_stack_oracle_members_are_box_oracles():
     """A z-slice stack of one slice is the box structure factor of that slice."""
     import numpy as np
