@@ -61,8 +61,10 @@ namespace {
 // The covariances of real fields are Hermitian: at a mirrored point (i > nx/2, where the
 // reference's unpacking takes the conjugate of entry (nx-i, -j, -k)) both spectra have
 // negated imaginary parts, so the real covariance is the stored entry's and the
-// imaginary one its negation, to the bit.  The accumulators are therefore kept on the
-// half spectrum and unfolded at the output: half the traffic of a sample.
+// imaginary one its negation, to the bit where it is not zero (a difference of equal
+// products is +0.0 on both sides: the output subtracts from 0.0).  The accumulators are
+// therefore kept on the half spectrum and unfolded at the output: half the traffic of a
+// sample.
 struct SfArgs {
     int nv, ncov;
     int64_t half;                    // half-spectrum entries of all members
@@ -196,7 +198,7 @@ __global__ void __launch_bounds__(256) k_sf_finalize(SfFinArgs a) {
             omag[mo] = mag;
             if (mirror) {
                 ore[rm] = re;
-                oim[imm] = -im_;
+                oim[imm] = 0.0 - im_;
                 omag[mm] = mag;
             }
         }

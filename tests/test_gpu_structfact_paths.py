@@ -35,6 +35,19 @@ def test_routes_match_oracle(nvar, shape_xyz, ng):
     sf.close()
 
 
+@pytest.mark.parametrize("shape_xyz", [(6, 4, 5), (7, 3, 4)])
+def test_auto_pairs_have_positive_zero_imaginary_parts(shape_xyz):
+    """A variable with itself: the imaginary part is +0.0 at every point, the mirrored
+    ones too, as where each point's own products are subtracted."""
+    sf = StructFact(shape_xyz, ["a"], [1.0])
+    mf = MultiFab(shape_xyz, CELL, 1, 0, device="cuda")
+    mf.valid().copy_(torch.randn((1,) + shape_xyz[::-1], dtype=torch.float64, generator=torch.Generator().manual_seed(19)))
+    sf.fort_structure(mf)
+    im = sf.finalize()[1].valid(0)
+    assert (im == 0).all() and not torch.signbit(im).any()
+    sf.close()
+
+
 def test_outputs_of_more_than_2_31_values():
     """1030 pairs at 128^3 are 2.16e9 values per output, with the components from 1024 on
     beyond 32-bit offsets (about 70 GB in all).  Every pair is the same one."""
