@@ -128,6 +128,7 @@ int alloc_member(fhd_batch* b, Member& m) {
     const int ns = b->ns;
     const int rdt = b->mixed ? FHD_F32 : FHD_F64;
     const size_t re = b->mixed ? 4 : 8;
+    if (!offsets_fit(n, 1, rec_words(ns, rdt))) return FHD_ERR_BAD_ARG;   // the kernels index with 32 bits
     m.cup = mk(n, CELLN, NGC, 5 + ns, FHD_F64);
     m.cup2 = m.cup;
     for (int d = 0; d < 3; ++d) m.cupm[d] = m.cup2m[d] = mk(n, FACEN[d], NGC, 1, FHD_F64);

@@ -162,6 +162,13 @@ bool walls_ghosts_ok(const fhd_fab& cu, const fhd_fab* mom, const fhd_fab& prim,
 int ensure_scratch(fhd_ctx* c) {
     const int* n = c->prm.n_cells;
     const int nvars = 5 + c->prm.nspecies;
+    // four species in FP64 have more words in a cell record, and more components in D,
+    // than the caller's prim, whose size fab_ok has tested (the record from 511^3 on, D from
+    // 509^3)
+    const bool fields = c->refpipe || tile_fused(c->tile);
+    if (fields ? !offsets_fit(n, NGC, c->prm.nspecies * c->prm.nspecies)
+               : !offsets_fit(n, 1, rec_words(c->prm.nspecies, c->prm.precision == FHD_PREC_MIXED ? FHD_F32 : FHD_F64)))
+        return FHD_ERR_BAD_ARG;
     fhd_fab tmpl = make_fab(nullptr, n, CELLN, NGC, nvars, FHD_F64);
     const int64_t cellpts = fab_points(tmpl);
     int64_t fpts[3];

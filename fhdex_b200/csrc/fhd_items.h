@@ -52,4 +52,15 @@ inline Items make_items(int nx, int ny, int nz) {
     return t;
 }
 
+// Whether 32-bit offsets (component or word times stride, plus the point) reach every
+// element of a field of n cells grown by g, with comps components or words per cell.
+inline bool offsets_fit(const int n[3], int g, int comps) {
+    int64_t e = comps;
+    for (int d = 0; d < 3; ++d) {
+        e *= n[d] + 2 * (int64_t)g;
+        if (e > (int64_t)INT32_MAX + 1) return false;
+    }
+    return true;
+}
+
 }  // namespace fhd

@@ -37,6 +37,17 @@ int main() {
     for (uint32_t d : {1u, 2u, 3u, 0x40000000u, 0x7ffffffeu, 0x7fffffffu})
         for (uint32_t q : {0u, 1u, 0x7ffffffdu, 0x7ffffffeu, 0x7fffffffu})
             if (fast_div(d).div(q) != q / d) ++bad;
+    // offsets_fit against the last element's offset, at sizes around the line (16 words of a
+    // four-species cell record: 510^3 the largest cube, whose 14 components of prim fit too)
+    for (int s : {500, 509, 510, 511, 512, 520})
+        for (int comps : {4, 7, 14, 16})
+            for (int g : {0, 1, 2}) {
+                const int n[3] = {s, s, s};
+                const uint64_t e = s + 2 * g, last = e * e * e * comps - 1;
+                if (offsets_fit(n, g, comps) != (last <= 0x7fffffffull)) ++bad;
+            }
+    const int big[3] = {1 << 30, 1 << 30, 1 << 30}, c510[3] = {510, 510, 510}, c511[3] = {511, 511, 511};
+    if (offsets_fit(big, 0, 1) || !offsets_fit(c510, 1, 16) || offsets_fit(c511, 1, 16) || !offsets_fit(c511, 2, 14)) ++bad;
     std::printf("%ld wrong of %ld points and 5000000 divisors\n", bad, points);
     return bad != 0;
 }
