@@ -48,11 +48,13 @@ struct fhd_sf {
     bool own_stream = false;
     double* cov = nullptr;           // [2][ncov][nmem][mz][my][mx/2+1]: real then imaginary accumulators
     double2* spec = nullptr;         // [nvaru][nmem][mz][my][mx/2+1] half spectra
-    double* real = nullptr;          // [nvaru][nmem][mz][my][mx] dense copy of the variables (FFT input)
+    double* real = nullptr;          // [per_max][nmem][mz][my][mx] dense copy of the variables (FFT input)
     int* dpairs = nullptr;           // [2][ncov] pair -> unique-variable slot, then the variables' components
     double* dscale = nullptr;        // [ncov]
     cufftHandle plan = 0;
-    int per_plan = 0;                // variables per execution of the plan: all, or one where that plan failed
+    // variables per execution of the plan: all of them, or one where their dense copy would
+    // take more than the half grid saves (more variables than pairs) or that plan failed
+    int per_max = 0, per_plan = 0;
     bool have_plan = false;
 };
 
@@ -286,7 +288,7 @@ int sf_plan(fhd_sf* s) {
     int dims[3], oemb[3];
     for (int r = 0; r < rank; ++r) dims[r] = oemb[r] = s->m[rank - 1 - r];
     oemb[rank - 1] = s->m[0] / 2 + 1;
-    s->per_plan = (int64_t)s->nmem * (int64_t)s->varu.size() > INT32_MAX ? 1 : (int)s->varu.size();
+    s->per_plan = (int64_t)s->nmem * s->per_max > INT32_MAX ? 1 : s->per_max;
     for (;;) {
         rc = cufft_rc(cufftPlanMany(&s->plan, rank, dims, dims, 1, s->m[0] * s->m[1] * s->m[2], oemb, 1,
                                     (s->m[0] / 2 + 1) * s->m[1] * s->m[2], CUFFT_D2Z, s->nmem * s->per_plan));
@@ -416,6 +418,9 @@ int fhd_sf_create_stack(fhd_sf** out, const int n_cells[3], int kind, int nvar, 
         hp[s->ncov + c] = slot[s->pb[c]];
     }
     hp.insert(hp.end(), s->varu.begin(), s->varu.end());
+    // full-grid accumulators and one variable's copy took 2 ncov + 1 grids beside the
+    // spectra, the half-grid ones and per_max copies take ncov + per_max
+    s->per_max = (int)s->varu.size() <= s->ncov + 1 ? (int)s->varu.size() : 1;
     const int64_t N = (int64_t)s->n[0] * s->n[1] * s->n[2];
     const int64_t half = (int64_t)(s->m[0] / 2 + 1) * s->m[1] * s->m[2] * s->nmem;
     int rc = FHD_OK;
@@ -424,7 +429,7 @@ int fhd_sf_create_stack(fhd_sf** out, const int n_cells[3], int kind, int nvar, 
     if (!rc) s->own_stream = true;
     if (!rc && (cudaMalloc(&s->cov, sizeof(double) * 2 * s->ncov * half) != cudaSuccess ||
                 cudaMalloc(&s->spec, sizeof(double2) * s->varu.size() * half) != cudaSuccess ||
-                                cudaMalloc(&s->real, sizeof(double) * s->varu.size() * N) != cudaSuccess ||
+                cudaMalloc(&s->real, sizeof(double) * s->per_max * N) != cudaSuccess ||
                 cudaMalloc(&s->dpairs, sizeof(int) * hp.size()) != cudaSuccess ||
                 cudaMalloc(&s->dscale, sizeof(double) * s->ncov) != cudaSuccess))
         rc = FHD_ERR_OOM;

@@ -48,6 +48,33 @@ def test_auto_pairs_have_positive_zero_imaginary_parts(shape_xyz):
     sf.close()
 
 
+def test_pair_list_with_more_variables_than_pairs():
+    """Two pairs of four variables: one variable at a time through the transform, in no more
+    memory than two full grids per pair, the four half spectra and one dense copy, and the
+    same result as the two pairs each by itself (within the FFT's rounding: a plan of one
+    transform against one of two)."""
+    shape = (128, 120, 124)
+    cells, half = 128 * 120 * 124, 65 * 120 * 124
+    mf = MultiFab(shape, CELL, 4, 0, device="cuda")
+    mf.valid().copy_(torch.randn((4,) + shape[::-1], dtype=torch.float64, generator=torch.Generator().manual_seed(20)))
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    sf = StructFact(shape, list("abcd"), [1.0, 2.0], pairs=([0, 2], [1, 3]))
+    # (each of the allocations is rounded up to 2 MiB)
+    assert free - torch.cuda.mem_get_info()[0] <= 8 * (2 * 2 * cells + 4 * 2 * half + cells) + 6 * 2 ** 21
+    for _ in range(2):
+        sf.fort_structure(mf)
+    got = sf.finalize()
+    sf.close()
+    for c, (a, b) in enumerate([(0, 1), (2, 3)]):
+        one = StructFact(shape, list("abcd"), [1.0 + c], pairs=([a], [b]))
+        for _ in range(2):
+            one.fort_structure(mf)
+        for g, w in zip(got, one.finalize()):
+            assert (g.valid(c) - w.valid(0)).abs().max() < 1e-12 * w.valid(0).abs().max(), c
+        one.close()
+
+
 def test_outputs_of_more_than_2_31_values():
     """1030 pairs at 128^3 are 2.16e9 values per output, with the components from 1024 on
     beyond 32-bit offsets (about 70 GB in all).  Every pair is the same one."""
