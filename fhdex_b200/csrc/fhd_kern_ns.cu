@@ -165,7 +165,8 @@ int FHD_CAT(exact_convert_ns, FHD_NS)(const DevParams& P, fhd_fab prim, const fh
     a.status = status;
     a.img = img;
     const int64_t tot = a.it.n;
-    k_convert<FHD_NS><<<resident_grid<k_convert<FHD_NS>>(tot, 128), 128, 0, s>>>(a);
+    if (img) k_convert<FHD_NS, true><<<resident_grid<k_convert<FHD_NS, true>>(tot, 128), 128, 0, s>>>(a);
+    else k_convert<FHD_NS, false><<<resident_grid<k_convert<FHD_NS, false>>(tot, 128), 128, 0, s>>>(a);
     return cuda_rc(cudaGetLastError());
 }
 #endif
