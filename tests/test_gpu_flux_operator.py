@@ -7,19 +7,35 @@ import pytest
 import torch
 
 from fhdex_b200.context import Context
-from fhdex_b200.params import argon, stable_dt
+from fhdex_b200.params import argon, argon_single, mixture4, stable_dt
 from fhdex_b200.state import StagState, StepNoise
+from tests.helpers import compare_named
+from tests.test_gpu_lowdim import CASES as LOWDIM, DT as LOWDIM_DT
+from tests.test_gpu_walls import CASES as WALLS, DT as WALLS_DT
 
 pytestmark = pytest.mark.gpu
 
+CASES = {
+    "argon": lambda: argon((9, 8, 7), dx=8e-6, seed=81),
+    "argon_adv0_visc3": lambda: argon((8, 9, 7), dx=8e-6, advection_type=0, visc_type=3, zeta_ratio=0.5, seed=82),
+    "argon_adv1": lambda: argon((7, 9, 8), dx=8e-6, advection_type=1, seed=83),
+    "argon_no_noise": lambda: argon((9, 8, 7), dx=8e-6, stoch_stress_form=0, seed=84),
+    "single": lambda: argon_single((6, 7, 9), dx=8e-6, seed=85),
+    "mixture4": lambda: mixture4((7, 6, 5), dx=8e-6, seed=86),
+    "mixture4_large": lambda: mixture4((41, 37, 33), dx=8e-6, seed=87),
+    **WALLS,
+    **LOWDIM,
+}
+DT = {**WALLS_DT, **LOWDIM_DT}
 
-def prepared(p, steps=2):
+
+def prepared(p, steps=2, dt=None):
     """A state some steps into a run, with its coefficients, and a noise W."""
     st = StagState(p, "cuda")
     ctx = Context(p)
     ctx.init_state(st)
     for s in range(steps):
-        ctx.rk3_step(st, stable_dt(p), s)
+        ctx.rk3_step(st, dt or stable_dt(p), s)
     nz = StepNoise(p, "cuda")
     ctx.fill_step_noise(nz, steps)
     torch.cuda.synchronize()
@@ -38,6 +54,73 @@ def fluxes(st):
 def poison(st):
     for a in fluxes(st).values():
         a.fill_(-7.0)
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_later_calls_equal_the_first(name):
+    """A context's first call computes in kernels of their own, which recompute every stress
+    per face; the later ones go through the stage's kernels.  Bit for bit, on every box."""
+    st, nz = prepared(CASES[name](), dt=DT.get(name))
+    ctx = Context(st.p)
+    operator(ctx, st, nz)
+    first = {n: a.clone() for n, a in fluxes(st).items()}
+    for _ in range(2):
+        poison(st)
+        operator(ctx, st, nz)
+        for n, a in fluxes(st).items():
+            assert torch.equal(a, first[n]), n
+    assert ctx.status() == 0
+    assert all(torch.isfinite(a).all() for a in first.values())
+    ctx.close()
+
+
+@pytest.mark.parametrize("injected", [False, True])
+@pytest.mark.parametrize("name", list(WALLS) + list(LOWDIM))
+def test_by_products_leave_the_step_as_without(name, injected):
+    """Boxes with walls and quasi-1-D / 2-D runs: a step that returns its coefficients and
+    fluxes leaves the state of one that does not, bit for bit."""
+    st, nz = prepared(CASES[name](), dt=DT.get(name))
+    out = []
+    for aux in (False, True):
+        d = st.clone()
+        ctx = Context(st.p)
+        for s in (2, 3):
+            ctx.fill_step_noise(nz, s)
+            ctx.rk3_step(d, DT.get(name) or stable_dt(st.p), s, noise=nz if injected else None, aux=aux)
+        assert ctx.status() == 0
+        ctx.close()
+        out.append(d)
+    bad, _ = compare_named(out[1].named(), out[0].named())
+    assert not bad, bad[:6]
+
+
+def test_calls_on_two_streams():
+    """Calls that share the scratch from two streams in turn, each behind the other."""
+    p = argon((44, 40, 36), dx=8e-6, seed=88)
+    a, nz = prepared(p)
+    b, _ = prepared(p.replace(seed=89), steps=3)
+    ctx = Context(p)
+    want = []
+    for st in (a, b):
+        fresh = Context(p)
+        operator(fresh, st, nz)
+        want.append({n: v.clone() for n, v in fluxes(st).items()})
+        fresh.close()
+        operator(ctx, st, nz)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for s in streams:
+        s.wait_stream(torch.cuda.current_stream())
+    for _ in range(20):
+        for s, st in zip(streams, (a, b)):
+            with torch.cuda.stream(s):
+                poison(st)
+                operator(ctx, st, nz)
+    torch.cuda.synchronize()
+    for st, w in zip((a, b), want):
+        for n, v in fluxes(st).items():
+            assert torch.equal(v, w[n]), n
+    assert ctx.status() == 0
+    ctx.close()
 
 
 def test_a_call_waits_for_the_last_on_a_recycled_stream():
