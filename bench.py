@@ -65,6 +65,12 @@ STATS_TRAFFIC_BYTES_PER_CELL = {"2": 1639.1}
 STAGE_FP64_FLOPS_PER_CELL = {"2:fp64": 3042.4}
 
 
+def count_launches(prof, p):
+    """Kernel launches in the profiled steps: one per bracketed scope (the passes of a box
+    with walls are at least that), and k_chem inside each stage's cellprep scope."""
+    return sum(v[1] for v in prof.values()) + (prof["cellprep"][1] if p.nreaction > 0 else 0)
+
+
 def measured_peak():
     try:
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
@@ -567,13 +573,10 @@ def run_ours(args):
     ms = replicas.max_over_ranks(ms, env, device=f"cuda:{local}")
     cells = p.n_cells[0] * p.n_cells[1] * p.n_cells[2]
     value = replicas.whole_job_rate(cells * args.steps, env, ms)
-    # every bracketed profile scope is one launch, except the face-flux scope (3 launches)
-    launches = sum(v[1] for v in prof.values()) + 2 * prof["faces"][1]
-    if p.nreaction > 0:  # k_chem runs inside each stage's cellprep scope
-        launches += prof["cellprep"][1]
+    launches = count_launches(prof, p)
 
     # roofline of the dominant kernel group: one RK stage = k_cellprep + k_taus +
-    # 3 x k_faces + k_update (conversion, transport coefficients, calculateFluxStag
+    # k_faces + k_update (conversion, transport coefficients, calculateFluxStag
     # and the stage update of the reference).
     # Algorithmic bytes per stage: the conserved state S = 5 + nspecies doubles per
     # cell read once (stage 1) or twice (U^s and U^0, stages 2-3) and written once;
@@ -592,7 +595,7 @@ def run_ours(args):
             "traffic_source": "ncu, 128^3, one timed step, per cell, scaled to this box" if traffic else None,
             "traffic_gbs": traffic * cells / avg_stage_s / 1e9 if traffic else None,
             "kernel": ("RK stage (k_cellprep + k_stage_zm), per stage" if prof["fused"][1] else
-                       "RK stage (k_cellprep + k_taus + 3x k_faces + k_update), per stage"),
+                       "RK stage (k_cellprep + k_taus + k_faces + k_update), per stage"),
             "kernel_ms_per_launch": 1e3 * avg_stage_s,
             "algorithmic_bytes_per_launch": alg_bytes,
             "step_breakdown_ms": {k: v[0] / args.steps for k, v in prof.items()}}

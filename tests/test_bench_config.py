@@ -37,6 +37,16 @@ def test_workload_description(p, word):
     assert cfg["n_cells"] == [8, 8, 8] and cfg["nspecies"] == p.nspecies
 
 
+def test_launch_count_of_a_periodic_step():
+    """13 launches: four kernels in each of three stages and the conversion (the faces of the
+    three directions are one launch); the chemistry source adds one per stage."""
+    b = load_bench()
+    prof = {k: (1.0, 3) for k in ("cellprep", "taus", "faces", "update")}
+    prof.update(convert=(0.1, 1), ghosts=(0.0, 0), aux_fluxes=(0.0, 0), fused=(0.0, 0))
+    assert b.count_launches(prof, argon(8)) == 13
+    assert b.count_launches(prof, no2_dimerization(8)) == 16
+
+
 @pytest.mark.parametrize("gas,ns,nreaction", [("argon", 1, 0), ("argon", 2, 0), ("argon", 4, 0), ("no2", 2, 2)])
 def test_make_params(gas, ns, nreaction):
     b = load_bench()
