@@ -62,9 +62,14 @@ inline int resident_grid(int64_t items, int block) {
     return (int)g;
 }
 
-// blocks per direction of the face kernel: together as many as the SMs hold at once
+// Blocks per direction of the face kernel: together as many as the SMs hold at once, each
+// over several chunks of its direction.  Quasi-1-D and 2-D runs (dim < 3): a block per chunk.
+// Their transverse faces cost next to nothing, so the blocks of those directions end early
+// and would leave the others' on a third (two thirds) of the SMs: faces per step, 256^3
+// argon, 1-D 6.9 against 12.9 ms, 2-D 10.2 against 12.9; 128x96x80 with four species, 1-D 1.29
+// against 2.74, 2-D 2.16 against 2.82.
 template <auto K>
-inline int face_grid(const int N[3], int block) {
+inline int face_grid(const int N[3], int block, int dim) {
     int64_t most = 0;
     for (int d = 0; d < 3; ++d) {
         const int64_t f = (int64_t)(N[0] + (d == 0)) * (N[1] + (d == 1)) * (N[2] + (d == 2));
@@ -72,7 +77,7 @@ inline int face_grid(const int N[3], int block) {
     }
     int64_t g = (most + block - 1) / block;
     const int cap = resident_blocks<K>(block) / 3;
-    if (g > cap) g = cap;
+    if (dim == 3 && g > cap) g = cap;
     return (int)(g < 1 ? 1 : g);
 }
 
@@ -355,7 +360,9 @@ inline int stage_block(const StageCall& c) {
 // Up to 4 blocks of points per SM (about 42^3) the launch's time is one thread's chain of
 // loads and FP64 operations: four threads per point cut it (argon FP64, per step: 16^3 30.6
 // against 38.3 us with one, 32^3 32.4 against 38.6, 40^3 38.3 against 42.2; 44^3 44.3 against
-// 43.2, 64^3 91 against 83, 128^3 512 against 393: there the kernel streams).  Not packed
+// 43.2, 64^3 91 against 83, 128^3 512 against 393: there the kernel streams).  Four
+// species and the mixed path alike (16^3 31.6 against 41.7 and 25.2 against 36.6 us, 40^3
+// 44.0 against 46.1 and 37.6 against 37.4).  Not packed
 // (walls, low dimensions, allocation-free) a small box takes one thread with all the
 // registers it wants.
 template <int NS, class R, int NZ, bool PACK>
@@ -379,7 +386,11 @@ int launch_stage_part_t(const StageCall& c, int part) {
         // Staged up to five waves of its blocks (about 76^3): 16^3 argon FP64 26.1 against
         // 38.6 us per step, 64^3 75.0 against 87.5, 72^3 103.9 against 116.9; even at 80^3
         // (143); beyond, L1 holds more of the neighbours' operands than the columns leave
-        // of it, 88^3 184 against 181, 128^3 535 against 511.
+        // of it, 88^3 184 against 181, 128^3 535 against 511.  The same line for the other
+        // species counts (16^3 25.7 against 38 us, 64^3 69 to 81 against 83 to 93) and in
+        // mixed precision (24.7 to 25.8 against 35 to 36; 61 to 66 against 74 to 77).
+        // Without noise there is less to overlap: mixed, 64^3 56 against 53 and 72^3 78
+        // against 68, 3 % of those steps at most.
         constexpr auto S = k_taus_staged<NS, R, NZ>;
         constexpr int bytes = TausStage<NS, R>::bytes;
         const int wave = staged_blocks<S>(kStagedThreads, bytes);
@@ -393,7 +404,7 @@ int launch_stage_part_t(const StageCall& c, int part) {
 #define FHD_FACES(BS, MINB)                                                                             \
         {                                                                                               \
             constexpr auto K = k_faces<NS, R, NZ, BS, MINB, false, false, true>;                        \
-            const int per = face_grid<K>(c.P.n, BS);                                                    \
+            const int per = face_grid<K>(c.P.n, BS, 3);                                                 \
             K<<<3 * per, BS, 0, c.stream>>>(a, per, StageAux<false>{});                                 \
         }
         switch (t) {
@@ -420,7 +431,7 @@ int launch_stage_plain_t(const StageCall& c, int part) {
         k_taus<NS, double, NZ><<<grid_for(a.it_taus.n, 128), 128, 0, c.stream>>>(a, StageAux<false>{});
     } else if (part == 1) {
         constexpr auto K = k_faces<NS, double, NZ, 128, 4>;
-        const int per = face_grid<K>(c.P.n, 128);
+        const int per = face_grid<K>(c.P.n, 128, 3);
         K<<<3 * per, 128, 0, c.stream>>>(a, per, StageAux<false>{});
     } else {
         launch_update(a, c.stream);
@@ -485,7 +496,7 @@ int launch_aux_stage_t(const StageCall& c, int part) {
         k_taus<NS, double, NZ, WL, true, PACK><<<grid_for(a.it_taus.n, 128), 128, 0, c.stream>>>(a, x);
     } else {
         constexpr auto K = k_faces<NS, double, NZ, 128, (WL && NS > 2 ? 4 : 8), WL, true, PACK>;
-        const int per = face_grid<K>(c.P.n, 128);
+        const int per = face_grid<K>(c.P.n, 128, c.P.dim);
         K<<<3 * per, 128, 0, c.stream>>>(a, per, x);
     }
     return cuda_rc(cudaGetLastError());
@@ -502,7 +513,7 @@ int launch_walls_part_t(const StageCall& c, int part) {
         // register cap: 64 up to two species (the periodic autotuner's choice at 256^3;
         // 128 was measured twice as slow for the wall variant), 128 above
         constexpr int MB = NS <= 2 ? 8 : 4;
-        const int per = face_grid<k_faces<NS, double, NZ, 128, MB, true>>(c.P.n, 128);
+        const int per = face_grid<k_faces<NS, double, NZ, 128, MB, true>>(c.P.n, 128, c.P.dim);
         k_faces<NS, double, NZ, 128, MB, true><<<3 * per, 128, 0, c.stream>>>(a, per, StageAux<false>{});
     } else {
         launch_update(a, c.stream);

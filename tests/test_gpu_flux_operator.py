@@ -7,7 +7,7 @@ import pytest
 import torch
 
 from fhdex_b200.context import Context
-from fhdex_b200.params import argon, argon_single, mixture4, stable_dt
+from fhdex_b200.params import argon, argon_single, mixture4, stable_dt, with_walls
 from fhdex_b200.state import StagState, StepNoise
 from tests.helpers import compare_named
 from tests.test_gpu_lowdim import CASES as LOWDIM, DT as LOWDIM_DT
@@ -26,6 +26,13 @@ CASES = {
     **WALLS,
     **LOWDIM,
 }
+# more faces than the SMs hold threads at once: the face kernel's grid of these runs
+LARGE = {
+    "large_1d": lambda: argon((250, 33, 32), dx=8e-6, seed=91).replace(do_1D=1),
+    "large_2d_walls": lambda: with_walls(mixture4((129, 130, 16), dx=8e-6, seed=92),
+                                         x=dict(vel=2, therm=2, mass=1, t=(263.0, 283.0))).replace(do_2D=1),
+}
+CASES.update(LARGE)
 DT = {**WALLS_DT, **LOWDIM_DT}
 
 
@@ -75,7 +82,7 @@ def test_later_calls_equal_the_first(name):
 
 
 @pytest.mark.parametrize("injected", [False, True])
-@pytest.mark.parametrize("name", list(WALLS) + list(LOWDIM))
+@pytest.mark.parametrize("name", list(WALLS) + list(LOWDIM) + list(LARGE))
 def test_by_products_leave_the_step_as_without(name, injected):
     """Boxes with walls and quasi-1-D / 2-D runs: a step that returns its coefficients and
     fluxes leaves the state of one that does not, bit for bit."""
