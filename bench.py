@@ -51,18 +51,18 @@ METRIC = "cell-updates/s (RK3 steps x cells)"
 UNIT = "cell-updates/s"
 
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of one RK stage
-# (k_cellprep + k_taus + 3 x k_faces + k_update) per cell, keyed
+# (k_cellprep + k_taus + k_faces + k_update) per cell, keyed
 # "nspecies:precision": ncu, 128^3, one full timed step captured, scaled to the
 # box by the cell count (every operand exceeds L2 at both sizes).  Absent for
 # configurations not captured.
-STAGE_TRAFFIC_BYTES_PER_CELL = {"2:fp64": 1592.1, "2:mixed": 1232.5}
+STAGE_TRAFFIC_BYTES_PER_CELL = {"2:fp64": 1139.3, "2:mixed": 936.0}
 # DRAM traffic of one statistics update per cell (all flags), keyed "nspecies":
 # ncu, 128^3, the three statistics kernels captured, scaled by the cell count.
 STATS_TRAFFIC_BYTES_PER_CELL = {"2": 1639.1}
 # FP64 flops of one RK stage per cell (dadd + dmul + 2 x dfma thread instructions
-# of k_cellprep, k_taus, 3 x k_faces and k_update; ncu at 128^3, divided by the
+# of k_cellprep, k_taus, k_faces and k_update; ncu at 128^3, divided by the
 # cells), keyed "nspecies:precision".
-STAGE_FP64_FLOPS_PER_CELL = {"2:fp64": 3042.4}
+STAGE_FP64_FLOPS_PER_CELL = {"2:fp64": 3027.8}
 
 
 def count_launches(prof, p):
@@ -450,7 +450,7 @@ def step_extras(args, p, dt, local, peak, peak_kind):
     nb = args.bench_batch_steps
     batched = {"config": {"members": args.members, "sizes": "half 32^3, half 64^3", "gas": "argon (2 species)",
                           "T0": "U(250, 350) K", "rho0": "U(1e-3, 3e-3) g/cm^3", "steps": nb,
-                          "launch": "fp64 / mixed: 23 batched kernels per step, one CUDA graph replay per step; "
+                          "launch": "fp64 / mixed: 20 batched kernels per step, one CUDA graph replay per step; "
                                     "*_persistent: one persistent launch per step (k_batch_persist), graph replay"}}
     members = None
     for prec, key in ((0, "fp64"), (1, "mixed")):
@@ -916,16 +916,18 @@ def run_sf(args):
     torch.cuda.synchronize()
     ms = e0.elapsed_time(e1) / args.steps
     avg_ms = None
-    if stack is not None:   # the output loop, once (it runs at plot time, not per sample)
+    if stack is not None:   # the output loop, once after an untimed call (it runs at plot time, not per sample)
+        sf.stack_average()
         e0.record()
         sf.stack_average()
         e1.record()
         torch.cuda.synchronize()
         avg_ms = e0.elapsed_time(e1)
     cells = p.n_cells[0] * p.n_cells[1] * p.n_cells[2]
-    # per point: pack (read + write 8 B), FFT (read 8 B, write the 8 B half spectrum) and
-    # the accumulation's spectrum read (8 B) per variable; covariance read + write per pair
-    alg = cells * (40 * nvar + 32 * sf.ncov)
+    # per point: FFT (read 8 B, write the 8 B half spectrum) and the accumulation's spectrum
+    # read (8 B) per variable, for pencils the dense copy (read + write 8 B); per pair the
+    # half grid's real and imaginary covariances, read and written
+    alg = cells * ((40 if stack == "x_pencils" else 24) * nvar + 16 * sf.ncov)
     peak, peak_kind = measured_peak()
     achieved = alg / (ms / 1e3) / 1e9
     print(json.dumps({"mode": "sf", "metric": "structure-factor samples x cells / s", "unit": "cell-samples/s",
@@ -938,7 +940,8 @@ def run_sf(args):
                       "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                                    "frac": achieved / peak, "peak_kind": peak_kind,
                                    "algorithmic_bytes_per_launch": alg,
-                                   "kernel": "4 x (k_sf_pack + cuFFT D2Z) + k_sf_accumulate"}}), flush=True)
+                                   "kernel": ("k_sf_pack + " if stack == "x_pencils" else "") +
+                                             "cuFFT D2Z of all variables + k_sf_accumulate"}}), flush=True)
     sf.close()
 
 
@@ -1013,7 +1016,7 @@ def run_ensemble(args):
                       "face_tile_regs": b.TILE_REGS[tile], "autotune_face_ms_per_stage": tune_ms,
                       "persistent_ms_per_step_by_regs": persist_ms or None,
                       "launch": ("one persistent launch per step (k_batch_persist), graph replay" if args.persistent
-                                 else "23 batched kernels per step, one CUDA graph replay per step"),
+                                 else "20 batched kernels per step, one CUDA graph replay per step"),
                       "equilibrium": eq}), flush=True)
 
 
