@@ -153,9 +153,10 @@ static __global__ void __launch_bounds__(256) k_stats_means_b(StatsArgs a) {
 
 // pass C: one thread per point of [0, n]^3.  As in pass B, operands are loaded in
 // groups before the stores they feed, so each thread keeps many loads in flight.  The
-// groups are of at most about 18 values, which lets 128 registers hold them: with all 26
+// groups are of at most about 18 values under a cap of 168 registers (12 warps per SM; no
+// spills for two species, 88 B for four): 408 us at 144x112x96, two species.  With all 26
 // covariances and both moments in one group each the kernel took 242 registers, eight
-// warps per SM (438 us at 144x112x96, two species, 4.3 TB/s of algorithmic bytes).
+// warps per SM, 438 us; at 128 registers, 180 B of spills, the update was slower again.
 template <int NS>
 static __global__ void __launch_bounds__(128, 3) k_stats_vars(StatsArgs a) {
     const RunParams& P = a.P;

@@ -227,7 +227,12 @@ int fhd_transport_coeffs(fhd_ctx* ctx, fhd_fab prim, fhd_fab eta, fhd_fab zeta,
 /* calculateFluxStag: fluxStag.cpp:5-1868 (declared
  * compressible_functions_stag.H:127-143).  edgeflux[6] = {edgeflux_x[0..1],
  * edgeflux_y[0..1], edgeflux_z[0..1]}; stochedge[3] = {xy, xz, yz} combined
- * noise; stochface[3]/stochcen[3] combined noise W (already weighted). */
+ * noise; stochface[3]/stochcen[3] combined noise W (already weighted).
+ * From its second call on the context keeps a scratch of the stresses in device
+ * memory (12 doubles per point of the box, about), allocated in stream order behind
+ * the first call's kernels, which compute without it; so do calls under capture and
+ * where no memory is left, with the same results.  Calls on several streams take the
+ * scratch in turn. */
 int fhd_flux_stag(fhd_ctx* ctx, fhd_fab cu, const fhd_fab mom[3], fhd_fab prim,
                   const fhd_fab vel[3], fhd_fab eta, fhd_fab zeta, fhd_fab kappa,
                   fhd_fab chi, fhd_fab D, const fhd_fab faceflux[3],
@@ -389,7 +394,9 @@ int fhd_batch_set_persistent(fhd_batch* batch, int enable, int tile);
  * expiry the member's status becomes FHD_ERR_TIMEOUT and every block stops taking
  * work for that step.  hold_phase >= 0 (0 .. 23) is a failure-injection hook for
  * tests: that phase's completions are never published, so the next phase's wait
- * runs out; -1 turns it off. */
+ * runs out; -1 turns it off.  A step has 20 phases where every member's update and
+ * conversion store the periodic ghosts (per stage cells, stresses, faces x / y / z,
+ * update; then the conversion and the step counter), 24 with ghost fills. */
 int fhd_batch_set_wait_limit(fhd_batch* batch, double seconds, int hold_phase);
 /* Latched device status of one member (waits for the stream). */
 int fhd_batch_member_status(fhd_batch* batch, int member);
@@ -540,8 +547,8 @@ int fhd_stats_stag(fhd_ctx* ctx, fhd_fab cu, fhd_fab prim, const fhd_fab vel[3],
  * nvar (nvar + 1) / 2 pairs (A = j, B = i for i <= j) as the reference's define
  * without pairs does (StructFact.cpp:45-69).  var_scaling has one entry per pair
  * (the result is divided by it).  The accumulators live in device memory owned
- * by the object (2 x ncov doubles per
- * point of the half spectrum). */
+ * by the object (2 x ncov doubles per point of the half spectrum).  A box of 2^31
+ * and more cells gives FHD_ERR_UNSUPPORTED. */
 typedef struct fhd_sf fhd_sf;
 int fhd_sf_create(fhd_sf** sf, const int n_cells[3], int nvar, int ncov, const int* pairA, const int* pairB,
                   const double* var_scaling, int device);
@@ -567,8 +574,9 @@ int fhd_sf_finalize(fhd_sf* sf, fhd_fab cov_real, fhd_fab cov_imag, fhd_fab cov_
  * i at y = i / n_cells[1], z = i % n_cells[1] of n_cells[0] x 1 x 1,
  * ExtractXPencil; needs n_cells[1] == n_cells[2], since for other shapes that
  * enumeration reads pencils outside the box).  All members and variables
- * transform in one batched cuFFT (one per variable where its work area does not fit).  fhd_sf_fort_structure takes the whole box's
- * variables fab and samples every member; fhd_sf_stack_average is the
+ * transform in one batched cuFFT (one per variable where its work area does not
+ * fit, or with more variables than pairs).  fhd_sf_fort_structure takes the whole
+ * box's variables fab and samples every member; fhd_sf_stack_average is the
  * reference's output loop: zeroed mag (ncov comps) and realimag (2 ncov comps:
  * real then imaginary) fabs of the member shape, AddToExternal of every member
  * in order (its Finalize, StructFact.cpp:979-1009), then mult by 1/members.
